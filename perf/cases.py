@@ -66,28 +66,28 @@ def _case(model, dtype, requests, shortest, longest, new, sampling="greedy"):
 def listed():
     return [
         # the smallest calls: a handful of launches on a few kilobytes, in true 32-bit
-        dict(_case("tiny-a", "float32", 3, 5, 31, 16), name="tiny a, 3 requests"),
+        dict(_case("tiny-a", "float32", 3, 5, 31, 16), name="tiny a: 3 requests"),
         # prompts cut by a budget of 32 tokens, sampled with a repetition penalty
-        dict(_case("tiny-b", "float32", 5, 1, 100, 24, "default"), name="tiny b, 5 requests, sampled"),
+        dict(_case("tiny-b", "float32", 5, 1, 100, 24, "default"), name="tiny b: 5 requests sampled"),
         # a 32-bit run of a real model, what a bfloat16 deployment is checked against
-        dict(_case("0.6b", "float32", 2, 77, 150, 12), name="0.6b float32, 2 requests"),
+        dict(_case("0.6b", "float32", 2, 77, 150, 12), name="0.6b float32: 2 requests"),
         # one user at a small model: latency of a step
-        dict(_case("0.6b", "bfloat16", 1, 61, 61, 64), name="0.6b, 1 user"),
+        dict(_case("0.6b", "bfloat16", 1, 61, 61, 64), name="0.6b: 1 user"),
         # a burst of requests of all lengths: portions of prompts beside decoded tokens
-        dict(_case("0.6b", "bfloat16", 96, 1, 1024, 24), name="0.6b, burst of 96"),
+        dict(_case("0.6b", "bfloat16", 96, 1, 1024, 24), name="0.6b: burst of 96"),
         # two long documents and a summary of each
-        dict(_case("0.6b", "bfloat16", 2, 9001, 12000, 32), name="0.6b, 2 long documents"),
+        dict(_case("0.6b", "bfloat16", 2, 9001, 12000, 32), name="0.6b: 2 long documents"),
         # one user, a page of prompt
-        dict(_case("8b", "bfloat16", 1, 512, 512, 48), name="8b, 1 user"),
+        dict(_case("8b", "bfloat16", 1, 512, 512, 48), name="8b: 1 user"),
         # the benchmark's batch
-        dict(_case("8b", "bfloat16", 8, 512, 512, 48), name="8b, 8 requests"),
+        dict(_case("8b", "bfloat16", 8, 512, 512, 48), name="8b: 8 requests"),
         # a busy server with short prompts
-        dict(_case("8b", "bfloat16", 64, 33, 200, 32), name="8b, 64 requests"),
+        dict(_case("8b", "bfloat16", 64, 33, 200, 32), name="8b: 64 requests"),
         # time to the first token of a long and of a short prompt
-        dict(_case("8b", "bfloat16", 1, 2048, 2048, 1), name="8b, prompt of 2048"),
-        dict(_case("8b", "bfloat16", 1, 203, 203, 1, "top"), name="8b, prompt of 203"),
+        dict(_case("8b", "bfloat16", 1, 2048, 2048, 1), name="8b: prompt of 2048"),
+        dict(_case("8b", "bfloat16", 1, 203, 203, 1, "top"), name="8b: prompt of 203"),
         # wide layers, pages of 16
-        dict(_case("32b-4", "bfloat16", 6, 1500, 2500, 16), name="32b 4 layers, 6 requests"),
+        dict(_case("32b-4", "bfloat16", 6, 1500, 2500, 16), name="32b 4 layers: 6 requests"),
     ]
 
 
