@@ -9,17 +9,17 @@
 //            and V pages of the request's block table (2-D TMA boxes of one page x 64 columns,
 //            128-byte swizzle), keys and values in rings of two stages each, the keys one tile
 //            ahead of the values;
-//   warp 1 and the last ISSUERS - 1 warps issue tcgen05.mma: S_g = Q_g K^T into tensor memory, and
-//            O_g += P_g V (P_g read from tensor memory, V as an N-contiguous operand) once the
-//            probabilities are there; the scores of tile g's next key tile follow its P V at once.
-//            A thread can issue one tcgen05.mma per 196 cycles, whatever its size (measured), and
-//            the products of a tile's chain (scores -> softmax -> P V -> next scores) lie on the
-//            critical path: every product's K steps are therefore dealt to ISSUERS threads of
-//            different warps, which walk the products in the same order.  Two hand-overs keep the
-//            tensor pipe's order right: the P V steps of a tile must all be issued before the first
-//            step of its next scores (which overwrites P), and that first step (it overwrites S)
-//            before the other steps of the same scores.  O starts as zeros, so that no P V step
-//            is the first one;
+//   warp 1   one thread issues tcgen05.mma: S_g = Q_g K^T into tensor memory, and O_g += P_g V (P_g
+//            read from tensor memory, V as an N-contiguous operand) as the probabilities arrive, in
+//            two halves of 64 keys, so that the first half of a product runs beside the exponentials
+//            of the second; the scores of tile g's next key tile follow its P V at once.  (The
+//            thread is chosen by elect.sync.  With `lane == 0` in its place the compiler cannot keep
+//            the MMAs' operands in uniform registers and a thread issues one MMA per 196 cycles,
+//            measured, more than the 64 that an MMA of 128 x 128 x 16 takes: three issuing threads
+//            with hand-overs between them were needed then.  32 heads over 8, 2,048 / 4,096 tokens:
+//            73.0 / 198.8 us with the three, 66.3 / 170.0 with the one; 2,048 queries at the end of
+//            12,000 keys, 16 heads: 225 -> 191 us.)  The tensor core takes a thread's
+//            MMAs in order: the next scores overwrite P_g after its P V has read it;
 //   warps 2-5 (tile 0) and 6-9 (tile 1), one thread per row: read the row of S from tensor memory,
 //            mask (key j is visible to the query at position p iff j <= p and, with a window
 //            W > 0, j > p - W: serve.py:668-680; with a chunk C > 0, j / C == p / C; with slopes, head
@@ -47,13 +47,9 @@ static_assert(D == 64 || D == 128, "the tcgen05 prefill kernel takes head sizes 
 constexpr int BM = 128;                      // rows of a query tile
 constexpr int BN = 128;                      // keys of a tile
 constexpr int GROUPS = 2;                    // query tiles of a block
-#ifndef TS_ATTN_ISSUERS
-#define TS_ATTN_ISSUERS 3
-#endif
-constexpr int ISSUERS = TS_ATTN_ISSUERS;     // threads that issue the MMAs of every product
+constexpr int P_PARTS = 2;                   // the probabilities of a key tile are handed over in this many parts
 constexpr int SOFTMAX_WARP0 = 2;             // warps 2..9: one thread per row of the two query tiles
-constexpr int EXTRA_WARP0 = SOFTMAX_WARP0 + GROUPS * 4;     // warps 10..: issuers 1.. (issuer 0 is warp 1)
-constexpr int THREADS = 32 * (EXTRA_WARP0 + ISSUERS - 1);
+constexpr int THREADS = 32 * (SOFTMAX_WARP0 + GROUPS * 4);
 constexpr int K_STAGES = 2;
 constexpr int V_STAGES = 2;
 constexpr int DCH = D / 64;                  // 64-column chunks of a head
@@ -89,12 +85,30 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// two floats in one 64-bit register: one instruction adds or multiplies both
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack_f32x2(float lo, float hi) {
+  f32x2 v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ float low_f32(f32x2 v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float high_f32(f32x2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ f32x2 fma_f32x2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 v;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+  return v;
+}
+__device__ __forceinline__ f32x2 add_f32x2(f32x2 a, f32x2 b) {
+  f32x2 v;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+  return v;
+}
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-// (10 warps take the registers of 12, three per scheduler: 168 registers a thread)
 __global__ void __launch_bounds__(THREADS, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, TcAttnParams p) {
@@ -110,33 +124,26 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   uint64_t* v_full = k_empty + K_STAGES;         // [V_STAGES]
   uint64_t* v_empty = v_full + V_STAGES;         // [V_STAGES] the stage's values are added to both O
   uint64_t* s_full = v_empty + V_STAGES;         // [GROUPS] S_g holds the scores of a key tile
-  uint64_t* p_full = s_full + GROUPS;            // [GROUPS] P_g is in tensor memory, O_g is rescaled
-  uint64_t* o_ready = p_full + GROUPS;           // [GROUPS] O_g holds the sum over the key tiles so far
-  uint64_t* pv_issued = o_ready + GROUPS;        // [GROUPS] every issuer has issued its P V steps of the key tile
-  uint64_t* s_first = pv_issued + GROUPS;        // [GROUPS] the first step of the scores (it overwrites S_g) is issued
-  uint64_t* o_zeroed = s_first + GROUPS;         // [GROUPS] O_g holds zeros
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_zeroed + GROUPS);
+  uint64_t* p_full = s_full + GROUPS;            // [GROUPS][P_PARTS] the part of P_g is in tensor memory, O_g is rescaled
+  uint64_t* o_ready = p_full + GROUPS * P_PARTS; // [GROUPS] O_g holds the sum over the key tiles so far
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_ready + GROUPS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(smem_u32(q_full), 1);
-    // (every issuer commits its own MMAs: what they complete counts ISSUERS arrivals)
     for (int s = 0; s < K_STAGES; ++s) {
       mbar_init(smem_u32(&k_full[s]), 1);
-      mbar_init(smem_u32(&k_empty[s]), ISSUERS);
+      mbar_init(smem_u32(&k_empty[s]), 1);
     }
     for (int s = 0; s < V_STAGES; ++s) {
       mbar_init(smem_u32(&v_full[s]), 1);
-      mbar_init(smem_u32(&v_empty[s]), ISSUERS);
+      mbar_init(smem_u32(&v_empty[s]), 1);
     }
     for (int g = 0; g < GROUPS; ++g) {
-      mbar_init(smem_u32(&s_full[g]), ISSUERS);
-      mbar_init(smem_u32(&p_full[g]), 4);
-      mbar_init(smem_u32(&o_ready[g]), ISSUERS);
-      mbar_init(smem_u32(&pv_issued[g]), ISSUERS);
-      mbar_init(smem_u32(&s_first[g]), 1);
-      mbar_init(smem_u32(&o_zeroed[g]), 4);
+      mbar_init(smem_u32(&s_full[g]), 1);
+      for (int h = 0; h < P_PARTS; ++h) mbar_init(smem_u32(&p_full[g * P_PARTS + h]), 4);
+      mbar_init(smem_u32(&o_ready[g]), 1);
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -227,77 +234,59 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         if (traced && lane == 0) timeline_mark_thread(30, t);
       }
     }
-  } else if (warp == 1 || warp >= EXTRA_WARP0) {
-    if (lane == 0 && n_tiles > 0) {
-      // issuer `me` of ISSUERS: its share of the K steps of every product, products in one order
-      const int me = warp == 1 ? 0 : warp - EXTRA_WARP0 + 1;
+  } else if (warp == 1) {
+    if (n_tiles > 0 && elect_one()) {
       constexpr uint32_t idesc_qk = make_idesc(BM, BN, false);
       constexpr uint32_t idesc_pv = make_idesc(BM, D, true);
-      constexpr int QK_STEPS = D / 16, PV_STEPS = BN / 16;
-      const int qk_lo = me * QK_STEPS / ISSUERS, qk_hi = (me + 1) * QK_STEPS / ISSUERS;
-      const int pv_lo = me * PV_STEPS / ISSUERS, pv_hi = (me + 1) * PV_STEPS / ISSUERS;
+      constexpr int QK_STEPS = D / 16, PV_STEPS = BN / 16 / P_PARTS;
       const uint64_t q_desc = smem_desc(smem_u32(Qs)), k_desc = smem_desc(smem_u32(Ks));
       const uint64_t v_desc = smem_desc_mn(smem_u32(Vs), CHUNK_BYTES);
-      // S_g = Q_g K^T of key tile t.  `after_pv`: the P V of tile g's previous key tile read P_g
-      // from S_g's columns; all of its steps must be in the pipe before step 0 here.
-      auto scores = [&](int g, int t, bool after_pv) -> bool {
+      // S_g = Q_g K^T of key tile t (the P V of tile g's previous key tile, which reads P_g from S_g's
+      // columns, is in the pipe before it)
+      auto scores = [&](int g, int t) -> bool {
         const int s = t % K_STAGES;
         if (!mbar_spin_wait(smem_u32(&k_full[s]), (t / K_STAGES) & 1, abort_flag)) return false;
-        if (me == 0) {
-          if (after_pv && !mbar_spin_wait(smem_u32(&pv_issued[g]), (t - 1) & 1, abort_flag)) return false;
-        } else {
-          if (!mbar_spin_wait(smem_u32(&s_first[g]), t & 1, abort_flag)) return false;
-        }
         tcgen05_fence_after();
-        if (traced && me == 0) timeline_mark_thread(10 + g, t);
+        if (traced) timeline_mark_thread(10 + g, t);
         // descriptors: a base made once, plus the operand's offset in 16-byte units (the address is
-        // the descriptor's low field; shared memory ends below its range).  An issuing thread is
-        // one serial chain of instructions: whatever it computes per MMA delays every MMA.
+        // the descriptor's low field; shared memory ends below its range)
         const uint64_t qd = q_desc + g * (Q_BYTES >> 4), kd = k_desc + s * (KV_BYTES >> 4);
 #pragma unroll
         for (int k = 0; k < QK_STEPS; ++k) {
-          if (k < qk_lo || k >= qk_hi) continue;
           const uint64_t off = ((k / 4) * CHUNK_BYTES + (k % 4) * 32) >> 4;
           umma(tmem_base + g * BN, qd + off, kd + off, idesc_qk, k > 0 ? 1u : 0u);
-          if (k == 0) {
-            // step 0 is in the pipe: the other issuers may add theirs
-            tcgen05_fence_before();
-            mbar_arrive(smem_u32(&s_first[g]));
-          }
         }
         tcgen05_commit(smem_u32(&s_full[g]));
         if (g == groups - 1) tcgen05_commit(smem_u32(&k_empty[s]));
         return true;
       };
-      // O_g += P_g V of key tile t
+      // O_g += P_g V of key tile t, a part of the keys at a time
       auto values = [&](int g, int t) -> bool {
         const int s = t % V_STAGES;
-        if (!mbar_spin_wait(smem_u32(&v_full[s]), (t / V_STAGES) & 1, abort_flag) ||
-            !mbar_spin_wait(smem_u32(&p_full[g]), t & 1, abort_flag))
-          return false;
-        tcgen05_fence_after();
-        if (traced && me == 0) timeline_mark_thread(12 + g, t);
+        if (!mbar_spin_wait(smem_u32(&v_full[s]), (t / V_STAGES) & 1, abort_flag)) return false;
         const uint64_t vd = v_desc + s * (KV_BYTES >> 4);
         const uint32_t o_addr = tmem_base + 2 * BN + g * 128, p_addr = tmem_base + g * BN;
 #pragma unroll
-        for (int k = 0; k < PV_STEPS; ++k) {
-          if (k < pv_lo || k >= pv_hi) continue;
-          umma_ts(o_addr, p_addr + k * 8, vd + ((k * 16 * 128) >> 4), idesc_pv, 1u);
+        for (int h = 0; h < P_PARTS; ++h) {
+          if (!mbar_spin_wait(smem_u32(&p_full[g * P_PARTS + h]), t & 1, abort_flag)) return false;
+          tcgen05_fence_after();
+          if (traced && h == 0) timeline_mark_thread(12 + g, t);
+#pragma unroll
+          for (int i = 0; i < PV_STEPS; ++i) {
+            const int k = h * PV_STEPS + i;
+            umma_ts(o_addr, p_addr + k * 8, vd + ((k * 16 * 128) >> 4), idesc_pv, t > 0 || k > 0 ? 1u : 0u);
+          }
         }
-        // this issuer's steps are in the pipe (the next scores of the tile wait for all issuers')
-        tcgen05_fence_before();
-        mbar_arrive(smem_u32(&pv_issued[g]));
         tcgen05_commit(smem_u32(&o_ready[g]));
         if (g == groups - 1) tcgen05_commit(smem_u32(&v_empty[s]));
         return true;
       };
       bool ok = mbar_spin_wait(smem_u32(q_full), 0, abort_flag);
-      for (int g = 0; ok && g < groups; ++g) ok = scores(g, 0, false);
-      for (int g = 0; ok && g < groups; ++g) ok = mbar_spin_wait(smem_u32(&o_zeroed[g]), 0, abort_flag);
+      for (int g = 0; ok && g < groups; ++g) ok = scores(g, 0);
       for (int t = 0; ok && t < n_tiles; ++t)
         for (int g = 0; ok && g < groups; ++g) {
           ok = values(g, t);
-          if (ok && t + 1 < n_tiles) ok = scores(g, t + 1, true);
+          if (ok && t + 1 < n_tiles) ok = scores(g, t + 1);
         }
     }
   } else {
@@ -321,18 +310,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       const bool tracer = traced && (threadIdx.x & 127) == 64;
       float m = -INFINITY, l = 0.f;
       bool ok = true;
-      {
-        // O_g starts as zeros: every P V step then accumulates, whichever issuer's comes first
-        float zeros[32];
-#pragma unroll
-        for (int e = 0; e < 32; ++e) zeros[e] = 0.f;
-#pragma unroll
-        for (int c = 0; c < D; c += 32) tmem_store32(tmem_o + lane_addr + c, zeros);
-        tmem_store_wait();
-        tcgen05_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&o_zeroed[g]));
-      }
       for (int t = 0; t < n_tiles; ++t) {
         const int j0 = tile_of(t) * BN;
         ok = mbar_wait(smem_u32(&s_full[g]), t & 1, abort_flag);
@@ -411,44 +388,44 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         const float alpha = ex2(m - m_safe);
         // (these scores were computed after the previous key tile's P V of this query tile, in
         // order: P_g has been read and the sum in O_g is complete)
-        // probabilities -> tensor memory, bfloat16 pairs over the first 64 columns of S_g: the A
-        // operand of O += P V
-        float sum4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int c = 0; c < BN; c += 64) {
-          float packed[32];
-#pragma unroll
-          for (int e = 0; e < 64; e += 2) {
-            const float p0 = ex2(fmaf(sv[c + e], sc, -m_safe));        // -inf gives 0
-            const float p1 = ex2(fmaf(sv[c + e + 1], sc, -m_safe));
-            sum4[(e / 2) & 3] += p0 + p1;
-            packed[e / 2] = __uint_as_float(pack2(p0, p1));
-          }
-          tmem_store32(tmem_s + lane_addr + c / 2, packed);
-        }
-        const float sum = (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
-        l = l * alpha + sum;
-        m = m_new;
-        if (tracer) timeline_mark_thread(22 + 4 * g, t);
         if (t > 0 && !__all_sync(0xffffffffu, alpha == 1.f)) {
-          float ov[D];
-#pragma unroll
-          for (int c = 0; c < D; c += 32) tmem_load32_nowait(tmem_o + lane_addr + c, ov + c);
-          tmem_load_wait();
-#pragma unroll
+          // 32 columns at a time: the row of S is still in registers
+#pragma unroll 1
           for (int c = 0; c < D; c += 32) {
             float v[32];
+            tmem_load32(tmem_o + lane_addr + c, v);
 #pragma unroll
-            for (int e = 0; e < 32; ++e) v[e] = ov[c + e] * alpha;
+            for (int e = 0; e < 32; ++e) v[e] *= alpha;
             tmem_store32(tmem_o + lane_addr + c, v);
           }
-          tmem_store_wait();
         }
-        tmem_store_wait();
-        tcgen05_fence_before();
-        __syncwarp();
+        // probabilities -> tensor memory, bfloat16 pairs over the first 64 columns of S_g: the A
+        // operand of O += P V, handed over in P_PARTS parts
+        f32x2 sum2[4] = {pack_f32x2(0.f, 0.f), pack_f32x2(0.f, 0.f), pack_f32x2(0.f, 0.f), pack_f32x2(0.f, 0.f)};
+        const f32x2 sc2 = pack_f32x2(sc, sc), minus_m2 = pack_f32x2(-m_safe, -m_safe);
+#pragma unroll
+        for (int h = 0; h < P_PARTS; ++h) {
+#pragma unroll
+          for (int c = h * (BN / P_PARTS); c < (h + 1) * (BN / P_PARTS); c += 32) {
+            float packed[16];
+#pragma unroll
+            for (int e = 0; e < 32; e += 2) {
+              const f32x2 x = fma_f32x2(pack_f32x2(sv[c + e], sv[c + e + 1]), sc2, minus_m2);
+              const float p0 = ex2(low_f32(x)), p1 = ex2(high_f32(x));        // -inf gives 0
+              sum2[(e / 2) & 3] = add_f32x2(sum2[(e / 2) & 3], pack_f32x2(p0, p1));
+              packed[e / 2] = __uint_as_float(pack2(p0, p1));
+            }
+            tmem_store16(tmem_s + lane_addr + c / 2, packed);
+          }
+          tmem_store_wait();
+          tcgen05_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&p_full[g * P_PARTS + h]));
+        }
+        const f32x2 sums = add_f32x2(add_f32x2(sum2[0], sum2[1]), add_f32x2(sum2[2], sum2[3]));
+        l = l * alpha + (low_f32(sums) + high_f32(sums));
+        m = m_new;
         if (tracer) timeline_mark_thread(23 + 4 * g, t);
-        if (lane == 0) mbar_arrive(smem_u32(&p_full[g]));
       }
       if (ok) {
         ok = mbar_wait(smem_u32(&o_ready[g]), (n_tiles - 1) & 1, abort_flag);

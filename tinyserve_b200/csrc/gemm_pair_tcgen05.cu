@@ -7,13 +7,11 @@
 // tensor memory, so every SM loads and reads only half of the weight tile.  Per 64-wide slice of
 // K each block's loader thread issues its TMA loads (128-byte swizzle, every block its own: no
 // cluster-wide copies) into a ring of five stages; both blocks' loads complete on the first
-// block's mbarrier.  Four threads of the first block issue
-// the four K steps of a stage (one thread issues a tcgen05.mma every 196 cycles at most, measured,
-// and an MMA of this size takes 128), all into the same accumulator, and commit the stage back to
-// both loaders.  Accumulators are double buffered (2 x 256 of the 512 columns): four epilogue
-// warps per block drain tile i (one thread per token row) while tile i + 1 is multiplied, zero
-// what they drained (every MMA accumulates, so no order among the issuing threads is needed) and
-// hand the buffer back.
+// block's mbarrier.  One thread of the first block (chosen by elect.sync, so that the MMAs' operands
+// stay in uniform registers: with `lane == 0` an MMA took 196 cycles to issue and four threads had to
+// share them) issues the four K steps of a stage and commits the stage back to both loaders.
+// Accumulators are double buffered (2 x 256 of the 512 columns): four epilogue warps per block drain
+// tile i (one thread per token row) while tile i + 1 is multiplied, and hand the buffer back.
 //
 // The epilogue warps reach global memory through tiles of 128 rows x 128 bytes in shared memory,
 // so that a warp's loads and stores cover whole lines; stores are not waited for, and the residual
@@ -27,9 +25,8 @@
 // pays.  A pair that holds part of such a tile adds its 32-bit partial tile to the tile's sum in
 // global memory (red.global.add; in the residual form the sum is the residual itself) and bumps the
 // tile's counter; the block that arrives last runs the epilogue on the sum.  Nobody waits for
-// anybody.  (The four issuing threads add into one accumulator in the order in which the tensor
-// core takes their instructions, and the parts of a cut tile in the order in which they arrive:
-// two runs agree to the rounding of a 32-bit sum, not bit by bit.)
+// anybody.  (The parts of a cut tile are added in the order in which they arrive: two runs agree to
+// the rounding of a 32-bit sum, not bit by bit.)
 //
 // Epilogues: plain (optional bias, optional RMSNorm factor per token row), gated (weight rows
 // alternate in blocks of 64, gate then up: out = act(gate) * up), residual (residual += result in
@@ -49,9 +46,8 @@ constexpr int BM = 128;              // token rows of a block (256 of the pair)
 constexpr int HALF_N = 256;          // weight rows of one MMA over the pair (128 in each block's shared memory)
 constexpr int BK = 64;               // K elements of a stage: 128 bytes, one swizzle row
 constexpr int A_BYTES = BM * BK * 2, B_BYTES = (HALF_N / 2) * BK * 2;
-constexpr int ISSUERS = BK / 16;     // one issuing thread per K step of a stage
-constexpr int LOAD_WARP = 4, ISSUE_WARP0 = 5;        // warps 0-3: epilogue; 4: loads; 5-8: issue (and epilogue)
-constexpr int THREADS = 32 * (ISSUE_WARP0 + ISSUERS);
+constexpr int K_STEPS = BK / 16;     // K steps of a stage
+constexpr int LOAD_WARP = 4, ISSUE_WARP0 = 5;        // warps 0-3: epilogue; 4: loads; 5: issues; 5-8: epilogue of the wide tile
 constexpr int TMEM_COLS = 512;
 constexpr int CHUNK = 32, CHUNKS = HALF_N / CHUNK;
 constexpr int TILE_BYTES = BM * 128; // an epilogue tile in shared memory: 128 rows of 128 bytes (32 float or 64 bfloat16)
@@ -68,6 +64,7 @@ template <int HALVES> struct Cfg {
   static constexpr int STAGES = HALVES == 1 ? 5 : 4;
   static constexpr int BUFFERS = 2 / HALVES;
   static constexpr int GROUPS = HALVES;            // epilogue groups of four warps, one per half
+  static constexpr int THREADS = 32 * (ISSUE_WARP0 + (HALVES == 1 ? 1 : 4));
   static constexpr int EPI_TILES = HALVES == 1 ? 2 : 1;      // tiles of each kind (accumulators in, rows out) per group
   static constexpr int ALL_TILES = 2 * GROUPS * EPI_TILES / HALVES;         // four, or two
   static constexpr size_t SMEM = 1024 + (size_t)STAGES * STAGE_BYTES + ALL_TILES * TILE_BYTES + 256;
@@ -137,13 +134,13 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster), "r"(x), "r"(y) : "memory");
 }
-// one MMA over the pair: D (both blocks' tensor memory) += A (128 rows of each block) * B (128 rows of each block)^T
-__device__ __forceinline__ void umma_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc) {
+// one MMA over the pair: D (both blocks' tensor memory) = or += A (128 rows of each block) * B (128 rows of each block)^T
+__device__ __forceinline__ void umma_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(1u) : "memory");
+      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
 }
 // arrives on the mbarrier at this shared-memory offset in both blocks once this thread's MMAs are done
 __device__ __forceinline__ void commit_pair(uint32_t bar) {
@@ -228,9 +225,6 @@ __device__ __forceinline__ bool epilogue_half(const PairParams& p, const Segment
   const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * HALF_N + g * HALF_N;
   // the other arrangement: unit u of rows rb + 16 j
   const int u = r_in & 7, rb = r_in >> 3;
-  float zeros[CHUNK];
-#pragma unroll
-  for (int e = 0; e < CHUNK; ++e) zeros[e] = 0.f;
   const bool partial = sg.parts > 1;                           // (tiles of 256 rows only)
   auto acc_tile = [&](int b) { return sh.acc + (b & (NT - 1)) * TILE_BYTES; };
   auto ost_tile = [&](int b) { return sh.ost + (b & (NT - 1)) * TILE_BYTES; };
@@ -261,7 +255,6 @@ __device__ __forceinline__ bool epilogue_half(const PairParams& p, const Segment
   tcgen05_fence_after();
   if (traced) timeline_mark_thread(41, sg.s1 - sg.s0);
   auto release_tmem = [&]() {
-    tmem_store_wait();
     tcgen05_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive_cluster(acc_empty0 + buf * 8);
@@ -273,7 +266,6 @@ __device__ __forceinline__ bool epilogue_half(const PairParams& p, const Segment
     for (int c = 0; c < CHUNKS; ++c) {
       float v[CHUNK];
       tmem_load32(acc + c * CHUNK, v);
-      tmem_store32(acc + c * CHUNK, zeros);
       tile_write_f32(acc_tile(c), r_in, v);
       epi_barrier(g);
       const bool col_ok = p.residual == nullptr || col0 + c * CHUNK + u * 4 < p.N;
@@ -313,13 +305,12 @@ __device__ __forceinline__ bool epilogue_half(const PairParams& p, const Segment
     for (int t = 0; t < p.x_tiles; ++t) ss += __ldcg(p.x_sumsq + (size_t)t * p.x_stride + own_row);
     row_scale = rsqrtf(ss / (float)p.K + p.x_eps);
   }
-  // chunk c of the accumulators of the row this thread owns: from tensor memory (zeroed behind),
+  // chunk c of the accumulators of the row this thread owns: from tensor memory,
   // or, for the block that finishes a cut tile, the sum of the parts (through a tile in shared
   // memory; the scratch is zeroed behind).  The four warps meet inside.
   auto take = [&](int c, int stage, float (&v)[CHUNK]) {
     if (!partial) {
       tmem_load32(acc + c * CHUNK, v);
-      tmem_store32(acc + c * CHUNK, zeros);
       return;
     }
     float4 a[8];
@@ -357,7 +348,6 @@ __device__ __forceinline__ bool epilogue_half(const PairParams& p, const Segment
       if (!partial) {
         float v[CHUNK];
         tmem_load32(acc + c * CHUNK, v);
-        tmem_store32(acc + c * CHUNK, zeros);
         tile_write_f32(acc_tile(c), r_in, v);
         epi_barrier(g);
       }
@@ -420,7 +410,6 @@ __device__ __forceinline__ bool epilogue_half(const PairParams& p, const Segment
       const int col = col0 + c * CHUNK;
       float v[CHUNK];
       tmem_load32(acc + c * CHUNK, v);
-      tmem_store32(acc + c * CHUNK, zeros);
 #pragma unroll
       for (int e = 0; e < CHUNK; ++e) {
         v[e] *= row_scale;
@@ -459,7 +448,7 @@ __device__ __forceinline__ bool epilogue_half(const PairParams& p, const Segment
 }
 
 template <int HALVES>
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(Cfg<HALVES>::THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, PairParams p) {
   using C = Cfg<HALVES>;
   extern __shared__ char smem_raw[];
@@ -481,10 +470,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) {
       mbar_init(smem_u32(&full[s]), 1);
-      mbar_init(smem_u32(&empty[s]), ISSUERS);
+      mbar_init(smem_u32(&empty[s]), 1);
     }
     for (int b = 0; b < 2; ++b) {
-      mbar_init(smem_u32(&acc_full[b]), ISSUERS);
+      mbar_init(smem_u32(&acc_full[b]), 1);
       mbar_init(smem_u32(&acc_empty[b]), 2 * 4 * C::GROUPS);     // every epilogue warp of both blocks
     }
     *abort_flag = 0;
@@ -512,34 +501,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   };
   const uint32_t acc_empty0 = map_to_rank(smem_u32(acc_empty), 0);
 
-  // Every accumulator starts at zero and every MMA accumulates: the warps that will drain a part
-  // of the tensor memory zero it now (and behind every chunk they drain) and hand it to the
-  // issuing threads.
-  const bool drains = warp < 4 || (HALVES == 2 && warp >= ISSUE_WARP0);
   const int group = warp < 4 ? 0 : 1, quarter = warp & 3;
   // group g's tiles: with tiles of 256 rows two of each kind, else one that serves as either
   EpiShared sh;
   sh.acc = tiles + (HALVES == 1 ? 0 : group * TILE_BYTES);
   sh.ost = tiles + (HALVES == 1 ? 2 * TILE_BYTES : group * TILE_BYTES);
-  if (drains) {
-    float zeros[CHUNK];
-#pragma unroll
-    for (int e = 0; e < CHUNK; ++e) zeros[e] = 0.f;
-    const uint32_t mine = tmem_base + ((uint32_t)(quarter * 32) << 16);
-    if (HALVES == 2) {
-      for (int c = 0; c < CHUNKS; ++c) tmem_store32(mine + group * HALF_N + c * CHUNK, zeros);
-    } else {
-      for (int c = 0; c < 2 * CHUNKS; ++c) tmem_store32(mine + c * CHUNK, zeros);
-    }
-    tmem_store_wait();
-    tcgen05_fence_before();
-    __syncwarp();
-    if (lane == 0) {
-      mbar_arrive_cluster(acc_empty0);
-      if (C::BUFFERS == 2) mbar_arrive_cluster(acc_empty0 + 8);
-    }
-  }
-
   if (warp == LOAD_WARP) {
     if (lane == 0) {
       const uint32_t full0 = map_to_rank(smem_u32(full), 0);     // the first block's barriers
@@ -565,7 +531,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       if (!ok) tell_partner();
     }
   } else if (warp >= ISSUE_WARP0) {
-    const int k_step = warp - ISSUE_WARP0;
     // bf16 x bf16 -> f32, both operands K-major, M = 256 over the pair, N = 256
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(HALF_N >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
     int stage = 0;
@@ -573,33 +538,35 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     bool ok = true;
     Segment sg;
     for (int i = 0; ok && segment_of(p, pair, i, sg); ++i) {
-      if (lane == 0 && rank == 0) {
+      if (warp == ISSUE_WARP0 && rank == 0 && elect_one()) {
         const int buf = C::BUFFERS == 2 ? (i & 1) : 0;
         const uint32_t parity = C::BUFFERS == 2 ? ((uint32_t)(i >> 1) & 1u) : ((uint32_t)i & 1u);
-        ok = mbar_wait(smem_u32(&acc_empty[buf]), parity, abort_flag);
+        // (a buffer is free at the start: the wait on the phase before the first returns at once)
+        ok = mbar_spin_wait(smem_u32(&acc_empty[buf]), parity ^ 1u, abort_flag);
         tcgen05_fence_after();
-        if (k_step == 0 && (pair % 24) == 0) timeline_mark_thread(50, i);
+        if ((pair % 24) == 0) timeline_mark_thread(50, i);
         const uint32_t d = tmem_base + buf * HALF_N;
         for (int s = sg.s0; ok && s < sg.s1; ++s) {
           ok = mbar_spin_wait(smem_u32(&full[stage]), phase, abort_flag);
           if (!ok) break;
           tcgen05_fence_after();
-          const uint32_t a = smem_u32(smem + (size_t)stage * C::STAGE_BYTES);
-          const uint64_t step = (uint64_t)((k_step * 32) >> 4);
+          const uint64_t a = smem_desc(smem_u32(smem + (size_t)stage * C::STAGE_BYTES));
 #pragma unroll
-          for (int h = 0; h < HALVES; ++h)
-            umma_pair(d + h * HALF_N, smem_desc(a) + step, smem_desc(a + A_BYTES + h * B_BYTES) + step, idesc);
+          for (int k = 0; k < K_STEPS; ++k)
+#pragma unroll
+            for (int h = 0; h < HALVES; ++h)
+              umma_pair(d + h * HALF_N, a + k * 2, a + ((A_BYTES + h * B_BYTES) >> 4) + k * 2, idesc, s > sg.s0 || k > 0 ? 1u : 0u);
           commit_pair(smem_u32(&empty[stage]));
           if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
         }
         if (ok) commit_pair(smem_u32(&acc_full[buf]));
-        if (k_step == 0 && (pair % 24) == 0) timeline_mark_thread(51, sg.s1 - sg.s0);
+        if ((pair % 24) == 0) timeline_mark_thread(51, sg.s1 - sg.s0);
         if (!ok) tell_partner();
       }
+      // the issuing thread's outcome is its warp's (which meets again here before the next election)
+      ok = __all_sync(0xffffffffu, ok) != 0;
       if (HALVES == 2) {
-        // the issuing warps drain the second half of the tile
-        __syncwarp();
-        ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+        // this warp and the next three drain the second half of the tile
         if (ok) ok = epilogue_half<HALVES>(p, sg, i, 1, quarter, lane, rank, tmem_base, acc_full, acc_empty0, sh, abort_flag, is_last);
       }
     }
@@ -674,7 +641,7 @@ int launch(const CUtensorMap& mx, const CUtensorMap& mw, const PairParams& p, cu
     configured = true;
   }
   const int blocks = 2 * (p.pairs < p.dp_tiles + p.tail_pairs ? p.pairs : p.dp_tiles + p.tail_pairs);
-  cudaError_t e = ts_launch_cluster(gemm_pair_kernel<HALVES>, dim3(blocks), dim3(THREADS), Cfg<HALVES>::SMEM, stream, dim3(2, 1, 1), mx, mw, p);
+  cudaError_t e = ts_launch_cluster(gemm_pair_kernel<HALVES>, dim3(blocks), dim3(Cfg<HALVES>::THREADS), Cfg<HALVES>::SMEM, stream, dim3(2, 1, 1), mx, mw, p);
   if (e != cudaSuccess) return ts_fail("gemm_pair (%d pairs): %s", p.pairs, cudaGetErrorString(e));
   return 0;
 }
@@ -693,7 +660,7 @@ TS_EXPORT int ts_gemm_pair_max_pairs() {
   if (cudaFuncSetAttribute(gemm_pair_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<1>::SMEM) != cudaSuccess) return 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2);
-  cfg.blockDim = dim3(THREADS);
+  cfg.blockDim = dim3(Cfg<1>::THREADS);
   cfg.dynamicSmemBytes = Cfg<1>::SMEM;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;

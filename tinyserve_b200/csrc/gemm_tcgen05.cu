@@ -6,11 +6,8 @@
 // the tensor core) and the tokens, padded to TILE_T in {16, 32, 64, 128}, as its N side.  The
 // accumulator D[128 weight rows x TILE_T tokens] lives in tensor memory.  Per 64-wide slice of K
 // one thread issues two TMA loads (W tile 128 x 64, x tile TILE_T x 64, 128-byte swizzle) into a
-// ring of shared-memory stages guarded by mbarriers; four threads of four warps issue one
-// tcgen05.mma (K = 16) each per slice, into an accumulator of their own, and commit the stage back
-// to the loader.  (One thread can issue a tcgen05.mma every 196 cycles, however small the MMA:
-// measured on B200.  Four issuing warps give four times the rate, which a block needs to keep
-// up with its share of the memory bandwidth when few blocks stream a product.)
+// ring of shared-memory stages guarded by mbarriers; one thread of another warp issues the slice's
+// four tcgen05.mma (K = 16) and commits the stage back to the loader.
 //
 // Shapes with few row tiles (N = 4096: 32 tiles for 148 SMs) are also cut along K.  Every block
 // then stores its partial tile to scratch and bumps the tile's counter; the block that arrives
@@ -38,8 +35,8 @@ namespace {
 using bf16 = __nv_bfloat16;
 constexpr int TILE_N = 128;          // weight rows of a block (MMA M)
 constexpr int BK = 64;               // K elements of a stage: 128 bytes, one swizzle row
-constexpr int ISSUERS = BK / 16;     // issuing threads: one per K step of a stage, each with its own accumulator
-constexpr int THREADS = 32 * (1 + ISSUERS);      // warp 0 loads, warps 1..4 issue, warps 0..3 do the epilogue
+constexpr int K_STEPS = BK / 16;     // MMAs of a stage
+constexpr int THREADS = 128;         // warp 0 loads, warp 1 issues, all four do the epilogue
 constexpr int W_STAGE_BYTES = TILE_N * BK * 2;
 
 // one of the products of the beside form
@@ -97,29 +94,13 @@ __host__ __device__ constexpr uint32_t instr_desc(int tile_t) {
   return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(tile_t >> 3) << 17) |
          (static_cast<uint32_t>(TILE_N >> 4) << 24);
 }
-// The four K steps of a stage go to four accumulators, one per issuing thread, which the
-// epilogue adds up.
-template <int TILE_T> struct Accs { static constexpr int N = ISSUERS; };
-
-template <int TILE_T>
-__device__ __forceinline__ void tmem_load8_sum(uint32_t addr, float (&v)[8]) {
-  tmem_load8(addr, v);
-#pragma unroll
-  for (int a = 1; a < Accs<TILE_T>::N; ++a) {
-    float t[8];
-    tmem_load8(addr + a * TILE_T, t);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] += t[i];
-  }
-}
-
 template <int TILE_T> struct Cfg {
   static constexpr int X_STAGE_BYTES = TILE_T * BK * 2;
   static constexpr int STAGE_BYTES = W_STAGE_BYTES + X_STAGE_BYTES;
   // two blocks share an SM: the ring and the barriers of a block stay below 113 KB
   static constexpr int RING = TS_GEMM_RING_KB * 1024;
   static constexpr int STAGES = RING / STAGE_BYTES < 2 ? 2 : (RING / STAGE_BYTES > 8 ? 8 : RING / STAGE_BYTES);
-  static constexpr int TMEM_COLS = Accs<TILE_T>::N * TILE_T < 32 ? 32 : Accs<TILE_T>::N * TILE_T;
+  static constexpr int TMEM_COLS = TILE_T < 32 ? 32 : TILE_T;
   static constexpr size_t SMEM = 1024 + (size_t)STAGES * STAGE_BYTES + 256;
 };
 
@@ -163,9 +144,9 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) {
       mbar_init(smem_u32(&full[s]), 1);
-      mbar_init(smem_u32(&empty[s]), ISSUERS);       // every issuing thread commits its own MMA
+      mbar_init(smem_u32(&empty[s]), 1);
     }
-    mbar_init(smem_u32(accum), ISSUERS);
+    mbar_init(smem_u32(accum), 1);
     *abort_flag = 0;
     *is_last = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -213,13 +194,12 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
         for (uint32_t w = 0; w < WAIT_LIMIT && !mbar_try_wait(bar, (i / C::STAGES) & 1); ++w) {}
       }
     }
-  } else if (warp >= 1 && lane == 0) {
-    // issuer `k` of four: the k-th K step (16 wide) of every stage, into accumulator k
-    const int k = warp - 1;
+  } else if (warp == 1 && elect_one()) {
+    // (chosen by elect.sync: with `lane == 0` in its place a thread issues one MMA per 196 cycles,
+    // because the compiler cannot keep its operands in uniform registers)
     pdl_wait();
     const uint32_t idesc = instr_desc(TILE_T);
     const uint64_t desc0 = smem_desc(smem_u32(smem));
-    const uint32_t acc = tmem_base + k * TILE_T;
     bool ok = true;
     for (int i = 0; i < nkb && ok; ++i) {
       const int s = i % C::STAGES;
@@ -228,16 +208,18 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
       tcgen05_fence_after();
       // one descriptor per operand and stage; a K step of 16 is 32 bytes = 2 address units on
       const uint64_t ad = desc0 + (uint64_t)s * (C::STAGE_BYTES >> 4), bd = ad + (W_STAGE_BYTES >> 4);
-      umma(acc, ad + 2 * k, bd + 2 * k, idesc, i > 0 ? 1u : 0u);
+#pragma unroll
+      for (int k = 0; k < K_STEPS; ++k) umma(tmem_base, ad + 2 * k, bd + 2 * k, idesc, i > 0 || k > 0 ? 1u : 0u);
       tcgen05_commit(smem_u32(&empty[s]));
     }
     if (ok && nkb > 0) tcgen05_commit(smem_u32(accum));
   } else {
     pdl_wait();
-    // (lanes 1.. of warps 1..4: they do not issue, they have time for the rows' norm factors)
-    const int idle = (warp - 1) * 31 + lane - 1;          // 0 .. 123 over the non-issuing lanes of warps 1..4
+    // (the lanes of warps 1..3 that do not issue have time for the rows' norm factors; two lanes
+    // take each row, so that one is left wherever the issuing lane is)
+    const int pair = (warp - 1) * 16 + (lane >> 1);       // 0 .. 47 over warps 1..3
     if (p.x_sumsq != nullptr && warp >= 1) {
-      for (int j = idle; j < TILE_T; j += 31 * ISSUERS) {
+      for (int j = pair; j < TILE_T; j += 48) {
         const int m = t_tile * TILE_T + j;
         float sum = 0.f;
         if (m < p.M)
@@ -254,13 +236,10 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
   if (have) have = mbar_spin_wait(smem_u32(accum), 0, abort_flag);
   have = __all_sync(0xffffffffu, have);      // tcgen05.ld is warp-wide: decide per warp
   tcgen05_fence_after();
-  // warps 0..3 own the 128 lanes of tensor memory (a warp reaches the quarter of its index mod 4);
-  // warp 4 only takes part in the barriers
-  const bool epi = warp < 4;
-  have = have && epi;
+  // warp w owns lanes 32 w .. 32 w + 31 of tensor memory
   const int n = n_tile * TILE_N + warp * 32 + lane;
   const int t0 = t_tile * TILE_T;
-  const uint32_t taddr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+  const uint32_t taddr = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
   if (p.residual != nullptr) {
     // residual form.  Every block of the cluster leaves its partial tile in its shared memory
     // (the ring is idle: all MMAs have completed); rank r then owns the tokens r, r + splits, ...:
@@ -270,20 +249,20 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
 #pragma unroll 1
     for (int c = 0; c < TILE_T; c += 8) {
       float v[8];
-      if (have) tmem_load8_sum<TILE_T>(taddr + c, v);
+      if (have) tmem_load8(taddr + c, v);
       else {
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = 0.f;
       }
-      if (epi) {
+      {
 #pragma unroll
         for (int i = 0; i < 8; ++i) red[(c + i) * TILE_N + threadIdx.x] = scaled ? v[i] * row_scale[c + i] : v[i];
       }
     }
-    const float wn = (epi && n < p.N) ? p.norm_w[n] : 0.f;
-    const float rs = (epi && n < p.N && p.res_scale.ptr != nullptr) ? p.res_scale[n] : 1.f;
+    const float wn = (n < p.N) ? p.norm_w[n] : 0.f;
+    const float rs = (n < p.N && p.res_scale.ptr != nullptr) ? p.res_scale[n] : 1.f;
     float wn2 = 0.f, bn = 0.f;
-    if (MULTI && epi && n < p.N) {
+    if (MULTI && n < p.N) {
       if (p.hprime2 != nullptr) wn2 = p.norm_w2[n];
       if (p.bias.ptr != nullptr) bn = p.bias[n];
     }
@@ -294,9 +273,9 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
       float part[8];
 #pragma unroll
       for (int s = 0; s < 8; ++s)
-        if (epi && s < p.splits) part[s] = cluster_load_f32(red + j * TILE_N + threadIdx.x, s);
+        if (s < p.splits) part[s] = cluster_load_f32(red + j * TILE_N + threadIdx.x, s);
       float sq = 0.f;
-      if (epi && n < p.N) {
+      if (n < p.N) {
         float sum = 0.f;
 #pragma unroll
         for (int s = 0; s < 8; ++s)
@@ -325,7 +304,7 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
 #pragma unroll
       for (int c = 0; c < TILE_T; c += 8) {
         float v[8];
-        if (have) tmem_load8_sum<TILE_T>(taddr + c, v);
+        if (have) tmem_load8(taddr + c, v);
         else {
 #pragma unroll
           for (int i = 0; i < 8; ++i) v[i] = 0.f;
@@ -334,7 +313,7 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
         for (int i = 0; i < 8; ++i) acc[c + i] = scaled ? v[i] * row_scale[c + i] : v[i];
       }
       float* up = reinterpret_cast<float*>(smem);               // [64][TILE_T + 1]
-      if (warp >= 2 && epi) {
+      if (warp >= 2) {
 #pragma unroll
         for (int i = 0; i < TILE_T; ++i) up[(threadIdx.x - 64) * (TILE_T + 1) + i] = acc[i];
       }
@@ -358,7 +337,7 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
 #pragma unroll 1
     for (int c = 0; c < TILE_T; c += 8) {
       float v[8];
-      if (have) tmem_load8_sum<TILE_T>(taddr + c, v);
+      if (have) tmem_load8(taddr + c, v);
       else {
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = 0.f;
@@ -369,7 +348,7 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
       }
 #pragma unroll
       for (int i = 0; i < 8; ++i) v[i] = plain_value(v[i] + bn, p.out_act);
-      if (epi && n < N) {
+      if (n < N) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const int m = t0 + c + i;
@@ -386,12 +365,12 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
 #pragma unroll 1
     for (int c = 0; c < TILE_T; c += 8) {
       float v[8];
-      if (have) tmem_load8_sum<TILE_T>(taddr + c, v);
+      if (have) tmem_load8(taddr + c, v);
       else {
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = 0.f;
       }
-      if (epi) {
+      {
 #pragma unroll
         for (int i = 0; i < 8; ++i) mine[(c + i) * TILE_N + warp * 32 + lane] = scaled ? v[i] * row_scale[c + i] : v[i];
       }
@@ -406,7 +385,7 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
         if (*is_last) p.counters[tile] = 0;
       }
       __syncthreads();
-      if (*is_last && epi) {
+      if (*is_last) {
         __threadfence();
         const float* base = p.partials + (size_t)tile * (TILE_T * TILE_N);
         const size_t split_stride = (size_t)tiles * (TILE_T * TILE_N);
