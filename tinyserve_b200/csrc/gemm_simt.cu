@@ -9,6 +9,8 @@
 // products each need to stay within 1e-4 of a float64 reference.)  Inputs may also be bfloat16
 // (products and sums still 32-bit).
 // tinyserve uses cuBLAS through nn.Linear for all of these (serve.py:828-829, 912-913, 1263).
+#include <type_traits>
+
 #include "common.cuh"
 
 TS_DEFINE_LAST_ERROR()
@@ -122,6 +124,165 @@ gemm_nt_kernel(const TI* __restrict__ A, const TI* __restrict__ W, const TI* __r
   }
 }
 
+// The product of a few rows of A (decode steps, the last rows before the vocabulary projection), in
+// which W is nearly all the bytes.  A thread owns one chain of SUM_BLOCK k (a "slot") of RT rows of W
+// for all of the MT rows of A, so that the sums are those of the tiled kernel bit by bit, and a block
+// covers CS chains of a row at a time: its threads are CS chains x 128 / CS groups of RT rows.  Slices
+// of STAGE_K k of every slot come through a ring of shared-memory stages (cp.async, 16 bytes a thread,
+// neighbouring threads on neighbouring bytes of a row); the stages of W that are fetched first do not
+// wait for the predecessor kernel.  The 16-byte unit u of slot s lies at u ^ (s & 7), so that
+// eight threads that read the same unit of eight slots touch all banks.  After the last slice of a
+// chain the chains' results go through shared memory to one thread per output, which adds them in
+// the order of k.
+// Bound by the bytes of W where MT is small, by shared-memory reads (1 + MT / RT per four fmaf x MT) above:
+// hence RT rows of W share the values of A.
+constexpr int SLOTS = 128;           // threads of a block: chains in flight x groups of rows
+constexpr int STAGE_K = 32;          // k of a slot that a stage holds: half a chain, 128 bytes
+constexpr int STAGE_UNITS = STAGE_K / 4;
+constexpr int GEMV_MAX_ROWS = 256, GEMV_MIN_BLOCKS = 128;
+constexpr int MAX_CHAINS_SHIFT = 4;  // up to 16 chains of a row at a time: 8 RT rows a block
+
+__device__ __forceinline__ void copy16_async(uint32_t dst, const void* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0));
+}
+
+template <int MT, int RT, int STAGES>
+__global__ void __launch_bounds__(SLOTS)
+gemv_nt_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
+               int M, int N, int K, size_t lda, size_t ldw, size_t ldc, int cs_shift) {
+  extern __shared__ __align__(16) char smem[];
+  const int cs = 1 << cs_shift, groups = SLOTS >> cs_shift;      // chains in flight, groups of rows
+  const int rows = groups * RT;
+  constexpr int W_BYTES = SLOTS * RT * STAGE_K * 4;
+  const int x_bytes = MT * cs * STAGE_K * 4;
+  const int stage_bytes = W_BYTES + x_bytes;
+  float* red = reinterpret_cast<float*>(smem + STAGES * stage_bytes);        // [MT][rows][cs + 1]
+  pdl_trigger();
+  const int n0 = blockIdx.x * rows, m0 = blockIdx.y * MT;
+  const int chains = (K + SUM_BLOCK - 1) / SUM_BLOCK;
+  const int passes = (chains + cs - 1) >> cs_shift;              // a pass: cs chains of every row, two stages
+  const int stages = 2 * passes;
+  const int tid = threadIdx.x;
+  const int c = tid & (cs - 1), g = tid >> cs_shift;
+
+  // unit i of a stage: slot i / 8 ((row, chain) with the chain fastest), 16 bytes i % 8 of it
+  auto load_w = [&](int st) {
+    const uint32_t base = static_cast<uint32_t>(__cvta_generic_to_shared(smem + (st % STAGES) * stage_bytes));
+    const int k0 = (st >> 1) * cs * SUM_BLOCK + (st & 1) * STAGE_K;
+#pragma unroll
+    for (int i = tid; i < SLOTS * RT * STAGE_UNITS; i += SLOTS) {
+      const int slot = i / STAGE_UNITS, u = i % STAGE_UNITS;
+      const int r = slot >> cs_shift, k = k0 + (slot & (cs - 1)) * SUM_BLOCK + u * 4;
+      const bool ok = n0 + r < N && k < K;
+      copy16_async(base + slot * (STAGE_K * 4) + ((u ^ (slot & 7)) << 4), W + (ok ? (size_t)(n0 + r) * ldw + k : 0), ok);
+    }
+  };
+  auto load_x = [&](int st) {
+    const uint32_t base = static_cast<uint32_t>(__cvta_generic_to_shared(smem + (st % STAGES) * stage_bytes + W_BYTES));
+    const int k0 = (st >> 1) * cs * SUM_BLOCK + (st & 1) * STAGE_K;
+    for (int i = tid; i < MT * cs * STAGE_UNITS; i += SLOTS) {
+      const int slot = i / STAGE_UNITS, u = i % STAGE_UNITS;
+      const int m = m0 + (slot >> cs_shift), k = k0 + (slot & (cs - 1)) * SUM_BLOCK + u * 4;
+      const bool ok = m < M && k < K;
+      copy16_async(base + slot * (STAGE_K * 4) + ((u ^ (slot & 7)) << 4), A + (ok ? (size_t)m * lda + k : 0), ok);
+    }
+  };
+  // the first stages of W, then (with the predecessor's results) those of A: a group of copies each
+  for (int st = 0; st < STAGES - 1; ++st)
+    if (st < stages) load_w(st);
+  pdl_wait();
+  for (int st = 0; st < STAGES - 1; ++st) {
+    if (st < stages) load_x(st);
+    asm volatile("cp.async.commit_group;\n" ::);       // (the first group holds every stage of W so far)
+  }
+
+  float part[RT][MT];
+#pragma unroll
+  for (int r = 0; r < RT; ++r)
+#pragma unroll
+    for (int m = 0; m < MT; ++m) part[r][m] = 0.f;
+  const int outputs = rows * MT;
+  float* totals = red + (size_t)outputs * (cs + 1);              // [MT][rows]
+  for (int st = 0; st < stages; ++st) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2));
+    __syncthreads();
+    // (the stage that everybody is done with)
+    if (st + STAGES - 1 < stages) {
+      load_w(st + STAGES - 1);
+      load_x(st + STAGES - 1);
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
+    const char* ws = smem + (st % STAGES) * stage_bytes;
+    const char* xs = ws + W_BYTES + c * (STAGE_K * 4);
+#pragma unroll(MT * RT >= 16 ? 2 : 4)
+    for (int u = 0; u < STAGE_UNITS; ++u) {
+      float4 w[RT];
+#pragma unroll
+      for (int r = 0; r < RT; ++r)
+        w[r] = *reinterpret_cast<const float4*>(ws + (r * SLOTS + tid) * (STAGE_K * 4) + ((u ^ (tid & 7)) << 4));
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+        // (slot m * cs + c of A: its low bits are c's, and m's where there are fewer than eight chains)
+        const float4 x = *reinterpret_cast<const float4*>(xs + (m << cs_shift) * (STAGE_K * 4) + ((u ^ (((m << cs_shift) + c) & 7)) << 4));
+#pragma unroll
+        for (int r = 0; r < RT; ++r) {
+          part[r][m] = fmaf(x.x, w[r].x, part[r][m]);
+          part[r][m] = fmaf(x.y, w[r].y, part[r][m]);
+          part[r][m] = fmaf(x.z, w[r].z, part[r][m]);
+          part[r][m] = fmaf(x.w, w[r].w, part[r][m]);
+        }
+      }
+    }
+    if (st & 1) {
+      // a chain of every slot is complete
+#pragma unroll
+      for (int r = 0; r < RT; ++r)
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+          red[(size_t)(m * rows + r * groups + g) * (cs + 1) + c] = part[r][m];
+          part[r][m] = 0.f;
+        }
+      __syncthreads();
+      for (int o = tid; o < outputs; o += SLOTS) {
+        float sum = st == 1 ? 0.f : totals[o];
+        for (int i = 0; i < cs; ++i) sum += red[(size_t)o * (cs + 1) + i];
+        if (st + 1 < stages) {
+          totals[o] = sum;
+        } else {
+          const int m = m0 + o / rows, n = n0 + o % rows;
+          if (m < M && n < N) C[(size_t)m * ldc + n] = bias ? sum + bias[n] : sum;
+        }
+      }
+    }
+  }
+}
+
+template <int MT, int RT, int STAGES>
+int launch_gemv(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, size_t lda, size_t ldw,
+                size_t ldc, cudaStream_t stream) {
+  const int chains = (K + SUM_BLOCK - 1) / SUM_BLOCK;
+  int cs_shift = 0;
+  while (cs_shift < MAX_CHAINS_SHIFT && (1 << cs_shift) < chains) ++cs_shift;
+  auto smem_of = [](int shift) {
+    const int cs = 1 << shift, outputs = (SLOTS >> shift) * RT * MT;
+    return (size_t)STAGES * (SLOTS * RT + MT * cs) * STAGE_K * 4 + (size_t)outputs * (cs + 2) * 4;
+  };
+  static bool configured = false;
+  if (!configured) {
+    size_t most = 0;
+    for (int s = 0; s <= MAX_CHAINS_SHIFT; ++s) most = smem_of(s) > most ? smem_of(s) : most;
+    cudaError_t e = cudaFuncSetAttribute(gemv_nt_kernel<MT, RT, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    if (e != cudaSuccess) return ts_fail("gemm_simt: %s", cudaGetErrorString(e));
+    configured = true;
+  }
+  const int rows = (SLOTS >> cs_shift) * RT;
+  dim3 grid((N + rows - 1) / rows, (M + MT - 1) / MT);
+  if (grid.y > 65535) return ts_fail("gemm: M = %d is too large", M);
+  TS_LAUNCH("gemm_simt", (gemv_nt_kernel<MT, RT, STAGES>), grid, SLOTS, smem_of(cs_shift), stream, A, W, bias, C, M, N, K,
+            lda, ldw, ldc, cs_shift);
+  return 0;
+}
+
 template <typename TI, typename TO>
 int launch(const void* A, const void* W, const void* bias, void* C, int M, int N, int K, size_t lda,
            size_t ldw, size_t ldc, cudaStream_t stream) {
@@ -132,6 +293,22 @@ int launch(const void* A, const void* W, const void* bias, void* C, int M, int N
   const TI* w = static_cast<const TI*>(W);
   const TI* b = static_cast<const TI*>(bias);
   TO* c = static_cast<TO*>(C);
+  if constexpr (std::is_same<TI, float>::value && std::is_same<TO, float>::value) {
+    // Up to GEMV_MAX_ROWS rows the chains of k are dealt to threads: the tiled kernel leaves most of the
+    // device idle (1024 x 2048 by 2 rows: 16 blocks, 193 us against 4.7 us; 4096 x 1024: 98 against 3.8; 128
+    // rows of 6144 x 1024: 228 against 118).  As many rows of A to a
+    // block as leave a block for nearly every SM: they share the reads of W.
+    if (vec && M <= GEMV_MAX_ROWS) {
+      const int chains = (K + SUM_BLOCK - 1) / SUM_BLOCK;
+      int cs = 1;
+      while (cs < (1 << MAX_CHAINS_SHIFT) && cs < chains) cs *= 2;
+      auto blocks = [&](int mt, int rt) { return (long long)((N + SLOTS / cs * rt - 1) / (SLOTS / cs * rt)) * ((M + mt - 1) / mt); };
+      if (M > 4 && blocks(8, 2) >= GEMV_MIN_BLOCKS) return launch_gemv<8, 2, 2>(a, w, b, c, M, N, K, lda, ldw, ldc, stream);
+      if (M > 2 && blocks(4, 2) >= GEMV_MIN_BLOCKS) return launch_gemv<4, 2, 2>(a, w, b, c, M, N, K, lda, ldw, ldc, stream);
+      if (blocks(2, 2) >= GEMV_MIN_BLOCKS) return launch_gemv<2, 2, 3>(a, w, b, c, M, N, K, lda, ldw, ldc, stream);
+      return launch_gemv<2, 1, 3>(a, w, b, c, M, N, K, lda, ldw, ldc, stream);
+    }
+  }
   if (M > 64) {
     dim3 grid((N + 127) / 128, (M + 127) / 128);
     if (grid.y > 65535) return ts_fail("gemm: M = %d is too large", M);
