@@ -1,0 +1,104 @@
+"""The 32-bit product of few rows (chains of k dealt to threads) against the sums that define it, bit by bit, and
+the sampler's rows over clusters of blocks against one row at a time and against a plain restatement."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def chain_sums(x, w, bias=None):
+    """fmaf over 64 consecutive k in order, the chains' results added in order, in 32-bit.  (A product of
+    two floats is exact in 64 bits, and the 64-bit sum of it with a float, rounded to 32 bits, is fmaf up to a
+    double rounding, which the operands below cannot show: they have 8 significant bits.)"""
+    x, w = x.double().cpu().numpy(), w.double().cpu().numpy()
+    total = np.zeros((x.shape[0], w.shape[0]), np.float32)
+    for k0 in range(0, x.shape[1], 64):
+        part = np.zeros_like(total)
+        for k in range(k0, min(k0 + 64, x.shape[1])):
+            part = (part.astype(np.float64) + x[:, k:k + 1] * w[None, :, k]).astype(np.float32)
+        total = total + part
+    return total if bias is None else total + bias.cpu().numpy()
+
+
+# K: less than a chain, whole chains, a ragged last chain, fewer and more chains than a block has in
+# flight at a time (16); N: edges of a block's rows; M: every width of the kernel and its edges
+@pytest.mark.parametrize("K", [4, 60, 64, 96, 160, 1024, 1100, 2052])
+@pytest.mark.parametrize("M,N", [(1, 1), (1, 8192), (2, 33), (3, 4100), (4, 17), (5, 2048), (8, 2056), (9, 100), (17, 1030), (64, 96), (256, 40)])
+def test_product_of_few_rows_is_the_chain_sum(M, N, K):
+    from tinyserve_b200.kernels import ops
+    if M * N * K > 2 ** 24:
+        pytest.skip("the restatement would take long; the shape's edges are covered by smaller ones")
+    g = torch.Generator().manual_seed(M * 7 + N * 3 + K)
+    x, w = (torch.randn(r, K, generator=g).bfloat16().float().cuda() for r in (M, N))
+    bias = torch.randn(N, generator=g).cuda()
+    out = ops.linear(x, w, bias)
+    np.testing.assert_array_equal(out.cpu().numpy(), chain_sums(x, w, bias))
+
+
+@pytest.mark.parametrize("M", [2, 5, 24, 300])
+def test_product_of_few_rows_takes_leading_dimensions(M):
+    from tinyserve_b200.kernels import ops
+    g = torch.Generator().manual_seed(M)
+    x, w = torch.randn(M, 144, generator=g).cuda(), torch.randn(96, 144, generator=g).cuda()
+    for k, at in ((128, 0), (128, 4), (126, 0), (128, 1)):          # aligned, aligned inside a row, a ragged K, unaligned
+        xs, ws = x[:, at:at + k], w[:, at:at + k]
+        want = ops.linear(xs.contiguous()[:1], ws.contiguous())
+        got = ops.linear(xs, ws)
+        assert torch.equal(got[:1], want)
+        torch.testing.assert_close(got.double(), xs.double() @ ws.double().T, rtol=0, atol=2e-5)
+
+
+def plain_sample(x, temp, k, p):
+    """The tokens that may be drawn: top-k with ties, then top-p over exact integer weights."""
+    y = (x * np.float32(1.0 / np.float32(temp))).astype(np.float32)
+    keep = np.ones(len(y), bool)
+    if 0 < k < len(y):
+        keep &= y >= np.sort(y)[-k]
+    if p < 1:
+        mx = y[keep].max()
+        weight = np.exp((y - mx).astype(np.float64)) * keep
+        order = np.argsort(-y, kind="stable")
+        before = np.cumsum(weight[order]) - weight[order]
+        keep_p = np.zeros_like(keep)
+        keep_p[order[before <= p * weight.sum()]] = True
+        keep &= keep_p
+    return keep
+
+
+@pytest.mark.parametrize("V", [1, 5, 257, 8191, 8192, 16384, 40000, 151936])
+@pytest.mark.parametrize("B", [1, 3, 40, 80, 150])
+def test_sampled_rows_do_not_depend_on_the_blocks_that_share_them(V, B):
+    """The number of blocks per row follows from the number of rows: a row alone, and the same row among
+    others, must give the same token, greedy or with any filter."""
+    from tinyserve_b200.kernels import ops
+    g = torch.Generator().manual_seed(V + B)
+    x = (torch.randn(B, V, generator=g) * 3).cuda()
+    x[:, V // 2] = x.max(dim=1).values                                # a tie for the largest
+    temp = torch.tensor([(0.0, 0.7, 1.3, 0.9)[i % 4] for i in range(B)]).cuda()
+    ks = torch.tensor([(0, 50, 0, 7)[i % 4] for i in range(B)], dtype=torch.int32).cuda()
+    ps = torch.tensor([(1.0, 0.9, 0.5, 1.0)[i % 4] for i in range(B)]).cuda()
+    streams, steps = torch.arange(B).cuda(), torch.arange(B, dtype=torch.int32).cuda()
+    together = ops.sample(x, temp, streams, steps, 11, top_k=ks, top_p=ps).cpu()
+    for i in sorted({0, 1 % B, 2 % B, 3 % B, B - 1}):
+        one = slice(i, i + 1)
+        alone = ops.sample(x[one], temp[one], streams[one], steps[one], 11, top_k=ks[one], top_p=ps[one]).cpu()
+        assert alone[0] == together[i]
+        row = x[i].cpu().numpy()
+        if temp[i] == 0:
+            assert together[i] == int(np.flatnonzero(row == row.max())[0])
+        else:
+            assert plain_sample(row, float(temp[i]), int(ks[i]), float(ps[i]))[int(together[i])]
+
+
+def test_rows_of_infinities_and_nans():
+    from tinyserve_b200.kernels import ops
+    x = torch.full((4, 20000), -float("inf")).cuda()
+    x[1, 12345] = float("inf")
+    x[2, 7] = 1.0
+    x[3] = 0.5
+    x[3, ::2] = float("nan")
+    zero, streams, steps = torch.zeros(4).cuda(), torch.arange(4).cuda(), torch.zeros(4, dtype=torch.int32).cuda()
+    assert ops.sample(x, zero, streams, steps, 1).tolist() == [0, 12345, 7, 1]
+    one = torch.ones(4).cuda()
+    assert ops.sample(x, one, streams, steps, 1).tolist()[1:3] == [12345, 7]

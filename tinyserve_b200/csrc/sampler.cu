@@ -1,4 +1,9 @@
-// Sampling from 32-bit logits, one block per row, everything on the device.
+// Sampling from 32-bit logits, everything on the device.  A row is read by a cluster of up to eight
+// blocks, a range of the vocabulary each, which combine their maxima and histograms through
+// distributed shared memory.  (A row of 151,936 logits is 600 KB: one block takes 18 us to read
+// it, and up to nine passes over it, most of whose histogram updates meet in a few bins, took 2.1 ms
+// with top-k and top-p.)  All that blocks combine is a maximum or an integer sum, so the result does
+// not depend on how many blocks share a row.
 //
 //   temperature == 0           -> argmax (serve.py:1521-1522)
 //   temperature > 0            -> x = logit / temperature, optional top-k (keep the k largest),
@@ -79,6 +84,19 @@ __device__ Best block_best(Best v, Best* scratch) {
   return scratch[0];
 }
 
+__device__ __forceinline__ uint32_t cluster_blocks() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ unsigned long long cluster_load_u64(const unsigned long long* own_shared, uint32_t rank) {
+  uint32_t local = static_cast<uint32_t>(__cvta_generic_to_shared(own_shared)), remote;
+  unsigned long long v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
+  asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(remote) : "memory");
+  return v;
+}
+
 __device__ float block_max_f(float v, float* scratch) {
   v = warp_max(v);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -92,6 +110,77 @@ __device__ float block_max_f(float v, float* scratch) {
   }
   __syncthreads();
   return scratch[32];
+}
+
+// The histograms of one radix pass: a block counts into its own, every block of the cluster then adds
+// up all of them.  Two buffers take turns, so that one cluster barrier per pass is enough: a
+// buffer is cleared two passes later, after the barrier that its last readers arrived at.
+struct Histogram {
+  unsigned long long own[2][256];
+  unsigned long long all[256];
+  unsigned int chosen;
+  unsigned long long before;       // what lies in bins above the chosen one
+};
+
+// hist[bin] += weight for the lanes with `on`.  `crowded`: most lanes fall into a few bins; lanes of one
+// bin then add up among themselves first (a weight above 2^32, which only infinite logits can have, goes
+// its own way).
+__device__ __forceinline__ void hist_add(unsigned long long* hist, bool on, uint32_t bin, unsigned long long weight, bool crowded) {
+  if (on && (!crowded || weight > (1ull << 32))) {
+    atomicAdd(&hist[bin], weight);
+    on = false;
+  }
+  if (!crowded) return;
+  const unsigned active = __ballot_sync(0xffffffffu, on);
+  if (!on) return;
+  const unsigned peers = __match_any_sync(active, bin);
+  const uint32_t lo = __reduce_add_sync(peers, (uint32_t)(weight & 0xFFFFFFu));
+  const uint32_t hi = __reduce_add_sync(peers, (uint32_t)(weight >> 24));
+  if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&hist[bin], ((unsigned long long)hi << 24) + lo);
+}
+
+// Sums of the cluster's histograms into h.all (every block for itself); called by all threads.
+__device__ void hist_combine(Histogram& h, int buf, uint32_t blocks) {
+  cluster_arrive();
+  cluster_wait();
+  if (threadIdx.x < 256) {
+    unsigned long long sum = 0;
+    for (uint32_t r = 0; r < blocks; ++r) sum += cluster_load_u64(&h.own[buf][threadIdx.x], r);
+    h.all[threadIdx.x] = sum;
+  }
+  __syncthreads();
+}
+
+// From the highest bin down: the first bin where before + bins above + the bin reaches `limit` (>= limit, or
+// > limit with `beyond`); h.chosen is that bin (0 if there is none), h.before = before + the bins above it
+// (all bins if there is none).
+__device__ void hist_choose(Histogram& h, unsigned long long before, unsigned long long limit, bool beyond) {
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    unsigned long long own = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) own += h.all[255 - (lane * 8 + i)];
+    unsigned long long upto = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long t = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += t;
+    }
+    const unsigned long long total = before + upto;
+    const unsigned hit = __ballot_sync(0xffffffffu, beyond ? total > limit : total >= limit);
+    if (hit == 0) {
+      if (lane == 31) { h.chosen = 0; h.before = total; }
+    } else if (lane == __ffs(hit) - 1) {
+      unsigned long long cum = total - own;
+      for (int i = 0; i < 8; ++i) {
+        const int bin = 255 - (lane * 8 + i);
+        const unsigned long long next = cum + h.all[bin];
+        if (beyond ? next > limit : next >= limit) { h.chosen = bin; h.before = cum; break; }
+        cum = next;
+      }
+    }
+  }
+  __syncthreads();
 }
 
 struct SampleArgs {
@@ -112,59 +201,92 @@ struct SampleArgs {
 __global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
   __shared__ Best best_scratch[32];
   __shared__ float f_scratch[33];
-  __shared__ unsigned long long hist[256];
-  __shared__ unsigned int sh_prefix;
-  __shared__ unsigned long long sh_above;
-  __shared__ unsigned long long sh_total;
+  __shared__ Histogram h;
+  __shared__ unsigned long long shared_word;      // what this block tells the cluster (a maximum, or its best token)
 
   pdl_trigger();
   pdl_wait();
-  const int row = blockIdx.x;
+  const uint32_t blocks = cluster_blocks(), rank = cluster_rank();
+  const int row = blockIdx.x / blocks;
   const float* x = a.logits + (size_t)row * a.row_stride;
   const int V = a.vocab;
+  // this block's range of the vocabulary, in whole groups of four tokens (one Philox call each)
+  const int per = ((V + 3) / 4 + blocks - 1) / blocks * 4;
+  const int v0 = min(V, (int)rank * per), v1 = min(V, v0 + per);
+  const bool aligned = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
   const float temp = a.temperature[row];
 
-  if (!(temp > 0.f)) {   // greedy
-    Best b{-INFINITY, 0x7fffffff};
-    for (int v = threadIdx.x; v < V; v += THREADS) b = better(b, Best{x[v], v});
+  // tokens v .. v + 3 of the row (v a multiple of four); -inf behind the range
+  auto load4 = [&](int v, float (&q)[4]) {
+    if (aligned && v + 3 < v1) {
+      const float4 t = *reinterpret_cast<const float4*>(x + v);
+      q[0] = t.x; q[1] = t.y; q[2] = t.z; q[3] = t.w;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) q[j] = v + j < v1 ? x[v + j] : -INFINITY;
+    }
+  };
+  // the best of all blocks' tokens; the first block writes it
+  auto finish = [&](Best b) {
     b = block_best(b, best_scratch);
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0) shared_word = (unsigned long long)__float_as_uint(b.value) << 32 | (uint32_t)b.index;
+    cluster_arrive();
+    cluster_wait();
+    if (rank == 0 && threadIdx.x == 0) {
+      for (uint32_t r = 1; r < blocks; ++r) {
+        const unsigned long long w = cluster_load_u64(&shared_word, r);
+        b = better(b, Best{__uint_as_float((uint32_t)(w >> 32)), (int)(uint32_t)w});
+      }
       a.out[row] = b.index;
       if (a.slot_tokens) a.slot_tokens[a.slots[row]] = b.index;
     }
+    // no block leaves while the first may still read its shared memory
+    cluster_arrive();
+    cluster_wait();
+  };
+
+  if (!(temp > 0.f)) {   // greedy
+    Best b{-INFINITY, 0x7fffffff};
+#pragma unroll 4
+    for (int base = v0 + threadIdx.x * 4; base < v1; base += THREADS * 4) {
+      float q[4];
+      load4(base, q);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (base + j < v1) b = better(b, Best{q[j], base + j});
+    }
+    finish(b);
     return;
   }
   const float inv_temp = 1.f / temp;
   const int k = a.top_k ? a.top_k[row] : 0;
   const float top_p = a.top_p ? a.top_p[row] : 1.f;
   uint32_t keep_from = 0;   // tokens with sort_key(x / temp) >= keep_from are kept
+  int buf = 0;
 
   if (k > 0 && k < V) {
     // radix select of the k-th largest key, one byte per pass
     uint32_t prefix = 0, mask = 0;
     unsigned long long remaining = (unsigned long long)k;
-    for (int byte = 3; byte >= 0; --byte) {
-      for (int i = threadIdx.x; i < 256; i += THREADS) hist[i] = 0ull;
+    for (int byte = 3; byte >= 0; --byte, buf ^= 1) {
+      if (threadIdx.x < 256) h.own[buf][threadIdx.x] = 0ull;
       __syncthreads();
-      for (int v = threadIdx.x; v < V; v += THREADS) {
-        const uint32_t key = sort_key(x[v] * inv_temp);
-        if ((key & mask) == prefix) atomicAdd(&hist[(key >> (8 * byte)) & 255u], 1ull);
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        unsigned long long cum = 0;
-        int chosen = 0;
-        for (int b = 255; b >= 0; --b) {
-          if (cum + hist[b] >= remaining) { chosen = b; break; }
-          cum += hist[b];
+      for (int base = v0; base < v1; base += THREADS * 4) {
+        const int v = base + threadIdx.x * 4;
+        float q[4];
+        load4(v, q);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t key = sort_key(q[j] * inv_temp);
+          hist_add(h.own[buf], v + j < v1 && (key & mask) == prefix, (key >> (8 * byte)) & 255u, 1ull, byte == 3);
         }
-        sh_prefix = prefix | ((uint32_t)chosen << (8 * byte));
-        sh_above = remaining - cum;
       }
-      __syncthreads();
-      prefix = sh_prefix;
-      remaining = sh_above;
+      hist_combine(h, buf, blocks);
+      hist_choose(h, 0ull, remaining, false);
+      prefix |= h.chosen << (8 * byte);
+      remaining -= h.before;
       mask |= 0xFFu << (8 * byte);
+      __syncthreads();
     }
     keep_from = prefix;
   }
@@ -172,45 +294,49 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
   if (top_p < 1.f) {
     // weights exp(x - max) as 32.32 fixed point: sums are exact and order-independent
     float mx = -INFINITY;
-    for (int v = threadIdx.x; v < V; v += THREADS) {
-      const float y = x[v] * inv_temp;
-      if (sort_key(y) >= keep_from) mx = fmaxf(mx, y);
+    for (int base = v0 + threadIdx.x * 4; base < v1; base += THREADS * 4) {
+      float q[4];
+      load4(base, q);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float y = q[j] * inv_temp;
+        if (base + j < v1 && sort_key(y) >= keep_from) mx = fmaxf(mx, y);
+      }
     }
     mx = block_max_f(mx, f_scratch);
+    if (threadIdx.x == 0) shared_word = __float_as_uint(mx);
+    cluster_arrive();
+    cluster_wait();
+    for (uint32_t r = 0; r < blocks; ++r) mx = fmaxf(mx, __uint_as_float((uint32_t)cluster_load_u64(&shared_word, r)));
     uint32_t prefix = 0, mask = 0;
-    unsigned long long above = 0;
-    for (int byte = 3; byte >= 0; --byte) {
-      for (int i = threadIdx.x; i < 256; i += THREADS) hist[i] = 0ull;
+    unsigned long long above = 0, limit = 0;
+    for (int byte = 3; byte >= 0; --byte, buf ^= 1) {
+      if (threadIdx.x < 256) h.own[buf][threadIdx.x] = 0ull;
       __syncthreads();
-      for (int v = threadIdx.x; v < V; v += THREADS) {
-        const float y = x[v] * inv_temp;
-        const uint32_t key = sort_key(y);
-        if (key >= keep_from && (key & mask) == prefix) {
-          const unsigned long long w = (unsigned long long)(expf(y - mx) * 4294967296.f);
-          atomicAdd(&hist[(key >> (8 * byte)) & 255u], w);
+      for (int base = v0; base < v1; base += THREADS * 4) {
+        const int v = base + threadIdx.x * 4;
+        float q[4];
+        load4(v, q);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float y = q[j] * inv_temp;
+          const uint32_t key = sort_key(y);
+          const bool on = v + j < v1 && key >= keep_from && (key & mask) == prefix;
+          const unsigned long long w = on ? (unsigned long long)(expf(y - mx) * 4294967296.f) : 0ull;
+          hist_add(h.own[buf], on && w != 0ull, (key >> (8 * byte)) & 255u, w, byte == 3);
         }
       }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        if (byte == 3) {
-          unsigned long long total = 0;
-          for (int b = 0; b < 256; ++b) total += hist[b];
-          sh_total = (unsigned long long)((double)top_p * (double)total);
-        }
-        const unsigned long long lim = sh_total;
-        unsigned long long cum = above;
-        int chosen = 0;
-        for (int b = 255; b >= 0; --b) {
-          if (cum + hist[b] > lim) { chosen = b; break; }
-          cum += hist[b];
-        }
-        sh_prefix = prefix | ((uint32_t)chosen << (8 * byte));
-        sh_above = cum;
+      hist_combine(h, buf, blocks);
+      if (byte == 3) {
+        unsigned long long total = 0;
+        for (int b = 0; b < 256; ++b) total += h.all[b];
+        limit = (unsigned long long)((double)top_p * (double)total);
       }
-      __syncthreads();
-      prefix = sh_prefix;
-      above = sh_above;
+      hist_choose(h, above, limit, true);
+      prefix |= h.chosen << (8 * byte);
+      above = h.before;
       mask |= 0xFFu << (8 * byte);
+      __syncthreads();
     }
     keep_from = max(keep_from, prefix);
   }
@@ -220,23 +346,21 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
   const unsigned long long stream = a.stream[row];
   const uint32_t step = a.step[row];
   Best b{-INFINITY, 0x7fffffff};
-  for (int base = threadIdx.x * 4; base < V; base += THREADS * 4) {
+  for (int base = v0 + threadIdx.x * 4; base < v1; base += THREADS * 4) {
     uint32_t c[4] = {(uint32_t)(base >> 2), step, (uint32_t)stream, (uint32_t)(stream >> 32)};
     philox4x32_10(c, k0, k1);
+    float q[4];
+    load4(base, q);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int v = base + j;
-      if (v < V) {
-        const float y = x[v] * inv_temp;
+      if (v < v1) {
+        const float y = q[j] * inv_temp;
         if (sort_key(y) >= keep_from) b = better(b, Best{y + gumbel(c[j]), v});
       }
     }
   }
-  b = block_best(b, best_scratch);
-  if (threadIdx.x == 0) {
-    a.out[row] = b.index;
-    if (a.slot_tokens) a.slot_tokens[a.slots[row]] = b.index;
-  }
+  finish(b);
 }
 
 // logits[row, id] = logit > 0 ? logit / penalty : logit * penalty for every listed id (>= 0);
@@ -270,7 +394,14 @@ TS_EXPORT int ts_sample(const float* logits, long long row_stride, int num_rows,
   TS_REQUIRE(temperature && stream_ids && steps && out, "sample: missing argument");
   TS_REQUIRE((slot_tokens == nullptr) == (slots == nullptr), "sample: slot_tokens and slots come together");
   SampleArgs a{logits, row_stride, vocab, temperature, top_k, top_p, stream_ids, steps, seed, out, slot_tokens, slots};
-  TS_LAUNCH("sample", sample_kernel, num_rows, THREADS, 0, stream, a);
+  // Blocks per row: as many as fill the device's 2 x 148 places for blocks of this size, eight at most
+  // (the portable cluster), a range of at least 4,096 tokens each: below, a cluster barrier costs more
+  // than the tokens it saves reading.
+  int blocks = 1;
+  while (blocks < 8 && vocab / (2 * blocks) >= 4096 && (long long)num_rows * 2 * blocks <= 296) blocks *= 2;
+  TS_REQUIRE((long long)num_rows * blocks <= 2147483647LL, "sample: too many rows");
+  cudaError_t e = ts_launch_cluster(sample_kernel, dim3(num_rows * blocks), dim3(THREADS), 0, stream, dim3(blocks, 1, 1), a);
+  if (e != cudaSuccess) return ts_fail("sample: %s", cudaGetErrorString(e));
   return 0;
 }
 
