@@ -1,4 +1,4 @@
-"""The 32-bit product of few rows (chains of k dealt to threads) against the sums that define it, bit by bit, and
+"""The 32-bit products (chains of k dealt to threads) against the sums that define it, bit by bit, and
 the sampler's rows over clusters of blocks against one row at a time and against a plain restatement."""
 import numpy as np
 import pytest
@@ -24,16 +24,25 @@ def chain_sums(x, w, bias=None):
 # K: less than a chain, whole chains, a ragged last chain, fewer and more chains than a block has in
 # flight at a time (16); N: edges of a block's rows; M: every width of the kernel and its edges
 @pytest.mark.parametrize("K", [4, 60, 64, 96, 160, 1024, 1100, 2052])
-@pytest.mark.parametrize("M,N", [(1, 1), (1, 8192), (2, 33), (3, 4100), (4, 17), (5, 2048), (8, 2056), (9, 100), (17, 1030), (64, 96), (256, 40)])
+@pytest.mark.parametrize("M,N", [(1, 1), (1, 8192), (2, 33), (3, 4100), (4, 17), (5, 2048), (8, 2056), (9, 100), (17, 1030), (64, 96), (256, 40), (640, 1100)])
 def test_product_of_few_rows_is_the_chain_sum(M, N, K):
     from tinyserve_b200.kernels import ops
-    if M * N * K > 2 ** 24:
+    if M * N * K > 2 ** 24 and (M < 640 or K > 96):
         pytest.skip("the restatement would take long; the shape's edges are covered by smaller ones")
     g = torch.Generator().manual_seed(M * 7 + N * 3 + K)
     x, w = (torch.randn(r, K, generator=g).bfloat16().float().cuda() for r in (M, N))
     bias = torch.randn(N, generator=g).cuda()
     out = ops.linear(x, w, bias)
     np.testing.assert_array_equal(out.cpu().numpy(), chain_sums(x, w, bias))
+
+
+@pytest.mark.parametrize("M,N,K", [(640, 1100, 1100), (641, 1087, 2052), (65, 12224, 260), (1030, 600, 300)])
+def test_rows_of_large_products_are_those_of_few_rows(M, N, K):
+    """Tiles of many rows (whole and ragged, whole rounds of four chains and not) against the kernel for few."""
+    from tinyserve_b200.kernels import ops
+    g = torch.Generator().manual_seed(M)
+    x, w, bias = torch.randn(M, K, generator=g).cuda(), torch.randn(N, K, generator=g).cuda(), torch.randn(N, generator=g).cuda()
+    assert torch.equal(ops.linear(x, w, bias), torch.cat([ops.linear(rows.contiguous(), w, bias) for rows in x.split(8)]))
 
 
 @pytest.mark.parametrize("M", [2, 5, 24, 300])

@@ -124,6 +124,162 @@ gemm_nt_kernel(const TI* __restrict__ A, const TI* __restrict__ W, const TI* __r
   }
 }
 
+// The tiled product with the chains of k dealt to CHAIN_GROUPS groups of threads, for float operands: a
+// block has a tile of 64 x 64 outputs, 64 threads of 8 x 8 outputs each take one chain of SUM_BLOCK k
+// of it, and four chains are under way side by side.  After every four chains the groups' results
+// meet in shared memory, where each output is added up in the order of k: the sums are those of the other kernels
+// bit by bit.  Slices of 16 k of every chain come through a ring of stages by cp.async, K fastest, in
+// rows of 64 bytes whose 16-byte unit u lies at u ^ (row / 2 & 3).
+// Bound by the multiply-add units (half of their rate: 36 TFLOP/s at 24576 x 4096 by 1,024 rows, where the tiled
+// kernel reached 21) and, for few tiles, by the chain of a block.  227 rows: 6144 x 1024 209 -> 109 us, 4096 x 1024
+// 217 -> 74; 1,024 rows of 1024 x 3072 588 -> 214.
+constexpr int CHAIN_GROUPS = 4, TILE = 64, SLICE = 16, SPLIT_STAGES = 2;
+constexpr int SPLIT_THREADS = 64 * CHAIN_GROUPS;
+constexpr int SLICE_BYTES = TILE * SLICE * 4;                        // of one operand and chain
+constexpr int SPLIT_STAGE_BYTES = 2 * CHAIN_GROUPS * SLICE_BYTES;    // 32 KB
+constexpr size_t SPLIT_SMEM = (size_t)SPLIT_STAGES * SPLIT_STAGE_BYTES;       // the ring; behind it the chains' results, a quarter of the tile
+constexpr size_t SPLIT_RED_BYTES = (size_t)CHAIN_GROUPS * 16 * TILE * 4;
+constexpr size_t SPLIT_TOTAL_BYTES = (size_t)TILE * TILE * 4;        // and the outputs' sums so far
+
+__device__ __forceinline__ void copy16_async(uint32_t dst, const void* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0));
+}
+
+__global__ void __launch_bounds__(SPLIT_THREADS, 2)
+gemm_nt_chains_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
+                      float* __restrict__ C, int M, int N, int K, size_t lda, size_t ldw, size_t ldc) {
+  extern __shared__ __align__(16) char smem[];
+  pdl_trigger();
+  const int tid = threadIdx.x, grp = tid >> 6, t = tid & 63;
+  // 8 x 8 outputs of a thread: rows ty + 8 i, columns tx + 8 j
+  const int tx = t & 7, ty = t >> 3;
+  const int m0 = blockIdx.y * TILE, n0 = blockIdx.x * TILE;
+  const int chains = (K + SUM_BLOCK - 1) / SUM_BLOCK;
+  const int rounds = (chains + CHAIN_GROUPS - 1) / CHAIN_GROUPS;
+  constexpr int PER_ROUND = SUM_BLOCK / SLICE;
+  const int stages = rounds * PER_ROUND;
+  auto load = [&](int st, bool of_w) {
+    const uint32_t base = static_cast<uint32_t>(__cvta_generic_to_shared(smem + (st % SPLIT_STAGES) * SPLIT_STAGE_BYTES)) +
+                          (of_w ? CHAIN_GROUPS * SLICE_BYTES : 0);
+    const float* src = of_w ? W : A;
+    const size_t ld = of_w ? ldw : lda;
+    const int row0 = of_w ? n0 : m0, rows = of_w ? N : M;
+#pragma unroll
+    for (int i = tid; i < CHAIN_GROUPS * TILE * SLICE / 4; i += SPLIT_THREADS) {
+      const int u = i & 3, r = (i >> 2) & (TILE - 1), c = i >> 8;
+      const int k = ((st / PER_ROUND) * CHAIN_GROUPS + c) * SUM_BLOCK + (st % PER_ROUND) * SLICE + u * 4;
+      const bool ok = row0 + r < rows && k < K;
+      copy16_async(base + c * SLICE_BYTES + r * (SLICE * 4) + ((u ^ ((r >> 1) & 3)) << 4), src + (ok ? (size_t)(row0 + r) * ld + k : 0), ok);
+    }
+  };
+  for (int st = 0; st < SPLIT_STAGES - 1; ++st)
+    if (st < stages) load(st, true);
+  pdl_wait();
+  for (int st = 0; st < SPLIT_STAGES - 1; ++st) {
+    if (st < stages) load(st, false);
+    asm volatile("cp.async.commit_group;\n" ::);
+  }
+  float part[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) part[i][j] = 0.f;
+  float* red = reinterpret_cast<float*>(smem + SPLIT_SMEM);        // [CHAIN_GROUPS][16][TILE]
+  float* totals = red + SPLIT_RED_BYTES / 4;                       // [TILE][TILE], an element always by the same thread
+  for (int rd = 0; rd < rounds; ++rd) {
+#pragma unroll 1
+    for (int q = 0; q < PER_ROUND; ++q) {
+      const int st = rd * PER_ROUND + q;
+      asm volatile("cp.async.wait_group %0;\n" ::"n"(SPLIT_STAGES - 2));
+      __syncthreads();
+      // (the stage that everybody is done with)
+      if (st + SPLIT_STAGES - 1 < stages) {
+        load(st + SPLIT_STAGES - 1, true);
+        load(st + SPLIT_STAGES - 1, false);
+      }
+      asm volatile("cp.async.commit_group;\n" ::);
+      const char* as = smem + (st % SPLIT_STAGES) * SPLIT_STAGE_BYTES + grp * SLICE_BYTES;
+      const char* ws = as + CHAIN_GROUPS * SLICE_BYTES;
+#pragma unroll
+      for (int u = 0; u < SLICE / 4; ++u) {
+        // (half of the rows at a time: the registers hold two blocks a multiprocessor)
+#pragma unroll
+        for (int half = 0; half < 8; half += 4) {
+          float4 a[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int r = (half + i) * 8 + ty;
+            a[i] = *reinterpret_cast<const float4*>(as + r * (SLICE * 4) + ((u ^ ((r >> 1) & 3)) << 4));
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const int r = j * 8 + tx;
+            const float4 w = *reinterpret_cast<const float4*>(ws + r * (SLICE * 4) + ((u ^ ((r >> 1) & 3)) << 4));
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              part[half + i][j] = fmaf(a[i].x, w.x, part[half + i][j]);
+              part[half + i][j] = fmaf(a[i].y, w.y, part[half + i][j]);
+              part[half + i][j] = fmaf(a[i].z, w.z, part[half + i][j]);
+              part[half + i][j] = fmaf(a[i].w, w.w, part[half + i][j]);
+            }
+          }
+        }
+      }
+    }
+    // a chain of every group is complete: its results go through shared memory, a quarter of the tile's
+    // rows (16) at a time, to the thread that adds up the output
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      if (h > 0) __syncthreads();
+#pragma unroll
+      for (int i2 = 0; i2 < 2; ++i2) {
+        const int i = h * 2 + i2;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          red[(grp * 16 + i2 * 8 + ty) * TILE + j * 8 + tx] = part[i][j];
+          part[i][j] = 0.f;
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int o = 0; o < 4; ++o) {
+        const int at = o * SPLIT_THREADS + tid;
+        float sum = rd == 0 ? 0.f : totals[h * 16 * TILE + at];
+#pragma unroll
+        for (int c = 0; c < CHAIN_GROUPS; ++c) sum += red[c * 16 * TILE + at];
+        totals[h * 16 * TILE + at] = sum;
+      }
+    }
+  }
+  // output o of quarter h: row h * 16 + at / TILE of the tile
+#pragma unroll
+  for (int h = 0; h < 4; ++h)
+#pragma unroll
+    for (int o = 0; o < 4; ++o) {
+      const int at = o * SPLIT_THREADS + tid;
+      const int m = m0 + h * 16 + at / TILE, n = n0 + at % TILE;
+      if (m < M && n < N) {
+        const float sum = totals[h * 16 * TILE + at];
+        C[(size_t)m * ldc + n] = bias ? sum + bias[n] : sum;
+      }
+    }
+}
+
+int launch_chains(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, size_t lda, size_t ldw,
+                  size_t ldc, cudaStream_t stream) {
+  constexpr size_t smem = SPLIT_SMEM + SPLIT_RED_BYTES + SPLIT_TOTAL_BYTES;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_nt_chains_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return ts_fail("gemm_simt: %s", cudaGetErrorString(e));
+    configured = true;
+  }
+  dim3 grid((N + TILE - 1) / TILE, (M + TILE - 1) / TILE);
+  if (grid.y > 65535) return ts_fail("gemm: M = %d is too large", M);
+  TS_LAUNCH("gemm_simt", gemm_nt_chains_kernel, grid, SPLIT_THREADS, smem, stream, A, W, bias, C, M, N, K, lda, ldw, ldc);
+  return 0;
+}
+
 // The product of a few rows of A (decode steps, the last rows before the vocabulary projection), in
 // which W is nearly all the bytes.  A thread owns one chain of SUM_BLOCK k (a "slot") of RT rows of W
 // for all of the MT rows of A, so that the sums are those of the tiled kernel bit by bit, and a block
@@ -139,12 +295,9 @@ gemm_nt_kernel(const TI* __restrict__ A, const TI* __restrict__ W, const TI* __r
 constexpr int SLOTS = 128;           // threads of a block: chains in flight x groups of rows
 constexpr int STAGE_K = 32;          // k of a slot that a stage holds: half a chain, 128 bytes
 constexpr int STAGE_UNITS = STAGE_K / 4;
-constexpr int GEMV_MAX_ROWS = 256, GEMV_MIN_BLOCKS = 128;
+constexpr int GEMV_WIDTH = 8;        // most rows of A of a block
+constexpr int GEMV_MIN_BLOCKS = 128;
 constexpr int MAX_CHAINS_SHIFT = 4;  // up to 16 chains of a row at a time: 8 RT rows a block
-
-__device__ __forceinline__ void copy16_async(uint32_t dst, const void* src, bool valid) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0));
-}
 
 template <int MT, int RT, int STAGES>
 __global__ void __launch_bounds__(SLOTS)
@@ -294,16 +447,22 @@ int launch(const void* A, const void* W, const void* bias, void* C, int M, int N
   const TI* b = static_cast<const TI*>(bias);
   TO* c = static_cast<TO*>(C);
   if constexpr (std::is_same<TI, float>::value && std::is_same<TO, float>::value) {
-    // Up to GEMV_MAX_ROWS rows the chains of k are dealt to threads: the tiled kernel leaves most of the
-    // device idle (1024 x 2048 by 2 rows: 16 blocks, 193 us against 4.7 us; 4096 x 1024: 98 against 3.8; 128
-    // rows of 6144 x 1024: 228 against 118).  As many rows of A to a
-    // block as leave a block for nearly every SM: they share the reads of W.
-    if (vec && M <= GEMV_MAX_ROWS) {
+    if (vec) {
+      // Both kernels below deal the chains of k to threads, one for few rows, one for many; whichever the
+      // estimate says ends sooner.  The first does about 13.8 TFLOP/s where it fills the device; the other takes
+      // 41 us per 1,024 k where a multiprocessor has one block, 36 us a block where it has more (measured: 4096 x 1024 by
+      // 48 / 64 / 128 / 512 rows 35 / 42 / 81 / 325 us against 41 / 42 / 65 / 143; 24576 x 4096 by 24 / 48 rows
+      // 309 / 609 against 422 / 425).
+      const double few = 1e-12 / 13.8 * 2.0 * M * N * K * 1e6;
+      const long long tiles = (long long)((N + TILE - 1) / TILE) * ((M + TILE - 1) / TILE);
+      const double many = K / 1024.0 * (tiles <= 148 ? 41.0 : 36.0 * ((tiles + 147) / 148));
+      if (M > GEMV_WIDTH && many < few) return launch_chains(a, w, b, c, M, N, K, lda, ldw, ldc, stream);
+      // As many rows of A to a block as leave a block for nearly every multiprocessor: they share the reads of W.
       const int chains = (K + SUM_BLOCK - 1) / SUM_BLOCK;
       int cs = 1;
       while (cs < (1 << MAX_CHAINS_SHIFT) && cs < chains) cs *= 2;
       auto blocks = [&](int mt, int rt) { return (long long)((N + SLOTS / cs * rt - 1) / (SLOTS / cs * rt)) * ((M + mt - 1) / mt); };
-      if (M > 4 && blocks(8, 2) >= GEMV_MIN_BLOCKS) return launch_gemv<8, 2, 2>(a, w, b, c, M, N, K, lda, ldw, ldc, stream);
+      if (M > 4 && blocks(GEMV_WIDTH, 2) >= GEMV_MIN_BLOCKS) return launch_gemv<GEMV_WIDTH, 2, 2>(a, w, b, c, M, N, K, lda, ldw, ldc, stream);
       if (M > 2 && blocks(4, 2) >= GEMV_MIN_BLOCKS) return launch_gemv<4, 2, 2>(a, w, b, c, M, N, K, lda, ldw, ldc, stream);
       if (blocks(2, 2) >= GEMV_MIN_BLOCKS) return launch_gemv<2, 2, 3>(a, w, b, c, M, N, K, lda, ldw, ldc, stream);
       return launch_gemv<2, 1, 3>(a, w, b, c, M, N, K, lda, ldw, ldc, stream);
