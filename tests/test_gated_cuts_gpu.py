@@ -1,0 +1,50 @@
+"""The gated product of a few tokens whose K is cut inside clusters, against the product and the activation in 64 bits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+# N (gate and up rows): one row tile, several, 48 (the gate/up product of a small model), 147 (the most that are cut);
+# K: one slice and a ragged one (no cut), cuts of unequal length, eight cuts
+@pytest.mark.parametrize("N,K", [(128, 64), (128, 2048), (256, 1096), (640, 520), (6144, 1024), (147 * 128, 512)])
+@pytest.mark.parametrize("M", [1, 2, 7, 8, 9, 15, 16])
+@pytest.mark.parametrize("activation,limit", [("silu", 0.0), ("gelu_tanh", 0.0), ("bounded_swish", 0.5)])
+def test_gated_product_of_few_row_tiles(M, N, K, activation, limit):
+    from tinyserve_b200.kernels import ops
+    g = torch.Generator().manual_seed(M + N + K)
+    x = torch.randn(M, K, generator=g).bfloat16().cuda()
+    w = (torch.randn(N, K, generator=g) * K ** -0.5).bfloat16().cuda()
+    blocks = w.double().view(N // 128, 2, 64, K)
+    gate, up = ((x.double() @ blocks[:, i].reshape(N // 2, K).T) for i in (0, 1))
+    if activation == "silu":
+        want = torch.nn.functional.silu(gate) * up
+    elif activation == "gelu_tanh":
+        want = torch.nn.functional.gelu(gate, approximate="tanh") * up
+    else:
+        gate, up = gate.clamp(max=limit), up.clamp(-limit, limit)
+        want = gate * torch.sigmoid(1.702 * gate) * (up + 1)
+    got = ops.gated_linear(x, w, activation, ops.GATED_BLOCK, limit)
+    assert got.dtype == torch.bfloat16 and got.shape == want.shape
+    # one rounding to bfloat16 (2^-9 of the value) and 32-bit sums of K terms of about 1 / sqrt(K)
+    assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 4e-6).all()
+    assert torch.equal(got, ops.gated_linear(x, w, activation, ops.GATED_BLOCK, limit)), "the same bits every time"
+    assert ops.gemm_tcgen05_error() == 0
+
+
+@pytest.mark.parametrize("M", [1, 5, 16])
+def test_rows_without_their_norm_factor(M):
+    from tinyserve_b200.kernels import ops
+    g = torch.Generator().manual_seed(M)
+    x, o = torch.randn(M, 1024, generator=g).bfloat16().cuda(), (torch.randn(1024, 1024, generator=g) * 0.03).bfloat16().cuda()
+    w = (torch.randn(768, 1024, generator=g) * 0.03).bfloat16().cuda()
+    norm = (1 + 0.1 * torch.randn(1024, generator=g)).bfloat16().cuda()
+    residual = torch.randn(M, 1024, generator=g).cuda()
+    rows = ops.add_rmsnorm(ops.linear(x, o, allow_pending=True), residual, norm, 1e-6, torch.bfloat16, scaled_ok=True)
+    assert isinstance(rows, ops.ScaledRows)
+    got = ops.gated_linear(rows, w, "silu", ops.GATED_BLOCK).double()
+    h = rows.data.double() * torch.rsqrt(residual.double().square().mean(1, keepdim=True) + 1e-6)
+    blocks = w.double().view(6, 2, 64, 1024)
+    gate, up = ((h @ blocks[:, i].reshape(384, 1024).T) for i in (0, 1))
+    want = torch.nn.functional.silu(gate) * up
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()

@@ -69,7 +69,7 @@ struct GemmParams {
   VecParam norm_w;
   bf16* hprime;
   float* sumsq_out;
-  // Gated form (no K cuts, up to 64 tokens): the weight rows alternate in blocks of 64, gate rows
+  // Gated form (up to 64 tokens; with K cuts, a cluster of them, up to 16): the weight rows alternate in blocks of 64, gate rows
   // then the matching up rows, so a 128-row tile holds both; out [M, N / 2] = act(gate) * up.
   int gated_act;        // 0: off; else the activation's code + 1
   float gated_limit;    // the bound of a bounded activation (gated_value)
@@ -296,6 +296,46 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
     // no block leaves while a peer may still read its shared memory
     cluster_arrive();
     cluster_wait();
+  } else if (p.gated_act != 0 && p.splits > 1) {
+    // gated form with K cuts (up to 16 tokens): the cuts of a row tile are a cluster, as in the residual form; rank r
+    // adds up the tokens r, r + splits, ... and applies the activation
+    if constexpr (TILE_T <= SUMSQ_STRIDE) {
+      float* red = reinterpret_cast<float*>(smem);               // [TILE_T][TILE_N], read by the cluster
+      float* sums = red + TILE_T * TILE_N;                       // [TILE_T][TILE_N], this block's tokens
+#pragma unroll 1
+      for (int c = 0; c < TILE_T; c += 8) {
+        float v[8];
+        if (have) tmem_load8(taddr + c, v);
+        else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) v[i] = 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) red[(c + i) * TILE_N + threadIdx.x] = scaled ? v[i] * row_scale[c + i] : v[i];
+      }
+      cluster_arrive();
+      cluster_wait();
+      for (int j = split; j < TILE_T && t0 + j < p.M; j += p.splits) {
+        float part[8];
+#pragma unroll
+        for (int s = 0; s < 8; ++s)
+          if (s < p.splits) part[s] = cluster_load_f32(red + j * TILE_N + threadIdx.x, s);
+        float sum = 0.f;
+#pragma unroll
+        for (int s = 0; s < 8; ++s)
+          if (s < p.splits) sum += part[s];
+        sums[j * TILE_N + threadIdx.x] = sum;
+      }
+      // (the peers' shared memory is read: they may leave)
+      cluster_arrive();
+      __syncthreads();
+      for (int j = split + p.splits * (threadIdx.x >> 6); j < TILE_T && t0 + j < p.M; j += 2 * p.splits) {
+        const int col = threadIdx.x & 63;
+        static_cast<bf16*>(p.out)[(size_t)(t0 + j) * p.ldc + n_tile * 64 + col] =
+            __float2bfloat16_rn(gated_value(sums[j * TILE_N + col], sums[j * TILE_N + 64 + col], p.gated_act - 1, p.gated_limit));
+      }
+      cluster_wait();
+    }
   } else if (p.gated_act != 0) {
     if constexpr (TILE_T <= 64) {
       // lanes 0..63 hold gate rows, lanes 64..127 the up rows of the same output columns: the up
@@ -449,7 +489,7 @@ int launch(const MAPS& maps, const GemmParams& p, dim3 grid, cudaStream_t stream
     if (e != cudaSuccess) return ts_fail("gemm_tcgen05: %s", cudaGetErrorString(e));
     configured = true;
   }
-  if (p.residual != nullptr) {
+  if (p.residual != nullptr || (p.gated_act != 0 && p.splits > 1)) {
     // the K cuts of a row tile are the blocks of one cluster
     cudaError_t e = ts_launch_cluster(gemm_wx_kernel<TILE_T, MAPS>, grid, dim3(THREADS), Cfg<TILE_T>::SMEM, stream,
                                       dim3(1, 1, p.splits), maps, p);
@@ -518,8 +558,8 @@ TS_EXPORT int ts_gemm_tcgen05(const void* x, const void* w, void* out, int M, in
 // are one thread-block cluster): residual [M, N] (float, contiguous) += x w^T; hprime [M, N]
 // (bfloat16) = residual * norm_w; sumsq_out [N / 128 rounded up][16] = the sums of residual^2
 // over each 128 columns, for the product that takes hprime as its x.
-// gated_act != 0 (up to 64 tokens, splits == 1, bfloat16 out [M, N / 2], ldc its leading
-// dimension, N a multiple of 128): the rows of w alternate in blocks of 64, gate rows then the
+// gated_act != 0 (up to 64 tokens, splits == 1, or up to 16 tokens and splits <= 8, one cluster a row tile, without
+// partials and counters; bfloat16 out [M, N / 2], ldc its leading dimension, N a multiple of 128): the rows of w alternate in blocks of 64, gate rows then the
 // matching up rows; out = act(gate) * up with act = gated_act - 1 (0 SiLU, 1 GELU-tanh, 2 the
 // bounded form of gated_value with gated_limit as its bound).
 // res_scale (residual form; [N] float or bfloat16, or nullptr): residual += (x w^T) * res_scale.
@@ -531,8 +571,8 @@ TS_EXPORT int ts_gemm_tcgen05_fused(const void* x, const void* w, void* out, int
                                     int res_scale_is_f32, cudaStream_t stream) {
   TS_REQUIRE((x_sumsq == nullptr && residual == nullptr) || M <= SUMSQ_STRIDE,
              "gemm_tcgen05: the scaled-rows and residual forms take up to %d tokens, got %d", SUMSQ_STRIDE, M);
-  TS_REQUIRE(gated_act == 0 || (gated_act <= ACT_COUNT && (gated_act - 1 != ACT_BOUNDED_SWISH || gated_limit > 0.f) && M <= 64 && splits == 1 && out && !out_f32 && !residual && N % 128 == 0),
-             "gemm_tcgen05: the gated form takes up to 64 tokens, no K cuts, a bfloat16 output and whole 128-row tiles");
+  TS_REQUIRE(gated_act == 0 || (gated_act <= ACT_COUNT && (gated_act - 1 != ACT_BOUNDED_SWISH || gated_limit > 0.f) && M <= 64 && (splits == 1 || (M <= SUMSQ_STRIDE && splits <= 8)) && out && !out_f32 && !residual && N % 128 == 0),
+             "gemm_tcgen05: the gated form takes up to 64 tokens (with up to 8 K cuts up to 16), a bfloat16 output and whole 128-row tiles");
   TS_REQUIRE(x_sumsq == nullptr || x_tiles > 0, "gemm_tcgen05: sums of squares without their tile count");
   TS_REQUIRE(residual == nullptr || (norm_w && hprime && sumsq_out && splits <= 8),
              "gemm_tcgen05: the residual form needs the norm's weight, both outputs and at most 8 cuts");
@@ -552,7 +592,7 @@ int gemm_tiled(const void* x, const void* w, void* out, int M, int N, int K, lon
   TS_REQUIRE(K % 8 == 0 && ldx % 8 == 0 && ldw % 8 == 0, "gemm_tcgen05: K and the leading dimensions must be multiples of 8 (16-byte rows for TMA), got K=%d", K);
   TS_REQUIRE((reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0, "gemm_tcgen05: operands must be 16-byte aligned");
   TS_REQUIRE(splits >= 1 && splits <= 64, "gemm_tcgen05: splits out of range");
-  TS_REQUIRE(residual != nullptr || splits == 1 || (partials && (counters || out == nullptr)), "gemm_tcgen05: split-K needs scratch and counters");
+  TS_REQUIRE(residual != nullptr || gated_act != 0 || splits == 1 || (partials && (counters || out == nullptr)), "gemm_tcgen05: split-K needs scratch and counters");
   TS_REQUIRE(residual != nullptr || out != nullptr || splits > 1, "gemm_tcgen05: without an output the partial tiles must be asked for (splits > 1)");
   const int tile_t = tile_tokens(M);
   Maps1 maps;
