@@ -8,9 +8,13 @@ from __future__ import annotations
 
 import zlib
 
+import numpy as np
 import torch
 
 from ..kernels import ops
+
+
+_TORCH = {np.float32: torch.float32, np.int32: torch.int32, np.int64: torch.int64}
 
 
 def stream_of(request_id, params) -> int:
@@ -37,30 +41,35 @@ class Sampler:
         self._rows = max_rows
         self._flip = 0
 
-    def _settings(self, temps, ks, ps, streams, steps):
-        """The per-row settings as device tensors, through one pinned staging buffer and one copy
-        (two buffers take turns: the copy of the step before may still be pending)."""
-        n = len(temps)
-        if self._staging is None or n > self._rows:
-            self._rows = max(self._rows, n, 8)
-            words = 6 * self._rows                    # float32 temp, float32 top_p, int32 top_k, int32 steps, int64 streams
+    def _stage(self, *columns):
+        """Columns of 32-bit (or, as int64, 64-bit) values as device tensors, through one pinned staging
+        buffer and one copy (two buffers take turns: the copy of the step before may still be pending; an
+        event per buffer keeps a host that runs further ahead from overwriting one)."""
+        sizes = [c.nbytes // 4 for c in columns]
+        offsets, words = [], 0
+        for size in sizes:
+            offsets.append(words)
+            words += (size + 3) // 4 * 4
+        if self._staging is None or words > self._staging[0].numel():
+            room = max(words, 6 * max(self._rows, 8), 2 * self._staging[0].numel() if self._staging else 0)
             pin = torch.device(self.device).type == "cuda"
-            self._staging = [(torch.zeros(words, dtype=torch.int32).pin_memory() if pin
-                              else torch.zeros(words, dtype=torch.int32)) for _ in range(2)]
-            self._device_words = torch.zeros(words, dtype=torch.int32, device=self.device)
-        R = self._rows
-        host = self._staging[self._flip]
-        self._flip ^= 1
+            self._staging = [(torch.zeros(room, dtype=torch.int32).pin_memory() if pin
+                              else torch.zeros(room, dtype=torch.int32)) for _ in range(2)]
+            self._device_words = torch.zeros(room, dtype=torch.int32, device=self.device)
+            self._copied = [None, None]
+        at_buffer, self._flip = self._flip, self._flip ^ 1
+        host, copied = self._staging[at_buffer], self._copied[at_buffer]
+        if copied is not None:
+            copied.synchronize()
         h = host.numpy()
-        h[0:n].view("float32")[:] = temps
-        h[R:R + n].view("float32")[:] = ps
-        h[2 * R:2 * R + n] = ks
-        h[3 * R:3 * R + n] = steps
-        h[4 * R:4 * R + 2 * n].view("int64")[:] = streams
-        d = self._device_words
-        d.copy_(host, non_blocking=True)
-        return (d[0:n].view(torch.float32), d[R:R + n].view(torch.float32), d[2 * R:2 * R + n],
-                d[3 * R:3 * R + n], d[4 * R:4 * R + 2 * n].view(torch.int64))
+        for column, at, size in zip(columns, offsets, sizes):
+            h[at:at + size] = column.reshape(-1).view(np.int32)
+        self._device_words[:words].copy_(host[:words], non_blocking=True)
+        if self._device_words.is_cuda:
+            self._copied[at_buffer] = copied or torch.cuda.Event()
+            self._copied[at_buffer].record()
+        return [self._device_words[at:at + size].view(_TORCH[column.dtype.type]).view(column.shape)
+                for column, at, size in zip(columns, offsets, sizes)]
 
     def _greedy_args(self, n):
         """Device tensors for an all-greedy batch (temperature 0 ignores the noise arguments)."""
@@ -95,16 +104,17 @@ class Sampler:
                 pen_rows.append(i)
                 pen_ids.append(ids)
                 pen_vals.append(float(p.repetition_penalty))
-        dev = self.device
-        if pen_rows:
-            width = max(len(x) for x in pen_ids)
-            table = torch.full((len(pen_rows), width), -1, dtype=torch.int32)
-            for j, ids in enumerate(pen_ids):
-                table[j, :len(ids)] = torch.tensor(ids, dtype=torch.int32)
-            ops.apply_repetition_penalty(logits, torch.tensor(pen_rows, dtype=torch.int32, device=dev),
-                                         table.to(dev), torch.tensor(pen_vals, dtype=torch.float32, device=dev))
         need_k = any(k > 0 for k, t in zip(ks, temps) if t > 0)
         need_p = any(p < 1.0 for p, t in zip(ps, temps) if t > 0)
-        d_temps, d_ps, d_ks, d_steps, d_streams = self._settings(temps, ks, ps, streams, steps)
+        columns = [np.array(temps, np.float32), np.array(ps, np.float32), np.array(ks, np.int32), np.array(steps, np.int32),
+                   np.array(streams, np.int64)]
+        if pen_rows:
+            table = np.full((len(pen_rows), max(len(x) for x in pen_ids)), -1, np.int32)
+            for row, ids in zip(table, pen_ids):
+                row[:len(ids)] = ids
+            columns += [np.array(pen_rows, np.int32), table, np.array(pen_vals, np.float32)]
+        d_temps, d_ps, d_ks, d_steps, d_streams, *penalty = self._stage(*columns)
+        if penalty:
+            ops.apply_repetition_penalty(logits, *penalty)
         return ops.sample(logits, d_temps, d_streams, d_steps, self.seed, top_k=d_ks if need_k else None,
                           top_p=d_ps if need_p else None, **feedback)
