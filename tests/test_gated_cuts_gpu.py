@@ -5,10 +5,10 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-# N (gate and up rows): one row tile, several, 48 (the gate/up product of a small model), 147 (the most that are cut);
+# N (gate and up rows): one row tile, several, 48 (the gate/up product of a small model), 147 (the most that are cut), 160 (one cut);
 # K: one slice and a ragged one (no cut), cuts of unequal length, eight cuts
-@pytest.mark.parametrize("N,K", [(128, 64), (128, 2048), (256, 1096), (640, 520), (6144, 1024), (147 * 128, 512)])
-@pytest.mark.parametrize("M", [1, 2, 7, 8, 9, 15, 16])
+@pytest.mark.parametrize("N,K", [(128, 64), (128, 2048), (256, 1096), (640, 520), (6144, 1024), (147 * 128, 512), (160 * 128, 256)])
+@pytest.mark.parametrize("M", [1, 2, 7, 8, 9, 15, 16, 17, 31, 32, 33, 63, 64])
 @pytest.mark.parametrize("activation,limit", [("silu", 0.0), ("gelu_tanh", 0.0), ("bounded_swish", 0.5)])
 def test_gated_product_of_few_row_tiles(M, N, K, activation, limit):
     from tinyserve_b200.kernels import ops

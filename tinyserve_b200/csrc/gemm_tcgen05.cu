@@ -69,7 +69,7 @@ struct GemmParams {
   VecParam norm_w;
   bf16* hprime;
   float* sumsq_out;
-  // Gated form (up to 64 tokens; with K cuts, a cluster of them, up to 16): the weight rows alternate in blocks of 64, gate rows
+  // Gated form (up to 64 tokens; the K cuts of a row tile are a cluster): the weight rows alternate in blocks of 64, gate rows
   // then the matching up rows, so a 128-row tile holds both; out [M, N / 2] = act(gate) * up.
   int gated_act;        // 0: off; else the activation's code + 1
   float gated_limit;    // the bound of a bounded activation (gated_value)
@@ -296,12 +296,14 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
     // no block leaves while a peer may still read its shared memory
     cluster_arrive();
     cluster_wait();
-  } else if (p.gated_act != 0 && p.splits > 1) {
-    // gated form with K cuts (up to 16 tokens): the cuts of a row tile are a cluster, as in the residual form; rank r
-    // adds up the tokens r, r + splits, ... and applies the activation
-    if constexpr (TILE_T <= SUMSQ_STRIDE) {
-      float* red = reinterpret_cast<float*>(smem);               // [TILE_T][TILE_N], read by the cluster
-      float* sums = red + TILE_T * TILE_N;                       // [TILE_T][TILE_N], this block's tokens
+  } else if (p.gated_act != 0) {
+    // gated form: the sums of the tile (with K cuts, a cluster of them as in the residual form: of the tokens rank,
+    // rank + splits, ..) in shared memory, where a thread finds its gate and its up row; neighbouring threads take
+    // neighbouring columns.  (A thread that kept its row's 64 sums in registers and only half of the threads at
+    // work took 23 us of a product of 64 tokens.)
+    if constexpr (TILE_T <= 64) {
+      float* red = reinterpret_cast<float*>(smem);               // [TILE_T][TILE_N] (the ring is idle), read by the cluster
+      float* sums = p.splits > 1 ? red + TILE_T * TILE_N : red;  // [TILE_T][TILE_N], this block's tokens
 #pragma unroll 1
       for (int c = 0; c < TILE_T; c += 8) {
         float v[8];
@@ -313,61 +315,32 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
 #pragma unroll
         for (int i = 0; i < 8; ++i) red[(c + i) * TILE_N + threadIdx.x] = scaled ? v[i] * row_scale[c + i] : v[i];
       }
-      cluster_arrive();
-      cluster_wait();
-      for (int j = split; j < TILE_T && t0 + j < p.M; j += p.splits) {
-        float part[8];
+      if (p.splits > 1) {
+        cluster_arrive();
+        cluster_wait();
+        for (int j = split; j < TILE_T && t0 + j < p.M; j += p.splits) {
+          float part[8];
 #pragma unroll
-        for (int s = 0; s < 8; ++s)
-          if (s < p.splits) part[s] = cluster_load_f32(red + j * TILE_N + threadIdx.x, s);
-        float sum = 0.f;
+          for (int s = 0; s < 8; ++s)
+            if (s < p.splits) part[s] = cluster_load_f32(red + j * TILE_N + threadIdx.x, s);
+          float sum = 0.f;
 #pragma unroll
-        for (int s = 0; s < 8; ++s)
-          if (s < p.splits) sum += part[s];
-        sums[j * TILE_N + threadIdx.x] = sum;
-      }
-      // (the peers' shared memory is read: they may leave)
-      cluster_arrive();
-      __syncthreads();
-      for (int j = split + p.splits * (threadIdx.x >> 6); j < TILE_T && t0 + j < p.M; j += 2 * p.splits) {
-        const int col = threadIdx.x & 63;
-        static_cast<bf16*>(p.out)[(size_t)(t0 + j) * p.ldc + n_tile * 64 + col] =
-            __float2bfloat16_rn(gated_value(sums[j * TILE_N + col], sums[j * TILE_N + 64 + col], p.gated_act - 1, p.gated_limit));
-      }
-      cluster_wait();
-    }
-  } else if (p.gated_act != 0) {
-    if constexpr (TILE_T <= 64) {
-      // lanes 0..63 hold gate rows, lanes 64..127 the up rows of the same output columns: the up
-      // half goes through shared memory (the ring is idle), the gate half activates and stores
-      float acc[TILE_T];
-#pragma unroll
-      for (int c = 0; c < TILE_T; c += 8) {
-        float v[8];
-        if (have) tmem_load8(taddr + c, v);
-        else {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) v[i] = 0.f;
+          for (int s = 0; s < 8; ++s)
+            if (s < p.splits) sum += part[s];
+          sums[j * TILE_N + threadIdx.x] = sum;
         }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) acc[c + i] = scaled ? v[i] * row_scale[c + i] : v[i];
-      }
-      float* up = reinterpret_cast<float*>(smem);               // [64][TILE_T + 1]
-      if (warp >= 2) {
-#pragma unroll
-        for (int i = 0; i < TILE_T; ++i) up[(threadIdx.x - 64) * (TILE_T + 1) + i] = acc[i];
+        // (the peers' shared memory is read: they may leave)
+        cluster_arrive();
       }
       __syncthreads();
-      const int col = n_tile * 64 + threadIdx.x, half_n = p.N / 2;
-      if (warp < 2 && col < half_n) {
-#pragma unroll
-        for (int i = 0; i < TILE_T; ++i) {
-          const int m = t0 + i;
-          if (m < p.M)
-            static_cast<bf16*>(p.out)[(size_t)m * p.ldc + col] =
-                __float2bfloat16_rn(gated_value(acc[i], up[threadIdx.x * (TILE_T + 1) + i], p.gated_act - 1, p.gated_limit));
-        }
+      const int col = threadIdx.x & 63;
+#pragma unroll 4
+      for (int j = split + p.splits * (threadIdx.x >> 6); j < TILE_T; j += 2 * p.splits) {
+        if (t0 + j < p.M)
+          static_cast<bf16*>(p.out)[(size_t)(t0 + j) * p.ldc + n_tile * 64 + col] =
+              __float2bfloat16_rn(gated_value(sums[j * TILE_N + col], sums[j * TILE_N + 64 + col], p.gated_act - 1, p.gated_limit));
       }
+      if (p.splits > 1) cluster_wait();
     }
   } else if (p.splits == 1) {
     const VecParam bias = beside ? p.seg[which].bias : p.bias;
@@ -558,8 +531,7 @@ TS_EXPORT int ts_gemm_tcgen05(const void* x, const void* w, void* out, int M, in
 // are one thread-block cluster): residual [M, N] (float, contiguous) += x w^T; hprime [M, N]
 // (bfloat16) = residual * norm_w; sumsq_out [N / 128 rounded up][16] = the sums of residual^2
 // over each 128 columns, for the product that takes hprime as its x.
-// gated_act != 0 (up to 64 tokens, splits == 1, or up to 16 tokens and splits <= 8, one cluster a row tile, without
-// partials and counters; bfloat16 out [M, N / 2], ldc its leading dimension, N a multiple of 128): the rows of w alternate in blocks of 64, gate rows then the
+// gated_act != 0 (up to 64 tokens and 8 cuts, which are one cluster a row tile, without partials and counters; bfloat16 out [M, N / 2], ldc its leading dimension, N a multiple of 128): the rows of w alternate in blocks of 64, gate rows then the
 // matching up rows; out = act(gate) * up with act = gated_act - 1 (0 SiLU, 1 GELU-tanh, 2 the
 // bounded form of gated_value with gated_limit as its bound).
 // res_scale (residual form; [N] float or bfloat16, or nullptr): residual += (x w^T) * res_scale.
@@ -571,8 +543,8 @@ TS_EXPORT int ts_gemm_tcgen05_fused(const void* x, const void* w, void* out, int
                                     int res_scale_is_f32, cudaStream_t stream) {
   TS_REQUIRE((x_sumsq == nullptr && residual == nullptr) || M <= SUMSQ_STRIDE,
              "gemm_tcgen05: the scaled-rows and residual forms take up to %d tokens, got %d", SUMSQ_STRIDE, M);
-  TS_REQUIRE(gated_act == 0 || (gated_act <= ACT_COUNT && (gated_act - 1 != ACT_BOUNDED_SWISH || gated_limit > 0.f) && M <= 64 && (splits == 1 || (M <= SUMSQ_STRIDE && splits <= 8)) && out && !out_f32 && !residual && N % 128 == 0),
-             "gemm_tcgen05: the gated form takes up to 64 tokens (with up to 8 K cuts up to 16), a bfloat16 output and whole 128-row tiles");
+  TS_REQUIRE(gated_act == 0 || (gated_act <= ACT_COUNT && (gated_act - 1 != ACT_BOUNDED_SWISH || gated_limit > 0.f) && M <= 64 && splits <= 8 && out && !out_f32 && !residual && N % 128 == 0),
+             "gemm_tcgen05: the gated form takes up to 64 tokens and 8 K cuts, a bfloat16 output and whole 128-row tiles");
   TS_REQUIRE(x_sumsq == nullptr || x_tiles > 0, "gemm_tcgen05: sums of squares without their tile count");
   TS_REQUIRE(residual == nullptr || (norm_w && hprime && sumsq_out && splits <= 8),
              "gemm_tcgen05: the residual form needs the norm's weight, both outputs and at most 8 cuts");

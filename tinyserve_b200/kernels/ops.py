@@ -711,12 +711,17 @@ def gated_activation(gate_up, activation="silu", block=0, limit=0.0):
 #: rows of gate and up alternate in blocks of this many in a fused gate/up weight: half a 128-row
 #: tile of the tcgen05 product
 GATED_BLOCK = 64
+#: Up to this many tokens the product of few tokens applies the activation itself, above half of it only where all
+#: row tiles run at once (two blocks a multiprocessor): the epilogue of a first wave keeps a second one from loading.
+#: 24576 x 4096 by 64 tokens 41.1 us with an activation kernel, 40.5 without; 6144 x 1024 17.2 and 11.6;
+#: 51200 x 5120 (400 tiles) by 32 tokens 87.1 and 86.7, by 64 94.7 and 96.1.
+GATED_MAX_TOKENS = 64
 
 
 def gated_linear(x, weight, activation="silu", block=0, limit=0.0):
     """act(gate) * up of x @ weight^T, [M, N / 2].  weight [N, K] holds gate rows then up rows
     (``block`` 0) or alternates them in blocks of ``block`` rows.  With blocks of GATED_BLOCK and up
-    to FUSED_MAX_TOKENS tokens the tcgen05 product does the activation in its epilogue; otherwise the product is followed by the activation kernel.  x may be the
+    to GATED_MAX_TOKENS tokens the tcgen05 product does the activation in its epilogue; otherwise the product is followed by the activation kernel.  x may be the
     ScaledRows that add_rmsnorm returned."""
     rows = x.data if isinstance(x, ScaledRows) else x
     N, K = weight.shape
@@ -730,7 +735,7 @@ def gated_linear(x, weight, activation="silu", block=0, limit=0.0):
         return _linear_pair(rows, weight, gated=code + 1, limit=limit, scale=x if rows is not x else None)
     if (block == GATED_BLOCK and N % 128 == 0 and isinstance(rows, torch.Tensor)
             and rows.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and _tcgen05_ok(rows, weight)
-            and rows.shape[0] <= FUSED_MAX_TOKENS):        # measured: at 64 tokens the epilogue costs 9 % of the step
+            and (rows.shape[0] <= GATED_MAX_TOKENS // 2 or (rows.shape[0] <= GATED_MAX_TOKENS and N <= 2 * num_sms() * 128))):
         _cuda(rows, weight)
         # (a product of few row tiles is cut along K inside clusters: 6144 x 1024 with its
         # activation: 8.9 -> 4.6 us for one token, 11.0 -> 6.0 for 16)
