@@ -35,6 +35,7 @@ static_assert(D % 16 == 0 && D >= 16 && D <= 256, "head size must be a multiple 
 constexpr int CH = D / 8;                 // 16-byte chunks of a row
 constexpr int ROW_BYTES = D * 2 + 16;     // rows are padded by one chunk: ldmatrix without conflicts
 constexpr int THREADS = 128;              // decode block
+constexpr int ALONE_TILES = 2;            // key tiles that one block walks without its cluster
 #ifndef TS_PREFILL_WARPS
 #define TS_PREFILL_WARPS 4
 #endif
@@ -562,7 +563,12 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
   const int first_tile = j_lo / BN, kept_tiles = min((keep + BN - 1) / BN, first_tile);
   const int total = (j_hi + BN - 1) / BN - first_tile + kept_tiles;
   auto tile_of = [&](int w) { return w < kept_tiles ? w : first_tile + (w - kept_tiles); };
-  const int per_split = (total + p.num_splits - 1) / p.num_splits;
+  // A short walk is one block's: the ranges of a cluster cost their merge (a cluster barrier and a round trip through
+  // distributed shared memory), a tile of 64 keys about 1 us.  One request, 16 heads over 8, 60 / 120 / 180 / 250 keys:
+  // 6.4 us in a cluster of eight, 4.5 / 5.4 / 6.5 / 7.7 alone.  (All blocks of the cluster see the same.)
+  const bool alone = p.cluster_merge && total <= ALONE_TILES;
+  const int per_split = alone ? total : (total + p.num_splits - 1) / p.num_splits;
+  if (alone && split > 0) return;
   const int walk_begin = split * per_split;
   const int n_tiles = max(0, min(total, walk_begin + per_split) - walk_begin);
   const int newest_tile = qpos / BN;
@@ -776,7 +782,7 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
       den = den * a + exp2f(sk - m_new);
       mx = m_new;
     }
-    if (p.num_splits == 1) {
+    if (p.num_splits == 1 || alone) {
       const float y = finished(den > 0.f ? num / den : 0.f, d, lanes);
       if (stores) p.out[((size_t)q_begin * p.H + head) * D + d] = __float2bfloat16_rn(y);
     } else if (p.cluster_merge) {
@@ -796,7 +802,7 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
       }
     }
   }
-  if (p.cluster_merge) {
+  if (p.cluster_merge && !alone) {
     // The blocks of a (request, KV group) are one cluster, rank = key range.  Each block merges
     // its share of the (head, dimension) pairs from all ranks' shared memory, in rank order.
     cluster_arrive();
