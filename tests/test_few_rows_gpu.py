@@ -58,6 +58,30 @@ def test_product_of_few_rows_takes_leading_dimensions(M):
         torch.testing.assert_close(got.double(), xs.double() @ ws.double().T, rtol=0, atol=2e-5)
 
 
+# both kernels that fetch W early (few rows; many rows, one wave of tiles and more), the weight made by the product just
+# before or by the one before that
+@pytest.mark.parametrize("between", [0, 1])
+@pytest.mark.parametrize("M,N,K", [(1, 2048, 1024), (8, 4096, 512), (200, 512, 1024), (1024, 1536, 1024)])
+def test_a_weight_may_be_the_product_before(M, N, K, between):
+    from tinyserve_b200.kernels import ops
+    g = torch.Generator().manual_seed(M)
+    x, a, b = (torch.randn(r, c, generator=g).cuda() for r, c in ((M, K), (N, 2048), (K, 2048)))
+    for _ in range(3):
+        stale = torch.full((N, K), float("nan"), device="cuda")            # what an early read of the weight finds
+        torch.cuda.synchronize()
+        del stale
+        w = ops.linear(a, b)
+        for _ in range(between):
+            ops.linear(x[:1], a[:, :K])
+        out = [ops.linear(x, w), ops.gated_linear(x, w), ops.activated_linear(x, w, "relu_squared")]
+        torch.cuda.synchronize()
+        want = [ops.linear(x, w, constant_weight=True), ops.gated_linear(x, w, constant_weight=True),
+                ops.activated_linear(x, w, "relu_squared", constant_weight=True)]
+        for got, expected in zip(out, want):
+            assert torch.equal(got, expected)
+    torch.testing.assert_close(w.double(), a.double() @ b.double().T, rtol=0, atol=2e-3)
+
+
 def plain_sample(x, temp, k, p):
     """The tokens that may be drawn: top-k with ties, then top-p over exact integer weights."""
     y = (x * np.float32(1.0 / np.float32(temp))).astype(np.float32)

@@ -147,7 +147,7 @@ __device__ __forceinline__ void copy16_async(uint32_t dst, const void* src, bool
 
 __global__ void __launch_bounds__(SPLIT_THREADS, 2)
 gemm_nt_chains_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
-                      float* __restrict__ C, int M, int N, int K, size_t lda, size_t ldw, size_t ldc) {
+                      float* __restrict__ C, int M, int N, int K, size_t lda, size_t ldw, size_t ldc, bool constant_w) {
   extern __shared__ __align__(16) char smem[];
   pdl_trigger();
   const int tid = threadIdx.x, grp = tid >> 6, t = tid & 63;
@@ -172,6 +172,9 @@ gemm_nt_chains_kernel(const float* __restrict__ A, const float* __restrict__ W, 
       copy16_async(base + c * SLICE_BYTES + r * (SLICE * 4) + ((u ^ ((r >> 1) & 3)) << 4), src + (ok ? (size_t)(row0 + r) * ld + k : 0), ok);
     }
   };
+  // (W is read ahead of the predecessors only where the caller says that none of them may have made it; a
+  // second wait returns at once)
+  if (!constant_w) pdl_wait();
   for (int st = 0; st < SPLIT_STAGES - 1; ++st)
     if (st < stages) load(st, true);
   pdl_wait();
@@ -266,7 +269,7 @@ gemm_nt_chains_kernel(const float* __restrict__ A, const float* __restrict__ W, 
 }
 
 int launch_chains(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, size_t lda, size_t ldw,
-                  size_t ldc, cudaStream_t stream) {
+                  size_t ldc, bool constant_w, cudaStream_t stream) {
   constexpr size_t smem = SPLIT_SMEM + SPLIT_RED_BYTES + SPLIT_TOTAL_BYTES;
   static bool configured = false;
   if (!configured) {
@@ -276,7 +279,7 @@ int launch_chains(const float* A, const float* W, const float* bias, float* C, i
   }
   dim3 grid((N + TILE - 1) / TILE, (M + TILE - 1) / TILE);
   if (grid.y > 65535) return ts_fail("gemm: M = %d is too large", M);
-  TS_LAUNCH("gemm_simt", gemm_nt_chains_kernel, grid, SPLIT_THREADS, smem, stream, A, W, bias, C, M, N, K, lda, ldw, ldc);
+  TS_LAUNCH("gemm_simt", gemm_nt_chains_kernel, grid, SPLIT_THREADS, smem, stream, A, W, bias, C, M, N, K, lda, ldw, ldc, constant_w);
   return 0;
 }
 
@@ -285,8 +288,8 @@ int launch_chains(const float* A, const float* W, const float* bias, float* C, i
 // for all of the MT rows of A, so that the sums are those of the tiled kernel bit by bit, and a block
 // covers CS chains of a row at a time: its threads are CS chains x 128 / CS groups of RT rows.  Slices
 // of STAGE_K k of every slot come through a ring of shared-memory stages (cp.async, 16 bytes a thread,
-// neighbouring threads on neighbouring bytes of a row); the stages of W that are fetched first do not
-// wait for the predecessor kernel.  The 16-byte unit u of slot s lies at u ^ (s & 7), so that
+// neighbouring threads on neighbouring bytes of a row); with a constant W its first stages do not
+// wait for the predecessor kernels.  The 16-byte unit u of slot s lies at u ^ (s & 7), so that
 // eight threads that read the same unit of eight slots touch all banks.  After the last slice of a
 // chain the chains' results go through shared memory to one thread per output, which adds them in
 // the order of k.
@@ -302,7 +305,7 @@ constexpr int MAX_CHAINS_SHIFT = 4;  // up to 16 chains of a row at a time: 8 RT
 template <int MT, int RT, int STAGES>
 __global__ void __launch_bounds__(SLOTS)
 gemv_nt_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
-               int M, int N, int K, size_t lda, size_t ldw, size_t ldc, int cs_shift) {
+               int M, int N, int K, size_t lda, size_t ldw, size_t ldc, int cs_shift, bool constant_w) {
   extern __shared__ __align__(16) char smem[];
   const int cs = 1 << cs_shift, groups = SLOTS >> cs_shift;      // chains in flight, groups of rows
   const int rows = groups * RT;
@@ -341,6 +344,7 @@ gemv_nt_kernel(const float* __restrict__ A, const float* __restrict__ W, const f
     }
   };
   // the first stages of W, then (with the predecessor's results) those of A: a group of copies each
+  if (!constant_w) pdl_wait();
   for (int st = 0; st < STAGES - 1; ++st)
     if (st < stages) load_w(st);
   pdl_wait();
@@ -412,7 +416,7 @@ gemv_nt_kernel(const float* __restrict__ A, const float* __restrict__ W, const f
 
 template <int MT, int RT, int STAGES>
 int launch_gemv(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, size_t lda, size_t ldw,
-                size_t ldc, cudaStream_t stream) {
+                size_t ldc, bool constant_w, cudaStream_t stream) {
   const int chains = (K + SUM_BLOCK - 1) / SUM_BLOCK;
   int cs_shift = 0;
   while (cs_shift < MAX_CHAINS_SHIFT && (1 << cs_shift) < chains) ++cs_shift;
@@ -432,13 +436,13 @@ int launch_gemv(const float* A, const float* W, const float* bias, float* C, int
   dim3 grid((N + rows - 1) / rows, (M + MT - 1) / MT);
   if (grid.y > 65535) return ts_fail("gemm: M = %d is too large", M);
   TS_LAUNCH("gemm_simt", (gemv_nt_kernel<MT, RT, STAGES>), grid, SLOTS, smem_of(cs_shift), stream, A, W, bias, C, M, N, K,
-            lda, ldw, ldc, cs_shift);
+            lda, ldw, ldc, cs_shift, constant_w);
   return 0;
 }
 
 template <typename TI, typename TO>
 int launch(const void* A, const void* W, const void* bias, void* C, int M, int N, int K, size_t lda,
-           size_t ldw, size_t ldc, cudaStream_t stream) {
+           size_t ldw, size_t ldc, bool constant_w, cudaStream_t stream) {
   const size_t align = 4 * sizeof(TI);
   const bool vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 &&
                    reinterpret_cast<uintptr_t>(A) % align == 0 && reinterpret_cast<uintptr_t>(W) % align == 0;
@@ -456,16 +460,16 @@ int launch(const void* A, const void* W, const void* bias, void* C, int M, int N
       const double few = 1e-12 / 13.8 * 2.0 * M * N * K * 1e6;
       const long long tiles = (long long)((N + TILE - 1) / TILE) * ((M + TILE - 1) / TILE);
       const double many = K / 1024.0 * (tiles <= 148 ? 41.0 : 36.0 * ((tiles + 147) / 148));
-      if (M > GEMV_WIDTH && many < few) return launch_chains(a, w, b, c, M, N, K, lda, ldw, ldc, stream);
+      if (M > GEMV_WIDTH && many < few) return launch_chains(a, w, b, c, M, N, K, lda, ldw, ldc, constant_w, stream);
       // As many rows of A to a block as leave a block for nearly every multiprocessor: they share the reads of W.
       const int chains = (K + SUM_BLOCK - 1) / SUM_BLOCK;
       int cs = 1;
       while (cs < (1 << MAX_CHAINS_SHIFT) && cs < chains) cs *= 2;
       auto blocks = [&](int mt, int rt) { return (long long)((N + SLOTS / cs * rt - 1) / (SLOTS / cs * rt)) * ((M + mt - 1) / mt); };
-      if (M > 4 && blocks(GEMV_WIDTH, 2) >= GEMV_MIN_BLOCKS) return launch_gemv<GEMV_WIDTH, 2, 2>(a, w, b, c, M, N, K, lda, ldw, ldc, stream);
-      if (M > 2 && blocks(4, 2) >= GEMV_MIN_BLOCKS) return launch_gemv<4, 2, 2>(a, w, b, c, M, N, K, lda, ldw, ldc, stream);
-      if (blocks(2, 2) >= GEMV_MIN_BLOCKS) return launch_gemv<2, 2, 3>(a, w, b, c, M, N, K, lda, ldw, ldc, stream);
-      return launch_gemv<2, 1, 3>(a, w, b, c, M, N, K, lda, ldw, ldc, stream);
+      if (M > 4 && blocks(GEMV_WIDTH, 2) >= GEMV_MIN_BLOCKS) return launch_gemv<GEMV_WIDTH, 2, 2>(a, w, b, c, M, N, K, lda, ldw, ldc, constant_w, stream);
+      if (M > 2 && blocks(4, 2) >= GEMV_MIN_BLOCKS) return launch_gemv<4, 2, 2>(a, w, b, c, M, N, K, lda, ldw, ldc, constant_w, stream);
+      if (blocks(2, 2) >= GEMV_MIN_BLOCKS) return launch_gemv<2, 2, 3>(a, w, b, c, M, N, K, lda, ldw, ldc, constant_w, stream);
+      return launch_gemv<2, 1, 3>(a, w, b, c, M, N, K, lda, ldw, ldc, constant_w, stream);
     }
   }
   if (M > 64) {
@@ -483,17 +487,18 @@ int launch(const void* A, const void* W, const void* bias, void* C, int M, int N
 
 }  // namespace
 
-// in_dtype: element type of A, W and bias; out_dtype: element type of C
+// in_dtype: element type of A, W and bias; out_dtype: element type of C; constant_w: no kernel that may still run
+// writes W (float32 products then fetch their first tiles of it before the kernels ahead of them are done)
 TS_EXPORT int ts_gemm_simt(int in_dtype, int out_dtype, const void* A, const void* W,
                            const void* bias, void* C, int M, int N, int K, long long lda,
-                           long long ldw, long long ldc, cudaStream_t stream) {
+                           long long ldw, long long ldc, int constant_w, cudaStream_t stream) {
   TS_REQUIRE(M > 0 && N > 0 && K > 0, "gemm: empty operand (M=%d N=%d K=%d)", M, N, K);
   TS_REQUIRE(lda >= K && ldw >= K && ldc >= N, "gemm: a leading dimension is smaller than its row");
   if (in_dtype == TS_F32 && out_dtype == TS_F32)
-    return launch<float, float>(A, W, bias, C, M, N, K, lda, ldw, ldc, stream);
+    return launch<float, float>(A, W, bias, C, M, N, K, lda, ldw, ldc, constant_w != 0, stream);
   if (in_dtype == TS_BF16 && out_dtype == TS_BF16)
-    return launch<__nv_bfloat16, __nv_bfloat16>(A, W, bias, C, M, N, K, lda, ldw, ldc, stream);
+    return launch<__nv_bfloat16, __nv_bfloat16>(A, W, bias, C, M, N, K, lda, ldw, ldc, constant_w != 0, stream);
   if (in_dtype == TS_BF16 && out_dtype == TS_F32)
-    return launch<__nv_bfloat16, float>(A, W, bias, C, M, N, K, lda, ldw, ldc, stream);
+    return launch<__nv_bfloat16, float>(A, W, bias, C, M, N, K, lda, ldw, ldc, constant_w != 0, stream);
   return ts_fail("gemm: unsupported dtypes in=%d out=%d", in_dtype, out_dtype);
 }

@@ -718,11 +718,11 @@ GATED_BLOCK = 64
 GATED_MAX_TOKENS = 64
 
 
-def gated_linear(x, weight, activation="silu", block=0, limit=0.0):
+def gated_linear(x, weight, activation="silu", block=0, limit=0.0, constant_weight=False):
     """act(gate) * up of x @ weight^T, [M, N / 2].  weight [N, K] holds gate rows then up rows
     (``block`` 0) or alternates them in blocks of ``block`` rows.  With blocks of GATED_BLOCK and up
     to GATED_MAX_TOKENS tokens the tcgen05 product does the activation in its epilogue; otherwise the product is followed by the activation kernel.  x may be the
-    ScaledRows that add_rmsnorm returned."""
+    ScaledRows that add_rmsnorm returned.  ``constant_weight``: as for ``linear``."""
     rows = x.data if isinstance(x, ScaledRows) else x
     N, K = weight.shape
     code, limit = activation_code(activation, limit)
@@ -742,7 +742,7 @@ def gated_linear(x, weight, activation="silu", block=0, limit=0.0):
         splits = min(gemm_splits(rows.shape[0], N, K, partials=True), FUSED_MAX_SPLITS)
         return _linear_tcgen05(rows, weight, False, splits=splits, gated=code + 1, limit=limit,
                                scale=x if rows is not x else None)
-    return gated_activation(linear(x, weight), activation, block, limit)
+    return gated_activation(linear(x, weight, constant_weight=constant_weight), activation, block, limit)
 
 
 def plain_activation_(x, activation):
@@ -757,14 +757,14 @@ def plain_activation_(x, activation):
     return x
 
 
-def activated_linear(x, weight, activation):
+def activated_linear(x, weight, activation, constant_weight=False):
     """act(x @ weight^T) [M, N]: in the tcgen05 product's epilogue for up to TCGEN05_MAX_TOKENS bfloat16 rows,
-    else the product followed by the activation in place."""
+    else the product followed by the activation in place.  ``constant_weight``: as for ``linear``."""
     x = materialize(x)
     if x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and activation in PLAIN_ACTIVATIONS and _tcgen05_ok(x, weight):
         _cuda(x, weight)
         return _linear_tcgen05(x, weight, False, plain=PLAIN_ACTIVATIONS[activation])
-    return plain_activation_(linear(x, weight), activation)
+    return plain_activation_(linear(x, weight, constant_weight=constant_weight), activation)
 
 
 def qk_norm_rope_kvwrite(qkv, positions, num_heads, num_kv_heads, head_dim, rotary=None,
@@ -1126,14 +1126,18 @@ def attention_from_qkv(qkv, positions, num_heads, num_kv_heads, head_dim, rotary
     return out
 
 
-def linear(x, weight, bias=None, out_float32=False, allow_partials=False, allow_pending=False):
+def linear(x, weight, bias=None, out_float32=False, allow_partials=False, allow_pending=False, constant_weight=False):
     """x [M, K] @ weight[N, K]^T (+ bias).  float32 operands: this package's 32-bit FMA kernel
     (no tensor cores, no reduced precision).  bfloat16 operands: this package's TMA + tcgen05
     kernel for up to TCGEN05_MAX_TOKENS rows (K and the leading dimensions multiples of 8), cuBLAS
     through torch above that, as in tinyserve (serve.py:828-829).  With ``allow_partials`` the
     result may be a SplitPartials (the caller hands it to add_rmsnorm, qk_norm_rope_kvwrite, or
     calls materialize); with ``allow_pending`` a PendingProduct (for add_rmsnorm, or materialize).
-    x may be the ScaledRows that add_rmsnorm returned."""
+    x may be the ScaledRows that add_rmsnorm returned.
+    ``constant_weight``: no kernel that may still run writes ``weight`` (a model's weights).  A float32 product
+    then fetches its first tiles of it while the kernels before it still run; without, the weight may be the
+    result of the product before.  The bfloat16 products of this package always fetch them so: a
+    bfloat16 weight that was computed on the device needs a synchronisation before its first product."""
     scale = None
     if isinstance(x, ScaledRows):
         scale, x = x, x.data
@@ -1172,10 +1176,10 @@ def linear(x, weight, bias=None, out_float32=False, allow_partials=False, allow_
         if out_float32:
             return torch.mm(x, weight.t(), out_dtype=torch.float32)
         return torch.mm(x, weight.t())
-    return _linear_simt(x, weight, bias, out_float32)
+    return _linear_simt(x, weight, bias, out_float32, constant_weight)
 
 
-def _linear_simt(x, weight, bias=None, out_float32=False):
+def _linear_simt(x, weight, bias=None, out_float32=False, constant_weight=False):
     """The 32-bit FMA product (float32 operands; it takes bfloat16 operands too)."""
     M, K = x.shape
     N = weight.shape[0]
@@ -1189,7 +1193,7 @@ def _linear_simt(x, weight, bias=None, out_float32=False):
     _check(lib, lib.ts_gemm_simt(c_int(_dt(x)), c_int(_DTYPE[out_dtype]), _ptr(x), _ptr(weight),
                                  _ptr(bias), _ptr(out), c_int(M), c_int(N), c_int(K),
                                  c_longlong(x.stride(0)), c_longlong(weight.stride(0)),
-                                 c_longlong(N), _stream()))
+                                 c_longlong(N), c_int(1 if constant_weight else 0), _stream()))
     return out
 
 
@@ -2202,10 +2206,10 @@ def branch_norm(x, residual, weight1, weight2, eps, out_dtype, rows=None, scaled
 
 class InputProduct:
     """A product a part starts with, described so that a block of two branches can run its parts' input
-    products in one launch: h @ weight^T (+ bias), in the compute type or 32-bit."""
+    products in one launch: h @ weight^T (+ bias), in the compute type or 32-bit.  ``constant_weight``: as for ``linear``."""
 
-    def __init__(self, weight, bias=None, out_float32=False):
-        self.weight, self.bias, self.out_float32 = weight, bias, out_float32
+    def __init__(self, weight, bias=None, out_float32=False, constant_weight=False):
+        self.weight, self.bias, self.out_float32, self.constant_weight = weight, bias, out_float32, constant_weight
 
 
 BESIDE_MAX_PRODUCTS = 3
@@ -2224,7 +2228,7 @@ def linear_beside(groups):
            and (not scaled or (len(scaled) == len(flat) and M <= FUSED_MAX_TOKENS
                                and all(h.sumsq is scaled[0].sumsq and h.eps == scaled[0].eps for h in scaled))))
     if not one:
-        return [[linear(h, p.weight, p.bias, out_float32=p.out_float32) for p in products] for h, products in groups]
+        return [[linear(h, p.weight, p.bias, out_float32=p.out_float32, constant_weight=p.constant_weight) for p in products] for h, products in groups]
     _cuda(*rows, *[p.weight for _, p in flat], *[p.bias for _, p in flat])
     outs = [torch.empty(M, p.weight.shape[0], dtype=torch.float32 if p.out_float32 else torch.bfloat16, device=rows[0].device)
             for _, p in flat]

@@ -247,7 +247,7 @@ class Attention(Mixer):
 
     def input_products(self):
         """The product this mixer starts with (the general form), for a block that runs it beside others."""
-        return [ops.InputProduct(self.w["qkv_proj.weight"], self.w.get("qkv_proj.bias"))] if self.general else None
+        return [ops.InputProduct(self.w["qkv_proj.weight"], self.w.get("qkv_proj.bias"), constant_weight=True)] if self.general else None
 
     def _query_rows(self, qkv, ctx, call, cache, view):
         """The attention kernels' query rows [T, heads, stored_dim] of this step's projected rows; keys and
@@ -299,15 +299,15 @@ class Attention(Mixer):
             out = ops.head_gate(out, qkv[:, v_end:] if self.head_gate else None, self.value_dim)
         else:
             out = out.view(out.shape[0], self.num_heads * self.value_dim)
-        return ops.linear(out, self.w["o_proj.weight"], self.w.get("o_proj.bias"), allow_pending=True)
+        return ops.linear(out, self.w["o_proj.weight"], self.w.get("o_proj.bias"), allow_pending=True, constant_weight=True)
 
     def _forward_general(self, h, ctx, call):
-        return self.forward_projected([ops.linear(h, self.w["qkv_proj.weight"], self.w.get("qkv_proj.bias"))], h, ctx, call)
+        return self.forward_projected([ops.linear(h, self.w["qkv_proj.weight"], self.w.get("qkv_proj.bias"), constant_weight=True)], h, ctx, call)
 
     def forward(self, h, ctx, call):
         if self.general:
             return self._forward_general(h, ctx, call)
-        qkv = ops.linear(h, self.w["qkv_proj.weight"], self.w.get("qkv_proj.bias"), allow_partials=True)
+        qkv = ops.linear(h, self.w["qkv_proj.weight"], self.w.get("qkv_proj.bias"), allow_partials=True, constant_weight=True)
         cache = ctx.cache(call.cache)
         view = ctx.group(cache.group)
         out = ops.attention_from_qkv(
@@ -316,7 +316,7 @@ class Attention(Mixer):
             self.k_norm.w["weight"] if self.k_norm is not None else None,
             self.q_norm.eps if self.q_norm is not None else 0.0,
             cache.k, cache.v, view, ctx, self.scale, self.window, write_cache=call.writes_cache)
-        return ops.linear(out.view(out.shape[0], self.q_size), self.w["o_proj.weight"], self.w.get("o_proj.bias"), allow_pending=True)
+        return ops.linear(out.view(out.shape[0], self.q_size), self.w["o_proj.weight"], self.w.get("o_proj.bias"), allow_pending=True, constant_weight=True)
 
 
 register_mixer("attention", Attention)

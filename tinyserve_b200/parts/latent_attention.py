@@ -99,7 +99,7 @@ class LatentAttention(Mixer):
 
     def forward(self, h, ctx, call):
         H, n, nr, nv, r = self.num_heads, self.head_dim, self.rot_dim, self.value_dim, self.kv_rank
-        proj = ops.materialize(ops.linear(h, self.w["in_proj.weight"]))
+        proj = ops.materialize(ops.linear(h, self.w["in_proj.weight"], constant_weight=True))
         cache = ctx.cache(call.cache)
         view = ctx.group(cache.group)
         rows = cache.tensors["latent"]
@@ -108,7 +108,7 @@ class LatentAttention(Mixer):
             proj, self.q_rank, self.w["q_norm.weight"], self.eps, kv_rank=r, rot_dim=nr,
             kv_weight=self.w["kv_norm.weight"] if writes else None, rotary=self.position, positions=ctx.positions,
             cache=rows if writes else None, slot_mapping=view.slot_mapping if writes else None)
-        q = ops.materialize(ops.linear(q_latent, self.w["q_up.weight"]))
+        q = ops.materialize(ops.linear(q_latent, self.w["q_up.weight"], constant_weight=True))
         T = q.shape[0]
         # the plain part of every head's query, carried into the latent space: [H, T, dim] x [H, dim, kv_rank]
         q_plain = q.view(T, H, n + nr)[:, :, :n].transpose(0, 1)
@@ -118,9 +118,9 @@ class LatentAttention(Mixer):
         # [H, T, kv_rank] x [H, kv_rank, vdim]: every head's weighted latent expanded to its values
         wide, w_uv = mixed[:, :, :r].transpose(0, 1), self.w["v_up.weight"].view(H, nv, r).transpose(1, 2)
         if not self.gate:
-            return ops.linear(ops.batched_matmul(wide, w_uv, side_by_side=True), self.w["o_proj.weight"], allow_pending=True)
+            return ops.linear(ops.batched_matmul(wide, w_uv, side_by_side=True), self.w["o_proj.weight"], allow_pending=True, constant_weight=True)
         gate = proj[:, self.q_rank + self.kv_size:]
-        return ops.linear(ops.gate_heads(ops.batched_matmul(wide, w_uv), gate), self.w["o_proj.weight"], allow_pending=True)
+        return ops.linear(ops.gate_heads(ops.batched_matmul(wide, w_uv), gate), self.w["o_proj.weight"], allow_pending=True, constant_weight=True)
 
 
 register_mixer("latent_attention", LatentAttention)

@@ -81,7 +81,7 @@ class MatrixStateMixer(Mixer):
         return StateSpec((self.num_heads, self.key_dim, self.value_dim), "float32")
 
     def _split(self, h):
-        proj = ops.materialize(ops.linear(h, self.w["in_proj.weight"]))
+        proj = ops.materialize(ops.linear(h, self.w["in_proj.weight"], constant_weight=True))
         qk, v = self.qk_size, self.v_size
         return proj, proj[:, :qk], proj[:, qk:2 * qk], proj[:, 2 * qk:2 * qk + v], proj[:, 2 * qk + v:2 * qk + 2 * v]
 
@@ -106,7 +106,7 @@ class Retention(MatrixStateMixer):
         out = ops.linear_attention(q, k, v, g, ctx.state(call.state), ctx, self.num_heads, self.key_dim,
                                    self.value_dim, ctx.dtype, decay=self.decay, rotary=self.position,
                                    k_scale=self.key_dim ** -0.5, eps=self.eps)
-        return ops.linear(out, self.w["o_proj.weight"], allow_pending=True)
+        return ops.linear(out, self.w["o_proj.weight"], allow_pending=True, constant_weight=True)
 
 
 class GatedLinearAttention(MatrixStateMixer):
@@ -136,11 +136,11 @@ class GatedLinearAttention(MatrixStateMixer):
     def forward(self, h, ctx, call):
         proj, q, k, v, g = self._split(h)
         low = proj[:, 2 * self.qk_size + 2 * self.v_size:]
-        z = ops.linear(low, self.w["decay_up.weight"], self.w["decay_up.bias"], out_float32=True)
+        z = ops.linear(low, self.w["decay_up.weight"], self.w["decay_up.bias"], out_float32=True, constant_weight=True)
         out = ops.linear_attention(q, k, v, g, ctx.state(call.state), ctx, self.num_heads, self.key_dim,
                                    self.value_dim, ctx.dtype, decay_logits=z, tau=self.tau,
                                    q_scale=self.key_dim ** -0.5, norm_weight=self.w["norm.weight"], eps=self.eps)
-        return ops.linear(out, self.w["o_proj.weight"], allow_pending=True)
+        return ops.linear(out, self.w["o_proj.weight"], allow_pending=True, constant_weight=True)
 
 
 class Lightning(MatrixStateMixer):
@@ -165,7 +165,7 @@ class Lightning(MatrixStateMixer):
         out = ops.linear_attention(q, k, v, g, ctx.state(call.state), ctx, self.num_heads, self.key_dim,
                                    self.value_dim, ctx.dtype, decay=self.decay, norm_weight=self.w["norm.weight"],
                                    eps=self.eps, input_activation="silu", gate_activation="sigmoid", joint_norm=True)
-        return ops.linear(out, self.w["o_proj.weight"], allow_pending=True)
+        return ops.linear(out, self.w["o_proj.weight"], allow_pending=True, constant_weight=True)
 
 
 class HGRN2(Mixer):
@@ -203,13 +203,13 @@ class HGRN2(Mixer):
         return StateSpec((self.num_heads, self.key_dim, self.value_dim), "float32")
 
     def forward(self, h, ctx, call):
-        proj = ops.materialize(ops.linear(h, self.w["in_proj.weight"]))
-        z = ops.linear(h, self.w["f_proj.weight"], self.w["f_proj.bias"], out_float32=True)
+        proj = ops.materialize(ops.linear(h, self.w["in_proj.weight"], constant_weight=True))
+        z = ops.linear(h, self.w["f_proj.weight"], self.w["f_proj.bias"], out_float32=True, constant_weight=True)
         out = ops.linear_attention(proj[:, :self.qk_size], None, proj[:, self.qk_size:], None, ctx.state(call.state), ctx,
                                    self.num_heads, self.key_dim, self.value_dim, ctx.dtype, decay_logits=z,
                                    lower=self.w["lower"], tied_key=True, input_activation="q",
                                    norm_weight=self.w["norm.weight"], eps=self.eps)
-        return ops.linear(out, self.w["o_proj.weight"], allow_pending=True)
+        return ops.linear(out, self.w["o_proj.weight"], allow_pending=True, constant_weight=True)
 
 
 class MLSTM(Mixer):
@@ -250,16 +250,16 @@ class MLSTM(Mixer):
                 "max": StateSpec((self.num_heads,), "float32")}
 
     def forward(self, h, ctx, call):
-        proj = ops.materialize(ops.linear(h, self.w["in_proj.weight"]))
+        proj = ops.materialize(ops.linear(h, self.w["in_proj.weight"], constant_weight=True))
         qk, v = self.qk_size, self.v_size
-        raw_gates = ops.linear(h, self.w["gates.weight"], self.w["gates.bias"], out_float32=True)
+        raw_gates = ops.linear(h, self.w["gates.weight"], self.w["gates.bias"], out_float32=True, constant_weight=True)
         keep, write, floor = ops.mlstm_gates(raw_gates, self.gate_cap, ctx.state(call.state_of("max")), ctx, self.num_heads)
         raw = ops.linear_attention(proj[:, :qk], proj[:, qk:2 * qk], proj[:, 2 * qk:2 * qk + v], None, ctx.state(call.state),
                                    ctx, self.num_heads, self.key_dim, self.state_cols, ctx.dtype, token_keep=keep,
                                    token_write=write, q_scale=self.key_dim ** -0.5, value_width=self.value_dim, raw=True)
         out = ops.mlstm_finish(raw, floor, self.w["norm.weight"], proj[:, 2 * qk + v:], self.eps, self.num_heads,
                                self.value_dim, ctx.dtype)
-        return ops.linear(out, self.w["o_proj.weight"], allow_pending=True)
+        return ops.linear(out, self.w["o_proj.weight"], allow_pending=True, constant_weight=True)
 
 
 class Mamba2(Mixer):
@@ -308,9 +308,9 @@ class Mamba2(Mixer):
     def forward(self, h, ctx, call):
         inner, C, H, GN = self.inner, self.conv_channels, self.num_heads, self.groups * self.state_dim
         weight = self.w["in_proj.weight"]
-        proj = ops.materialize(ops.linear(h, weight[:inner + C]))
+        proj = ops.materialize(ops.linear(h, weight[:inner + C], constant_weight=True))
         # the step sizes enter the recurrence: their product leaves in 32-bit
-        dt_raw = ops.linear(h, weight[inner + C:], out_float32=True)
+        dt_raw = ops.linear(h, weight[inner + C:], out_float32=True, constant_weight=True)
         conv_state = ctx.state(call.state_of("conv")) if self.taps > 1 else None
         xbc = ops.causal_conv(proj[:, inner:], self.w["conv.weight"], conv_state, ctx, ctx.dtype, bias=self.w["conv.bias"],
                               activation="silu")
@@ -321,7 +321,7 @@ class Mamba2(Mixer):
                                    step_sizes=(dt_raw, self.w["dt_bias"], self.w["a_log"]), qk_group=H // self.groups, raw=True)
         out = ops.ssm_finish(raw, x, self.w["skip"], proj[:, :inner], self.w["norm.weight"], self.norm_groups, self.eps, H,
                              self.value_dim, ctx.dtype)
-        return ops.linear(out, self.w["o_proj.weight"], allow_pending=True)
+        return ops.linear(out, self.w["o_proj.weight"], allow_pending=True, constant_weight=True)
 
 
 class GatedDeltaRule(Mixer):
@@ -367,7 +367,7 @@ class GatedDeltaRule(Mixer):
         return specs
 
     def input_products(self):
-        return [ops.InputProduct(self.w["in_proj.weight"]), ops.InputProduct(self.w["gates.weight"], None, True)]
+        return [ops.InputProduct(self.w["in_proj.weight"], constant_weight=True), ops.InputProduct(self.w["gates.weight"], None, True, constant_weight=True)]
 
     def forward_projected(self, projected, h, ctx, call):
         proj, logits = ops.materialize(projected[0]), projected[1]
@@ -377,7 +377,7 @@ class GatedDeltaRule(Mixer):
         out = ops.delta_rule(x[:, :qk], x[:, qk:2 * qk], x[:, 2 * qk:], proj[:, C:], logits, self.w["dt_bias"], self.w["a_log"],
                              ctx.state(call.state_of("")), ctx, self.num_heads, self.key_dim, self.value_dim, self.w["norm.weight"],
                              self.eps, ctx.dtype, q_scale=self.key_dim ** -0.5, qk_group=self.num_heads // self.num_kv_heads)
-        return ops.linear(out, self.w["o_proj.weight"], allow_pending=True)
+        return ops.linear(out, self.w["o_proj.weight"], allow_pending=True, constant_weight=True)
 
     def forward(self, h, ctx, call):
         return self.forward_projected(ops.linear_beside([(h, self.input_products())])[0], h, ctx, call)

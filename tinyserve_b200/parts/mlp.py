@@ -46,8 +46,8 @@ class GatedMLP(FeedForward):
     accepts_scaled_rows = True
 
     def forward(self, h, ctx):
-        act = ops.gated_linear(h, self.w["gate_up_proj.weight"], self.activation, self.block, self.limit)
-        return ops.linear(act, self.w["down_proj.weight"], allow_pending=True)
+        act = ops.gated_linear(h, self.w["gate_up_proj.weight"], self.activation, self.block, self.limit, constant_weight=True)
+        return ops.linear(act, self.w["down_proj.weight"], allow_pending=True, constant_weight=True)
 
 
 register_feed_forward("gated_mlp", GatedMLP)
@@ -75,14 +75,14 @@ class PolyNormMLP(FeedForward):
         }
 
     def input_products(self):
-        return [ops.InputProduct(self.w["up_proj.weight"], self.w["up_proj.bias"])]
+        return [ops.InputProduct(self.w["up_proj.weight"], self.w["up_proj.bias"], constant_weight=True)]
 
     def forward_projected(self, projected, h, ctx):
         act = ops.poly_norm(projected[0], self.w["act"], self.eps)
-        return ops.linear(act, self.w["down_proj.weight"], self.w["down_proj.bias"], allow_pending=True)
+        return ops.linear(act, self.w["down_proj.weight"], self.w["down_proj.bias"], allow_pending=True, constant_weight=True)
 
     def forward(self, h, ctx):
-        return self.forward_projected([ops.linear(h, p.weight, p.bias) for p in self.input_products()], h, ctx)
+        return self.forward_projected([ops.linear(h, p.weight, p.bias, constant_weight=True) for p in self.input_products()], h, ctx)
 
 
 register_feed_forward("poly_norm_mlp", PolyNormMLP)
@@ -106,8 +106,8 @@ class PlainMLP(FeedForward):
                 "down_proj.weight": ParamSpec((n, i), sources=(Source(f"{nm['down']}.weight", 0, n),))}
 
     def forward(self, h, ctx):
-        return ops.linear(ops.activated_linear(h, self.w["up_proj.weight"], self.activation), self.w["down_proj.weight"],
-                          allow_pending=True)
+        return ops.linear(ops.activated_linear(h, self.w["up_proj.weight"], self.activation, constant_weight=True), self.w["down_proj.weight"],
+                          allow_pending=True, constant_weight=True)
 
 
 register_feed_forward("plain_mlp", PlainMLP)

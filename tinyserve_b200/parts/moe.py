@@ -128,18 +128,18 @@ class MixtureOfExperts(FeedForward):
     def input_products(self):
         """Router and up-projections, for a block that runs them beside its mixer's input product (a step
         of few tokens, where all experts run on all tokens)."""
-        return [ops.InputProduct(self.w["router.weight"], out_float32=True), ops.InputProduct(self.w["up.weight"])]
+        return [ops.InputProduct(self.w["router.weight"], out_float32=True, constant_weight=True), ops.InputProduct(self.w["up.weight"], constant_weight=True)]
 
     def forward_projected(self, projected, h, ctx):
         return self._all_experts(projected[0], projected[1], h)
 
     def forward(self, h, ctx):
-        logits = ops.linear(h, self.w["router.weight"], out_float32=True)
+        logits = ops.linear(h, self.w["router.weight"], out_float32=True, constant_weight=True)
         if not isinstance(h, ops.ScaledRows) and self._grouped(h):
             gates, rest = self._route(self._biased(logits))
             return ops.moe_grouped(h, gates, self.w["up.weight"], self.w["down.weight"], self.top,
                                    gated=self.gated, activation=self.gate_activation, limit=self.limit, rest=rest)
-        return self._all_experts(logits, ops.linear(h, self.w["up.weight"]), h)
+        return self._all_experts(logits, ops.linear(h, self.w["up.weight"], constant_weight=True), h)
 
     def _biased(self, logits):
         if self.router_bias and self.router in CORRECTED_ROUTERS:
@@ -162,7 +162,7 @@ class MixtureOfExperts(FeedForward):
             ops.moe_activate_(a, None, self.num_experts, logits=logits, top=self.top)      # (routes in the same kernel)
         else:
             ops.moe_activate_(a, self._route(logits)[0], self.num_experts)
-        y = ops.linear(a, self.w["down.weight"], allow_pending=True)
+        y = ops.linear(a, self.w["down.weight"], allow_pending=True, constant_weight=True)
         return y if rest is None else ops.RowsAdded(y, rest, h.data if isinstance(h, ops.ScaledRows) else h)
 
 

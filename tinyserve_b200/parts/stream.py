@@ -31,7 +31,7 @@ class InputInjection(StreamOp):
         both = ops.stream_concat(residual, pending, first, ctx.dtype)
         # (the pass's vector rides as the product's bias: added in 32-bit in its epilogue, or by a
         # kernel of its own behind the library's product)
-        return ops.linear(both, self.w["in.weight"], self.w["step.weight"][arg], out_float32=True), None
+        return ops.linear(both, self.w["in.weight"], self.w["step.weight"][arg], out_float32=True, constant_weight=True), None
 
 
 register_stream_op("input_injection", InputInjection)
