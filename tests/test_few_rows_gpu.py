@@ -58,6 +58,23 @@ def test_product_of_few_rows_takes_leading_dimensions(M):
         torch.testing.assert_close(got.double(), xs.double() @ ws.double().T, rtol=0, atol=2e-5)
 
 
+@pytest.mark.parametrize("M", [65535 * 8, 65535 * 8 + 1, 65535 * 64 + 1, 65535 * 128])
+def test_products_of_very_many_rows(M):
+    """A grid has 65,535 blocks of rows at most, which every kernel reaches at another number of rows."""
+    from tinyserve_b200.kernels import ops
+    g = torch.Generator().manual_seed(3)
+    w = torch.randn(3, 8, generator=g).cuda()
+    x = torch.randn(1024, 8, generator=g).cuda().repeat(-(-M // 1024), 1)[:M]
+    out, want = ops.linear(x, w), ops.linear(x[:1024], w)
+    assert torch.equal(out, want.repeat(-(-M // 1024), 1)[:M])
+
+
+def test_more_rows_than_any_grid_covers_are_refused():
+    from tinyserve_b200.kernels import ops
+    with pytest.raises(RuntimeError, match="too large"):
+        ops.linear(torch.zeros(65535 * 128 + 1, 4, device="cuda"), torch.zeros(3, 4, device="cuda"))
+
+
 # both kernels that fetch W early (few rows; many rows, one wave of tiles and more), the weight made by the product just
 # before or by the one before that
 @pytest.mark.parametrize("between", [0, 1])

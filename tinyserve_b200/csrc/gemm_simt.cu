@@ -450,8 +450,11 @@ int launch(const void* A, const void* W, const void* bias, void* C, int M, int N
   const TI* w = static_cast<const TI*>(W);
   const TI* b = static_cast<const TI*>(bias);
   TO* c = static_cast<TO*>(C);
-  if constexpr (std::is_same<TI, float>::value && std::is_same<TO, float>::value) {
-    if (vec) {
+  constexpr bool chained = std::is_same<TI, float>::value && std::is_same<TO, float>::value;
+  if constexpr (chained) {
+    // (a grid has 65,535 blocks of rows at most: more rows than these kernels' blocks cover go to the wider ones)
+    auto fits = [&](int rows) { return ((long long)M + rows - 1) / rows <= 65535; };
+    if (vec && fits(TILE)) {
       // Both kernels below deal the chains of k to threads, one for few rows, one for many; whichever the
       // estimate says ends sooner.  The first does about 13.8 TFLOP/s where it fills the device; the other takes
       // 41 us per 1,024 k where a multiprocessor has one block, 36 us a block where it has more (measured: 4096 x 1024 by
@@ -460,7 +463,7 @@ int launch(const void* A, const void* W, const void* bias, void* C, int M, int N
       const double few = 1e-12 / 13.8 * 2.0 * M * N * K * 1e6;
       const long long tiles = (long long)((N + TILE - 1) / TILE) * ((M + TILE - 1) / TILE);
       const double many = K / 1024.0 * (tiles <= 148 ? 41.0 : 36.0 * ((tiles + 147) / 148));
-      if (M > GEMV_WIDTH && many < few) return launch_chains(a, w, b, c, M, N, K, lda, ldw, ldc, constant_w, stream);
+      if (M > GEMV_WIDTH && (many < few || !fits(GEMV_WIDTH))) return launch_chains(a, w, b, c, M, N, K, lda, ldw, ldc, constant_w, stream);
       // As many rows of A to a block as leave a block for nearly every multiprocessor: they share the reads of W.
       const int chains = (K + SUM_BLOCK - 1) / SUM_BLOCK;
       int cs = 1;
@@ -479,8 +482,13 @@ int launch(const void* A, const void* W, const void* bias, void* C, int M, int N
     else TS_LAUNCH("gemm_simt", (gemm_nt_kernel<TI, TO, 128, 128, 8, 8, false>), grid, THREADS, 0, stream, a, w, b, c, M, N, K, lda, ldw, ldc);
   } else {
     dim3 grid((N + 63) / 64, (M + 63) / 64);
-    if (vec) TS_LAUNCH("gemm_simt", (gemm_nt_kernel<TI, TO, 64, 64, 4, 4, true>), grid, THREADS, 0, stream, a, w, b, c, M, N, K, lda, ldw, ldc);
-    else TS_LAUNCH("gemm_simt", (gemm_nt_kernel<TI, TO, 64, 64, 4, 4, false>), grid, THREADS, 0, stream, a, w, b, c, M, N, K, lda, ldw, ldc);
+    if constexpr (!chained) {       // (aligned float operands of so few rows never come here)
+      if (vec) {
+        TS_LAUNCH("gemm_simt", (gemm_nt_kernel<TI, TO, 64, 64, 4, 4, true>), grid, THREADS, 0, stream, a, w, b, c, M, N, K, lda, ldw, ldc);
+        return 0;
+      }
+    }
+    TS_LAUNCH("gemm_simt", (gemm_nt_kernel<TI, TO, 64, 64, 4, 4, false>), grid, THREADS, 0, stream, a, w, b, c, M, N, K, lda, ldw, ldc);
   }
   return 0;
 }
