@@ -7,7 +7,11 @@
 // accumulator D[128 weight rows x TILE_T tokens] lives in tensor memory.  Per 64-wide slice of K
 // one thread issues two TMA loads (W tile 128 x 64, x tile TILE_T x 64, 128-byte swizzle) into a
 // ring of shared-memory stages guarded by mbarriers; one thread of another warp issues the slice's
-// four tcgen05.mma (K = 16) and commits the stage back to the loader.
+// four tcgen05.mma (K = 16), into four accumulators that the epilogue adds up, and commits the
+// stage back to the loader.  (The tensor core cuts a sum's low bits off at every tcgen05.mma: in one
+// accumulator, four times the steps, the error against 64 bits is 4 to 6.5 times as large.  38,000 x 4096
+// by 64 tokens: 1.0e-6 with four, 4.4e-6 with one; operands all positive 2.1e-6 and 13.7e-6.  Adding
+// them up costs nothing that shows for up to 32 tokens, 0.3 us for 33 to 64.)
 //
 // Shapes with few row tiles (N = 4096: 32 tiles for 148 SMs) are also cut along K.  Every block
 // then stores its partial tile to scratch and bumps the tile's counter; the block that arrives
@@ -94,13 +98,51 @@ __host__ __device__ constexpr uint32_t instr_desc(int tile_t) {
   return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(tile_t >> 3) << 17) |
          (static_cast<uint32_t>(TILE_N >> 4) << 24);
 }
+// Accumulators: step k of a stage goes to number k % ACCS, TILE_T columns on each.  (Two blocks share an SM and
+// trigger their successors before they allocate, so a block may take no more than half of the tensor memory: a
+// block of the successor could otherwise hold what a block that it waits for still needs.)
+template <int TILE_T> struct Accs { static constexpr int N = TILE_T <= 64 ? K_STEPS : 2; };
+
+// eight columns of the sums
+template <int TILE_T>
+__device__ __forceinline__ void tmem_load8_sum(uint32_t addr, float (&v)[8]) {
+  if constexpr (Accs<TILE_T>::N == 2) {
+    float u[8];
+    tmem_load8(addr, v);
+    tmem_load8(addr + TILE_T, u);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] += u[i];
+    return;
+  }
+  static_assert(K_STEPS == 4, "four accumulators are read at once");
+  uint32_t r[K_STEPS][8];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%32];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%33];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16,%17,%18,%19,%20,%21,%22,%23}, [%34];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%24,%25,%26,%27,%28,%29,%30,%31}, [%35];\n\t"
+      "tcgen05.wait::ld.sync.aligned;\n"
+      : "=r"(r[0][0]), "=r"(r[0][1]), "=r"(r[0][2]), "=r"(r[0][3]), "=r"(r[0][4]), "=r"(r[0][5]), "=r"(r[0][6]), "=r"(r[0][7]),
+        "=r"(r[1][0]), "=r"(r[1][1]), "=r"(r[1][2]), "=r"(r[1][3]), "=r"(r[1][4]), "=r"(r[1][5]), "=r"(r[1][6]), "=r"(r[1][7]),
+        "=r"(r[2][0]), "=r"(r[2][1]), "=r"(r[2][2]), "=r"(r[2][3]), "=r"(r[2][4]), "=r"(r[2][5]), "=r"(r[2][6]), "=r"(r[2][7]),
+        "=r"(r[3][0]), "=r"(r[3][1]), "=r"(r[3][2]), "=r"(r[3][3]), "=r"(r[3][4]), "=r"(r[3][5]), "=r"(r[3][6]), "=r"(r[3][7])
+      : "r"(addr), "r"(addr + TILE_T), "r"(addr + 2 * TILE_T), "r"(addr + 3 * TILE_T)
+      : "memory");
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    v[i] = __uint_as_float(r[0][i]);
+#pragma unroll
+    for (int a = 1; a < K_STEPS; ++a) v[i] += __uint_as_float(r[a][i]);
+  }
+}
+
 template <int TILE_T> struct Cfg {
   static constexpr int X_STAGE_BYTES = TILE_T * BK * 2;
   static constexpr int STAGE_BYTES = W_STAGE_BYTES + X_STAGE_BYTES;
   // two blocks share an SM: the ring and the barriers of a block stay below 113 KB
   static constexpr int RING = TS_GEMM_RING_KB * 1024;
   static constexpr int STAGES = RING / STAGE_BYTES < 2 ? 2 : (RING / STAGE_BYTES > 8 ? 8 : RING / STAGE_BYTES);
-  static constexpr int TMEM_COLS = TILE_T < 32 ? 32 : TILE_T;
+  static constexpr int TMEM_COLS = Accs<TILE_T>::N * TILE_T;
   static constexpr size_t SMEM = 1024 + (size_t)STAGES * STAGE_BYTES + 256;
 };
 
@@ -209,7 +251,7 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
       // one descriptor per operand and stage; a K step of 16 is 32 bytes = 2 address units on
       const uint64_t ad = desc0 + (uint64_t)s * (C::STAGE_BYTES >> 4), bd = ad + (W_STAGE_BYTES >> 4);
 #pragma unroll
-      for (int k = 0; k < K_STEPS; ++k) umma(tmem_base, ad + 2 * k, bd + 2 * k, idesc, i > 0 || k > 0 ? 1u : 0u);
+      for (int k = 0; k < K_STEPS; ++k) umma(tmem_base + k % Accs<TILE_T>::N * TILE_T, ad + 2 * k, bd + 2 * k, idesc, i > 0 || k >= Accs<TILE_T>::N ? 1u : 0u);
       tcgen05_commit(smem_u32(&empty[s]));
     }
     if (ok && nkb > 0) tcgen05_commit(smem_u32(accum));
@@ -249,7 +291,7 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
 #pragma unroll 1
     for (int c = 0; c < TILE_T; c += 8) {
       float v[8];
-      if (have) tmem_load8(taddr + c, v);
+      if (have) tmem_load8_sum<TILE_T>(taddr + c, v);
       else {
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = 0.f;
@@ -307,7 +349,7 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
 #pragma unroll 1
       for (int c = 0; c < TILE_T; c += 8) {
         float v[8];
-        if (have) tmem_load8(taddr + c, v);
+        if (have) tmem_load8_sum<TILE_T>(taddr + c, v);
         else {
 #pragma unroll
           for (int i = 0; i < 8; ++i) v[i] = 0.f;
@@ -350,7 +392,7 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
 #pragma unroll 1
     for (int c = 0; c < TILE_T; c += 8) {
       float v[8];
-      if (have) tmem_load8(taddr + c, v);
+      if (have) tmem_load8_sum<TILE_T>(taddr + c, v);
       else {
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = 0.f;
@@ -378,7 +420,7 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
 #pragma unroll 1
     for (int c = 0; c < TILE_T; c += 8) {
       float v[8];
-      if (have) tmem_load8(taddr + c, v);
+      if (have) tmem_load8_sum<TILE_T>(taddr + c, v);
       else {
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = 0.f;
