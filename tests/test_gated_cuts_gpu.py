@@ -32,19 +32,24 @@ def test_gated_product_of_few_row_tiles(M, N, K, activation, limit):
     assert ops.gemm_tcgen05_error() == 0
 
 
-@pytest.mark.parametrize("M", [1, 5, 16])
+@pytest.mark.parametrize("M", [1, 5, 16, 17, 40, 64])
 def test_rows_without_their_norm_factor(M):
+    """Up to 16 rows from the product for few tokens; more (which only the paired product makes) are normalised first."""
     from tinyserve_b200.kernels import ops
     g = torch.Generator().manual_seed(M)
     x, o = torch.randn(M, 1024, generator=g).bfloat16().cuda(), (torch.randn(1024, 1024, generator=g) * 0.03).bfloat16().cuda()
     w = (torch.randn(768, 1024, generator=g) * 0.03).bfloat16().cuda()
     norm = (1 + 0.1 * torch.randn(1024, generator=g)).bfloat16().cuda()
     residual = torch.randn(M, 1024, generator=g).cuda()
-    rows = ops.add_rmsnorm(ops.linear(x, o, allow_pending=True), residual, norm, 1e-6, torch.bfloat16, scaled_ok=True)
+    rows = ops.add_rmsnorm(ops.PendingProduct(x, o, wide=M > 16), residual, norm, 1e-6, torch.bfloat16, scaled_ok=True)
     assert isinstance(rows, ops.ScaledRows)
     got = ops.gated_linear(rows, w, "silu", ops.GATED_BLOCK).double()
     h = rows.data.double() * torch.rsqrt(residual.double().square().mean(1, keepdim=True) + 1e-6)
     blocks = w.double().view(6, 2, 64, 1024)
     gate, up = ((h @ blocks[:, i].reshape(384, 1024).T) for i in (0, 1))
     want = torch.nn.functional.silu(gate) * up
-    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()
+    if M > 16:
+        # five roundings to bfloat16 of 2^-9 at most each: the normalised rows' (in gate and in up), gate's, up's, the result's
+        assert (got - want).norm() <= 5 * 2.0 ** -9 * want.norm()
+    else:
+        assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()

@@ -735,6 +735,7 @@ def gated_linear(x, weight, activation="silu", block=0, limit=0.0, constant_weig
         return _linear_pair(rows, weight, gated=code + 1, limit=limit, scale=x if rows is not x else None)
     if (block == GATED_BLOCK and N % 128 == 0 and isinstance(rows, torch.Tensor)
             and rows.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and _tcgen05_ok(rows, weight)
+            and (rows is x or rows.shape[0] <= FUSED_MAX_TOKENS)          # (norm factors come for so many rows)
             and (rows.shape[0] <= GATED_MAX_TOKENS // 2 or (rows.shape[0] <= GATED_MAX_TOKENS and N <= 2 * num_sms() * 128))):
         _cuda(rows, weight)
         # (a product of few row tiles is cut along K inside clusters: 6144 x 1024 with its
