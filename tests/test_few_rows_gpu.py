@@ -141,6 +141,29 @@ def test_sampled_rows_do_not_depend_on_the_blocks_that_share_them(V, B):
             assert plain_sample(row, float(temp[i]), int(ks[i]), float(ps[i]))[int(together[i])]
 
 
+# the longest row that one block reads for its maximum, and one more; the fewest tokens that get a cluster; odd rows;
+# numbers of rows around those whose clusters of eight, four and two have a place at once
+@pytest.mark.parametrize("V", [8188, 8192, 32768, 32769, 50257])
+@pytest.mark.parametrize("B", [1, 14, 15, 16, 17, 18, 19, 33, 37, 38, 74, 75, 148, 149])
+def test_maximum_of_rows_by_any_number_of_blocks(V, B):
+    from tinyserve_b200.kernels import ops
+    g = torch.Generator(device="cuda").manual_seed(V + B)
+    x = torch.randn(B, V, generator=g, device="cuda")
+    at = torch.randint(V, (B,), generator=g, device="cuda")
+    x[torch.arange(B), at] = 9.0
+    x[:, V - 1] = 9.0                                                    # a tie: the lower index wins
+    zero, one = torch.zeros(B, device="cuda"), torch.full((B,), 1e-3, device="cuda")
+    streams, steps = torch.arange(B, device="cuda"), torch.zeros(B, dtype=torch.int32, device="cuda")
+    assert torch.equal(ops.sample(x, zero, streams, steps, 5), at.int())
+    x[:, V - 1] = 0.0
+    x[torch.arange(B), at] = 9.0
+    # at so low a temperature the noise cannot lift another token over the largest
+    assert torch.equal(ops.sample(x, one, streams, steps, 5), at.int())
+    mixed = torch.where(streams % 2 == 0, zero, one)
+    keep = torch.full((B,), 3, dtype=torch.int32, device="cuda")
+    assert torch.equal(ops.sample(x, mixed, streams, steps, 5, top_k=keep, top_p=torch.full((B,), 0.5, device="cuda")), at.int())
+
+
 def test_rows_of_infinities_and_nans():
     from tinyserve_b200.kernels import ops
     x = torch.full((4, 20000), -float("inf")).cuda()

@@ -1,9 +1,8 @@
-// Sampling from 32-bit logits, everything on the device.  A row is read by a cluster of up to eight
-// blocks, a range of the vocabulary each, which combine their maxima and histograms through
-// distributed shared memory.  (A row of 151,936 logits is 600 KB: one block takes 18 us to read
-// it, and up to nine passes over it, most of whose histogram updates meet in a few bins, took 2.1 ms
-// with top-k and top-p.)  All that blocks combine is a maximum or an integer sum, so the result does
-// not depend on how many blocks share a row.
+// Sampling from 32-bit logits, everything on the device.  A row is read by one block or by a cluster of up
+// to eight, a range of the vocabulary each, which combine their maxima and histograms through
+// distributed shared memory.  All that blocks combine is a maximum or an integer sum, so the result does
+// not depend on how many blocks share a row.  One row of 151,936 logits (600 KB) by one block / by eight:
+// greedy 9.1 / 4.8 us, with a temperature 65 / 12, with top-p 322 / 62, with top-k and top-p 463 / 90.
 //
 //   temperature == 0           -> argmax (serve.py:1521-1522)
 //   temperature > 0            -> x = logit / temperature, optional top-k (keep the k largest),
@@ -18,6 +17,8 @@
 // (v / 4, step, stream_lo, stream_hi); u = ((word >> 9) + 0.5) * 2^-23; g = -log(-log(u)).
 // tinyserve draws from torch's global generator instead (serve.py:1546, tinykernels.py:1866).
 // Ties go to the lowest token id.  Top-k keeps every token that ties with the k-th largest.
+#include <atomic>
+
 #include "common.cuh"
 
 TS_DEFINE_LAST_ERROR()
@@ -25,6 +26,9 @@ TS_DEFINE_LAST_ERROR()
 namespace {
 
 constexpr int THREADS = 1024;
+// The longest row of which one block finds the maximum as fast as a cluster (16,384 / 32,000 / 65,536 tokens: 2.6 / 3.6 /
+// 4.8 us by one block, 3.6 / 3.9 / 4.1 by the best of two, four and eight).
+constexpr int GREEDY_ALONE = 32768;
 
 __device__ __forceinline__ void philox4x32_10(uint32_t (&c)[4], uint32_t k0, uint32_t k1) {
 #pragma unroll
@@ -140,12 +144,21 @@ __device__ __forceinline__ void hist_add(unsigned long long* hist, bool on, uint
 }
 
 // Sums of the cluster's histograms into h.all (every block for itself); called by all threads.
+template <bool CLUSTER>
 __device__ void hist_combine(Histogram& h, int buf, uint32_t blocks) {
-  cluster_arrive();
-  cluster_wait();
+  if constexpr (CLUSTER) {
+    cluster_arrive();
+    cluster_wait();
+  } else {
+    __syncthreads();
+  }
   if (threadIdx.x < 256) {
     unsigned long long sum = 0;
-    for (uint32_t r = 0; r < blocks; ++r) sum += cluster_load_u64(&h.own[buf][threadIdx.x], r);
+    if constexpr (CLUSTER) {
+      for (uint32_t r = 0; r < blocks; ++r) sum += cluster_load_u64(&h.own[buf][threadIdx.x], r);
+    } else {
+      sum = h.own[buf][threadIdx.x];
+    }
     h.all[threadIdx.x] = sum;
   }
   __syncthreads();
@@ -198,6 +211,9 @@ struct SampleArgs {
   const int* slots;
 };
 
+// CLUSTER false: a row is one block's, which then has nothing to wait for (a cluster of one costs 0.8 to 1 us:
+// 512 tokens greedy 1.8 us, 2.8 as a cluster).
+template <bool CLUSTER>
 __global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
   __shared__ Best best_scratch[32];
   __shared__ float f_scratch[33];
@@ -206,13 +222,14 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
 
   pdl_trigger();
   pdl_wait();
-  const uint32_t blocks = cluster_blocks(), rank = cluster_rank();
+  const uint32_t blocks = CLUSTER ? cluster_blocks() : 1u, rank = CLUSTER ? cluster_rank() : 0u;
   const int row = blockIdx.x / blocks;
   const float* x = a.logits + (size_t)row * a.row_stride;
   const int V = a.vocab;
   // this block's range of the vocabulary, in whole groups of four tokens (one Philox call each)
   const int per = ((V + 3) / 4 + blocks - 1) / blocks * 4;
-  const int v0 = min(V, (int)rank * per), v1 = min(V, v0 + per);
+  int v0 = min(V, (int)rank * per), v1 = min(V, v0 + per);
+  bool alone = false;       // the first block has the row to itself
   const bool aligned = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
   const float temp = a.temperature[row];
 
@@ -229,26 +246,49 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
   // the best of all blocks' tokens; the first block writes it
   auto finish = [&](Best b) {
     b = block_best(b, best_scratch);
-    if (threadIdx.x == 0) shared_word = (unsigned long long)__float_as_uint(b.value) << 32 | (uint32_t)b.index;
-    cluster_arrive();
-    cluster_wait();
+    if (CLUSTER && !alone) {
+      if (threadIdx.x == 0) shared_word = (unsigned long long)__float_as_uint(b.value) << 32 | (uint32_t)b.index;
+      cluster_arrive();
+      cluster_wait();
+      if (rank == 0 && threadIdx.x == 0)
+        for (uint32_t r = 1; r < blocks; ++r) {
+          const unsigned long long w = cluster_load_u64(&shared_word, r);
+          b = better(b, Best{__uint_as_float((uint32_t)(w >> 32)), (int)(uint32_t)w});
+        }
+    }
     if (rank == 0 && threadIdx.x == 0) {
-      for (uint32_t r = 1; r < blocks; ++r) {
-        const unsigned long long w = cluster_load_u64(&shared_word, r);
-        b = better(b, Best{__uint_as_float((uint32_t)(w >> 32)), (int)(uint32_t)w});
-      }
       a.out[row] = b.index;
       if (a.slot_tokens) a.slot_tokens[a.slots[row]] = b.index;
     }
-    // no block leaves while the first may still read its shared memory
-    cluster_arrive();
-    cluster_wait();
+    if (CLUSTER && !alone) {
+      // no block leaves while the first may still read its shared memory
+      cluster_arrive();
+      cluster_wait();
+    }
   };
 
   if (!(temp > 0.f)) {   // greedy
+    // a short row is the first block's (nobody has met in the cluster so far)
+    alone = CLUSTER && V <= GREEDY_ALONE;
+    if (alone) {
+      if (rank > 0) return;
+      v0 = 0;
+      v1 = V;
+    }
     Best b{-INFINITY, 0x7fffffff};
-#pragma unroll 4
-    for (int base = v0 + threadIdx.x * 4; base < v1; base += THREADS * 4) {
+    int base = v0 + threadIdx.x * 4;
+    // four loads in flight per thread
+    for (; aligned && base < v1 - 3 * THREADS * 4 - 3; base += 4 * THREADS * 4) {
+      float4 t[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) t[i] = *reinterpret_cast<const float4*>(x + base + i * THREADS * 4);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int v = base + i * THREADS * 4;
+        b = better(better(better(better(b, Best{t[i].x, v}), Best{t[i].y, v + 1}), Best{t[i].z, v + 2}), Best{t[i].w, v + 3});
+      }
+    }
+    for (; base < v1; base += THREADS * 4) {
       float q[4];
       load4(base, q);
 #pragma unroll
@@ -281,7 +321,7 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
           hist_add(h.own[buf], v + j < v1 && (key & mask) == prefix, (key >> (8 * byte)) & 255u, 1ull, byte == 3);
         }
       }
-      hist_combine(h, buf, blocks);
+      hist_combine<CLUSTER>(h, buf, blocks);
       hist_choose(h, 0ull, remaining, false);
       prefix |= h.chosen << (8 * byte);
       remaining -= h.before;
@@ -304,10 +344,12 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
       }
     }
     mx = block_max_f(mx, f_scratch);
-    if (threadIdx.x == 0) shared_word = __float_as_uint(mx);
-    cluster_arrive();
-    cluster_wait();
-    for (uint32_t r = 0; r < blocks; ++r) mx = fmaxf(mx, __uint_as_float((uint32_t)cluster_load_u64(&shared_word, r)));
+    if constexpr (CLUSTER) {
+      if (threadIdx.x == 0) shared_word = __float_as_uint(mx);
+      cluster_arrive();
+      cluster_wait();
+      for (uint32_t r = 0; r < blocks; ++r) mx = fmaxf(mx, __uint_as_float((uint32_t)cluster_load_u64(&shared_word, r)));
+    }
     uint32_t prefix = 0, mask = 0;
     unsigned long long above = 0, limit = 0;
     for (int byte = 3; byte >= 0; --byte, buf ^= 1) {
@@ -326,7 +368,7 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
           hist_add(h.own[buf], on && w != 0ull, (key >> (8 * byte)) & 255u, w, byte == 3);
         }
       }
-      hist_combine(h, buf, blocks);
+      hist_combine<CLUSTER>(h, buf, blocks);
       if (byte == 3) {
         unsigned long long total = 0;
         for (int b = 0; b < 256; ++b) total += h.all[b];
@@ -382,6 +424,28 @@ __global__ void repetition_penalty_kernel(float* logits, long long row_stride, i
   }
 }
 
+// how many clusters of this many blocks the current device holds at once (0 if it does not say)
+int max_clusters(int blocks) {
+  constexpr int DEVICES = 64;
+  static std::atomic<int> known[DEVICES][9];       // the number + 1
+  int device = 0, n = 0;
+  if (cudaGetDevice(&device) != cudaSuccess) return 0;
+  if (device < DEVICES && (n = known[device][blocks].load(std::memory_order_relaxed)) > 0) return n - 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(THREADS);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = blocks;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, sample_kernel<true>, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
+  if (device < DEVICES) known[device][blocks].store(n + 1, std::memory_order_relaxed);
+  return n;
+}
+
 }  // namespace
 
 TS_EXPORT int ts_sample(const float* logits, long long row_stride, int num_rows, int vocab,
@@ -394,13 +458,17 @@ TS_EXPORT int ts_sample(const float* logits, long long row_stride, int num_rows,
   TS_REQUIRE(temperature && stream_ids && steps && out, "sample: missing argument");
   TS_REQUIRE((slot_tokens == nullptr) == (slots == nullptr), "sample: slot_tokens and slots come together");
   SampleArgs a{logits, row_stride, vocab, temperature, top_k, top_p, stream_ids, steps, seed, out, slot_tokens, slots};
-  // Blocks per row: as many as fill the device's 2 x 148 places for blocks of this size, eight at most
-  // (the portable cluster), a range of at least 4,096 tokens each: below, a cluster barrier costs more
-  // than the tokens it saves reading.
+  // Blocks per row: as many (1, 2, 4 or 8, the portable cluster) as leave every row's cluster a place at once (a second
+  // wave doubles the time: 16 rows of 151,936 tokens with top-k and top-p 147 us in clusters of four, 178 in
+  // clusters of eight, of which 15 fit), a range of at least 2,048 tokens each and no cluster below 8,192
+  // (with top-k and top-p 8,192 tokens 40 / 33 us by one block / by four, 4,096 tokens 29 / 32 by one / by two).
   int blocks = 1;
-  while (blocks < 8 && vocab / (2 * blocks) >= 4096 && (long long)num_rows * 2 * blocks <= 296) blocks *= 2;
-  TS_REQUIRE((long long)num_rows * blocks <= 2147483647LL, "sample: too many rows");
-  cudaError_t e = ts_launch_cluster(sample_kernel, dim3(num_rows * blocks), dim3(THREADS), 0, stream, dim3(blocks, 1, 1), a);
+  while (blocks < 8 && vocab >= 8192 && vocab / (2 * blocks) >= 2048 && num_rows <= max_clusters(2 * blocks)) blocks *= 2;
+  if (blocks == 1) {
+    TS_LAUNCH("sample", sample_kernel<false>, num_rows, THREADS, 0, stream, a);
+    return 0;
+  }
+  cudaError_t e = ts_launch_cluster(sample_kernel<true>, dim3(num_rows * blocks), dim3(THREADS), 0, stream, dim3(blocks, 1, 1), a);
   if (e != cudaSuccess) return ts_fail("sample: %s", cudaGetErrorString(e));
   return 0;
 }
