@@ -1,4 +1,4 @@
-"""How close the 32-bit sums of the bfloat16 product for few tokens are to 64 bits."""
+"""The 32-bit sums of the bfloat16 product for few tokens: how close they are to 64 bits, and the order of their parts."""
 import pytest
 import torch
 
@@ -19,4 +19,22 @@ def test_sums_of_one_sign(M, K):
     w = torch.rand(N, K, generator=g, device="cuda").bfloat16()
     out, want = ops.linear(x, w, out_float32=True).double(), x.double() @ w.double().T
     assert ((out - want).norm() / want.norm()).item() <= K / 64 * 2.0 ** -24
+    assert ops.gemm_tcgen05_error() == 0
+
+
+@pytest.mark.parametrize("splits", [2, 3, 4, 5, 8, 9, 16])
+@pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 64, 100])
+def test_parts_add_up_in_order(M, splits):
+    """The block that arrives last adds the parts in the order of K, several at a time: the same bits as one by one."""
+    from tinyserve_b200.kernels import ops
+    N, K = 640, 16 * 64
+    g = torch.Generator(device="cuda").manual_seed(M + splits)
+    x, w = (torch.randn(r, K, generator=g, device="cuda").bfloat16() for r in (M, N))
+    parts = ops._linear_tcgen05(x, w, False, splits=splits, partials_only=True)
+    tile = ops._tile_t(M)
+    buffer = parts.data.view(splits, N // 128, tile, 128)
+    want = torch.zeros(M, N, device="cuda")
+    for s in range(splits):
+        want += buffer[s].permute(1, 0, 2).reshape(tile, N)[:M]
+    assert torch.equal(ops._linear_tcgen05(x, w, True, splits=splits), want)
     assert ops.gemm_tcgen05_error() == 0

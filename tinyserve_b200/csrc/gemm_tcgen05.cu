@@ -147,7 +147,7 @@ template <int TILE_T> struct Cfg {
 };
 
 template <int TILE_T, typename MAPS>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, 2)
 gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmParams p) {
   using C = Cfg<TILE_T>;
   constexpr bool MULTI = sizeof(MAPS) != sizeof(Maps1);
@@ -447,20 +447,30 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
         const VecParam bias = beside ? p.seg[which].bias : p.bias;
         const int ldc = beside ? p.seg[which].ldc : p.ldc, out_f32 = beside ? p.seg[which].out_f32 : p.out_f32;
         const float bn = (bias.ptr != nullptr && n < N) ? bias[n] : 0.f;
-        // eight columns at a time, so that eight chains of loads are in flight per thread
+        // eight columns of four parts at a time, so that up to 32 loads are in flight per thread (a part at a time a
+        // block waits once per part: 1024 x 3072 by 32 tokens, eight parts, 29.1 us, as it is 11.8)
+        constexpr int COLS = 8, PARTS = 4;
 #pragma unroll 1
-        for (int c0 = 0; c0 < TILE_T && t0 + c0 < p.M; c0 += 8) {
-          float sum[8];
+        for (int c0 = 0; c0 < TILE_T && t0 + c0 < p.M; c0 += COLS) {
+          float sum[COLS];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) sum[i] = bn;
-          for (int s = 0; s < p.splits; ++s) {
-            const float* src = base + s * split_stride + c0 * TILE_N + warp * 32 + lane;
+          for (int i = 0; i < COLS; ++i) sum[i] = bn;
+#pragma unroll 1
+          for (int s0 = 0; s0 < p.splits; s0 += PARTS) {
+            const float* src = base + s0 * split_stride + c0 * TILE_N + warp * 32 + lane;
+            float part[PARTS][COLS];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) sum[i] += __ldcg(src + i * TILE_N);
+            for (int s = 0; s < PARTS; ++s)
+#pragma unroll
+              for (int i = 0; i < COLS; ++i) part[s][i] = s0 + s < p.splits ? __ldcg(src + s * split_stride + i * TILE_N) : 0.f;
+#pragma unroll
+            for (int s = 0; s < PARTS; ++s)
+#pragma unroll
+              for (int i = 0; i < COLS; ++i) sum[i] += part[s][i];
           }
           if (n < N) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < COLS; ++i) {
               const int m = t0 + c0 + i;
               if (m < p.M) {
                 const float y = plain_value(sum[i], p.out_act);
