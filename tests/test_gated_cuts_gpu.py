@@ -32,6 +32,21 @@ def test_gated_product_of_few_row_tiles(M, N, K, activation, limit):
     assert ops.gemm_tcgen05_error() == 0
 
 
+@pytest.mark.parametrize("splits", [1, 2, 3, 4, 5, 6, 7, 8])
+@pytest.mark.parametrize("M", [1, 16, 31, 64])
+def test_any_number_of_cuts(M, splits):
+    """Cuts of unequal length, and one without a slice (5 cuts of 16 slices)."""
+    from tinyserve_b200.kernels import ops
+    g = torch.Generator().manual_seed(M)
+    x, w = torch.randn(M, 1024, generator=g).bfloat16().cuda(), (torch.randn(640, 1024, generator=g) / 32).bfloat16().cuda()
+    blocks = w.double().view(5, 2, 64, 1024)
+    gate, up = ((x.double() @ blocks[:, i].reshape(320, 1024).T) for i in (0, 1))
+    want = torch.nn.functional.silu(gate) * up
+    got = ops._linear_tcgen05(x, w, False, splits=splits, gated=ops.ACTIVATIONS["silu"] + 1)
+    assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 4e-6).all()
+    assert ops.gemm_tcgen05_error() == 0
+
+
 @pytest.mark.parametrize("M", [1, 5, 16, 17, 40, 64])
 def test_rows_without_their_norm_factor(M):
     """Up to 16 rows from the product for few tokens; more (which only the paired product makes) are normalised first."""

@@ -341,7 +341,7 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
   } else if (p.gated_act != 0) {
     // gated form: the sums of the tile (with K cuts, a cluster of them as in the residual form: of the tokens rank,
     // rank + splits, ..) in shared memory, where a thread finds its gate and its up row; neighbouring threads take
-    // neighbouring columns.  (A thread that kept its row's 64 sums in registers and only half of the threads at
+    // neighbouring pairs of columns.  (A thread that kept its row's 64 sums in registers and only half of the threads at
     // work took 23 us of a product of 64 tokens.)
     if constexpr (TILE_T <= 64) {
       float* red = reinterpret_cast<float*>(smem);               // [TILE_T][TILE_N] (the ring is idle), read by the cluster
@@ -375,12 +375,15 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
         cluster_arrive();
       }
       __syncthreads();
-      const int col = threadIdx.x & 63;
+      const int col = (threadIdx.x & 31) * 2;
 #pragma unroll 4
-      for (int j = split + p.splits * (threadIdx.x >> 6); j < TILE_T; j += 2 * p.splits) {
-        if (t0 + j < p.M)
-          static_cast<bf16*>(p.out)[(size_t)(t0 + j) * p.ldc + n_tile * 64 + col] =
-              __float2bfloat16_rn(gated_value(sums[j * TILE_N + col], sums[j * TILE_N + 64 + col], p.gated_act - 1, p.gated_limit));
+      for (int j = split + p.splits * (threadIdx.x >> 5); j < TILE_T; j += 4 * p.splits) {
+        if (t0 + j < p.M) {
+          const float2 g = *reinterpret_cast<const float2*>(sums + j * TILE_N + col);
+          const float2 u = *reinterpret_cast<const float2*>(sums + j * TILE_N + 64 + col);
+          *reinterpret_cast<__nv_bfloat162*>(static_cast<bf16*>(p.out) + (size_t)(t0 + j) * p.ldc + n_tile * 64 + col) =
+              __floats2bfloat162_rn(gated_value(g.x, u.x, p.gated_act - 1, p.gated_limit), gated_value(g.y, u.y, p.gated_act - 1, p.gated_limit));
+        }
       }
       if (p.splits > 1) cluster_wait();
     }
@@ -525,6 +528,35 @@ int launch(const MAPS& maps, const GemmParams& p, dim3 grid, cudaStream_t stream
   return 0;
 }
 
+// The device counts one block of this kernel a multiprocessor; as many share one as their shared memory allows
+// (gated product of one token: 64 row tiles in clusters of two / four 9.1 / 7.9 us, 72 in clusters of three / four, of
+// which 66 fit, 14.4 / 19.3).
+template <int TILE_T>
+int max_clusters(int blocks) {
+  int n = 0, counted = 0, device = 0, shared = 0, reserved = 0;
+  cudaFuncAttributes attributes;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(1, 1, blocks);
+  cfg.blockDim = dim3(THREADS);
+  cfg.dynamicSmemBytes = Cfg<TILE_T>::SMEM;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = blocks;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaFuncSetAttribute(gemm_wx_kernel<TILE_T, Maps1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<TILE_T>::SMEM) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, gemm_wx_kernel<TILE_T, Maps1>, &cfg) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&counted, gemm_wx_kernel<TILE_T, Maps1>, THREADS, Cfg<TILE_T>::SMEM) != cudaSuccess ||
+      cudaFuncGetAttributes(&attributes, gemm_wx_kernel<TILE_T, Maps1>) != cudaSuccess || cudaGetDevice(&device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&shared, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, device) != cudaSuccess || counted < 1) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n / counted * (shared / (int)(Cfg<TILE_T>::SMEM + attributes.sharedSizeBytes + reserved));
+}
+
 int tile_tokens(int M) { return M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128)); }
 
 // the kernels with several operand pairs are built for up to 64 tokens
@@ -543,6 +575,16 @@ TS_EXPORT int ts_gemm_tcgen05_error() {
   int flag = 0;
   if (cudaMemcpyFromSymbol(&flag, g_error_flag, sizeof(int)) != cudaSuccess) return -1;
   return flag;
+}
+
+// How many clusters of `splits` blocks of the product of M tokens the current device holds at once (0 if it does not say).
+TS_EXPORT int ts_gemm_tcgen05_max_clusters(int M, int splits) {
+  switch (tile_tokens(M)) {
+    case 16: return max_clusters<16>(splits);
+    case 32: return max_clusters<32>(splits);
+    case 64: return max_clusters<64>(splits);
+    default: return max_clusters<128>(splits);
+  }
 }
 
 // scratch floats that `splits` > 1 needs
@@ -597,6 +639,7 @@ TS_EXPORT int ts_gemm_tcgen05_fused(const void* x, const void* w, void* out, int
              "gemm_tcgen05: the scaled-rows and residual forms take up to %d tokens, got %d", SUMSQ_STRIDE, M);
   TS_REQUIRE(gated_act == 0 || (gated_act <= ACT_COUNT && (gated_act - 1 != ACT_BOUNDED_SWISH || gated_limit > 0.f) && M <= 64 && splits <= 8 && out && !out_f32 && !residual && N % 128 == 0),
              "gemm_tcgen05: the gated form takes up to 64 tokens and 8 K cuts, a bfloat16 output and whole 128-row tiles");
+  TS_REQUIRE(gated_act == 0 || (ldc % 2 == 0 && (reinterpret_cast<uintptr_t>(out) & 3) == 0), "gemm_tcgen05: the gated form stores pairs of columns");
   TS_REQUIRE(x_sumsq == nullptr || x_tiles > 0, "gemm_tcgen05: sums of squares without their tile count");
   TS_REQUIRE(residual == nullptr || (norm_w && hprime && sumsq_out && splits <= 8),
              "gemm_tcgen05: the residual form needs the norm's weight, both outputs and at most 8 cuts");

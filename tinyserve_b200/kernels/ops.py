@@ -5,6 +5,7 @@ must live on a CUDA device and a missing compiler or library raises."""
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from ctypes import c_float, c_int, c_longlong, c_ulonglong, c_void_p
 
@@ -353,6 +354,35 @@ def gemm_splits(M, N, K, partials=False):
             splits = min(splits, 2)
     per = -(-slices // splits)
     return -(-slices // per)           # no cut without a slice
+
+
+_clusters: dict = {}
+
+
+def gemm_max_clusters(M, splits):
+    """How many clusters of ``splits`` blocks of the product of M tokens the device holds at once."""
+    key = (_tile_t(M), splits)
+    if key not in _clusters:
+        _clusters[key] = _gemm_tcgen05().ts_gemm_tcgen05_max_clusters(c_int(M), c_int(splits))
+    return _clusters[key]
+
+
+@functools.lru_cache(maxsize=4096)
+def gated_splits(M, N, K):
+    """Cuts along K of the gated product, the blocks of a cluster per row tile: the number whose estimate ends first,
+    in us.  A slice of K costs a block 0.2 and more the more blocks share the memory; the epilogue of an uncut tile
+    0.065 a token; the cuts of one 0.1 each to meet and 0.37 a token to add up, each cut its share of the tokens.
+    Only numbers whose clusters all have a place at once: 96 row tiles (12288 x 2048) of 64 tokens
+    take 32.8 us in clusters of three, of which 90 fit, 24.8 in clusters of two, 17.7 uncut; one token 14.5, 11.3
+    and 11.3; 48 row tiles (6144 x 1024) of one token 5.6 uncut, 4.6 in clusters of four, 8.3 of six."""
+    tiles, slices = -(-N // 128), -(-K // 64)
+
+    def estimate(splits):
+        epilogue = 0.065 * M if splits == 1 else 0.2 + 0.1 * splits + 0.37 * -(-M // splits)
+        return -(-slices // splits) * max(0.2, 0.15 + 0.0018 * tiles * splits) + epilogue
+
+    return min([1] + [s for s in range(2, min(slices // 2, FUSED_MAX_SPLITS) + 1) if tiles <= gemm_max_clusters(M, s)],
+               key=estimate)
 
 
 def gemm_tcgen05_error() -> int:
@@ -738,10 +768,7 @@ def gated_linear(x, weight, activation="silu", block=0, limit=0.0, constant_weig
             and (rows is x or rows.shape[0] <= FUSED_MAX_TOKENS)          # (norm factors come for so many rows)
             and (rows.shape[0] <= GATED_MAX_TOKENS // 2 or (rows.shape[0] <= GATED_MAX_TOKENS and N <= 2 * num_sms() * 128))):
         _cuda(rows, weight)
-        # (a product of few row tiles is cut along K inside clusters: 6144 x 1024 with its
-        # activation: 8.9 -> 4.6 us for one token, 11.0 -> 6.0 for 16)
-        splits = min(gemm_splits(rows.shape[0], N, K, partials=True), FUSED_MAX_SPLITS)
-        return _linear_tcgen05(rows, weight, False, splits=splits, gated=code + 1, limit=limit,
+        return _linear_tcgen05(rows, weight, False, splits=gated_splits(rows.shape[0], N, K), gated=code + 1, limit=limit,
                                scale=x if rows is not x else None)
     return gated_activation(linear(x, weight, constant_weight=constant_weight), activation, block, limit)
 
