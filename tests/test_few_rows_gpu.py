@@ -58,6 +58,20 @@ def test_product_of_few_rows_takes_leading_dimensions(M):
         torch.testing.assert_close(got.double(), xs.double() @ ws.double().T, rtol=0, atol=2e-5)
 
 
+# a short K, where the rule goes over to the tiled kernel (first and last of each line: either side of it)
+@pytest.mark.parametrize("M,N,K", [(8, 32000, 16), (40, 32000, 16), (64, 32000, 200), (65, 4096, 16), (512, 9000, 4), (4096, 64, 64), (4096, 64, 320),
+                                   (20000, 33, 16), (20000, 256, 96), (20000, 256, 200), (100000, 8, 32), (100000, 8, 260)])
+def test_rows_of_products_of_a_short_k(M, N, K):
+    from tinyserve_b200.kernels import ops
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x, w, bias = (torch.randn(*s, generator=g, device="cuda") for s in ((M, K), (N, K), (N,)))
+    out = ops.linear(x, w, bias)
+    for rows in (torch.arange(8), torch.arange(M - 8, M), torch.randint(M, (8,)), torch.randint(M, (3,))):
+        rows = rows.cuda()
+        assert torch.equal(out[rows], ops.linear(x[rows].contiguous(), w, bias))
+        torch.testing.assert_close(out[rows].double(), x[rows].double() @ w.double().T + bias.double(), rtol=0, atol=2e-4)
+
+
 @pytest.mark.parametrize("M", [65535 * 8, 65535 * 8 + 1, 65535 * 64 + 1, 65535 * 128])
 def test_products_of_very_many_rows(M):
     """A grid has 65,535 blocks of rows at most, which every kernel reaches at another number of rows."""

@@ -9,6 +9,8 @@
 // products each need to stay within 1e-4 of a float64 reference.)  Inputs may also be bfloat16
 // (products and sums still 32-bit).
 // tinyserve uses cuBLAS through nn.Linear for all of these (serve.py:828-829, 912-913, 1263).
+#include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "common.cuh"
@@ -440,6 +442,18 @@ int launch_gemv(const float* A, const float* W, const float* bias, float* C, int
   return 0;
 }
 
+// of the current device (148 if it does not say)
+int multiprocessors() {
+  constexpr int DEVICES = 64;
+  static std::atomic<int> known[DEVICES];
+  int device = 0, n = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || device >= DEVICES) return 148;
+  if ((n = known[device].load(std::memory_order_relaxed)) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || n <= 0) return 148;
+  known[device].store(n, std::memory_order_relaxed);
+  return n;
+}
+
 template <typename TI, typename TO>
 int launch(const void* A, const void* W, const void* bias, void* C, int M, int N, int K, size_t lda,
            size_t ldw, size_t ldc, bool constant_w, cudaStream_t stream) {
@@ -455,24 +469,43 @@ int launch(const void* A, const void* W, const void* bias, void* C, int M, int N
     // (a grid has 65,535 blocks of rows at most: more rows than these kernels' blocks cover go to the wider ones)
     auto fits = [&](int rows) { return ((long long)M + rows - 1) / rows <= 65535; };
     if (vec && fits(TILE)) {
-      // Both kernels below deal the chains of k to threads, one for few rows, one for many; whichever the
-      // estimate says ends sooner.  The first does about 13.8 TFLOP/s where it fills the device; the other takes
-      // 41 us per 1,024 k where a multiprocessor has one block, 36 us a block where it has more (measured: 4096 x 1024 by
-      // 48 / 64 / 128 / 512 rows 35 / 42 / 81 / 325 us against 41 / 42 / 65 / 143; 24576 x 4096 by 24 / 48 rows
-      // 309 / 609 against 422 / 425).
-      const double few = 1e-12 / 13.8 * 2.0 * M * N * K * 1e6;
-      const long long tiles = (long long)((N + TILE - 1) / TILE) * ((M + TILE - 1) / TILE);
-      const double many = K / 1024.0 * (tiles <= 148 ? 41.0 : 36.0 * ((tiles + 147) / 148));
-      if (M > GEMV_WIDTH && (many < few || !fits(GEMV_WIDTH))) return launch_chains(a, w, b, c, M, N, K, lda, ldw, ldc, constant_w, stream);
-      // As many rows of A to a block as leave a block for nearly every multiprocessor: they share the reads of W.
-      const int chains = (K + SUM_BLOCK - 1) / SUM_BLOCK;
+      // Estimates in us; the three kernels give the same bits.
+      // few: the kernel for few rows, 13.8 TFLOP/s where it fills the device, for what its blocks compute: whole groups of
+      // rows of W, whole passes of chains.  many: the chains kernel, a round of four chains in 10.25 us where a
+      // multiprocessor has one block, in 9 a block where it has more (measured: 4096 x 1024 by 48 / 64 / 128 / 512 rows
+      // 35 / 42 / 81 / 325 us against 41 / 42 / 65 / 143; 24576 x 4096 by 24 / 48 rows 309 / 609 against 422 / 425).
+      const int chains = (K + SUM_BLOCK - 1) / SUM_BLOCK, sms = multiprocessors();
       int cs = 1;
       while (cs < (1 << MAX_CHAINS_SHIFT) && cs < chains) cs *= 2;
       auto blocks = [&](int mt, int rt) { return (long long)((N + SLOTS / cs * rt - 1) / (SLOTS / cs * rt)) * ((M + mt - 1) / mt); };
-      if (M > 4 && blocks(GEMV_WIDTH, 2) >= GEMV_MIN_BLOCKS) return launch_gemv<GEMV_WIDTH, 2, 2>(a, w, b, c, M, N, K, lda, ldw, ldc, constant_w, stream);
-      if (M > 2 && blocks(4, 2) >= GEMV_MIN_BLOCKS) return launch_gemv<4, 2, 2>(a, w, b, c, M, N, K, lda, ldw, ldc, constant_w, stream);
-      if (blocks(2, 2) >= GEMV_MIN_BLOCKS) return launch_gemv<2, 2, 3>(a, w, b, c, M, N, K, lda, ldw, ldc, constant_w, stream);
-      return launch_gemv<2, 1, 3>(a, w, b, c, M, N, K, lda, ldw, ldc, constant_w, stream);
+      const int passes = (chains + cs - 1) / cs, group = SLOTS / cs * 2;
+      const double few = 2.0 * M * ((N + group - 1) / group * (double)group) * (passes * cs * SUM_BLOCK) / 13.8e6;
+      const long long tiles = (long long)((N + TILE - 1) / TILE) * ((M + TILE - 1) / TILE);
+      const double many = (chains + CHAIN_GROUPS - 1) / CHAIN_GROUPS * (tiles <= sms ? 10.25 : 9.0 * ((tiles + sms - 1) / sms));
+      // As many rows of A to a block as leave a block for nearly every multiprocessor: they share the reads of W.
+      const int width = M > 4 && blocks(GEMV_WIDTH, 2) >= GEMV_MIN_BLOCKS ? GEMV_WIDTH : M > 2 && blocks(4, 2) >= GEMV_MIN_BLOCKS ? 4 : 2;
+      const int height = width > 2 || blocks(2, 2) >= GEMV_MIN_BLOCKS ? 2 : 1;
+      const bool chained_tiles = M > GEMV_WIDTH && (many < few || !fits(GEMV_WIDTH));
+      // Both work in whole chains and rounds, the tiled kernel in slices of 16 k (2.75 us for a tile of 128 x 128; 64 x 64 up
+      // to 64 rows): the better one for a short K.  M x N x K, us, the other kernel's first: 100,000 x 8 x 16 314 / 23,
+      // 512 x 32,000 x 4 214 / 33, 20,000 x 256 x 96 83 / 54, 4,096 x 64 x 64 16 / 12, but 4,096 x 128 x 128 15 / 24.
+      const double ours = chained_tiles ? many : 1.0 + std::max(1.4 * few, 0.45 * passes * width * height);
+      const int slices = (K + BK - 1) / BK;
+      double tiled;
+      if (M > 64) {
+        const long long t = (long long)((N + 127) / 128) * ((M + 127) / 128);
+        tiled = 2.5 + 2.75 * slices * ((t + sms - 1) / sms) + (double)t / sms;
+      } else {
+        const double t = (double)((N + 63) / 64) / sms;
+        tiled = 1.0 + std::max(1.65, 0.75 * t) * slices + 0.3 * t;
+      }
+      if (tiled >= 0.95 * ours) {
+        if (chained_tiles) return launch_chains(a, w, b, c, M, N, K, lda, ldw, ldc, constant_w, stream);
+        if (width == GEMV_WIDTH) return launch_gemv<GEMV_WIDTH, 2, 2>(a, w, b, c, M, N, K, lda, ldw, ldc, constant_w, stream);
+        if (width == 4) return launch_gemv<4, 2, 2>(a, w, b, c, M, N, K, lda, ldw, ldc, constant_w, stream);
+        if (height == 2) return launch_gemv<2, 2, 3>(a, w, b, c, M, N, K, lda, ldw, ldc, constant_w, stream);
+        return launch_gemv<2, 1, 3>(a, w, b, c, M, N, K, lda, ldw, ldc, constant_w, stream);
+      }
     }
   }
   if (M > 64) {
@@ -482,13 +515,8 @@ int launch(const void* A, const void* W, const void* bias, void* C, int M, int N
     else TS_LAUNCH("gemm_simt", (gemm_nt_kernel<TI, TO, 128, 128, 8, 8, false>), grid, THREADS, 0, stream, a, w, b, c, M, N, K, lda, ldw, ldc);
   } else {
     dim3 grid((N + 63) / 64, (M + 63) / 64);
-    if constexpr (!chained) {       // (aligned float operands of so few rows never come here)
-      if (vec) {
-        TS_LAUNCH("gemm_simt", (gemm_nt_kernel<TI, TO, 64, 64, 4, 4, true>), grid, THREADS, 0, stream, a, w, b, c, M, N, K, lda, ldw, ldc);
-        return 0;
-      }
-    }
-    TS_LAUNCH("gemm_simt", (gemm_nt_kernel<TI, TO, 64, 64, 4, 4, false>), grid, THREADS, 0, stream, a, w, b, c, M, N, K, lda, ldw, ldc);
+    if (vec) TS_LAUNCH("gemm_simt", (gemm_nt_kernel<TI, TO, 64, 64, 4, 4, true>), grid, THREADS, 0, stream, a, w, b, c, M, N, K, lda, ldw, ldc);
+    else TS_LAUNCH("gemm_simt", (gemm_nt_kernel<TI, TO, 64, 64, 4, 4, false>), grid, THREADS, 0, stream, a, w, b, c, M, N, K, lda, ldw, ldc);
   }
   return 0;
 }
