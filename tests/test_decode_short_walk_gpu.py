@@ -40,6 +40,26 @@ def test_decode_attention_of_short_walks(head_dim, page, lengths, window, keep_f
     assert ops.attention_mma_error(D) == 0
 
 
+@pytest.mark.parametrize("D", [80, 96, 256])
+@pytest.mark.parametrize("B", [12, 16])
+def test_short_walks_of_wide_heads_in_small_clusters(D, B):
+    """Clusters of three (12 requests) and of two (16): either side of the number of tiles that a block walks alone."""
+    from tinyserve_b200.kernels import ops
+    H, page = 8, 16
+    lengths = ([1, 63, 64, 65, 127, 128, 129, 192] * 2)[:B]
+    assert ops.decode_splits(B, 1024, H, H) == (3 if B == 12 else 2)
+    g = torch.Generator().manual_seed(D + B)
+    k, v = (torch.randn(B * 12 + 1, H, page, D, generator=g).bfloat16().cuda() for _ in range(2))
+    q = torch.randn(B, H, D, generator=g).bfloat16().cuda()
+    table = (torch.randperm(B * 12, generator=g) + 1).int().view(B, 12).cuda()
+    ctx = NS(cu_q=torch.arange(B + 1, dtype=torch.int32).cuda(), kv_lens=torch.tensor(lengths, dtype=torch.int32).cuda(),
+             num_requests=B, max_q_len=1, max_kv_len=1024)
+    out, want = (ops.paged_attention(q, k, v, NS(block_table=table, page_size=page), ctx, D ** -0.5, num_splits=n).float() for n in (None, 1))
+    # a probability is rounded to bfloat16 (2^-9) against its range's maximum on either side, and so is the result
+    assert (out - want).abs().max() <= 2.0 ** -8 * (want.abs().max() + v.float().abs().max())
+    assert ops.attention_mma_error(D) == 0
+
+
 @pytest.mark.parametrize("lengths", [[1], [64, 128, 129, 40], [127, 500]])
 def test_decode_attention_from_the_projection_of_short_walks(lengths):
     """The kernel that makes the newest key and value itself against the two kernels."""

@@ -35,7 +35,13 @@ static_assert(D % 16 == 0 && D >= 16 && D <= 256, "head size must be a multiple 
 constexpr int CH = D / 8;                 // 16-byte chunks of a row
 constexpr int ROW_BYTES = D * 2 + 16;     // rows are padded by one chunk: ldmatrix without conflicts
 constexpr int THREADS = 128;              // decode block
-constexpr int ALONE_TILES = 2;            // key tiles that one block walks without its cluster
+// Key tiles that one block walks without its cluster.  Two, but one in clusters of two blocks where the ranges come by
+// cp.async, the head is wide and the merge short (few query heads a key head).  Clusters of two, 16 requests, 128 keys,
+// in the cluster / alone: heads of 256, one query head 17.8 / 20.4 us, four 22.9 / 22.5, eight 29.7 / 25.3; by TMA
+// 14.1 / 13.1; heads of 96 6.5 / 6.8, of 80 6.2 / 5.8.  In clusters of three and more alone is always the faster.
+__device__ __forceinline__ int alone_tiles(int cluster, int group, bool tma) {
+  return cluster > 2 || D <= 80 || tma || group >= 4 ? 2 : 1;
+}
 #ifndef TS_PREFILL_WARPS
 #define TS_PREFILL_WARPS 4
 #endif
@@ -566,7 +572,7 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
   // A short walk is one block's: the ranges of a cluster cost their merge (a cluster barrier and a round trip through
   // distributed shared memory), a tile of 64 keys about 1 us.  One request, 16 heads over 8, 60 / 120 / 180 / 250 keys:
   // 6.4 us in a cluster of eight, 4.5 / 5.4 / 6.5 / 7.7 alone.  (All blocks of the cluster see the same.)
-  const bool alone = p.cluster_merge && total <= ALONE_TILES;
+  const bool alone = p.cluster_merge && total <= alone_tiles(p.num_splits, G, TMA);
   const int per_split = alone ? total : (total + p.num_splits - 1) / p.num_splits;
   if (alone && split > 0) return;
   const int walk_begin = split * per_split;
