@@ -534,6 +534,16 @@ def test_repetition_penalty():
     assert torch.allclose(logits.cpu(), want)
 
 
+@pytest.mark.parametrize("D", [64, 128])
+def test_prefill_attention_keeps_its_rows_in_registers(D):
+    """A row of 128 scores a thread leaves few registers; spilled ones cost up to 14 %."""
+    import ctypes
+    out = (ctypes.c_int * 8)()
+    assert ops()._attention_tcgen05(D).ts_attention_tcgen05_resources(out) == 0 and out[6] == 0
+    registers, threads, local = out[0], out[4], out[7]
+    assert local == 0 and -(-threads // 128) * 4 * 32 * registers <= 65536
+
+
 # ----------------------------------------------------------------------------- tcgen05 product
 @pytest.mark.parametrize("M,N,K", [(1, 128, 64), (8, 256, 256), (16, 384, 4096), (5, 200, 72), (17, 130, 136),
                                    (33, 4096, 1024), (64, 1000, 520), (100, 640, 192), (128, 128, 64),
