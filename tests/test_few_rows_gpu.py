@@ -58,6 +58,18 @@ def test_product_of_few_rows_takes_leading_dimensions(M):
         torch.testing.assert_close(got.double(), xs.double() @ ws.double().T, rtol=0, atol=2e-5)
 
 
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two devices")
+def test_products_on_two_devices_of_one_process():
+    from tinyserve_b200.kernels import ops
+    g = torch.Generator().manual_seed(1)
+    for M, N in ((1, 4096), (8, 4096), (600, 1024)):
+        x, w, results = torch.randn(M, 1024, generator=g), torch.randn(N, 1024, generator=g), []
+        for device in range(2):
+            with torch.cuda.device(device):
+                results.append(ops.linear(x.cuda(), w.cuda()).cpu())
+        assert torch.equal(*results)
+
+
 # a short K, where the rule goes over to the tiled kernel (first and last of each line: either side of it)
 @pytest.mark.parametrize("M,N,K", [(8, 32000, 16), (40, 32000, 16), (64, 32000, 200), (65, 4096, 16), (512, 9000, 4), (4096, 64, 64), (4096, 64, 320),
                                    (20000, 33, 16), (20000, 256, 96), (20000, 256, 200), (100000, 8, 32), (100000, 8, 260)])

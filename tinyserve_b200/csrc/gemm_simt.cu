@@ -270,15 +270,25 @@ gemm_nt_chains_kernel(const float* __restrict__ A, const float* __restrict__ W, 
     }
 }
 
+// Lets a kernel have this much dynamic shared memory, once per device of the process.
+template <typename Kernel>
+cudaError_t allow_shared(Kernel* kernel, size_t bytes, std::atomic<unsigned long long>& devices) {
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = device < 64 ? 1ull << device : 0ull;
+  if (devices.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) devices.fetch_or(bit, std::memory_order_relaxed);
+  return e;
+}
+
 int launch_chains(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, size_t lda, size_t ldw,
                   size_t ldc, bool constant_w, cudaStream_t stream) {
   constexpr size_t smem = SPLIT_SMEM + SPLIT_RED_BYTES + SPLIT_TOTAL_BYTES;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_nt_chains_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return ts_fail("gemm_simt: %s", cudaGetErrorString(e));
-    configured = true;
-  }
+  static std::atomic<unsigned long long> devices;
+  const cudaError_t e = allow_shared(gemm_nt_chains_kernel, smem, devices);
+  if (e != cudaSuccess) return ts_fail("gemm_simt: %s", cudaGetErrorString(e));
   dim3 grid((N + TILE - 1) / TILE, (M + TILE - 1) / TILE);
   if (grid.y > 65535) return ts_fail("gemm: M = %d is too large", M);
   TS_LAUNCH("gemm_simt", gemm_nt_chains_kernel, grid, SPLIT_THREADS, smem, stream, A, W, bias, C, M, N, K, lda, ldw, ldc, constant_w);
@@ -426,14 +436,11 @@ int launch_gemv(const float* A, const float* W, const float* bias, float* C, int
     const int cs = 1 << shift, outputs = (SLOTS >> shift) * RT * MT;
     return (size_t)STAGES * (SLOTS * RT + MT * cs) * STAGE_K * 4 + (size_t)outputs * (cs + 2) * 4;
   };
-  static bool configured = false;
-  if (!configured) {
-    size_t most = 0;
-    for (int s = 0; s <= MAX_CHAINS_SHIFT; ++s) most = smem_of(s) > most ? smem_of(s) : most;
-    cudaError_t e = cudaFuncSetAttribute(gemv_nt_kernel<MT, RT, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
-    if (e != cudaSuccess) return ts_fail("gemm_simt: %s", cudaGetErrorString(e));
-    configured = true;
-  }
+  size_t most = 0;
+  for (int s = 0; s <= MAX_CHAINS_SHIFT; ++s) most = std::max(most, smem_of(s));
+  static std::atomic<unsigned long long> devices;
+  const cudaError_t e = allow_shared(gemv_nt_kernel<MT, RT, STAGES>, most, devices);
+  if (e != cudaSuccess) return ts_fail("gemm_simt: %s", cudaGetErrorString(e));
   const int rows = (SLOTS >> cs_shift) * RT;
   dim3 grid((N + rows - 1) / rows, (M + MT - 1) / MT);
   if (grid.y > 65535) return ts_fail("gemm: M = %d is too large", M);
