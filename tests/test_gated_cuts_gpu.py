@@ -24,12 +24,32 @@ def test_gated_product_of_few_row_tiles(M, N, K, activation, limit):
     else:
         gate, up = gate.clamp(max=limit), up.clamp(-limit, limit)
         want = gate * torch.sigmoid(1.702 * gate) * (up + 1)
+    launches = ops.launch_count()
     got = ops.gated_linear(x, w, activation, ops.GATED_BLOCK, limit)
+    assert ops.launch_count() - launches == 1, "one kernel"
     assert got.dtype == torch.bfloat16 and got.shape == want.shape
     # one rounding to bfloat16 (2^-9 of the value) and 32-bit sums of K terms of about 1 / sqrt(K)
     assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 4e-6).all()
     assert torch.equal(got, ops.gated_linear(x, w, activation, ops.GATED_BLOCK, limit)), "the same bits every time"
     assert ops.gemm_tcgen05_error() == 0
+
+
+@pytest.mark.parametrize("M,kernels", [(32, 1), (33, 2), (64, 2)])
+def test_more_row_tiles_than_run_at_once(M, kernels):
+    """51,200 rows are 400 row tiles, more than two a multiprocessor: above 32 tokens the activation is a kernel of its own."""
+    from tinyserve_b200.kernels import ops
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x, w = torch.randn(M, 128, generator=g, device="cuda").bfloat16(), (torch.randn(51200, 128, generator=g, device="cuda") / 11).bfloat16()
+    blocks = w.double().view(400, 2, 64, 128)
+    gate, up = ((x.double() @ blocks[:, i].reshape(25600, 128).T) for i in (0, 1))
+    want = torch.nn.functional.silu(gate) * up
+    launches = ops.launch_count()
+    got = ops.gated_linear(x, w, "silu", ops.GATED_BLOCK).double()
+    assert ops.launch_count() - launches == kernels
+    # of two kernels gate and up are rounded to bfloat16 as well: 2^-9 each, silu's slope is at most 1.1 and its argument's
+    # rounding 2^-9 of it
+    bound = 2.0 ** -8 * want.abs() + 4e-6 + (kernels - 1) * 2.0 ** -8 * (want.abs() + 1.1 * gate.abs() * up.abs())
+    assert ((got - want).abs() <= bound).all()
 
 
 @pytest.mark.parametrize("splits", [1, 2, 3, 4, 5, 6, 7, 8])

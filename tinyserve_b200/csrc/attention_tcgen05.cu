@@ -13,12 +13,11 @@
 //            read from tensor memory, V as an N-contiguous operand) as the probabilities arrive, in
 //            two halves of 64 keys, so that the first half of a product runs beside the exponentials
 //            of the second; the scores of tile g's next key tile follow its P V at once.  (The
-//            thread is chosen by elect.sync.  With `lane == 0` in its place the compiler cannot keep
-//            the MMAs' operands in uniform registers and a thread issues one MMA per 196 cycles,
-//            measured, more than the 64 that an MMA of 128 x 128 x 16 takes: three issuing threads
-//            with hand-overs between them were needed then.  32 heads over 8, 2,048 / 4,096 tokens:
-//            73.0 / 198.8 us with the three, 66.3 / 170.0 with the one; 2,048 queries at the end of
-//            12,000 keys, 16 heads: 225 -> 191 us.)  The tensor core takes a thread's
+//            thread is chosen by elect.sync.  With `lane == 0` in its place a thread issues one MMA per
+//            196 cycles, measured, more than the 64 that an MMA of 128 x 128 x 16 takes: three issuing
+//            threads with hand-overs between them were needed then.  32 heads over 8, 2,048 tokens 71.4
+//            us with the three, 60 with the one; 2,048 queries at the end of 12,000 keys 426 and 350;
+//            32 requests of 64 tokens, 64 heads 41.1 and 40.3.)  The tensor core takes a thread's
 //            MMAs in order: the next scores overwrite P_g after its P V has read it;
 //   warps 2-5 (tile 0) and 6-9 (tile 1), one thread per row: read the row of S from tensor memory,
 //            mask (key j is visible to the query at position p iff j <= p and, with a window

@@ -7,9 +7,8 @@
 // tensor memory, so every SM loads and reads only half of the weight tile.  Per 64-wide slice of
 // K each block's loader thread issues its TMA loads (128-byte swizzle, every block its own: no
 // cluster-wide copies) into a ring of five stages; both blocks' loads complete on the first
-// block's mbarrier.  One thread of the first block (chosen by elect.sync, so that the MMAs' operands
-// stay in uniform registers: with `lane == 0` an MMA took 196 cycles to issue and four threads had to
-// share them) issues the four K steps of a stage and commits the stage back to both loaders.
+// block's mbarrier.  One thread of the first block (chosen by elect.sync: with `lane == 0` in its
+// place an MMA took 196 cycles to issue and four threads had to share them) issues the four K steps of a stage and commits the stage back to both loaders.
 // Accumulators are double buffered (2 x 256 of the 512 columns): four epilogue warps per block drain
 // tile i (one thread per token row) while tile i + 1 is multiplied, and hand the buffer back.
 //
@@ -57,7 +56,7 @@ constexpr int TILE_BYTES = BM * 128; // an epilogue tile in shared memory: 128 r
 // us to drain, which a mainloop of 64 slices of K still hides).  HALVES = 2: tiles of 256 x 512,
 // one accumulator of all 512 columns: a block loads 48 KB per eight MMAs instead of 32 KB per
 // four (with all SMs loading, the L2 delivers about 80 GB/s to each, which bounds the narrower
-// tile), and the epilogue runs while no MMA does, by the issuing warps as well.
+// tile), and the epilogue runs while no MMA does, by the issuing warp and the three after it as well.
 template <int HALVES> struct Cfg {
   static constexpr int TILE_N = HALF_N * HALVES;
   static constexpr int STAGE_BYTES = A_BYTES + HALVES * B_BYTES;

@@ -237,8 +237,7 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
       }
     }
   } else if (warp == 1 && elect_one()) {
-    // (chosen by elect.sync: with `lane == 0` in its place a thread issues one MMA per 196 cycles,
-    // because the compiler cannot keep its operands in uniform registers)
+    // (chosen by elect.sync: with `lane == 0` in its place a thread issues one MMA per 196 cycles)
     pdl_wait();
     const uint32_t idesc = instr_desc(TILE_T);
     const uint64_t desc0 = smem_desc(smem_u32(smem));

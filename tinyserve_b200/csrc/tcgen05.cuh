@@ -68,7 +68,9 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y) : "memory");
 }
 // True in one thread of a converged warp.  A branch on it tells the compiler that a single thread
-// runs what follows, so that the operands of tcgen05.mma stay in uniform registers.
+// runs what follows: a tcgen05.mma then takes as long to issue as the tensor core takes for it; behind
+// `lane == 0` every one took 196 cycles, whatever its size (presumably because its operands, which the
+// instruction wants in uniform registers, have to be brought there each time).
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(

@@ -159,8 +159,8 @@ class SplitPartials:
 _NO_PARTIALS = (c_void_p(0), c_int(0), c_int(0), c_int(0), c_int(0))
 
 #: up to this many tokens the product before a residual add + norm does the add itself
-#: (PendingProduct, ScaledRows), the gate/up product applies the activation in its epilogue and the
-#: decode attention kernel takes the q/k/v projection as it is
+#: (PendingProduct, ScaledRows) and the decode attention kernel takes the q/k/v projection as it is
+#: (the gate/up product applies the activation in its epilogue up to GATED_MAX_TOKENS)
 FUSED_MAX_TOKENS = 16
 FUSED_MAX_SPLITS = 8
 
@@ -743,7 +743,7 @@ def gated_activation(gate_up, activation="silu", block=0, limit=0.0):
 GATED_BLOCK = 64
 #: Up to this many tokens the product of few tokens applies the activation itself, above half of it only where all
 #: row tiles run at once (two blocks a multiprocessor): the epilogue of a first wave keeps a second one from loading.
-#: 24576 x 4096 by 64 tokens 41.1 us with an activation kernel, 40.5 without; 6144 x 1024 17.2 and 11.6;
+#: 24576 x 4096 by 64 tokens 43.0 us with an activation kernel, 41.4 without; 6144 x 1024 14.6 and 10.8;
 #: 51200 x 5120 (400 tiles) by 32 tokens 87.1 and 86.7, by 64 94.7 and 96.1.
 GATED_MAX_TOKENS = 64
 
@@ -751,7 +751,8 @@ GATED_MAX_TOKENS = 64
 def gated_linear(x, weight, activation="silu", block=0, limit=0.0, constant_weight=False):
     """act(gate) * up of x @ weight^T, [M, N / 2].  weight [N, K] holds gate rows then up rows
     (``block`` 0) or alternates them in blocks of ``block`` rows.  With blocks of GATED_BLOCK and up
-    to GATED_MAX_TOKENS tokens the tcgen05 product does the activation in its epilogue; otherwise the product is followed by the activation kernel.  x may be the
+    to GATED_MAX_TOKENS tokens (above half as many: of up to two row tiles a multiprocessor) the tcgen05 product
+    does the activation in its epilogue; otherwise the product is followed by the activation kernel.  x may be the
     ScaledRows that add_rmsnorm returned.  ``constant_weight``: as for ``linear``."""
     rows = x.data if isinstance(x, ScaledRows) else x
     N, K = weight.shape
