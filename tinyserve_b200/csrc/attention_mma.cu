@@ -34,14 +34,8 @@ constexpr int D = TS_HEAD_DIM;
 static_assert(D % 16 == 0 && D >= 16 && D <= 256, "head size must be a multiple of 16 up to 256");
 constexpr int CH = D / 8;                 // 16-byte chunks of a row
 constexpr int ROW_BYTES = D * 2 + 16;     // rows are padded by one chunk: ldmatrix without conflicts
-constexpr int THREADS = 128;              // decode block
-// Key tiles that one block walks without its cluster.  Two, but one in clusters of two blocks where the ranges come by
-// cp.async, the head is wide and the merge short (few query heads a key head).  Clusters of two, 16 requests, 128 keys,
-// in the cluster / alone: heads of 256, one query head 17.8 / 20.4 us, four 22.9 / 22.5, eight 29.7 / 25.3; by TMA
-// 14.1 / 13.1; heads of 96 6.5 / 6.8, of 80 6.2 / 5.8.  In clusters of three and more alone is always the faster.
-__device__ __forceinline__ int alone_tiles(int cluster, int group, bool tma) {
-  return cluster > 2 || D <= 80 || tma || group >= 4 ? 2 : 1;
-}
+constexpr int CLUSTER_MAX = 8;            // key ranges that merge in a cluster
+constexpr int ALONE_TILES = 4;            // key tiles that one block walks without its cluster
 #ifndef TS_PREFILL_WARPS
 #define TS_PREFILL_WARPS 4
 #endif
@@ -135,8 +129,8 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 // NKEYS keys from j0 on -> shared memory (keys and values); keys outside [j_lo, j_hi) and not below `keep` become zeros
 template <int NKEYS, int NTHREADS>
 __device__ __forceinline__ void load_kv_tile(char* ks, char* vs, const MmaAttnParams& p, const int* bt,
-                                             int kvh, int j0, int j_lo, int j_hi, int keep = 0) {
-  for (int i = threadIdx.x; i < NKEYS * CH; i += NTHREADS) {
+                                             int kvh, int j0, int j_lo, int j_hi, int keep, int thread) {
+  for (int i = thread; i < NKEYS * CH; i += NTHREADS) {
     const int key = i / CH, c = i % CH;
     const int j = j0 + key;
     const bool valid = (j >= j_lo || j < keep) && j < j_hi;
@@ -307,7 +301,7 @@ __global__ void __launch_bounds__(PRE_THREADS) attn_prefill_kernel(MmaAttnParams
   const int kept_tiles = min((keep + BN - 1) / BN, first_tile);
   const int walk_end = end_tile - first_tile + kept_tiles;
   auto tile_of = [&](int w) { return w < kept_tiles ? w : first_tile + (w - kept_tiles); };
-  load_kv_tile<BN, PRE_THREADS>(Ks, Vs, p, bt, kvh, tile_of(0) * BN, j_lo, j_hi, keep);
+  load_kv_tile<BN, PRE_THREADS>(Ks, Vs, p, bt, kvh, tile_of(0) * BN, j_lo, j_hi, keep, threadIdx.x);
   cp_async_commit();
 
   int pos[2], lo[2];
@@ -342,7 +336,7 @@ __global__ void __launch_bounds__(PRE_THREADS) attn_prefill_kernel(MmaAttnParams
     const int buf = walk & 1;
     if (walk + 1 < walk_end)
       load_kv_tile<BN, PRE_THREADS>(Ks + (buf ^ 1) * BN * ROW_BYTES, Vs + (buf ^ 1) * BN * ROW_BYTES, p, bt,
-                                    kvh, tile_of(walk + 1) * BN, j_lo, j_hi, keep);
+                                    kvh, tile_of(walk + 1) * BN, j_lo, j_hi, keep, threadIdx.x);
     cp_async_commit();
     cp_async_wait<1>();
     __syncthreads();
@@ -520,33 +514,167 @@ __device__ __forceinline__ void build_head(const MmaAttnParams& p, int t, int co
   }
 }
 
-// TMA false: key and value tiles come by cp.async, 16 bytes a thread, into padded rows (any head
+// The decode block.  One query against a few hundred keys is a chain of short phases, and what bounds it is how long
+// each of them takes, not bytes; so:
+// - Scores are made as S^T = K Q^T and outputs as O^T = V^T P^T: the keys (or the columns of V) are the 16 rows of an
+//   mma.sync and the heads its 8 columns, which needs half of the instructions (and registers for O) that heads as rows
+//   take while a KV group has up to 8 heads (NH = 1; NH = 2 for up to 16).  P turns from the one layout into the other by
+//   movmatrix.
+// - Eight warps in two groups: group g takes the tiles g, g + 2, .. of the block's walk, a warp 16 keys of a tile.  A group
+//   waits for its tiles alone and refills the stage that it has emptied; nothing in the walk is common to the block.
+//   Three stages and six mbarriers: tile i lies in stage i % 3 and is counted on barrier i % 6, which always belongs to
+//   the same group, so that no group can miss a phase.
+// - The warps' partial sums lie in shared memory in rows of D + 4 floats, which neither side's accesses collide on.
+// - Ranges that are a cluster send their sums to the rank that adds them up, into memory of their own: one cluster
+//   barrier lies between, and nobody has to wait for a reader before it leaves.
+// Heads as rows, four warps a tile, a merge by reading -> this, one launch after the other, us: 32 heads over 8, 540 keys, 1
+// request 9.1 -> 6.7, 8 13.4 -> 9.8, 16 15.3 -> 10.6; 64 of 130 keys 15.4 -> 11.8; 32 of 4,000 91 -> 77 (524 MB); 16 heads
+// over 8, 90 keys 6.5 -> 4.9, 2 of 10,500 24.2 -> 18.9; 64 over 8, pages of 16, 6 of 2,000 37.6 -> 25.9.
+//
+// TMA false: key and value tiles come by cp.async, 16 bytes a thread of the group, into padded rows (any head
 // size in steps of 16, any page size).  TMA true (head sizes in steps of 64, pages of 32 or 64
-// keys): one thread fetches whole pages as boxes of page x 64 columns with the 128-byte swizzle
-// and an mbarrier per stage counts their bytes; an SM streams about half as much again this way
+// keys): one warp of the group fetches whole pages as boxes of page x 64 columns with the 128-byte swizzle;
+// an SM streams about half as much again this way
 // as through its load/store unit's miss queue.  Whole pages come, also the keys past the
 // request's length in its last page: those are masked, and must hold finite numbers (the engine's
 // cache starts as zeros and only ever takes keys and values).
-template <bool TMA>
+constexpr int DEC_THREADS = 256, DEC_WARPS = DEC_THREADS / 32, DEC_GROUP = DEC_THREADS / 2;
+constexpr int DEC_BARRIERS = 2 * DEC_STAGES;
+constexpr int SUM_ROW = D + 4;                       // floats of a row of partial sums (4 mod 16: no bank conflicts)
+
+// the block's shared memory: query rows, stages, and what peers of a cluster send
+template <bool TMA> struct DecShared {
+  static constexpr int KV_TILE = TMA ? BN * D * 2 : BN * ROW_BYTES;      // bytes of the keys (or values) of a stage
+  static constexpr int Q_BYTES = 16 * ROW_BYTES;
+  static constexpr int ALIGN = TMA ? 1024 : 16;
+  // received sums: every rank's share of [heads][D], rounded up to pairs of columns, and maxima and sums of the rows
+  static constexpr int recv_floats(int heads) { return heads * D + 2 * CLUSTER_MAX + CLUSTER_MAX * heads * 2; }
+  static size_t bytes(int heads) { return Q_BYTES + ALIGN + (size_t)2 * DEC_STAGES * KV_TILE + recv_floats(heads) * 4; }
+};
+
+__device__ __forceinline__ uint32_t transposed(uint32_t a) {
+  uint32_t b;
+  asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(b) : "r"(a));
+  return b;
+}
+// arrives on the mbarrier once every cp.async of this thread so far has landed
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void group_barrier(int group) {
+  if (group == 0) asm volatile("bar.sync 1, %0;\n" ::"n"(DEC_GROUP) : "memory");
+  else asm volatile("bar.sync 2, %0;\n" ::"n"(DEC_GROUP) : "memory");
+}
+__device__ __forceinline__ void cluster_store_f32(float* own_shared, uint32_t rank, float v) {
+  uint32_t local = static_cast<uint32_t>(__cvta_generic_to_shared(own_shared)), remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
+}
+
+// sixteen keys (rows key0 .. of a tile) for the block's heads: scores, online softmax, outputs.  The lane holds the heads
+// 2t and 2t + 1 of every eight and of S^T the keys g and g + 8, of O^T the columns g and g + 8 of every sixteen.
+// `jbase` is the position of row key0; m, l: running maximum and this lane's part of the sum (log2 domain).
+template <bool SWZ, int NH, bool Q_REGS>
+__device__ __forceinline__ void decode_keys(float (&o)[NH][D / 16][4], float (&m)[NH][2], float (&l)[NH][2],
+                                            const uint32_t (*qf)[NH][2], const char* qs, const char* ks, const char* vs, int key0,
+                                            int jbase, int qpos, int j_lo, int keep, const MmaAttnParams& p,
+                                            const float (&sl)[NH][2], int lane) {
+  const int mi = lane >> 3, r = lane & 7, g = lane >> 2;
+  float s[NH][4];
+#pragma unroll
+  for (int nh = 0; nh < NH; ++nh)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) s[nh][e] = 0.f;
+#pragma unroll
+  for (int kstep = 0; kstep < D / 16; ++kstep) {
+    uint32_t a[4];
+    ldmatrix_x4(a, kv_piece<SWZ>(ks, key0 + (mi & 1) * 8 + r, kstep * 2 + (mi >> 1)));
+    if (Q_REGS) {
+#pragma unroll
+      for (int nh = 0; nh < NH; ++nh) mma_bf16(s[nh], a, qf[kstep][nh][0], qf[kstep][nh][1]);
+    } else {
+      // heads 0..7 (both halves of the step), then heads 8..15
+      uint32_t b[4];
+      ldmatrix_x4(b, smem_u32(qs + ((mi >> 1) * 8 + r) * ROW_BYTES + (kstep * 2 + (mi & 1)) * 16));
+#pragma unroll
+      for (int nh = 0; nh < NH; ++nh) mma_bf16(s[nh], a, b[2 * nh], b[2 * nh + 1]);
+    }
+  }
+  bool seen[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int j = jbase + g + 8 * h;
+    seen[h] = j <= qpos && (j >= j_lo || j < keep);
+  }
+  uint32_t pf[NH][2];
+#pragma unroll
+  for (int nh = 0; nh < NH; ++nh) {
+    float alpha[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      float mx = -INFINITY;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float v = s[nh][2 * h + e];
+        if (p.cap2 > 0.f) v = p.cap2 * soft_tanh(v * p.cap_in);      // (the same for every thread of the launch)
+        else v *= p.scale_log2;
+        if (p.slopes) v = fmaf(sl[nh][e], (float)(jbase + g + 8 * h - qpos), v);
+        if (!seen[h]) v = -INFINITY;
+        s[nh][2 * h + e] = v;
+        mx = fmaxf(mx, v);
+      }
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+      const float m_new = fmaxf(m[nh][e], mx);
+      const float m_safe = m_new == -INFINITY ? 0.f : m_new;
+      alpha[e] = fast_exp2(m[nh][e] - m_safe);      // m = -inf gives 0
+      m[nh][e] = m_new;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) s[nh][2 * h + e] = fast_exp2(s[nh][2 * h + e] - m_safe);
+      l[nh][e] = fmaf(l[nh][e], alpha[e], s[nh][e] + s[nh][2 + e]);
+    }
+    pf[nh][0] = transposed(pack_bf16(s[nh][0], s[nh][1]));
+    pf[nh][1] = transposed(pack_bf16(s[nh][2], s[nh][3]));
+#pragma unroll
+    for (int dp = 0; dp < D / 16; ++dp)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[nh][dp][e] *= alpha[e & 1];
+  }
+#pragma unroll
+  for (int dp = 0; dp < D / 16; ++dp) {
+    uint32_t a[4];
+    ldmatrix_x4_trans(a, kv_piece<SWZ>(vs, key0 + (mi >> 1) * 8 + r, dp * 2 + (mi & 1)));
+#pragma unroll
+    for (int nh = 0; nh < NH; ++nh) mma_bf16(o[nh][dp], a, pf[nh][0], pf[nh][1]);
+  }
+}
+
+template <bool TMA, int NH>
 __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const CUtensorMap* map_k,
                                                  const CUtensorMap* map_v) {
+  using S = DecShared<TMA>;
+  constexpr int KV_TILE = S::KV_TILE;
+  constexpr bool Q_REGS = D <= 128 && NH == 1;
   extern __shared__ __align__(16) char smem[];
-  constexpr int KV_TILE = TMA ? BN * D * 2 : BN * ROW_BYTES;      // bytes of the keys (or values) of a stage
   char* Qs = smem;                                   // [16][ROW_BYTES]
-  char* Ks = TMA ? reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(Qs + 16 * ROW_BYTES) + 1023) & ~uintptr_t(1023))
-                 : Qs + 16 * ROW_BYTES;              // [DEC_STAGES][KV_TILE]
+  char* Ks = TMA ? reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(Qs + S::Q_BYTES) + 1023) & ~uintptr_t(1023))
+                 : Qs + S::Q_BYTES;                  // [DEC_STAGES][KV_TILE]
   char* Vs = Ks + DEC_STAGES * KV_TILE;              // [DEC_STAGES][KV_TILE]
-  __shared__ uint64_t full[DEC_STAGES];              // (TMA) the stage's bytes have landed
+  float* recv = reinterpret_cast<float*>(Vs + DEC_STAGES * KV_TILE);       // peers' sums: [rank][this block's share]
+  __shared__ uint64_t full[DEC_BARRIERS];            // the tile's bytes have landed
   __shared__ int abort_flag_s;
   volatile int* abort_flag = &abort_flag_s;
-  if (TMA && threadIdx.x == 0) {
-    for (int s = 0; s < DEC_STAGES; ++s) mbar_init(smem_u32(&full[s]), 1);
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < DEC_BARRIERS; ++s) mbar_init(smem_u32(&full[s]), TMA ? 1 : DEC_GROUP);
     abort_flag_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  if (TMA) __syncthreads();
+  __syncthreads();
 
   pdl_trigger();
+  // (peers may be written to once they have all started; the wait for that comes before the first such write)
+  if (p.cluster_merge) cluster_arrive();
   // The lengths, the block table and every cached key but the newest were written before this
   // step's kernels began: the first tiles are fetched before pdl_wait(), while the kernels that
   // make this token's query, key and value still run.  The tile with the newest key and the
@@ -557,8 +685,8 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
   const int q_begin = p.cu_q[b];
   if (p.cu_q[b + 1] - q_begin != 1) return;
   const int kv_len = p.kv_lens[b];
-  const int G = p.H / p.Hkv, g0 = head_tile * 16, ng = min(16, G - g0);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2;
+  const int G = p.H / p.Hkv, g0 = head_tile * 8 * NH, ng = min(8 * NH, G - g0);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, group = warp >> 2;
   const int* bt = p.block_table + (size_t)b * p.max_blocks;
   const int qpos = kv_len - 1;
   const int j_hi = kv_len;
@@ -569,10 +697,8 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
   const int first_tile = j_lo / BN, kept_tiles = min((keep + BN - 1) / BN, first_tile);
   const int total = (j_hi + BN - 1) / BN - first_tile + kept_tiles;
   auto tile_of = [&](int w) { return w < kept_tiles ? w : first_tile + (w - kept_tiles); };
-  // A short walk is one block's: the ranges of a cluster cost their merge (a cluster barrier and a round trip through
-  // distributed shared memory), a tile of 64 keys about 1 us.  One request, 16 heads over 8, 60 / 120 / 180 / 250 keys:
-  // 6.4 us in a cluster of eight, 4.5 / 5.4 / 6.5 / 7.7 alone.  (All blocks of the cluster see the same.)
-  const bool alone = p.cluster_merge && total <= alone_tiles(p.num_splits, G, TMA);
+  // A short walk is one block's: the ranges of a cluster cost their merge.  (All blocks of the cluster see the same.)
+  const bool alone = p.cluster_merge && total <= ALONE_TILES;
   const int per_split = alone ? total : (total + p.num_splits - 1) / p.num_splits;
   if (alone && split > 0) return;
   const int walk_begin = split * per_split;
@@ -582,23 +708,23 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
   // fetched before the wait, without that key, which this block makes itself
   const bool from_qkv = p.from_qkv != 0;
   const int j_load = from_qkv ? j_hi - 1 : j_hi;
-  const int late_tile = from_qkv ? -1 : newest_tile;
   const bool has_newest = from_qkv && total - 1 >= walk_begin && total - 1 < walk_begin + n_tiles;   // (the walk ends with it)
   __shared__ __align__(16) bf16 newest_kv[2 * D];
 
-  // tile `tile` of the keys and values into stage `stage`
-  auto load_tile = [&](int stage, int tile, int j_end) {
+  // tile i of this block's walk into its stage, by the group that is not going to read it (the one that emptied the stage)
+  auto load_tile = [&](int i) {
+    const int tile = tile_of(walk_begin + i), stage = i % DEC_STAGES;
+    const uint32_t bar = smem_u32(&full[i % DEC_BARRIERS]);
     if (TMA) {
       // the boxes of a tile (pages x 64-column chunks x keys/values) are dealt to the lanes of
-      // warp 0, so that issuing them costs the block one box's time, not sixteen; lane 0's
+      // the group's first warp, so that issuing them costs the block one box's time, not sixteen; lane 0's
       // arrival carries the tile's byte count, so the stage cannot complete before it
-      if (threadIdx.x < 32) {
+      if ((warp & 3) == 0) {
         const int pages_per_tile = BN >> p.page_shift, boxes = pages_per_tile * (D / 64) * 2;
-        const uint32_t bar = smem_u32(&full[stage]);
-        if (threadIdx.x == 0) mbar_expect_tx(bar, 2 * KV_TILE);
+        if (lane == 0) mbar_expect_tx(bar, 2 * KV_TILE);
         __syncwarp();
-        for (int i = threadIdx.x; i < boxes; i += 32) {
-          const int values = i & 1, c = (i >> 1) % (D / 64), pg = (i >> 1) / (D / 64);
+        for (int k = lane; k < boxes; k += 32) {
+          const int values = k & 1, c = (k >> 1) % (D / 64), pg = (k >> 1) / (D / 64);
           const int j = tile * BN + (pg << p.page_shift);
           const int page = j < j_hi ? bt[j >> p.page_shift] : 0;                        // past the end: the null page
           const int row = (values ? page * p.Hv + kvh / p.v_share : page * p.Hkv + kvh) << p.page_shift;
@@ -607,12 +733,15 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
         }
       }
     } else {
-      load_kv_tile<BN, THREADS>(Ks + stage * KV_TILE, Vs + stage * KV_TILE, p, bt, kvh, tile * BN, j_lo, j_end, keep);
+      load_kv_tile<BN, DEC_GROUP>(Ks + stage * KV_TILE, Vs + stage * KV_TILE, p, bt, kvh, tile * BN, j_lo, j_load, keep,
+                                  threadIdx.x & (DEC_GROUP - 1));
+      cp_async_arrive(bar);
     }
   };
+  const int late = from_qkv ? -1 : newest_tile;      // its newest key is there after the wait only
 #pragma unroll
-  for (int s = 0; s < DEC_STAGES - 1; ++s)
-    if (s < n_tiles && tile_of(walk_begin + s) != late_tile) load_tile(s, tile_of(walk_begin + s), j_load);
+  for (int s = 0; s < DEC_STAGES; ++s)
+    if (s < n_tiles && group == ((s + 1) & 1) && tile_of(walk_begin + s) != late) load_tile(s);
   // the timeline build follows the blocks of one (request, KV group): marks 40.. with the key
   // range as their value
   const bool traced = blockIdx.x == 0 && blockIdx.z == 0 && threadIdx.x == 0;
@@ -625,7 +754,7 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
     load_angles(hq, p, pos_q, lane);
     load_weights(hq, p.q_weight, p.has_norm, lane);
     hk = hq;
-    if (has_newest) load_weights(hk, p.k_weight, p.has_norm, lane);
+    if (has_newest && warp == 0) load_weights(hk, p.k_weight, p.has_norm, lane);
   }
   if (traced) timeline_mark_thread(41, split);          // constants fetched
   pdl_wait();
@@ -634,7 +763,7 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
     // the heads this block makes, dealt to the warps in turn: the newest key (norm, rotary) and
     // value where this block holds them, then the query rows; rows past the group are zero
     const int extra = has_newest ? 2 : 0;
-    for (int i = warp; i < extra + 16; i += THREADS / 32) {
+    for (int i = warp; i < extra + 8 * NH; i += DEC_WARPS) {
       if (i < extra) {
         build_head(p, q_begin, (p.H + (i == 0 ? 0 : p.Hkv) + kvh) * D, i == 0, hk, lane, newest_kv + i * D);
         continue;
@@ -647,136 +776,143 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
         for (int d = lane * 2; d < D; d += 64) *reinterpret_cast<uint32_t*>(row + d) = 0u;
       }
     }
-    __syncthreads();
-    if (has_newest && head_tile == 0 && slot >= 0) {
-      const size_t page = slot >> p.page_shift, in_page = slot & p.page_mask;
-      const size_t at = (((page * p.Hkv + kvh) << p.page_shift) + in_page) * D;
-      for (int d = threadIdx.x * 2; d < 2 * D; d += THREADS * 2) {
-        bf16* dst = d < D ? p.k_cache_out + at + d : p.v_cache_out + at + (d - D);
-        *reinterpret_cast<uint32_t*>(dst) = *reinterpret_cast<const uint32_t*>(newest_kv + d);
-      }
-    }
   } else {
-    for (int i = threadIdx.x; i < 16 * CH; i += THREADS) {
+    for (int i = threadIdx.x; i < 8 * NH * CH; i += DEC_THREADS) {
       const int r = i / CH, c = i % CH;
-      const bool valid = r < ng;
-      const bf16* src = valid ? p.q + ((size_t)q_begin * p.H + kvh * G + g0 + r) * D + c * 8 : p.q;
-      cp_async16(smem_u32(Qs + r * ROW_BYTES + c * 16), src, valid);
+      const uint4 q = r < ng ? *reinterpret_cast<const uint4*>(p.q + ((size_t)q_begin * p.H + kvh * G + g0 + r) * D + c * 8)
+                             : make_uint4(0u, 0u, 0u, 0u);
+      *reinterpret_cast<uint4*>(Qs + r * ROW_BYTES + c * 16) = q;
     }
-  }
 #pragma unroll
-  for (int s = 0; s < DEC_STAGES - 1; ++s) {
-    if (s < n_tiles && tile_of(walk_begin + s) == late_tile) load_tile(s, tile_of(walk_begin + s), j_hi);
-    // the first group holds the query and all of these tiles; the others stay empty, so that the
-    // loop below finds as many groups as it counts on
-    cp_async_commit();
+    for (int s = 0; s < DEC_STAGES; ++s)
+      if (s < n_tiles && group == ((s + 1) & 1) && tile_of(walk_begin + s) == late) load_tile(s);
   }
-  if (TMA) {        // only the query rows came by cp.async
-    cp_async_wait<0>();
-    __syncthreads();
+  __syncthreads();
+  if (has_newest && head_tile == 0 && slot >= 0) {
+    const size_t page = slot >> p.page_shift, in_page = slot & p.page_mask;
+    const size_t at = (((page * p.Hkv + kvh) << p.page_shift) + in_page) * D;
+    for (int d = threadIdx.x * 2; d < 2 * D; d += DEC_THREADS * 2) {
+      bf16* dst = d < D ? p.k_cache_out + at + d : p.v_cache_out + at + (d - D);
+      *reinterpret_cast<uint32_t*>(dst) = *reinterpret_cast<const uint32_t*>(newest_kv + d);
+    }
   }
   if (traced) timeline_mark_thread(43, split);          // query rows (and the newest key) made
-  int pos[2], lo[2];
-  float sl[2];
+  const int t = lane & 3;
+  float sl[NH][2], m[NH][2], l[NH][2], o[NH][D / 16][4];
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    pos[h] = g + 8 * h < ng ? qpos : -1;
-    lo[h] = j_lo;
-    sl[h] = p.slopes && g + 8 * h < ng ? p.slopes[kvh * G + g0 + g + 8 * h] * LOG2E : 0.f;
-  }
-  float o[D / 8][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+  for (int nh = 0; nh < NH; ++nh) {
 #pragma unroll
-  for (int dt = 0; dt < D / 8; ++dt)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) o[dt][e] = 0.f;
-  uint32_t qf[Q_IN_REGS ? D / 16 : 1][4];
-
-  for (int it = 0; it < n_tiles; ++it) {
-    const int nxt = it + DEC_STAGES - 1;
-    if (nxt < n_tiles) load_tile(nxt % DEC_STAGES, tile_of(walk_begin + nxt), j_load);
-    if (TMA) {
-      // bounded; a wait that ran out raises the block's abort flag and the status word, the loop
-      // goes on over whatever the stage holds, and the block stores no output at the end
-      mbar_wait(smem_u32(&full[it % DEC_STAGES]), (it / DEC_STAGES) & 1, abort_flag);
-    } else {
-      cp_async_commit();
-      cp_async_wait<DEC_STAGES - 1>();
+    for (int e = 0; e < 2; ++e) {
+      const int r = nh * 8 + 2 * t + e;
+      sl[nh][e] = p.slopes && r < ng ? p.slopes[kvh * G + g0 + r] * LOG2E : 0.f;
+      m[nh][e] = -INFINITY;
+      l[nh][e] = 0.f;
     }
-    __syncthreads();
-    if (has_newest && tile_of(walk_begin + it) == newest_tile) {
-      // the newest key and value take their row of the tile (the copy left zeros or stale bytes there)
-      const int row = qpos - newest_tile * BN, buf_n = it % DEC_STAGES;
-      for (int d = threadIdx.x * 2; d < 2 * D; d += THREADS * 2) {
-        const int e = d < D ? d : d - D;          // element of the head; two neighbours per thread
-        char* tile = (d < D ? Ks : Vs) + (size_t)buf_n * KV_TILE;
+#pragma unroll
+    for (int dp = 0; dp < D / 16; ++dp)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[nh][dp][e] = 0.f;
+  }
+  uint32_t qf[Q_REGS ? D / 16 : 1][NH][2];
+  if (Q_REGS) {
+    const int mi = lane >> 3, r = lane & 7;
+#pragma unroll
+    for (int k2 = 0; k2 < D / 32; ++k2) {              // two steps of 16 columns at once
+      uint32_t b[4];
+      ldmatrix_x4(b, smem_u32(Qs + r * ROW_BYTES + (k2 * 4 + mi) * 16));
+      qf[2 * k2][0][0] = b[0]; qf[2 * k2][0][1] = b[1];
+      qf[2 * k2 + 1][0][0] = b[2]; qf[2 * k2 + 1][0][1] = b[3];
+    }
+    if (D % 32 != 0) {
+      uint32_t b[4];
+      ldmatrix_x4(b, smem_u32(Qs + r * ROW_BYTES + ((D / 16 - 1) * 2 + (mi & 1)) * 16));
+      qf[D / 16 - 1][0][0] = b[0]; qf[D / 16 - 1][0][1] = b[1];
+    }
+  }
+
+  const int key0 = (warp & 3) * 16;
+  for (int it = group; it < n_tiles; it += 2) {
+    const int stage = it % DEC_STAGES;
+    // bounded; a wait that ran out raises the block's abort flag and the status word, the loop
+    // goes on over whatever the stage holds, and the block stores no output at the end
+    mbar_wait(smem_u32(&full[it % DEC_BARRIERS]), (it / DEC_BARRIERS) & 1, abort_flag);
+    __syncwarp();
+    char* ks = Ks + stage * KV_TILE;
+    char* vs = Vs + stage * KV_TILE;
+    const int jbase = tile_of(walk_begin + it) * BN + key0;
+    if (has_newest && qpos >= jbase && qpos < jbase + 16) {
+      // the newest key and value take their row of the tile (the copy left zeros or stale bytes there), which no other warp reads
+      const int row = qpos - jbase + key0;
+      for (int d = lane * 2; d < 2 * D; d += 64) {
+        const int e = d < D ? d : d - D;          // element of the head; two neighbours per lane
+        char* tile = d < D ? ks : vs;
         char* dst = TMA ? tile + (e / 64) * (BN * 128) + row * 128 + ((((e % 64) / 8) ^ (row & 7)) << 4) + (e % 8) * 2
                         : tile + row * ROW_BYTES + e * 2;
         *reinterpret_cast<uint32_t*>(dst) = *reinterpret_cast<const uint32_t*>(newest_kv + d);
       }
-      __syncthreads();
+      __syncwarp();
     }
-    if (Q_IN_REGS && it == 0) {
-      const int mi = lane >> 3, r = lane & 7;
-#pragma unroll
-      for (int kstep = 0; kstep < D / 16; ++kstep)
-        ldmatrix_x4(qf[kstep], smem_u32(Qs + ((mi & 1) * 8 + r) * ROW_BYTES + (kstep * 2 + (mi >> 1)) * 16));
+    if (jbase < j_hi) decode_keys<TMA, NH, Q_REGS>(o, m, l, qf, Qs, ks, vs, key0, jbase, qpos, j_lo, keep, p, sl, lane);
+    if (it + DEC_STAGES < n_tiles) {
+      group_barrier(group);
+      load_tile(it + DEC_STAGES);
     }
-    const int buf = it % DEC_STAGES;
-    const int jbase = tile_of(walk_begin + it) * BN + warp * 16;
-    if (jbase < j_hi) {
-      float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-      qk_tile<2, TMA>(s, Qs, qf, Ks + buf * KV_TILE, warp * 16, lane);
-      if (p.slopes) softmax_tile<2, true, true>(s, o, m, l, pos, lo, jbase, p.scale_log2, lane, keep, sl, p.cap2, p.cap_in);
-      else softmax_tile<2>(s, o, m, l, pos, lo, jbase, p.scale_log2, lane, keep, nullptr, p.cap2, p.cap_in);
-      pv_tile<2, TMA>(o, s, Vs + buf * KV_TILE, warp * 16, lane);
-    }
-    __syncthreads();
   }
-  cp_async_wait<0>();
   __syncthreads();
   if (traced) timeline_mark_thread(44, split);          // all key tiles done
 
-  // merge the four warps' partial softmax through shared memory (the K buffers are free now)
-  float* sm_o = reinterpret_cast<float*>(Ks);                  // [4][16][D]
-  float* sm_ml = sm_o + 4 * 16 * D;                            // [4][16][2]
-  float* cl_ml = sm_ml + 4 * 16 * 2;                           // [16][2] of the block, for its cluster
+  // merge the warps' partial softmax through shared memory (the stages are free now)
+  float* sm_o = reinterpret_cast<float*>(Ks);                  // [DEC_WARPS][ng][SUM_ROW]
+  float* sm_ml = sm_o + DEC_WARPS * 8 * NH * SUM_ROW;          // [DEC_WARPS][8 NH][2]
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    float sum = l[h];
-    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-    const int r = g + 8 * h;
+  for (int nh = 0; nh < NH; ++nh)
 #pragma unroll
-    for (int dt = 0; dt < D / 8; ++dt) {
-      sm_o[(warp * 16 + r) * D + dt * 8 + 2 * (lane & 3)] = o[dt][2 * h];
-      sm_o[(warp * 16 + r) * D + dt * 8 + 2 * (lane & 3) + 1] = o[dt][2 * h + 1];
+    for (int e = 0; e < 2; ++e) {
+      const int r = nh * 8 + 2 * t + e;
+      float sum = l[nh][e];
+      sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+      if (r < ng) {
+        float* row = sm_o + (warp * ng + r) * SUM_ROW + (lane >> 2);
+#pragma unroll
+        for (int dp = 0; dp < D / 16; ++dp) {
+          row[dp * 16] = o[nh][dp][e];
+          row[dp * 16 + 8] = o[nh][dp][2 + e];
+        }
+        if ((lane >> 2) == 0) {
+          sm_ml[(warp * 8 * NH + r) * 2] = m[nh][e];
+          sm_ml[(warp * 8 * NH + r) * 2 + 1] = sum;
+        }
+      }
     }
-    if ((lane & 3) == 0) {
-      sm_ml[(warp * 16 + r) * 2] = m[h];
-      sm_ml[(warp * 16 + r) * 2 + 1] = sum;
-    }
-  }
   __syncthreads();
-  const bool stores = !TMA || abort_flag_s == 0;
+  const bool stores = abort_flag_s == 0;
   // (a turned output needs its column's mate, which is the neighbour lane's: both lanes of a pair are in or out)
   auto finished = [&](float v, int d, unsigned lanes) {
     if (!p.turn.cos) return v;
     const float mate = __shfl_xor_sync(lanes, v, 1);
     return p.turn.value(v, mate, d, qpos);
   };
-  for (int i = threadIdx.x; i < ng * D; i += THREADS) {
+  const bool merged = p.cluster_merge && !alone;
+  const int per_rank = ((ng * D + p.num_splits - 1) / p.num_splits + 1) & ~1;       // (whole column pairs)
+  float* recv_ml = recv + 8 * NH * D + 2 * CLUSTER_MAX;                             // [rank][8 NH][2]
+  if (merged) cluster_wait();                           // all peers have started
+  for (int i = threadIdx.x; i < ng * D; i += DEC_THREADS) {
     const unsigned lanes = ~0u >> (32 - min(32, ng * D - (i - lane)));        // the warp's lanes that take part
     const int r = i / D, d = i % D;
-    float mx = -INFINITY;
+    float mw[DEC_WARPS], mx = -INFINITY;
 #pragma unroll
-    for (int w = 0; w < 4; ++w) mx = fmaxf(mx, sm_ml[(w * 16 + r) * 2]);
+    for (int w = 0; w < DEC_WARPS; ++w) {
+      mw[w] = sm_ml[(w * 8 * NH + r) * 2];
+      mx = fmaxf(mx, mw[w]);
+    }
     float num = 0.f, den = 0.f;
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      const float mw = sm_ml[(w * 16 + r) * 2];
-      const float wgt = mw == -INFINITY ? 0.f : exp2f(mw - mx);
-      num = fmaf(wgt, sm_o[(w * 16 + r) * D + d], num);
-      den = fmaf(wgt, sm_ml[(w * 16 + r) * 2 + 1], den);
+    for (int w = 0; w < DEC_WARPS; ++w) {
+      const float wgt = mw[w] == -INFINITY ? 0.f : exp2f(mw[w] - mx);
+      num = fmaf(wgt, sm_o[(w * ng + r) * SUM_ROW + d], num);
+      den = fmaf(wgt, sm_ml[(w * 8 * NH + r) * 2 + 1], den);
     }
     const int head = kvh * G + g0 + r;
     if (p.sinks && split == 0) {
@@ -791,12 +927,13 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
     if (p.num_splits == 1 || alone) {
       const float y = finished(den > 0.f ? num / den : 0.f, d, lanes);
       if (stores) p.out[((size_t)q_begin * p.H + head) * D + d] = __float2bfloat16_rn(y);
-    } else if (p.cluster_merge) {
-      // this thread has read its four values of (r, d); the first warp's place now holds their sum
-      sm_o[r * D + d] = num;
-      if (d == 0) {
-        cl_ml[r * 2] = mx;
-        cl_ml[r * 2 + 1] = den;
+    } else if (merged) {
+      // to the rank that adds this element up, at its place among this range's
+      const int owner = i / per_rank;
+      cluster_store_f32(recv + split * per_rank + (i - owner * per_rank), owner, num);
+      if (d < p.num_splits) {                           // (every thread of the row holds the same maximum and sum)
+        cluster_store_f32(recv_ml + (split * 8 * NH + r) * 2, d, mx);
+        cluster_store_f32(recv_ml + (split * 8 * NH + r) * 2 + 1, d, den);
       }
     } else {
       // partial rows go by token, or by the entry of the request list when there is one
@@ -808,56 +945,43 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
       }
     }
   }
-  if (p.cluster_merge && !alone) {
+  if (merged) {
     // The blocks of a (request, KV group) are one cluster, rank = key range.  Each block merges
-    // its share of the (head, dimension) pairs from all ranks' shared memory, in rank order.
+    // its share of the (head, dimension) pairs, in rank order.
     cluster_arrive();
     cluster_wait();
-    const int per_rank = ((ng * D + p.num_splits - 1) / p.num_splits + 1) & ~1;       // (whole column pairs)
     const int i_end = min(ng * D, (split + 1) * per_rank);
-    for (int i = split * per_rank + threadIdx.x; i < i_end; i += THREADS) {
+    for (int i = split * per_rank + threadIdx.x; i < i_end; i += DEC_THREADS) {
       const unsigned lanes = ~0u >> (32 - min(32, i_end - (i - lane)));
       const int r = i / D, d = i % D;
-      float ms[8], ls[8], os[8];
-#pragma unroll
-      for (int s = 0; s < 8; ++s)
-        if (s < p.num_splits) {
-          ms[s] = cluster_load_f32(cl_ml + r * 2, s);
-          ls[s] = cluster_load_f32(cl_ml + r * 2 + 1, s);
-          os[s] = cluster_load_f32(sm_o + r * D + d, s);
-        }
       float mx = -INFINITY;
-#pragma unroll
-      for (int s = 0; s < 8; ++s)
-        if (s < p.num_splits) mx = fmaxf(mx, ms[s]);
+      for (int s = 0; s < p.num_splits; ++s) mx = fmaxf(mx, recv_ml[(s * 8 * NH + r) * 2]);
       float num = 0.f, den = 0.f;
-#pragma unroll
-      for (int s = 0; s < 8; ++s)
-        if (s < p.num_splits) {
-          const float wgt = ms[s] == -INFINITY ? 0.f : exp2f(ms[s] - mx);
-          num = fmaf(wgt, os[s], num);
-          den = fmaf(wgt, ls[s], den);
-        }
+      for (int s = 0; s < p.num_splits; ++s) {
+        const float ms = recv_ml[(s * 8 * NH + r) * 2];
+        const float wgt = ms == -INFINITY ? 0.f : exp2f(ms - mx);
+        num = fmaf(wgt, recv[s * per_rank + (i - split * per_rank)], num);
+        den = fmaf(wgt, recv_ml[(s * 8 * NH + r) * 2 + 1], den);
+      }
       const float y = finished(den > 0.f ? num / den : 0.f, d, lanes);
       if (stores) p.out[((size_t)q_begin * p.H + kvh * G + g0 + r) * D + d] = __float2bfloat16_rn(y);
     }
-    if (traced) timeline_mark_thread(45, split);        // merged and stored
-    // no block leaves while a peer may still read its shared memory
-    cluster_arrive();
-    cluster_wait();
-    if (traced) timeline_mark_thread(46, split);
-    return;
   }
+  if (traced) timeline_mark_thread(45, split);          // merged and stored
 }
 
-__global__ void __launch_bounds__(THREADS) attn_decode_kernel(MmaAttnParams p) {
-  attn_decode_body<false>(p, nullptr, nullptr);
+// (two blocks share a multiprocessor where their shared memory lets them: heads of up to 128)
+constexpr int DEC_MIN_BLOCKS = D <= 128 ? 2 : 1;
+template <int NH>
+__global__ void __launch_bounds__(DEC_THREADS, DEC_MIN_BLOCKS) attn_decode_kernel(MmaAttnParams p) {
+  attn_decode_body<false, NH>(p, nullptr, nullptr);
 }
 constexpr bool TMA_HEAD = D % 64 == 0;        // boxes are 64 columns wide
-__global__ void __launch_bounds__(THREADS)
+template <int NH>
+__global__ void __launch_bounds__(DEC_THREADS, DEC_MIN_BLOCKS)
 attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                        MmaAttnParams p) {
-  attn_decode_body<TMA_HEAD>(p, &map_k, &map_v);
+  attn_decode_body<TMA_HEAD, NH>(p, &map_k, &map_v);
 }
 
 // out[row] = sum_s 2^(m_s - m) o_s / sum_s 2^(m_s - m) l_s over the key ranges of a row
@@ -989,6 +1113,27 @@ TS_EXPORT int ts_paged_attention_mma_from_qkv(const void* qkv, const float* part
 }
 
 namespace {
+template <bool TMA, int NH>
+int launch_decode(const MmaAttnParams& p, const CUtensorMap& mk, const CUtensorMap& mv, dim3 grid, cudaStream_t stream) {
+  constexpr bool BY_TMA = TMA && TMA_HEAD;
+  const size_t smem = DecShared<BY_TMA>::bytes(8 * NH);
+  static bool configured = false;
+  if (!configured) {
+    const cudaError_t e = BY_TMA ? cudaFuncSetAttribute(attn_decode_tma_kernel<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                                 : cudaFuncSetAttribute(attn_decode_kernel<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return ts_fail("attn_decode: %s", cudaGetErrorString(e));
+    configured = true;
+  }
+  const dim3 block(DEC_THREADS), cluster(1, grid.y, 1);
+  cudaError_t e;
+  if (BY_TMA) e = p.cluster_merge ? ts_launch_cluster(attn_decode_tma_kernel<NH>, grid, block, smem, stream, cluster, mk, mv, p)
+                                  : ts_launch(attn_decode_tma_kernel<NH>, grid, block, smem, stream, mk, mv, p);
+  else e = p.cluster_merge ? ts_launch_cluster(attn_decode_kernel<NH>, grid, block, smem, stream, cluster, p)
+                           : ts_launch(attn_decode_kernel<NH>, grid, block, smem, stream, p);
+  if (e != cudaSuccess) return ts_fail("attn_decode (%d key ranges): %s", (int)grid.y, cudaGetErrorString(e));
+  return 0;
+}
+
 int paged_attention_mma_impl(const MmaAttnParams* from_qkv, const void* q, void* out, const void* k_cache,
                              const void* v_cache, const int* block_table, const int* cu_q, const int* kv_lens,
                              int num_tokens, int num_requests, int max_q_len, int H, int Hkv, int page_size,
@@ -1021,7 +1166,9 @@ int paged_attention_mma_impl(const MmaAttnParams* from_qkv, const void* q, void*
   const int G = H / Hkv;
   cudaError_t e;
   if (decode_only) {
-    p.heads_per_tile = 16; p.queries_per_tile = 1; p.head_tiles = (G + 15) / 16;
+    // up to 8 heads of a KV group a block, up to 16 where there are more
+    const int nh = G <= 8 ? 1 : 2;
+    p.heads_per_tile = 8 * nh; p.queries_per_tile = 1; p.head_tiles = (G + 8 * nh - 1) / (8 * nh);
     // whole pages by TMA where the sizes allow it
     // (pages of 32 and 64 keys: measured on B200, 64 requests x 4096 keys, pages of 64: 6.67 TB/s by
     // TMA against 5.78 by cp.async; with pages of 16 both reach 5.4: the 4 KB pieces are what limits)
@@ -1042,27 +1189,13 @@ int paged_attention_mma_impl(const MmaAttnParams* from_qkv, const void* q, void*
                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS,
                    "paged_attention_mma: cuTensorMapEncodeTiled failed for the cache");
     }
-    const size_t smem = tma ? (size_t)16 * ROW_BYTES + 1024 + (size_t)2 * DEC_STAGES * BN * D * 2
-                            : (size_t)(16 + 2 * DEC_STAGES * BN) * ROW_BYTES;
-    static bool configured = false, configured_tma = false;
-    if (!(tma ? configured_tma : configured)) {
-      e = tma ? cudaFuncSetAttribute(attn_decode_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-              : cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return ts_fail("paged_attention_mma: %s", cudaGetErrorString(e));
-      (tma ? configured_tma : configured) = true;
-    }
     // tile_req / tile_q0 here: the one-token requests of a mixed batch and their tokens
     const int count = tile_req ? num_tiles : num_requests;
-    dim3 grid(Hkv * p.head_tiles, num_splits, count);
-    if (decode_only == 2 && num_splits > 1 && num_splits <= 8) {
-      p.cluster_merge = 1;
-      e = tma ? ts_launch_cluster(attn_decode_tma_kernel, grid, dim3(THREADS), smem, stream, dim3(1, num_splits, 1), mk, mv, p)
-              : ts_launch_cluster(attn_decode_kernel, grid, dim3(THREADS), smem, stream, dim3(1, num_splits, 1), p);
-      if (e != cudaSuccess) return ts_fail("attn_decode (clusters of %d): %s", num_splits, cudaGetErrorString(e));
-      return 0;
-    }
-    if (tma) TS_LAUNCH("attn_decode_tma", attn_decode_tma_kernel, grid, THREADS, smem, stream, mk, mv, p);
-    else TS_LAUNCH("attn_decode", attn_decode_kernel, grid, THREADS, smem, stream, p);
+    const dim3 grid(Hkv * p.head_tiles, num_splits, count);
+    p.cluster_merge = decode_only == 2 && num_splits > 1 && num_splits <= CLUSTER_MAX;
+    const int failed = tma ? (nh == 1 ? launch_decode<true, 1>(p, mk, mv, grid, stream) : launch_decode<true, 2>(p, mk, mv, grid, stream))
+                           : (nh == 1 ? launch_decode<false, 1>(p, mk, mv, grid, stream) : launch_decode<false, 2>(p, mk, mv, grid, stream));
+    if (failed || p.cluster_merge) return failed;
     if (num_splits > 1) {
       TS_LAUNCH("attention_combine", attention_combine_kernel, (tile_req ? count : num_tokens) * H,
                 D >= 128 ? 128 : (D >= 64 ? 64 : 32), 0, stream,
