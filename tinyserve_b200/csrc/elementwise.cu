@@ -1351,83 +1351,91 @@ __global__ void qk_norm_rope_kvwrite_rows_kernel(const T* __restrict__ qkv, T* _
   }
 }
 
-// The same for head sizes 64, 128 and 256, with four neighbouring elements of each half per lane
-// (8- or 16-byte accesses): LPH = D / 8 lanes share a head, a warp works on 32 / LPH heads at once.
-template <typename T, int LPH>
-__global__ void qk_norm_rope_kvwrite_rows4_kernel(const T* __restrict__ qkv, T* __restrict__ q_out,
-                                                  const int* __restrict__ positions, RopeArgs rope,
-                                                  VecParam qw, VecParam kw, int has_norm, float eps,
-                                                  int H, int Hkv, T* __restrict__ k_cache,
-                                                  T* __restrict__ v_cache,
-                                                  const int* __restrict__ slot_mapping, int page_size,
-                                                  int heads_total) {
-  constexpr int D = LPH * 8, HALF = D / 2, HPW = 32 / LPH, U = 3;
+// The same for head sizes 64, 128 and 256, with eight neighbouring elements of each half per lane (16-byte accesses for
+// bfloat16): LPH = D / 16 lanes share a head.  A lane keeps its head for TOK tokens, so that a norm's weights are fetched
+// once for all of them, before the wait, and all tokens' rows are in flight together.  Bound by bytes (the rows read and
+// written once); a block per token, whose warps walked its heads with 8-byte accesses, spent its time on what it fetched
+// before the first row.  That form -> this one, heads of 128, 8 key heads, us: 2,048 tokens of 16 / 32 / 64 heads 11.2 ->
+// 5.9, 12.3 -> 10.0, 21.2 -> 14.7; 4,096 of 32 30.6 -> 25.3 (201 MB); 512 of 32 4.5 -> 3.0.
+template <typename T> struct Raw8 { uint4 part[sizeof(T) / 2]; };      // eight elements as they lie in memory
+template <typename T, int LPH, int TOK>
+__global__ void __launch_bounds__(512, sizeof(T) == 2 ? 2 : 1)
+qk_norm_rope_kvwrite_rows8_kernel(const T* __restrict__ qkv, T* __restrict__ q_out,
+                                  const int* __restrict__ positions, RopeArgs rope,
+                                  VecParam qw, VecParam kw, int has_norm, float eps,
+                                  int H, int Hkv, T* __restrict__ k_cache, T* __restrict__ v_cache,
+                                  const int* __restrict__ slot_mapping, int page_size, int heads_total, int num_tokens) {
+  constexpr int D = LPH * 16, HALF = D / 2, HPW = 32 / LPH;
   pdl_trigger();
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int sub = lane / LPH, j = 4 * (lane % LPH);
-  const int t = blockIdx.x;
-  const int pos = positions[t];
-  const int slot = slot_mapping ? slot_mapping[t] : -1;
-  float c[4], sn[4], wqa[4], wqb[4], wka[4], wkb[4];
-  Quad<float>::load(rope.cos + (size_t)pos * HALF + j, c);
-  Quad<float>::load(rope.sin + (size_t)pos * HALF + j, sn);
+  const int head = (blockIdx.y * warps + warp) * HPW + lane / LPH, j = 8 * (lane % LPH);
+  const bool in = head < heads_total, is_q = head < H, is_v = head >= H + Hkv;
+  const int t0 = blockIdx.x * TOK;
+  int pos[TOK], slot[TOK];
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    wqa[e] = has_norm ? qw[j + e] : 1.f;
-    wqb[e] = has_norm ? qw[HALF + j + e] : 1.f;
-    wka[e] = has_norm ? kw[j + e] : 1.f;
-    wkb[e] = has_norm ? kw[HALF + j + e] : 1.f;
+  for (int k = 0; k < TOK; ++k) {
+    const int t = min(t0 + k, num_tokens - 1);
+    pos[k] = positions[t];
+    slot[k] = slot_mapping ? slot_mapping[t] : -1;
+  }
+  float wa[8], wb[8];
+  if (has_norm && in && !is_v) {
+    const VecParam w = is_q ? qw : kw;
+    if (w.is_f32) {
+      load8(static_cast<const float*>(w.ptr) + j, wa);
+      load8(static_cast<const float*>(w.ptr) + HALF + j, wb);
+    } else {
+      load8(static_cast<const __nv_bfloat16*>(w.ptr) + j, wa);
+      load8(static_cast<const __nv_bfloat16*>(w.ptr) + HALF + j, wb);
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) wa[e] = wb[e] = 1.f;
   }
   pdl_wait();
-  const size_t page = slot >= 0 ? slot / page_size : 0, in_page = slot >= 0 ? slot % page_size : 0;
-  const T* row = qkv + (size_t)t * (H + 2 * Hkv) * D;
-  for (int base = warp * HPW; base < heads_total; base += warps * HPW * U) {
-    float a[U][4], b[U][4];
+  Raw8<T> raw_a[TOK], raw_b[TOK];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int head = base + sub + u * warps * HPW;
-      if (head < heads_total) {
-        Quad<T>::load(row + (size_t)head * D + j, a[u]);
-        Quad<T>::load(row + (size_t)head * D + HALF + j, b[u]);
-      } else {
+  for (int k = 0; k < TOK; ++k) {
+    const T* src = qkv + ((size_t)min(t0 + k, num_tokens - 1) * (H + 2 * Hkv) + (in ? head : 0)) * D + j;
+    raw_a[k] = *reinterpret_cast<const Raw8<T>*>(src);
+    raw_b[k] = *reinterpret_cast<const Raw8<T>*>(src + HALF);
+  }
+  const int kvh = is_q ? 0 : (is_v ? head - H - Hkv : head - H);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) a[u][e] = b[u][e] = 0.f;
-      }
+  for (int k = 0; k < TOK; ++k) {
+    float a[8], b[8], acc = 0.f;
+    load8(reinterpret_cast<const T*>(&raw_a[k]), a);
+    load8(reinterpret_cast<const T*>(&raw_b[k]), b);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc += a[e] * a[e] + b[e] * b[e];
+#pragma unroll
+    for (int o = LPH / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (!in || t0 + k >= num_tokens || (!is_q && slot[k] < 0)) continue;
+    T* dst;
+    if (is_q) {
+      dst = q_out + ((size_t)(t0 + k) * H + head) * D;
+    } else {
+      const size_t page = slot[k] / page_size, in_page = slot[k] % page_size;
+      dst = (is_v ? v_cache : k_cache) + ((page * Hkv + kvh) * page_size + in_page) * D;
     }
+    if (!is_v) {
+      float c[8], sn[8];
+      load8(rope.cos + (size_t)pos[k] * HALF + j, c);
+      load8(rope.sin + (size_t)pos[k] * HALF + j, sn);
+      const float rstd = has_norm ? rsqrtf(acc / (float)D + eps) : 1.f;
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int head = base + sub + u * warps * HPW;
-      float acc = 0.f;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc += a[u][e] * a[u][e] + b[u][e] * b[u][e];
-#pragma unroll
-      for (int o = LPH / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (head >= heads_total) continue;
-      const bool is_q = head < H, is_v = head >= H + Hkv;
-      if (!is_q && slot < 0) continue;
-      const int kvh = is_q ? 0 : (is_v ? head - H - Hkv : head - H);
-      T* dst = is_q ? q_out + ((size_t)t * H + head) * D
-                    : (is_v ? v_cache : k_cache) + ((page * Hkv + kvh) * page_size + in_page) * D;
-      float oa[4], ob[4];
-      if (is_v) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) { oa[e] = a[u][e]; ob[e] = b[u][e]; }
-      } else {
-        const float rstd = has_norm ? rsqrtf(acc / (float)D + eps) : 1.f;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          float x0 = a[u][e], x1 = b[u][e];
-          if (has_norm) {
-            x0 *= rstd * (is_q ? wqa[e] : wka[e]);
-            x1 *= rstd * (is_q ? wqb[e] : wkb[e]);
-          }
-          oa[e] = x0 * c[e] - x1 * sn[e];
-          ob[e] = x1 * c[e] + x0 * sn[e];
+      for (int e = 0; e < 8; ++e) {
+        float x0 = a[e], x1 = b[e];
+        if (has_norm) {
+          x0 *= rstd * wa[e];
+          x1 *= rstd * wb[e];
         }
+        a[e] = x0 * c[e] - x1 * sn[e];
+        b[e] = x1 * c[e] + x0 * sn[e];
       }
-      Quad<T>::store(dst + j, oa);
-      Quad<T>::store(dst + HALF + j, ob);
     }
+    store8(dst + j, a);
+    store8(dst + HALF + j, b);
   }
 }
 
@@ -1468,23 +1476,34 @@ TS_EXPORT int ts_qk_norm_rope_kvwrite(int dtype, const void* qkv, void* q_out, c
   TS_LAUNCH("qk_norm_rope_kvwrite", (qk_norm_rope_kvwrite_rows_kernel<T, STEPS>), dim3(num_tokens), warps * 32, 0, \
             stream, (const T*)qkv, (T*)q_out, positions, rope, qw, kw, has_norm, eps, H, Hkv, D, (T*)k_cache, \
             (T*)v_cache, slot_mapping, page_size, heads_total)
-#define TS_ROPE_ROWS4(T, LPH)                                                                         \
-  TS_LAUNCH("qk_norm_rope_kvwrite", (qk_norm_rope_kvwrite_rows4_kernel<T, LPH>), dim3(num_tokens), warps * 32, 0, \
-            stream, (const T*)qkv, (T*)q_out, positions, rope, qw, kw, has_norm, eps, H, Hkv, (T*)k_cache,  \
-            (T*)v_cache, slot_mapping, page_size, heads_total)
   const bool aligned16 = (reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(q_out) |
                           reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache) |
-                          reinterpret_cast<uintptr_t>(cos) | reinterpret_cast<uintptr_t>(sin)) % 16 == 0;
-  if (vec && aligned16 && num_tokens >= 256 && partials == nullptr && (D == 64 || D == 128 || D == 256) &&
+                          reinterpret_cast<uintptr_t>(cos) | reinterpret_cast<uintptr_t>(sin) |
+                          reinterpret_cast<uintptr_t>(q_weight) | reinterpret_cast<uintptr_t>(k_weight)) % 16 == 0;
+  // From 128 tokens on (16 / 32 / 64 heads, us, a warp per head -> eight elements per lane: 96 tokens 1.6 -> 1.8, 2.0 -> 2.2,
+  // 3.2 -> 2.3; 203 tokens 2.9 -> 2.3, 3.8 -> 2.2, 5.5 -> 2.3); from 512 on there are blocks enough for two tokens each.
+  constexpr int ROWS8_MIN = 128, ROWS8_TOK = 2;
+  if (vec && aligned16 && num_tokens >= ROWS8_MIN && partials == nullptr && (D == 64 || D == 128 || D == 256) &&
       (dtype == TS_F32 || dtype == TS_BF16)) {
+    const int per_warp = 512 / D, need = (heads_total + per_warp - 1) / per_warp;
+    const int tok = num_tokens >= 512 ? ROWS8_TOK : 1;
+    const int parts = (need + 15) / 16, block_warps = (need + parts - 1) / parts;
+    const dim3 rows_grid((num_tokens + tok - 1) / tok, parts);
+#define TS_ROPE_ROWS8(T, LPH, TOK)                                                                     \
+  TS_LAUNCH("qk_norm_rope_kvwrite", (qk_norm_rope_kvwrite_rows8_kernel<T, LPH, TOK>), rows_grid, block_warps * 32, 0, \
+            stream, (const T*)qkv, (T*)q_out, positions, rope, qw, kw, has_norm, eps, H, Hkv, (T*)k_cache,  \
+            (T*)v_cache, slot_mapping, page_size, heads_total, num_tokens)
+#define TS_ROPE_ROWS8_D(T, TOK) \
+  do { if (D == 64) TS_ROPE_ROWS8(T, 4, TOK); else if (D == 128) TS_ROPE_ROWS8(T, 8, TOK); else TS_ROPE_ROWS8(T, 16, TOK); } while (0)
     if (dtype == TS_F32) {
-      if (D == 64) TS_ROPE_ROWS4(float, 8); else if (D == 128) TS_ROPE_ROWS4(float, 16); else TS_ROPE_ROWS4(float, 32);
+      if (tok == 1) TS_ROPE_ROWS8_D(float, 1); else TS_ROPE_ROWS8_D(float, ROWS8_TOK);
     } else {
-      if (D == 64) TS_ROPE_ROWS4(__nv_bfloat16, 8); else if (D == 128) TS_ROPE_ROWS4(__nv_bfloat16, 16); else TS_ROPE_ROWS4(__nv_bfloat16, 32);
+      if (tok == 1) TS_ROPE_ROWS8_D(__nv_bfloat16, 1); else TS_ROPE_ROWS8_D(__nv_bfloat16, ROWS8_TOK);
     }
+#undef TS_ROPE_ROWS8_D
+#undef TS_ROPE_ROWS8
     return 0;
   }
-#undef TS_ROPE_ROWS4
   if (vec && num_tokens >= 256 && partials == nullptr && D <= 256 && (dtype == TS_F32 || dtype == TS_BF16)) {
     const int steps = (D / 4 + 31) / 32;
     if (dtype == TS_F32) {
