@@ -64,6 +64,7 @@ struct MmaAttnParams {
   int num_splits, window;
   int keep_first;           // with a window: keys below this stay visible
   const float* sinks;       // [H] or null
+  int num_tokens;           // T
   int chunk;                // > 0: a query at position i sees key j only if i / chunk == j / chunk (no window then)
   const float* slopes;      // [H] or null: slopes[h] * (i - j) is taken off head h's scaled score
   TurnBack turn;            // outputs turned back by their query's position; cos null: none
@@ -665,6 +666,27 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
   __shared__ uint64_t full[DEC_BARRIERS];            // the tile's bytes have landed
   __shared__ int abort_flag_s;
   volatile int* abort_flag = &abort_flag_s;
+  // The block starts when a block of the projection leaves its place, so what comes before its wait is on the critical
+  // path, and under the stream of weights a load takes more than a microsecond.  Everything that can be asked for at once
+  // is: the lengths, the first pages of the request's table, the norms' weights and, as long as the token's number is
+  // not known, position and slot of token b (with one token a request it is that one).  The angles are the only second trip.
+  // with a request list block z handles its entry z (the one-token requests of a mixed batch)
+  const int b = p.tile_req ? p.tile_req[blockIdx.z] : blockIdx.z, split = blockIdx.y;
+  const int kvh = blockIdx.x / p.head_tiles, head_tile = blockIdx.x % p.head_tiles;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, group = warp >> 2;
+  const int* bt = p.block_table + (size_t)b * p.max_blocks;
+  const int q_begin = p.cu_q[b], q_end = p.cu_q[b + 1], kv_len = p.kv_lens[b];
+  const int first_pages = TMA && lane < p.max_blocks ? bt[lane] : 0;
+  // from the projection itself the newest key never comes from the cache: every tile may be
+  // fetched before the wait, without that key, which this block makes itself
+  const bool from_qkv = p.from_qkv != 0;
+  int slot = -1, pos_q = 0;
+  HeadConsts hq, hk;
+  if (from_qkv) {
+    if (b < p.num_tokens) { pos_q = p.positions[b]; slot = p.slot_mapping[b]; }
+    load_weights(hq, p.q_weight, p.has_norm, lane);
+    if (warp == 0) load_weights(hk, p.k_weight, p.has_norm, lane);
+  }
   if (threadIdx.x == 0) {
     for (int s = 0; s < DEC_BARRIERS; ++s) mbar_init(smem_u32(&full[s]), TMA ? 1 : DEC_GROUP);
     abort_flag_s = 0;
@@ -679,15 +701,8 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
   // step's kernels began: the first tiles are fetched before pdl_wait(), while the kernels that
   // make this token's query, key and value still run.  The tile with the newest key and the
   // query follow after it.
-  // with a request list block z handles its entry z (the one-token requests of a mixed batch)
-  const int b = p.tile_req ? p.tile_req[blockIdx.z] : blockIdx.z, split = blockIdx.y;
-  const int kvh = blockIdx.x / p.head_tiles, head_tile = blockIdx.x % p.head_tiles;
-  const int q_begin = p.cu_q[b];
-  if (p.cu_q[b + 1] - q_begin != 1) return;
-  const int kv_len = p.kv_lens[b];
+  if (q_end - q_begin != 1) return;
   const int G = p.H / p.Hkv, g0 = head_tile * 8 * NH, ng = min(8 * NH, G - g0);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, group = warp >> 2;
-  const int* bt = p.block_table + (size_t)b * p.max_blocks;
   const int qpos = kv_len - 1;
   const int j_hi = kv_len;
   const int j_lo = p.chunk > 0 ? max(0, qpos) / p.chunk * p.chunk : (p.window > 0 ? max(0, qpos - p.window + 1) : 0);
@@ -704,9 +719,6 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
   const int walk_begin = split * per_split;
   const int n_tiles = max(0, min(total, walk_begin + per_split) - walk_begin);
   const int newest_tile = qpos / BN;
-  // from the projection itself the newest key never comes from the cache: every tile may be
-  // fetched before the wait, without that key, which this block makes itself
-  const bool from_qkv = p.from_qkv != 0;
   const int j_load = from_qkv ? j_hi - 1 : j_hi;
   const bool has_newest = from_qkv && total - 1 >= walk_begin && total - 1 < walk_begin + n_tiles;   // (the walk ends with it)
   __shared__ __align__(16) bf16 newest_kv[2 * D];
@@ -723,10 +735,13 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
         const int pages_per_tile = BN >> p.page_shift, boxes = pages_per_tile * (D / 64) * 2;
         if (lane == 0) mbar_expect_tx(bar, 2 * KV_TILE);
         __syncwarp();
-        for (int k = lane; k < boxes; k += 32) {
-          const int values = k & 1, c = (k >> 1) % (D / 64), pg = (k >> 1) / (D / 64);
-          const int j = tile * BN + (pg << p.page_shift);
-          const int page = j < j_hi ? bt[j >> p.page_shift] : 0;                        // past the end: the null page
+        for (int k0 = 0; k0 < boxes; k0 += 32) {
+          const int k = k0 + lane, values = k & 1, c = (k >> 1) % (D / 64), pg = (k >> 1) / (D / 64);
+          const int j = tile * BN + (pg << p.page_shift), at = j >> p.page_shift;
+          int page = __shfl_sync(0xffffffffu, first_pages, at & 31);
+          if (k >= boxes) continue;
+          if (j >= j_hi) page = 0;                                                      // past the end: the null page
+          else if (at >= 32) page = bt[at];
           const int row = (values ? page * p.Hv + kvh / p.v_share : page * p.Hkv + kvh) << p.page_shift;
           const int off = stage * KV_TILE + c * (BN * 128) + (pg << p.page_shift) * 128;
           tma_load_2d(smem_u32((values ? Vs : Ks) + off), values ? map_v : map_k, bar, c * 64, row);
@@ -746,15 +761,11 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
   // range as their value
   const bool traced = blockIdx.x == 0 && blockIdx.z == 0 && threadIdx.x == 0;
   if (traced) timeline_mark_thread(40, split);          // first tiles on their way
-  int slot = -1;
-  HeadConsts hq, hk;
   if (from_qkv) {
-    const int pos_q = p.positions[q_begin];
-    slot = p.slot_mapping[q_begin];
+    if (q_begin != b) { pos_q = p.positions[q_begin]; slot = p.slot_mapping[q_begin]; }
     load_angles(hq, p, pos_q, lane);
-    load_weights(hq, p.q_weight, p.has_norm, lane);
-    hk = hq;
-    if (has_newest && warp == 0) load_weights(hk, p.k_weight, p.has_norm, lane);
+#pragma unroll
+    for (int s = 0; s < ROPE_STEPS; ++s) { hk.c[s] = hq.c[s]; hk.sn[s] = hq.sn[s]; }
   }
   if (traced) timeline_mark_thread(41, split);          // constants fetched
   pdl_wait();
@@ -1157,7 +1168,7 @@ int paged_attention_mma_impl(const MmaAttnParams* from_qkv, const void* q, void*
   p.tile_q0 = tile_q0;
   TS_REQUIRE((tile_req == nullptr) == (tile_q0 == nullptr) && (tile_req == nullptr || num_tiles > 0),
              "paged_attention_mma: the work list is incomplete");
-  p.H = H; p.Hkv = Hkv; p.max_blocks = max_blocks;
+  p.H = H; p.Hkv = Hkv; p.max_blocks = max_blocks; p.num_tokens = num_tokens;
   p.v_share = v_share; p.Hv = Hkv / v_share;
   p.page_shift = 0;
   while ((1 << p.page_shift) < page_size) ++p.page_shift;
