@@ -1357,7 +1357,10 @@ __global__ void qk_norm_rope_kvwrite_rows_kernel(const T* __restrict__ qkv, T* _
 // written once); a block per token, whose warps walked its heads with 8-byte accesses, spent its time on what it fetched
 // before the first row.  That form -> this one, heads of 128, 8 key heads, us: 2,048 tokens of 16 / 32 / 64 heads 11.2 ->
 // 5.9, 12.3 -> 10.0, 21.2 -> 14.7; 4,096 of 32 30.6 -> 25.3 (201 MB); 512 of 32 4.5 -> 3.0.
-template <typename T> struct Raw8 { uint4 part[sizeof(T) / 2]; };      // eight elements as they lie in memory
+// eight elements as they lie in memory (of the type that load8 reads them by)
+template <typename T> struct Raw8;
+template <> struct Raw8<float> { float4 part[2]; };
+template <> struct Raw8<__nv_bfloat16> { uint4 part; };
 template <typename T, int LPH, int TOK>
 __global__ void __launch_bounds__(512, sizeof(T) == 2 ? 2 : 1)
 qk_norm_rope_kvwrite_rows8_kernel(const T* __restrict__ qkv, T* __restrict__ q_out,
