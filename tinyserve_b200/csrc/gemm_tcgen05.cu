@@ -264,6 +264,7 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
         const int m = t_tile * TILE_T + j;
         float sum = 0.f;
         if (m < p.M)
+#pragma unroll 8
           for (int t = 0; t < p.x_tiles; ++t) sum += __ldcg(p.x_sumsq + (size_t)t * SUMSQ_STRIDE + m);
         row_scale[j] = rsqrtf(sum / (float)p.K + p.x_eps);
       }

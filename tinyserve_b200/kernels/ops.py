@@ -202,7 +202,7 @@ class PendingProduct:
 
 class ScaledRows:
     """Rows that still lack their RMSNorm factor: ``data`` [M, N] holds residual * norm_weight in
-    bfloat16 and ``sumsq`` [tiles, 16] the sums of residual^2 over each 128 columns.  ``linear``
+    bfloat16 and ``sumsq`` [tiles, 16] the sums of residual^2 over each 128 (or 16) columns.  ``linear``
     takes it as x and scales every token's result by rsqrt(sum / N + eps) in its epilogue, which
     is the same product as with normalised rows; ``materialize()`` gives the normalised rows."""
 
@@ -322,6 +322,47 @@ def _gemm():
 
 def _gemm_tcgen05():
     return build.load_unit("gemm_tcgen05.cu")
+
+
+def _gemv():
+    return build.load_unit("gemv_mma.cu")
+
+
+#: Products of up to this many tokens whose weights the device holds in registers at once run on the kernel that loads
+#: them there before its dependency wait (csrc/gemv_mma.cu).
+GEMV_MAX_TOKENS = 8
+GEMV_MAX_BYTES = 1 << 24
+GEMV_MAX_K = 4096
+
+
+def _gemv_fits(M, N, K, gated=False, residual=False):
+    """The residual form leaves sums of squares per 16 columns, which the next product adds up: up to 64 of them."""
+    return (M <= GEMV_MAX_TOKENS and 2 * N * K <= GEMV_MAX_BYTES and K <= (GEMV_MAX_K // 2 if gated else GEMV_MAX_K)
+            and (not gated or N % 128 == 0) and (not residual or (N % 16 == 0 and N <= 1024)))
+
+
+def _linear_gemv(x, weight, out_float32=False, partials_only=False, scale=None, gated=0, limit=0.0, residual=None, norm_weight=None):
+    """The product of up to GEMV_MAX_TOKENS tokens (operands as for the tcgen05 kernel); see ``_linear_tcgen05`` for the
+    arguments.  ``residual`` with ``norm_weight``: returns (hprime, sumsq) of the new residual."""
+    M, K = x.shape
+    N = weight.shape[0]
+    out = partials = hprime = sumsq = None
+    if residual is not None:
+        hprime = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)
+        sumsq = torch.empty(N // 16, 16, dtype=torch.float32, device=x.device)
+    elif partials_only:
+        partials = torch.empty(-(-N // 128) * 16 * 128, dtype=torch.float32, device=x.device)
+    else:
+        out = torch.empty(M, N // 2 if gated else N, dtype=torch.float32 if out_float32 else torch.bfloat16, device=x.device)
+    lib = _gemv()
+    _check(lib, lib.ts_gemv_mma(
+        _ptr(x), _ptr(weight), _ptr(out), _ptr(partials), c_int(M), c_int(N), c_int(K), c_longlong(x.stride(0)), c_longlong(weight.stride(0)),
+        c_longlong(out.stride(0) if out is not None else 0), c_int(1 if out_float32 else 0), *(scale.args() if scale is not None else _NO_SCALE),
+        _ptr(residual), _ptr(norm_weight), c_int(_vec_flag(norm_weight, torch.bfloat16) if norm_weight is not None else 0),
+        _ptr(hprime), _ptr(sumsq), c_int(gated), c_float(limit), _stream()))
+    if residual is not None:
+        return hprime, sumsq
+    return SplitPartials(partials, 1, M, N, 16, torch.bfloat16) if partials_only else out
 
 
 _counters: dict = {}
@@ -585,7 +626,7 @@ def units_for(head_dims, key_dims=(), delta_dims=()) -> list:
     """The (source, defines) units a model with these attention head sizes, these key sizes of
     its matrix-state mixers and these of its delta-rule mixers needs."""
     units = [("elementwise.cu", {}), ("gemm_simt.cu", {}), ("gemm_tcgen05.cu", {}), ("gemm_pair_tcgen05.cu", {}),
-             ("sampler.cu", {}), ("latent_moe.cu", {}), ("sequence.cu", {}), ("streams.cu", {})]
+             ("gemv_mma.cu", {}), ("sampler.cu", {}), ("latent_moe.cu", {}), ("sequence.cu", {}), ("streams.cu", {})]
     units += [("attention_simt.cu", {"TS_HEAD_DIM": d}) for d in sorted(set(head_dims))]
     units += [("attention_mma.cu", _mma_defines(d)) for d in sorted(set(head_dims))
               if d <= MMA_MAX_HEAD_DIM]
@@ -651,6 +692,9 @@ def _product_add_residual(pending, residual, weight, eps, x_scale=None):
     if pending.wide:
         hprime, sumsq = _linear_pair(x, w, residual=residual, norm_weight=weight)
         return ScaledRows(hprime, sumsq, tiles, eps)
+    if x_scale is None and _gemv_fits(M, N, K, residual=True):
+        hprime, sumsq = _linear_gemv(x, w, residual=residual, norm_weight=weight)
+        return ScaledRows(hprime, sumsq, sumsq.shape[0], eps)
     hprime = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)
     sumsq = torch.empty(tiles, 16, dtype=torch.float32, device=x.device)
     lib = _gemm_tcgen05()
@@ -769,6 +813,8 @@ def gated_linear(x, weight, activation="silu", block=0, limit=0.0, constant_weig
             and (rows is x or rows.shape[0] <= FUSED_MAX_TOKENS)          # (norm factors come for so many rows)
             and (rows.shape[0] <= GATED_MAX_TOKENS // 2 or (rows.shape[0] <= GATED_MAX_TOKENS and N <= 2 * num_sms() * 128))):
         _cuda(rows, weight)
+        if _gemv_fits(rows.shape[0], N, K, gated=True):
+            return _linear_gemv(rows, weight, gated=code + 1, limit=limit, scale=x if rows is not x else None)
         return _linear_tcgen05(rows, weight, False, splits=gated_splits(rows.shape[0], N, K), gated=code + 1, limit=limit,
                                scale=x if rows is not x else None)
     return gated_activation(linear(x, weight, constant_weight=constant_weight), activation, block, limit)
@@ -1189,6 +1235,8 @@ def linear(x, weight, bias=None, out_float32=False, allow_partials=False, allow_
             if scale is not None:
                 x, scale = scale.materialize(), None
             return _linear_tcgen05(x, weight, out_float32, bias=bias)
+        if _gemv_fits(M, N, K):
+            return _linear_gemv(x, weight, out_float32, partials_only=allow_partials and not out_float32, scale=scale)
         if (allow_partials or allow_pending) and not out_float32 \
                 and gemm_splits(x.shape[0], weight.shape[0], x.shape[1], partials=True) > 1:
             return _linear_tcgen05(x, weight, False, partials_only=True, scale=scale)
