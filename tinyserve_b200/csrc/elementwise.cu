@@ -1361,9 +1361,16 @@ __global__ void qk_norm_rope_kvwrite_rows_kernel(const T* __restrict__ qkv, T* _
 template <typename T> struct Raw8;
 template <> struct Raw8<float> { float4 part[2]; };
 template <> struct Raw8<__nv_bfloat16> { uint4 part; };
+// (not loads that the compiler may take for constant and bring forward over the dependency wait)
+__device__ __forceinline__ Raw8<float> load_raw8(const float* p) {
+  return Raw8<float>{{__ldcg(reinterpret_cast<const float4*>(p)), __ldcg(reinterpret_cast<const float4*>(p) + 1)}};
+}
+__device__ __forceinline__ Raw8<__nv_bfloat16> load_raw8(const __nv_bfloat16* p) {
+  return Raw8<__nv_bfloat16>{__ldcg(reinterpret_cast<const uint4*>(p))};
+}
 template <typename T, int LPH, int TOK>
 __global__ void __launch_bounds__(512, sizeof(T) == 2 ? 2 : 1)
-qk_norm_rope_kvwrite_rows8_kernel(const T* __restrict__ qkv, T* __restrict__ q_out,
+qk_norm_rope_kvwrite_rows8_kernel(const T* qkv, T* __restrict__ q_out,
                                   const int* __restrict__ positions, RopeArgs rope,
                                   VecParam qw, VecParam kw, int has_norm, float eps,
                                   int H, int Hkv, T* __restrict__ k_cache, T* __restrict__ v_cache,
@@ -1400,8 +1407,8 @@ qk_norm_rope_kvwrite_rows8_kernel(const T* __restrict__ qkv, T* __restrict__ q_o
 #pragma unroll
   for (int k = 0; k < TOK; ++k) {
     const T* src = qkv + ((size_t)min(t0 + k, num_tokens - 1) * (H + 2 * Hkv) + (in ? head : 0)) * D + j;
-    raw_a[k] = *reinterpret_cast<const Raw8<T>*>(src);
-    raw_b[k] = *reinterpret_cast<const Raw8<T>*>(src + HALF);
+    raw_a[k] = load_raw8(src);
+    raw_b[k] = load_raw8(src + HALF);
   }
   const int kvh = is_q ? 0 : (is_v ? head - H - Hkv : head - H);
 #pragma unroll
