@@ -35,7 +35,13 @@ static_assert(D % 16 == 0 && D >= 16 && D <= 256, "head size must be a multiple 
 constexpr int CH = D / 8;                 // 16-byte chunks of a row
 constexpr int ROW_BYTES = D * 2 + 16;     // rows are padded by one chunk: ldmatrix without conflicts
 constexpr int CLUSTER_MAX = 8;            // key ranges that merge in a cluster
-constexpr int ALONE_TILES = 4;            // key tiles that one block walks without its cluster
+// Key tiles that one block walks without its cluster.  Two, but one in clusters of two blocks where the ranges come by
+// cp.async, the head is wide and the merge short (few query heads a key head).  Clusters of two, 16 requests, 128 keys,
+// in the cluster / alone: heads of 256, one query head 17.8 / 20.4 us, four 22.9 / 22.5, eight 29.7 / 25.3; by TMA
+// 14.1 / 13.1; heads of 96 6.5 / 6.8, of 80 6.2 / 5.8.  In clusters of three and more alone is always the faster.
+__device__ __forceinline__ int alone_tiles(int cluster, int group, bool tma) {
+  return cluster > 2 || D <= 80 || tma || group >= 4 ? 2 : 1;
+}
 #ifndef TS_PREFILL_WARPS
 #define TS_PREFILL_WARPS 4
 #endif
@@ -515,32 +521,28 @@ __device__ __forceinline__ void build_head(const MmaAttnParams& p, int t, int co
   }
 }
 
-// The decode block.  One query against a few hundred keys is a chain of short phases, and what bounds it is how long
-// each of them takes, not bytes; so:
+// The decode block whose query rows and newest keys are there already (a kernel of its own made them).
 // - Scores are made as S^T = K Q^T and outputs as O^T = V^T P^T: the keys (or the columns of V) are the 16 rows of an
 //   mma.sync and the heads its 8 columns, which needs half of the instructions (and registers for O) that heads as rows
 //   take while a KV group has up to 8 heads (NH = 1; NH = 2 for up to 16).  P turns from the one layout into the other by
 //   movmatrix.
-// - Eight warps in two groups: group g takes the tiles g, g + 2, .. of the block's walk, a warp 16 keys of a tile.  A group
-//   waits for its tiles alone and refills the stage that it has emptied; nothing in the walk is common to the block.
-//   Three stages and six mbarriers: tile i lies in stage i % 3 and is counted on barrier i % 6, which always belongs to
-//   the same group, so that no group can miss a phase.
+// - A warp takes 16 keys of every tile and waits for the tile's bytes itself; the block meets only where a stage is filled
+//   again.
 // - The warps' partial sums lie in shared memory in rows of D + 4 floats, which neither side's accesses collide on.
 // - Ranges that are a cluster send their sums to the rank that adds them up, into memory of their own: one cluster
 //   barrier lies between, and nobody has to wait for a reader before it leaves.
-// Heads as rows, four warps a tile, a merge by reading -> this, one launch after the other, us: 32 heads over 8, 540 keys, 1
-// request 9.1 -> 6.7, 8 13.4 -> 9.8, 16 15.3 -> 10.6; 64 of 130 keys 15.4 -> 11.8; 32 of 4,000 91 -> 77 (524 MB); 16 heads
-// over 8, 90 keys 6.5 -> 4.9, 2 of 10,500 24.2 -> 18.9; 64 over 8, pages of 16, 6 of 2,000 37.6 -> 25.9.
+// Bound by bytes where there are many requests: @A@
+// Eight warps on two tiles at once: 2,199 us.  (The block that makes its rows itself, below, keeps heads as rows: in
+// a decode step of few requests this form of it was 2.5 us slower a layer, although it is 2.4 us faster with nothing around it.)
 //
-// TMA false: key and value tiles come by cp.async, 16 bytes a thread of the group, into padded rows (any head
+// TMA false: key and value tiles come by cp.async, 16 bytes a thread, into padded rows (any head
 // size in steps of 16, any page size).  TMA true (head sizes in steps of 64, pages of 32 or 64
-// keys): one warp of the group fetches whole pages as boxes of page x 64 columns with the 128-byte swizzle;
+// keys): one warp fetches whole pages as boxes of page x 64 columns with the 128-byte swizzle;
 // an SM streams about half as much again this way
 // as through its load/store unit's miss queue.  Whole pages come, also the keys past the
 // request's length in its last page: those are masked, and must hold finite numbers (the engine's
 // cache starts as zeros and only ever takes keys and values).
-constexpr int DEC_THREADS = 256, DEC_WARPS = DEC_THREADS / 32, DEC_GROUP = DEC_THREADS / 2;
-constexpr int DEC_BARRIERS = 2 * DEC_STAGES;
+constexpr int DEC_THREADS = 128, DEC_WARPS = DEC_THREADS / 32;
 constexpr int SUM_ROW = D + 4;                       // floats of a row of partial sums (4 mod 16: no bank conflicts)
 
 // the block's shared memory: query rows, stages, and what peers of a cluster send
@@ -561,10 +563,6 @@ __device__ __forceinline__ uint32_t transposed(uint32_t a) {
 // arrives on the mbarrier once every cp.async of this thread so far has landed
 __device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void group_barrier(int group) {
-  if (group == 0) asm volatile("bar.sync 1, %0;\n" ::"n"(DEC_GROUP) : "memory");
-  else asm volatile("bar.sync 2, %0;\n" ::"n"(DEC_GROUP) : "memory");
 }
 __device__ __forceinline__ void cluster_store_f32(float* own_shared, uint32_t rank, float v) {
   uint32_t local = static_cast<uint32_t>(__cvta_generic_to_shared(own_shared)), remote;
@@ -663,32 +661,18 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
                  : Qs + S::Q_BYTES;                  // [DEC_STAGES][KV_TILE]
   char* Vs = Ks + DEC_STAGES * KV_TILE;              // [DEC_STAGES][KV_TILE]
   float* recv = reinterpret_cast<float*>(Vs + DEC_STAGES * KV_TILE);       // peers' sums: [rank][this block's share]
-  __shared__ uint64_t full[DEC_BARRIERS];            // the tile's bytes have landed
+  __shared__ uint64_t full[DEC_STAGES];              // the tile's bytes have landed
   __shared__ int abort_flag_s;
   volatile int* abort_flag = &abort_flag_s;
-  // The block starts when a block of the projection leaves its place, so what comes before its wait is on the critical
-  // path, and under the stream of weights a load takes more than a microsecond.  Everything that can be asked for at once
-  // is: the lengths, the first pages of the request's table, the norms' weights and, as long as the token's number is
-  // not known, position and slot of token b (with one token a request it is that one).  The angles are the only second trip.
   // with a request list block z handles its entry z (the one-token requests of a mixed batch)
   const int b = p.tile_req ? p.tile_req[blockIdx.z] : blockIdx.z, split = blockIdx.y;
   const int kvh = blockIdx.x / p.head_tiles, head_tile = blockIdx.x % p.head_tiles;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, group = warp >> 2;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int* bt = p.block_table + (size_t)b * p.max_blocks;
   const int q_begin = p.cu_q[b], q_end = p.cu_q[b + 1], kv_len = p.kv_lens[b];
-  const int first_pages = TMA && lane < p.max_blocks ? bt[lane] : 0;
-  // from the projection itself the newest key never comes from the cache: every tile may be
-  // fetched before the wait, without that key, which this block makes itself
-  const bool from_qkv = p.from_qkv != 0;
-  int slot = -1, pos_q = 0;
-  HeadConsts hq, hk;
-  if (from_qkv) {
-    if (b < p.num_tokens) { pos_q = p.positions[b]; slot = p.slot_mapping[b]; }
-    load_weights(hq, p.q_weight, p.has_norm, lane);
-    if (warp == 0) load_weights(hk, p.k_weight, p.has_norm, lane);
-  }
+  const int first_pages = TMA && lane < p.max_blocks ? bt[lane] : 0;       // (one trip to memory for what the first tiles need)
   if (threadIdx.x == 0) {
-    for (int s = 0; s < DEC_BARRIERS; ++s) mbar_init(smem_u32(&full[s]), TMA ? 1 : DEC_GROUP);
+    for (int s = 0; s < DEC_STAGES; ++s) mbar_init(smem_u32(&full[s]), TMA ? 1 : DEC_THREADS);
     abort_flag_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
@@ -713,25 +697,21 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
   const int total = (j_hi + BN - 1) / BN - first_tile + kept_tiles;
   auto tile_of = [&](int w) { return w < kept_tiles ? w : first_tile + (w - kept_tiles); };
   // A short walk is one block's: the ranges of a cluster cost their merge.  (All blocks of the cluster see the same.)
-  const bool alone = p.cluster_merge && total <= ALONE_TILES;
+  const bool alone = p.cluster_merge && total <= alone_tiles(p.num_splits, G, TMA);
   const int per_split = alone ? total : (total + p.num_splits - 1) / p.num_splits;
   if (alone && split > 0) return;
   const int walk_begin = split * per_split;
   const int n_tiles = max(0, min(total, walk_begin + per_split) - walk_begin);
   const int newest_tile = qpos / BN;
-  const int j_load = from_qkv ? j_hi - 1 : j_hi;
-  const bool has_newest = from_qkv && total - 1 >= walk_begin && total - 1 < walk_begin + n_tiles;   // (the walk ends with it)
-  __shared__ __align__(16) bf16 newest_kv[2 * D];
-
-  // tile i of this block's walk into its stage, by the group that is not going to read it (the one that emptied the stage)
+  // tile i of this block's walk into its stage
   auto load_tile = [&](int i) {
     const int tile = tile_of(walk_begin + i), stage = i % DEC_STAGES;
-    const uint32_t bar = smem_u32(&full[i % DEC_BARRIERS]);
+    const uint32_t bar = smem_u32(&full[stage]);
     if (TMA) {
       // the boxes of a tile (pages x 64-column chunks x keys/values) are dealt to the lanes of
-      // the group's first warp, so that issuing them costs the block one box's time, not sixteen; lane 0's
+      // the first warp, so that issuing them costs the block one box's time, not sixteen; lane 0's
       // arrival carries the tile's byte count, so the stage cannot complete before it
-      if ((warp & 3) == 0) {
+      if (warp == 0) {
         const int pages_per_tile = BN >> p.page_shift, boxes = pages_per_tile * (D / 64) * 2;
         if (lane == 0) mbar_expect_tx(bar, 2 * KV_TILE);
         __syncwarp();
@@ -748,65 +728,30 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
         }
       }
     } else {
-      load_kv_tile<BN, DEC_GROUP>(Ks + stage * KV_TILE, Vs + stage * KV_TILE, p, bt, kvh, tile * BN, j_lo, j_load, keep,
-                                  threadIdx.x & (DEC_GROUP - 1));
+      load_kv_tile<BN, DEC_THREADS>(Ks + stage * KV_TILE, Vs + stage * KV_TILE, p, bt, kvh, tile * BN, j_lo, j_hi, keep, threadIdx.x);
       cp_async_arrive(bar);
     }
   };
-  const int late = from_qkv ? -1 : newest_tile;      // its newest key is there after the wait only
+  // (the newest key is there after the wait only)
 #pragma unroll
   for (int s = 0; s < DEC_STAGES; ++s)
-    if (s < n_tiles && group == ((s + 1) & 1) && tile_of(walk_begin + s) != late) load_tile(s);
+    if (s < n_tiles && tile_of(walk_begin + s) != newest_tile) load_tile(s);
   // the timeline build follows the blocks of one (request, KV group): marks 40.. with the key
   // range as their value
   const bool traced = blockIdx.x == 0 && blockIdx.z == 0 && threadIdx.x == 0;
   if (traced) timeline_mark_thread(40, split);          // first tiles on their way
-  if (from_qkv) {
-    if (q_begin != b) { pos_q = p.positions[q_begin]; slot = p.slot_mapping[q_begin]; }
-    load_angles(hq, p, pos_q, lane);
-#pragma unroll
-    for (int s = 0; s < ROPE_STEPS; ++s) { hk.c[s] = hq.c[s]; hk.sn[s] = hq.sn[s]; }
-  }
-  if (traced) timeline_mark_thread(41, split);          // constants fetched
   pdl_wait();
   if (traced) timeline_mark_thread(42, split);          // the projection is there
-  if (from_qkv) {
-    // the heads this block makes, dealt to the warps in turn: the newest key (norm, rotary) and
-    // value where this block holds them, then the query rows; rows past the group are zero
-    const int extra = has_newest ? 2 : 0;
-    for (int i = warp; i < extra + 8 * NH; i += DEC_WARPS) {
-      if (i < extra) {
-        build_head(p, q_begin, (p.H + (i == 0 ? 0 : p.Hkv) + kvh) * D, i == 0, hk, lane, newest_kv + i * D);
-        continue;
-      }
-      const int r = i - extra;
-      bf16* row = reinterpret_cast<bf16*>(Qs + r * ROW_BYTES);
-      if (r < ng) {
-        build_head(p, q_begin, (kvh * G + g0 + r) * D, true, hq, lane, row);
-      } else {
-        for (int d = lane * 2; d < D; d += 64) *reinterpret_cast<uint32_t*>(row + d) = 0u;
-      }
-    }
-  } else {
-    for (int i = threadIdx.x; i < 8 * NH * CH; i += DEC_THREADS) {
-      const int r = i / CH, c = i % CH;
-      const uint4 q = r < ng ? *reinterpret_cast<const uint4*>(p.q + ((size_t)q_begin * p.H + kvh * G + g0 + r) * D + c * 8)
-                             : make_uint4(0u, 0u, 0u, 0u);
-      *reinterpret_cast<uint4*>(Qs + r * ROW_BYTES + c * 16) = q;
-    }
+  for (int i = threadIdx.x; i < 8 * NH * CH; i += DEC_THREADS) {
+    const int r = i / CH, c = i % CH;
+    const uint4 q = r < ng ? __ldcg(reinterpret_cast<const uint4*>(p.q + ((size_t)q_begin * p.H + kvh * G + g0 + r) * D + c * 8))
+                           : make_uint4(0u, 0u, 0u, 0u);
+    *reinterpret_cast<uint4*>(Qs + r * ROW_BYTES + c * 16) = q;
+  }
 #pragma unroll
-    for (int s = 0; s < DEC_STAGES; ++s)
-      if (s < n_tiles && group == ((s + 1) & 1) && tile_of(walk_begin + s) == late) load_tile(s);
-  }
+  for (int s = 0; s < DEC_STAGES; ++s)
+    if (s < n_tiles && tile_of(walk_begin + s) == newest_tile) load_tile(s);
   __syncthreads();
-  if (has_newest && head_tile == 0 && slot >= 0) {
-    const size_t page = slot >> p.page_shift, in_page = slot & p.page_mask;
-    const size_t at = (((page * p.Hkv + kvh) << p.page_shift) + in_page) * D;
-    for (int d = threadIdx.x * 2; d < 2 * D; d += DEC_THREADS * 2) {
-      bf16* dst = d < D ? p.k_cache_out + at + d : p.v_cache_out + at + (d - D);
-      *reinterpret_cast<uint32_t*>(dst) = *reinterpret_cast<const uint32_t*>(newest_kv + d);
-    }
-  }
   if (traced) timeline_mark_thread(43, split);          // query rows (and the newest key) made
   const int t = lane & 3;
   float sl[NH][2], m[NH][2], l[NH][2], o[NH][D / 16][4];
@@ -841,31 +786,18 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
     }
   }
 
-  const int key0 = (warp & 3) * 16;
-  for (int it = group; it < n_tiles; it += 2) {
+  const int key0 = warp * 16;
+  for (int it = 0; it < n_tiles; ++it) {
     const int stage = it % DEC_STAGES;
     // bounded; a wait that ran out raises the block's abort flag and the status word, the loop
     // goes on over whatever the stage holds, and the block stores no output at the end
-    mbar_wait(smem_u32(&full[it % DEC_BARRIERS]), (it / DEC_BARRIERS) & 1, abort_flag);
+    mbar_wait(smem_u32(&full[stage]), (it / DEC_STAGES) & 1, abort_flag);
     __syncwarp();
-    char* ks = Ks + stage * KV_TILE;
-    char* vs = Vs + stage * KV_TILE;
     const int jbase = tile_of(walk_begin + it) * BN + key0;
-    if (has_newest && qpos >= jbase && qpos < jbase + 16) {
-      // the newest key and value take their row of the tile (the copy left zeros or stale bytes there), which no other warp reads
-      const int row = qpos - jbase + key0;
-      for (int d = lane * 2; d < 2 * D; d += 64) {
-        const int e = d < D ? d : d - D;          // element of the head; two neighbours per lane
-        char* tile = d < D ? ks : vs;
-        char* dst = TMA ? tile + (e / 64) * (BN * 128) + row * 128 + ((((e % 64) / 8) ^ (row & 7)) << 4) + (e % 8) * 2
-                        : tile + row * ROW_BYTES + e * 2;
-        *reinterpret_cast<uint32_t*>(dst) = *reinterpret_cast<const uint32_t*>(newest_kv + d);
-      }
-      __syncwarp();
-    }
-    if (jbase < j_hi) decode_keys<TMA, NH, Q_REGS>(o, m, l, qf, Qs, ks, vs, key0, jbase, qpos, j_lo, keep, p, sl, lane);
+    if (jbase < j_hi)
+      decode_keys<TMA, NH, Q_REGS>(o, m, l, qf, Qs, Ks + stage * KV_TILE, Vs + stage * KV_TILE, key0, jbase, qpos, j_lo, keep, p, sl, lane);
     if (it + DEC_STAGES < n_tiles) {
-      group_barrier(group);
+      __syncthreads();
       load_tile(it + DEC_STAGES);
     }
   }
@@ -981,8 +913,280 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
   if (traced) timeline_mark_thread(45, split);          // merged and stored
 }
 
+// The decode block that makes its query rows, newest key and value itself from the fused projection (a few requests): a
+// chain of short phases, each a trip to memory or a meeting.  Heads are the 16 rows of the MMAs here; four warps take 16
+// keys each of every tile.  The merge through padded rows and, in a cluster, by sending: @B@
+template <bool TMA>
+__device__ __forceinline__ void attn_decode_qkv_body(const MmaAttnParams& p, const CUtensorMap* map_k,
+                                                 const CUtensorMap* map_v) {
+  extern __shared__ __align__(16) char smem[];
+  constexpr int KV_TILE = TMA ? BN * D * 2 : BN * ROW_BYTES;      // bytes of the keys (or values) of a stage
+  char* Qs = smem;                                   // [16][ROW_BYTES]
+  char* Ks = TMA ? reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(Qs + 16 * ROW_BYTES) + 1023) & ~uintptr_t(1023))
+                 : Qs + 16 * ROW_BYTES;              // [DEC_STAGES][KV_TILE]
+  char* Vs = Ks + DEC_STAGES * KV_TILE;              // [DEC_STAGES][KV_TILE]
+  __shared__ uint64_t full[DEC_STAGES];              // (TMA) the stage's bytes have landed
+  __shared__ int abort_flag_s;
+  volatile int* abort_flag = &abort_flag_s;
+  if (TMA && threadIdx.x == 0) {
+    for (int s = 0; s < DEC_STAGES; ++s) mbar_init(smem_u32(&full[s]), 1);
+    abort_flag_s = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  if (TMA) __syncthreads();
+
+  pdl_trigger();
+  if (p.cluster_merge) cluster_arrive();
+  // The lengths, the block table and every cached key but the newest were written before this
+  // step's kernels began: the first tiles are fetched before pdl_wait(), while the kernels that
+  // make this token's query, key and value still run.  The tile with the newest key and the
+  // query follow after it.
+  const int b = blockIdx.z, split = blockIdx.y;
+  const int kvh = blockIdx.x / p.head_tiles, head_tile = blockIdx.x % p.head_tiles;
+  const int q_begin = p.cu_q[b];
+  if (p.cu_q[b + 1] - q_begin != 1) return;
+  const int kv_len = p.kv_lens[b];
+  const int G = p.H / p.Hkv, g0 = head_tile * 16, ng = min(16, G - g0);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2;
+  const int* bt = p.block_table + (size_t)b * p.max_blocks;
+  const int qpos = kv_len - 1;
+  const int j_hi = kv_len;
+  const int j_lo = p.window > 0 ? max(0, qpos - p.window + 1) : 0;
+  const int first_tile = j_lo / BN, total = (j_hi + BN - 1) / BN - first_tile;
+  auto tile_of = [&](int w) { return first_tile + w; };
+  // A short walk is one block's: the ranges of a cluster cost their merge (a cluster barrier and a round trip through
+  // distributed shared memory), a tile of 64 keys about 1 us.  One request, 16 heads over 8, 60 / 120 / 180 / 250 keys:
+  // 6.4 us in a cluster of eight, 4.5 / 5.4 / 6.5 / 7.7 alone.  (All blocks of the cluster see the same.)
+  const bool alone = p.cluster_merge && total <= alone_tiles(p.num_splits, G, TMA);
+  const int per_split = alone ? total : (total + p.num_splits - 1) / p.num_splits;
+  if (alone && split > 0) return;
+  const int walk_begin = split * per_split;
+  const int n_tiles = max(0, min(total, walk_begin + per_split) - walk_begin);
+  const int newest_tile = qpos / BN;
+  // the newest key never comes from the cache: every tile may be fetched before the wait, without that
+  // key, which this block makes itself
+  const int j_load = j_hi - 1;
+  const bool has_newest = total - 1 >= walk_begin && total - 1 < walk_begin + n_tiles;   // (the walk ends with it)
+  __shared__ __align__(16) bf16 newest_kv[2 * D];
+
+  // tile `tile` of the keys and values into stage `stage`
+  auto load_tile = [&](int stage, int tile) {
+    if (TMA) {
+      // the boxes of a tile (pages x 64-column chunks x keys/values) are dealt to the lanes of
+      // warp 0, so that issuing them costs the block one box's time, not sixteen; lane 0's
+      // arrival carries the tile's byte count, so the stage cannot complete before it
+      if (threadIdx.x < 32) {
+        const int pages_per_tile = BN >> p.page_shift, boxes = pages_per_tile * (D / 64) * 2;
+        const uint32_t bar = smem_u32(&full[stage]);
+        if (threadIdx.x == 0) mbar_expect_tx(bar, 2 * KV_TILE);
+        __syncwarp();
+        for (int i = threadIdx.x; i < boxes; i += 32) {
+          const int values = i & 1, c = (i >> 1) % (D / 64), pg = (i >> 1) / (D / 64);
+          const int j = tile * BN + (pg << p.page_shift);
+          const int page = j < j_hi ? bt[j >> p.page_shift] : 0;                        // past the end: the null page
+          const int row = (page * p.Hkv + kvh) << p.page_shift;
+          const int off = stage * KV_TILE + c * (BN * 128) + (pg << p.page_shift) * 128;
+          tma_load_2d(smem_u32((values ? Vs : Ks) + off), values ? map_v : map_k, bar, c * 64, row);
+        }
+      }
+    } else {
+      load_kv_tile<BN, DEC_THREADS>(Ks + stage * KV_TILE, Vs + stage * KV_TILE, p, bt, kvh, tile * BN, j_lo, j_load, 0, threadIdx.x);
+    }
+  };
+#pragma unroll
+  for (int s = 0; s < DEC_STAGES - 1; ++s)
+    if (s < n_tiles) load_tile(s, tile_of(walk_begin + s));
+  // the timeline build follows the blocks of one (request, KV group): marks 40.. with the key
+  // range as their value
+  const bool traced = blockIdx.x == 0 && blockIdx.z == 0 && threadIdx.x == 0;
+  if (traced) timeline_mark_thread(40, split);          // first tiles on their way
+  const int pos_q = p.positions[q_begin], slot = p.slot_mapping[q_begin];
+  HeadConsts hq, hk;
+  load_angles(hq, p, pos_q, lane);
+  load_weights(hq, p.q_weight, p.has_norm, lane);
+  hk = hq;
+  if (has_newest) load_weights(hk, p.k_weight, p.has_norm, lane);
+  if (traced) timeline_mark_thread(41, split);          // constants fetched
+  pdl_wait();
+  if (traced) timeline_mark_thread(42, split);          // the projection is there
+  // the heads this block makes, dealt to the warps in turn: the newest key (norm, rotary) and
+  // value where this block holds them, then the query rows; rows past the group are zero
+  const int extra = has_newest ? 2 : 0;
+  for (int i = warp; i < extra + 16; i += DEC_WARPS) {
+    const int r = i - extra;
+    bf16* row = i < extra ? newest_kv + i * D : reinterpret_cast<bf16*>(Qs + r * ROW_BYTES);
+    if (i < extra || r < ng) {
+      const int head = i < extra ? p.H + (i == 0 ? 0 : p.Hkv) + kvh : kvh * G + g0 + r;
+      HeadConsts h = hq;
+#pragma unroll
+      for (int k = 0; k < ROPE_STEPS; ++k)
+        if (i < extra) { h.wa[k] = hk.wa[k]; h.wb[k] = hk.wb[k]; }
+      build_head(p, q_begin, head * D, i != 1 || extra == 0, h, lane, row);
+    } else {
+      for (int d = lane * 2; d < D; d += 64) *reinterpret_cast<uint32_t*>(row + d) = 0u;
+    }
+  }
+  __syncthreads();
+  if (has_newest && head_tile == 0 && slot >= 0) {
+    const size_t page = slot >> p.page_shift, in_page = slot & p.page_mask;
+    const size_t at = (((page * p.Hkv + kvh) << p.page_shift) + in_page) * D;
+    for (int d = threadIdx.x * 2; d < 2 * D; d += DEC_THREADS * 2) {
+      bf16* dst = d < D ? p.k_cache_out + at + d : p.v_cache_out + at + (d - D);
+      *reinterpret_cast<uint32_t*>(dst) = *reinterpret_cast<const uint32_t*>(newest_kv + d);
+    }
+  }
+  if (!TMA) {
+#pragma unroll
+    for (int s = 0; s < DEC_STAGES - 1; ++s) cp_async_commit();      // as many groups as the loop below counts on
+  }
+  if (traced) timeline_mark_thread(43, split);          // query rows (and the newest key) made
+  int pos[2], lo[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    pos[h] = g + 8 * h < ng ? qpos : -1;
+    lo[h] = j_lo;
+  }
+  float o[D / 8][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+#pragma unroll
+  for (int dt = 0; dt < D / 8; ++dt)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[dt][e] = 0.f;
+  uint32_t qf[Q_IN_REGS ? D / 16 : 1][4];
+
+  for (int it = 0; it < n_tiles; ++it) {
+    const int nxt = it + DEC_STAGES - 1;
+    if (nxt < n_tiles) load_tile(nxt % DEC_STAGES, tile_of(walk_begin + nxt));
+    if (TMA) {
+      // bounded; a wait that ran out raises the block's abort flag and the status word, the loop
+      // goes on over whatever the stage holds, and the block stores no output at the end
+      mbar_wait(smem_u32(&full[it % DEC_STAGES]), (it / DEC_STAGES) & 1, abort_flag);
+    } else {
+      cp_async_commit();
+      cp_async_wait<DEC_STAGES - 1>();
+    }
+    __syncthreads();
+    if (has_newest && tile_of(walk_begin + it) == newest_tile) {
+      // the newest key and value take their row of the tile (the copy left zeros or stale bytes there)
+      const int row = qpos - newest_tile * BN, buf_n = it % DEC_STAGES;
+      for (int d = threadIdx.x * 2; d < 2 * D; d += DEC_THREADS * 2) {
+        const int e = d < D ? d : d - D;          // element of the head; two neighbours per thread
+        char* tile = (d < D ? Ks : Vs) + (size_t)buf_n * KV_TILE;
+        char* dst = TMA ? tile + (e / 64) * (BN * 128) + row * 128 + ((((e % 64) / 8) ^ (row & 7)) << 4) + (e % 8) * 2
+                        : tile + row * ROW_BYTES + e * 2;
+        *reinterpret_cast<uint32_t*>(dst) = *reinterpret_cast<const uint32_t*>(newest_kv + d);
+      }
+      __syncthreads();
+    }
+    if (Q_IN_REGS && it == 0) {
+      const int mi = lane >> 3, r = lane & 7;
+#pragma unroll
+      for (int kstep = 0; kstep < D / 16; ++kstep)
+        ldmatrix_x4(qf[kstep], smem_u32(Qs + ((mi & 1) * 8 + r) * ROW_BYTES + (kstep * 2 + (mi >> 1)) * 16));
+    }
+    const int buf = it % DEC_STAGES;
+    const int jbase = tile_of(walk_begin + it) * BN + warp * 16;
+    if (jbase < j_hi) {
+      float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+      qk_tile<2, TMA>(s, Qs, qf, Ks + buf * KV_TILE, warp * 16, lane);
+      softmax_tile<2>(s, o, m, l, pos, lo, jbase, p.scale_log2, lane);
+      pv_tile<2, TMA>(o, s, Vs + buf * KV_TILE, warp * 16, lane);
+    }
+    __syncthreads();
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+  if (traced) timeline_mark_thread(44, split);          // all key tiles done
+
+  // merge the four warps' partial softmax through shared memory (the K buffers are free now)
+  constexpr int SROW = D + 8;                                  // (8 mod 16: two floats a lane do not collide)
+  float* sm_o = reinterpret_cast<float*>(Ks);                  // [4][16][SROW]
+  float* sm_ml = sm_o + 4 * 16 * SROW;                         // [4][16][2]
+  float* recv = reinterpret_cast<float*>(Vs + DEC_STAGES * KV_TILE);
+  float* recv_ml = recv + 16 * D + 32;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    float sum = l[h];
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    const int r = g + 8 * h;
+    if (r < ng) {
+#pragma unroll
+      for (int dt = 0; dt < D / 8; ++dt)
+        *reinterpret_cast<float2*>(sm_o + (warp * 16 + r) * SROW + dt * 8 + 2 * (lane & 3)) = make_float2(o[dt][2 * h], o[dt][2 * h + 1]);
+    }
+    if ((lane & 3) == 0) {
+      sm_ml[(warp * 16 + r) * 2] = m[h];
+      sm_ml[(warp * 16 + r) * 2 + 1] = sum;
+    }
+  }
+  __syncthreads();
+  const bool stores = !TMA || abort_flag_s == 0;
+  const int per_rank = ((ng * D + p.num_splits - 1) / p.num_splits + 1) & ~1;       // (whole column pairs)
+  if (p.cluster_merge && !alone) cluster_wait();
+#pragma unroll 1
+  for (int i = threadIdx.x; i < ng * D; i += DEC_THREADS) {
+    const int r = i / D, d = i % D;
+    float mx = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) mx = fmaxf(mx, sm_ml[(w * 16 + r) * 2]);
+    float num = 0.f, den = 0.f;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const float mw = sm_ml[(w * 16 + r) * 2];
+      const float wgt = mw == -INFINITY ? 0.f : exp2f(mw - mx);
+      num = fmaf(wgt, sm_o[(w * 16 + r) * SROW + d], num);
+      den = fmaf(wgt, sm_ml[(w * 16 + r) * 2 + 1], den);
+    }
+    const int head = kvh * G + g0 + r;
+    if (p.num_splits == 1 || alone) {
+      const float y = den > 0.f ? num / den : 0.f;
+      if (stores) p.out[((size_t)q_begin * p.H + head) * D + d] = __float2bfloat16_rn(y);
+    } else if (p.cluster_merge) {
+      const int owner = i / per_rank;
+      cluster_store_f32(recv + split * per_rank + (i - owner * per_rank), owner, num);
+      if (d < p.num_splits) {
+        cluster_store_f32(recv_ml + (split * 16 + r) * 2, d, mx);
+        cluster_store_f32(recv_ml + (split * 16 + r) * 2 + 1, d, den);
+      }
+    } else {
+      const size_t row = (size_t)q_begin * p.H + head;
+      p.part_o[(row * p.num_splits + split) * D + d] = num;
+      if (d == 0) {
+        p.part_ml[(row * p.num_splits + split) * 2] = mx;
+        p.part_ml[(row * p.num_splits + split) * 2 + 1] = den;
+      }
+    }
+  }
+  if (p.cluster_merge && !alone) {
+    // The blocks of a (request, KV group) are one cluster, rank = key range.  Each block merges
+    // its share of the (head, dimension) pairs from all ranks' shared memory, in rank order.
+    cluster_arrive();
+    cluster_wait();
+    const int i_end = min(ng * D, (split + 1) * per_rank);
+    for (int i = split * per_rank + threadIdx.x; i < i_end; i += DEC_THREADS) {
+      const int r = i / D, d = i % D;
+      float mx = -INFINITY;
+#pragma unroll 1
+      for (int k = 0; k < p.num_splits; ++k) mx = fmaxf(mx, recv_ml[(k * 16 + r) * 2]);
+      float num = 0.f, den = 0.f;
+#pragma unroll 1
+      for (int k = 0; k < p.num_splits; ++k) {
+        const float ms = recv_ml[(k * 16 + r) * 2];
+        const float wgt = ms == -INFINITY ? 0.f : exp2f(ms - mx);
+        num = fmaf(wgt, recv[k * per_rank + (i - split * per_rank)], num);
+        den = fmaf(wgt, recv_ml[(k * 16 + r) * 2 + 1], den);
+      }
+      const float y = den > 0.f ? num / den : 0.f;
+      if (stores) p.out[((size_t)q_begin * p.H + kvh * G + g0 + r) * D + d] = __float2bfloat16_rn(y);
+    }
+    if (traced) timeline_mark_thread(45, split);        // merged and stored
+    return;
+  }
+}
+
 // (two blocks share a multiprocessor where their shared memory lets them: heads of up to 128)
 constexpr int DEC_MIN_BLOCKS = D <= 128 ? 2 : 1;
+__global__ void __launch_bounds__(DEC_THREADS) attn_decode_qkv_kernel(MmaAttnParams p) { attn_decode_qkv_body<false>(p, nullptr, nullptr); }
 template <int NH>
 __global__ void __launch_bounds__(DEC_THREADS, DEC_MIN_BLOCKS) attn_decode_kernel(MmaAttnParams p) {
   attn_decode_body<false, NH>(p, nullptr, nullptr);
@@ -993,6 +1197,11 @@ __global__ void __launch_bounds__(DEC_THREADS, DEC_MIN_BLOCKS)
 attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                        MmaAttnParams p) {
   attn_decode_body<TMA_HEAD, NH>(p, &map_k, &map_v);
+}
+__global__ void __launch_bounds__(DEC_THREADS)
+attn_decode_qkv_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
+                           MmaAttnParams p) {
+  attn_decode_qkv_body<TMA_HEAD>(p, &map_k, &map_v);
 }
 
 // out[row] = sum_s 2^(m_s - m) o_s / sum_s 2^(m_s - m) l_s over the key ranges of a row
@@ -1124,25 +1333,29 @@ TS_EXPORT int ts_paged_attention_mma_from_qkv(const void* qkv, const float* part
 }
 
 namespace {
-template <bool TMA, int NH>
-int launch_decode(const MmaAttnParams& p, const CUtensorMap& mk, const CUtensorMap& mv, dim3 grid, cudaStream_t stream) {
-  constexpr bool BY_TMA = TMA && TMA_HEAD;
-  const size_t smem = DecShared<BY_TMA>::bytes(8 * NH);
+// one of the decode kernels; NH 0: the one that makes its rows from the projection
+template <bool TMA, int NH, typename... Args>
+int launch_decode_kernel(void (*kernel)(Args...), const MmaAttnParams& p, dim3 grid, cudaStream_t stream, Args... args) {
+  const size_t smem = DecShared<TMA>::bytes(NH == 1 ? 8 : 16);
   static bool configured = false;
   if (!configured) {
-    const cudaError_t e = BY_TMA ? cudaFuncSetAttribute(attn_decode_tma_kernel<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                                 : cudaFuncSetAttribute(attn_decode_kernel<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return ts_fail("attn_decode: %s", cudaGetErrorString(e));
     configured = true;
   }
-  const dim3 block(DEC_THREADS), cluster(1, grid.y, 1);
-  cudaError_t e;
-  if (BY_TMA) e = p.cluster_merge ? ts_launch_cluster(attn_decode_tma_kernel<NH>, grid, block, smem, stream, cluster, mk, mv, p)
-                                  : ts_launch(attn_decode_tma_kernel<NH>, grid, block, smem, stream, mk, mv, p);
-  else e = p.cluster_merge ? ts_launch_cluster(attn_decode_kernel<NH>, grid, block, smem, stream, cluster, p)
-                           : ts_launch(attn_decode_kernel<NH>, grid, block, smem, stream, p);
+  const cudaError_t e = p.cluster_merge ? ts_launch_cluster(kernel, grid, dim3(DEC_THREADS), smem, stream, dim3(1, grid.y, 1), args...)
+                                        : ts_launch(kernel, grid, dim3(DEC_THREADS), smem, stream, args...);
   if (e != cudaSuccess) return ts_fail("attn_decode (%d key ranges): %s", (int)grid.y, cudaGetErrorString(e));
   return 0;
+}
+int launch_decode(int nh, bool tma, const MmaAttnParams& p, const CUtensorMap& mk, const CUtensorMap& mv, dim3 grid, cudaStream_t stream) {
+  if (tma)
+    return nh == 0   ? launch_decode_kernel<TMA_HEAD, 0>(attn_decode_qkv_tma_kernel, p, grid, stream, mk, mv, p)
+           : nh == 1 ? launch_decode_kernel<TMA_HEAD, 1>(attn_decode_tma_kernel<1>, p, grid, stream, mk, mv, p)
+                     : launch_decode_kernel<TMA_HEAD, 2>(attn_decode_tma_kernel<2>, p, grid, stream, mk, mv, p);
+  return nh == 0   ? launch_decode_kernel<false, 0>(attn_decode_qkv_kernel, p, grid, stream, p)
+         : nh == 1 ? launch_decode_kernel<false, 1>(attn_decode_kernel<1>, p, grid, stream, p)
+                   : launch_decode_kernel<false, 2>(attn_decode_kernel<2>, p, grid, stream, p);
 }
 
 int paged_attention_mma_impl(const MmaAttnParams* from_qkv, const void* q, void* out, const void* k_cache,
@@ -1177,9 +1390,9 @@ int paged_attention_mma_impl(const MmaAttnParams* from_qkv, const void* q, void*
   const int G = H / Hkv;
   cudaError_t e;
   if (decode_only) {
-    // up to 8 heads of a KV group a block, up to 16 where there are more
-    const int nh = G <= 8 ? 1 : 2;
-    p.heads_per_tile = 8 * nh; p.queries_per_tile = 1; p.head_tiles = (G + 8 * nh - 1) / (8 * nh);
+    // heads of a block: up to 8 of a KV group, up to 16 where there are more; always 16 rows from the projection
+    const int nh = p.from_qkv ? 0 : G <= 8 ? 1 : 2, heads = nh == 1 ? 8 : 16;
+    p.heads_per_tile = heads; p.queries_per_tile = 1; p.head_tiles = (G + heads - 1) / heads;
     // whole pages by TMA where the sizes allow it
     // (pages of 32 and 64 keys: measured on B200, 64 requests x 4096 keys, pages of 64: 6.67 TB/s by
     // TMA against 5.78 by cp.async; with pages of 16 both reach 5.4: the 4 KB pieces are what limits)
@@ -1204,8 +1417,7 @@ int paged_attention_mma_impl(const MmaAttnParams* from_qkv, const void* q, void*
     const int count = tile_req ? num_tiles : num_requests;
     const dim3 grid(Hkv * p.head_tiles, num_splits, count);
     p.cluster_merge = decode_only == 2 && num_splits > 1 && num_splits <= CLUSTER_MAX;
-    const int failed = tma ? (nh == 1 ? launch_decode<true, 1>(p, mk, mv, grid, stream) : launch_decode<true, 2>(p, mk, mv, grid, stream))
-                           : (nh == 1 ? launch_decode<false, 1>(p, mk, mv, grid, stream) : launch_decode<false, 2>(p, mk, mv, grid, stream));
+    const int failed = launch_decode(nh, tma, p, mk, mv, grid, stream);
     if (failed || p.cluster_merge) return failed;
     if (num_splits > 1) {
       TS_LAUNCH("attention_combine", attention_combine_kernel, (tile_req ? count : num_tokens) * H,
