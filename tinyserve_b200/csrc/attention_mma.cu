@@ -550,8 +550,8 @@ template <bool TMA> struct DecShared {
   static constexpr int KV_TILE = TMA ? BN * D * 2 : BN * ROW_BYTES;      // bytes of the keys (or values) of a stage
   static constexpr int Q_BYTES = 16 * ROW_BYTES;
   static constexpr int ALIGN = TMA ? 1024 : 16;
-  // received sums: every rank's share of [heads][D], rounded up to pairs of columns, and maxima and sums of the rows
-  static constexpr int recv_floats(int heads) { return heads * D + 2 * CLUSTER_MAX + CLUSTER_MAX * heads * 2; }
+  // received sums: every rank's share of [heads][D], rounded up to fours of columns, and maxima and sums of the rows
+  static constexpr int recv_floats(int heads) { return heads * D + 4 * CLUSTER_MAX + CLUSTER_MAX * heads * 2; }
   static size_t bytes(int heads) { return Q_BYTES + ALIGN + (size_t)2 * DEC_STAGES * KV_TILE + recv_floats(heads) * 4; }
 };
 
@@ -564,10 +564,101 @@ __device__ __forceinline__ uint32_t transposed(uint32_t a) {
 __device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void cluster_store_f32(float* own_shared, uint32_t rank, float v) {
+__device__ __forceinline__ uint32_t in_peer(const float* own_shared, uint32_t rank) {
   uint32_t local = static_cast<uint32_t>(__cvta_generic_to_shared(own_shared)), remote;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
+  return remote;
+}
+__device__ __forceinline__ void add_scaled4(float (&sum)[4], float factor, const float* shared) {
+  const float4 v = *reinterpret_cast<const float4*>(shared);
+  sum[0] = fmaf(factor, v.x, sum[0]); sum[1] = fmaf(factor, v.y, sum[1]);
+  sum[2] = fmaf(factor, v.z, sum[2]); sum[3] = fmaf(factor, v.w, sum[3]);
+}
+
+// The end of a decode block: the partial sums of its warps (sm_o: rows of STRIDE floats, `o_rows` rows a warp; sm_ml: maximum
+// and sum, ROWS rows a warp) become output rows, or partial rows in scratch, or go to the peers of the cluster, of whose
+// outputs this block makes its share, in rank order.  Four neighbouring columns a thread.  OPTIONS: sinks, turned outputs, a
+// request list.
+template <int ROWS, int STRIDE, bool OPTIONS>
+__device__ __forceinline__ void merge_block(const MmaAttnParams& p, const float* sm_o, int o_rows, const float* sm_ml, float* recv,
+                                            bool alone, bool stores, int ng, int head0, int q_begin, int split, int qpos) {
+  const bool merged = p.cluster_merge && !alone;
+  const int per_rank = ((ng * D + p.num_splits - 1) / p.num_splits + 3) & ~3;
+  float* recv_ml = recv + ROWS * D + 4 * CLUSTER_MAX;                               // [rank][ROWS][2]
+  auto write = [&](int r, int d, const float (&num)[4], float den) {
+    float y[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) y[e] = den > 0.f ? num[e] / den : 0.f;
+    if (OPTIONS && p.turn.cos) {
+      const float u[4] = {y[0], y[1], y[2], y[3]};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) y[e] = p.turn.value(u[e], u[e ^ 1], d + e, qpos);
+    }
+    if (stores)
+      *reinterpret_cast<uint2*>(p.out + ((size_t)q_begin * p.H + head0 + r) * D + d) = make_uint2(pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]));
+  };
+  if (merged) cluster_wait();                           // all peers have started
+#pragma unroll 1
+  for (int i = threadIdx.x * 4; i < ng * D; i += DEC_THREADS * 4) {
+    const int r = i / D, d = i % D;
+    float mw[DEC_WARPS], mx = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < DEC_WARPS; ++w) {
+      mw[w] = sm_ml[(w * ROWS + r) * 2];
+      mx = fmaxf(mx, mw[w]);
+    }
+    float num[4] = {0.f, 0.f, 0.f, 0.f}, den = 0.f;
+#pragma unroll
+    for (int w = 0; w < DEC_WARPS; ++w) {
+      const float wgt = mw[w] == -INFINITY ? 0.f : exp2f(mw[w] - mx);
+      add_scaled4(num, wgt, sm_o + (w * o_rows + r) * STRIDE + d);
+      den = fmaf(wgt, sm_ml[(w * ROWS + r) * 2 + 1], den);
+    }
+    if (OPTIONS && p.sinks && split == 0) {
+      // the sink joins the first key range's partial sum (log2 domain, like the maxima)
+      const float sk = p.sinks[head0 + r] * LOG2E;
+      const float m_new = fmaxf(mx, sk);
+      const float a = mx == -INFINITY ? 0.f : exp2f(mx - m_new);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) num[e] *= a;
+      den = den * a + exp2f(sk - m_new);
+      mx = m_new;
+    }
+    if (p.num_splits == 1 || alone) {
+      write(r, d, num, den);
+    } else if (merged) {
+      // to the rank that adds these columns up, at their place among this range's
+      const int owner = i / per_rank;
+      asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(in_peer(recv + split * per_rank + (i - owner * per_rank), owner)),
+                   "f"(num[0]), "f"(num[1]), "f"(num[2]), "f"(num[3]) : "memory");
+      // (every thread of the row holds the same maximum and sum)
+      for (int k = d / 4; k < p.num_splits; k += D / 4)
+        asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(in_peer(recv_ml + (split * ROWS + r) * 2, k)), "f"(mx), "f"(den) : "memory");
+    } else {
+      // partial rows go by token, or by the entry of the request list when there is one
+      const size_t row = ((size_t)(OPTIONS && p.tile_req ? (int)blockIdx.z : q_begin) * p.H + head0 + r) * p.num_splits + split;
+      *reinterpret_cast<float4*>(p.part_o + row * D + d) = make_float4(num[0], num[1], num[2], num[3]);
+      if (d == 0) *reinterpret_cast<float2*>(p.part_ml + row * 2) = make_float2(mx, den);
+    }
+  }
+  if (!merged) return;
+  cluster_arrive();
+  cluster_wait();
+  const int i_end = min(ng * D, (split + 1) * per_rank);
+#pragma unroll 1
+  for (int i = split * per_rank + threadIdx.x * 4; i < i_end; i += DEC_THREADS * 4) {
+    const int r = i / D;
+    float mx = -INFINITY;
+    for (int k = 0; k < p.num_splits; ++k) mx = fmaxf(mx, recv_ml[(k * ROWS + r) * 2]);
+    float num[4] = {0.f, 0.f, 0.f, 0.f}, den = 0.f;
+    for (int k = 0; k < p.num_splits; ++k) {
+      const float ms = recv_ml[(k * ROWS + r) * 2];
+      const float wgt = ms == -INFINITY ? 0.f : exp2f(ms - mx);
+      add_scaled4(num, wgt, recv + k * per_rank + (i - split * per_rank));
+      den = fmaf(wgt, recv_ml[(k * ROWS + r) * 2 + 1], den);
+    }
+    write(r, i % D, num, den);
+  }
 }
 
 // sixteen keys (rows key0 .. of a tile) for the block's heads: scores, online softmax, outputs.  The lane holds the heads
@@ -831,85 +922,7 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
     }
   __syncthreads();
   const bool stores = abort_flag_s == 0;
-  // (a turned output needs its column's mate, which is the neighbour lane's: both lanes of a pair are in or out)
-  auto finished = [&](float v, int d, unsigned lanes) {
-    if (!p.turn.cos) return v;
-    const float mate = __shfl_xor_sync(lanes, v, 1);
-    return p.turn.value(v, mate, d, qpos);
-  };
-  const bool merged = p.cluster_merge && !alone;
-  const int per_rank = ((ng * D + p.num_splits - 1) / p.num_splits + 1) & ~1;       // (whole column pairs)
-  float* recv_ml = recv + 8 * NH * D + 2 * CLUSTER_MAX;                             // [rank][8 NH][2]
-  if (merged) cluster_wait();                           // all peers have started
-  for (int i = threadIdx.x; i < ng * D; i += DEC_THREADS) {
-    const unsigned lanes = ~0u >> (32 - min(32, ng * D - (i - lane)));        // the warp's lanes that take part
-    const int r = i / D, d = i % D;
-    float mw[DEC_WARPS], mx = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < DEC_WARPS; ++w) {
-      mw[w] = sm_ml[(w * 8 * NH + r) * 2];
-      mx = fmaxf(mx, mw[w]);
-    }
-    float num = 0.f, den = 0.f;
-#pragma unroll
-    for (int w = 0; w < DEC_WARPS; ++w) {
-      const float wgt = mw[w] == -INFINITY ? 0.f : exp2f(mw[w] - mx);
-      num = fmaf(wgt, sm_o[(w * ng + r) * SUM_ROW + d], num);
-      den = fmaf(wgt, sm_ml[(w * 8 * NH + r) * 2 + 1], den);
-    }
-    const int head = kvh * G + g0 + r;
-    if (p.sinks && split == 0) {
-      // the sink joins the first key range's partial sum (log2 domain, like the maxima)
-      const float sk = p.sinks[head] * LOG2E;
-      const float m_new = fmaxf(mx, sk);
-      const float a = mx == -INFINITY ? 0.f : exp2f(mx - m_new);
-      num *= a;
-      den = den * a + exp2f(sk - m_new);
-      mx = m_new;
-    }
-    if (p.num_splits == 1 || alone) {
-      const float y = finished(den > 0.f ? num / den : 0.f, d, lanes);
-      if (stores) p.out[((size_t)q_begin * p.H + head) * D + d] = __float2bfloat16_rn(y);
-    } else if (merged) {
-      // to the rank that adds this element up, at its place among this range's
-      const int owner = i / per_rank;
-      cluster_store_f32(recv + split * per_rank + (i - owner * per_rank), owner, num);
-      if (d < p.num_splits) {                           // (every thread of the row holds the same maximum and sum)
-        cluster_store_f32(recv_ml + (split * 8 * NH + r) * 2, d, mx);
-        cluster_store_f32(recv_ml + (split * 8 * NH + r) * 2 + 1, d, den);
-      }
-    } else {
-      // partial rows go by token, or by the entry of the request list when there is one
-      const size_t row = (size_t)(p.tile_req ? (int)blockIdx.z : q_begin) * p.H + head;
-      p.part_o[(row * p.num_splits + split) * D + d] = num;
-      if (d == 0) {
-        p.part_ml[(row * p.num_splits + split) * 2] = mx;
-        p.part_ml[(row * p.num_splits + split) * 2 + 1] = den;
-      }
-    }
-  }
-  if (merged) {
-    // The blocks of a (request, KV group) are one cluster, rank = key range.  Each block merges
-    // its share of the (head, dimension) pairs, in rank order.
-    cluster_arrive();
-    cluster_wait();
-    const int i_end = min(ng * D, (split + 1) * per_rank);
-    for (int i = split * per_rank + threadIdx.x; i < i_end; i += DEC_THREADS) {
-      const unsigned lanes = ~0u >> (32 - min(32, i_end - (i - lane)));
-      const int r = i / D, d = i % D;
-      float mx = -INFINITY;
-      for (int s = 0; s < p.num_splits; ++s) mx = fmaxf(mx, recv_ml[(s * 8 * NH + r) * 2]);
-      float num = 0.f, den = 0.f;
-      for (int s = 0; s < p.num_splits; ++s) {
-        const float ms = recv_ml[(s * 8 * NH + r) * 2];
-        const float wgt = ms == -INFINITY ? 0.f : exp2f(ms - mx);
-        num = fmaf(wgt, recv[s * per_rank + (i - split * per_rank)], num);
-        den = fmaf(wgt, recv_ml[(s * 8 * NH + r) * 2 + 1], den);
-      }
-      const float y = finished(den > 0.f ? num / den : 0.f, d, lanes);
-      if (stores) p.out[((size_t)q_begin * p.H + kvh * G + g0 + r) * D + d] = __float2bfloat16_rn(y);
-    }
-  }
+  merge_block<8 * NH, SUM_ROW, true>(p, sm_o, ng, sm_ml, recv, alone, stores, ng, kvh * G + g0, q_begin, split, qpos);
   if (traced) timeline_mark_thread(45, split);          // merged and stored
 }
 
@@ -1102,7 +1115,6 @@ __device__ __forceinline__ void attn_decode_qkv_body(const MmaAttnParams& p, con
   float* sm_o = reinterpret_cast<float*>(Ks);                  // [4][16][SROW]
   float* sm_ml = sm_o + 4 * 16 * SROW;                         // [4][16][2]
   float* recv = reinterpret_cast<float*>(Vs + DEC_STAGES * KV_TILE);
-  float* recv_ml = recv + 16 * D + 32;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     float sum = l[h];
@@ -1121,72 +1133,13 @@ __device__ __forceinline__ void attn_decode_qkv_body(const MmaAttnParams& p, con
   }
   __syncthreads();
   const bool stores = !TMA || abort_flag_s == 0;
-  const int per_rank = ((ng * D + p.num_splits - 1) / p.num_splits + 1) & ~1;       // (whole column pairs)
-  if (p.cluster_merge && !alone) cluster_wait();
-#pragma unroll 1
-  for (int i = threadIdx.x; i < ng * D; i += DEC_THREADS) {
-    const int r = i / D, d = i % D;
-    float mx = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < 4; ++w) mx = fmaxf(mx, sm_ml[(w * 16 + r) * 2]);
-    float num = 0.f, den = 0.f;
-#pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      const float mw = sm_ml[(w * 16 + r) * 2];
-      const float wgt = mw == -INFINITY ? 0.f : exp2f(mw - mx);
-      num = fmaf(wgt, sm_o[(w * 16 + r) * SROW + d], num);
-      den = fmaf(wgt, sm_ml[(w * 16 + r) * 2 + 1], den);
-    }
-    const int head = kvh * G + g0 + r;
-    if (p.num_splits == 1 || alone) {
-      const float y = den > 0.f ? num / den : 0.f;
-      if (stores) p.out[((size_t)q_begin * p.H + head) * D + d] = __float2bfloat16_rn(y);
-    } else if (p.cluster_merge) {
-      const int owner = i / per_rank;
-      cluster_store_f32(recv + split * per_rank + (i - owner * per_rank), owner, num);
-      if (d < p.num_splits) {
-        cluster_store_f32(recv_ml + (split * 16 + r) * 2, d, mx);
-        cluster_store_f32(recv_ml + (split * 16 + r) * 2 + 1, d, den);
-      }
-    } else {
-      const size_t row = (size_t)q_begin * p.H + head;
-      p.part_o[(row * p.num_splits + split) * D + d] = num;
-      if (d == 0) {
-        p.part_ml[(row * p.num_splits + split) * 2] = mx;
-        p.part_ml[(row * p.num_splits + split) * 2 + 1] = den;
-      }
-    }
-  }
-  if (p.cluster_merge && !alone) {
-    // The blocks of a (request, KV group) are one cluster, rank = key range.  Each block merges
-    // its share of the (head, dimension) pairs from all ranks' shared memory, in rank order.
-    cluster_arrive();
-    cluster_wait();
-    const int i_end = min(ng * D, (split + 1) * per_rank);
-    for (int i = split * per_rank + threadIdx.x; i < i_end; i += DEC_THREADS) {
-      const int r = i / D, d = i % D;
-      float mx = -INFINITY;
-#pragma unroll 1
-      for (int k = 0; k < p.num_splits; ++k) mx = fmaxf(mx, recv_ml[(k * 16 + r) * 2]);
-      float num = 0.f, den = 0.f;
-#pragma unroll 1
-      for (int k = 0; k < p.num_splits; ++k) {
-        const float ms = recv_ml[(k * 16 + r) * 2];
-        const float wgt = ms == -INFINITY ? 0.f : exp2f(ms - mx);
-        num = fmaf(wgt, recv[k * per_rank + (i - split * per_rank)], num);
-        den = fmaf(wgt, recv_ml[(k * 16 + r) * 2 + 1], den);
-      }
-      const float y = den > 0.f ? num / den : 0.f;
-      if (stores) p.out[((size_t)q_begin * p.H + kvh * G + g0 + r) * D + d] = __float2bfloat16_rn(y);
-    }
-    if (traced) timeline_mark_thread(45, split);        // merged and stored
-    return;
-  }
+  merge_block<16, SROW, false>(p, sm_o, 16, sm_ml, recv, alone, stores, ng, kvh * G + g0, q_begin, split, qpos);
+  if (traced) timeline_mark_thread(45, split);          // merged and stored
 }
 
 // (two blocks share a multiprocessor where their shared memory lets them: heads of up to 128)
 constexpr int DEC_MIN_BLOCKS = D <= 128 ? 2 : 1;
-__global__ void __launch_bounds__(DEC_THREADS) attn_decode_qkv_kernel(MmaAttnParams p) { attn_decode_qkv_body<false>(p, nullptr, nullptr); }
+__global__ void __launch_bounds__(DEC_THREADS, DEC_MIN_BLOCKS) attn_decode_qkv_kernel(MmaAttnParams p) { attn_decode_qkv_body<false>(p, nullptr, nullptr); }
 template <int NH>
 __global__ void __launch_bounds__(DEC_THREADS, DEC_MIN_BLOCKS) attn_decode_kernel(MmaAttnParams p) {
   attn_decode_body<false, NH>(p, nullptr, nullptr);
@@ -1198,7 +1151,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                        MmaAttnParams p) {
   attn_decode_body<TMA_HEAD, NH>(p, &map_k, &map_v);
 }
-__global__ void __launch_bounds__(DEC_THREADS)
+__global__ void __launch_bounds__(DEC_THREADS, DEC_MIN_BLOCKS)
 attn_decode_qkv_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                            MmaAttnParams p) {
   attn_decode_qkv_body<TMA_HEAD>(p, &map_k, &map_v);
