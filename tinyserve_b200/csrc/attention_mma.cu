@@ -536,23 +536,22 @@ __device__ __forceinline__ void build_head(const MmaAttnParams& p, int t, int co
 // a decode step of few requests this form of it was 2.5 us slower a layer, although it is 2.4 us faster with nothing around it.)
 //
 // TMA false: key and value tiles come by cp.async, 16 bytes a thread, into padded rows (any head
-// size in steps of 16, any page size).  TMA true (head sizes in steps of 64, pages of 32 or 64
+// size in steps of 16, any page size).  TMA true (head sizes in steps of 64, pages of 16 to 64
 // keys): one warp fetches whole pages as boxes of page x 64 columns with the 128-byte swizzle;
 // an SM streams about half as much again this way
 // as through its load/store unit's miss queue.  Whole pages come, also the keys past the
-// request's length in its last page: those are masked, and must hold finite numbers (the engine's
-// cache starts as zeros and only ever takes keys and values).
+// request's length in its last page: their scores are masked and their values made zero in shared memory.
 constexpr int DEC_THREADS = 128, DEC_WARPS = DEC_THREADS / 32;
 constexpr int SUM_ROW = D + 4;                       // floats of a row of partial sums (4 mod 16: no bank conflicts)
 
-// the block's shared memory: query rows, stages, and what peers of a cluster send
-template <bool TMA> struct DecShared {
+// The block's shared memory: query rows, and over them, once they are read, what peers of a cluster send (heads of 128 by
+// cp.async: two blocks share a multiprocessor only so); then the stages.
+template <bool TMA, int ROWS> struct DecShared {
   static constexpr int KV_TILE = TMA ? BN * D * 2 : BN * ROW_BYTES;      // bytes of the keys (or values) of a stage
-  static constexpr int Q_BYTES = 16 * ROW_BYTES;
-  static constexpr int ALIGN = TMA ? 1024 : 16;
-  // received sums: every rank's share of [heads][D], rounded up to fours of columns, and maxima and sums of the rows
-  static constexpr int recv_floats(int heads) { return heads * D + 4 * CLUSTER_MAX + CLUSTER_MAX * heads * 2; }
-  static size_t bytes(int heads) { return Q_BYTES + ALIGN + (size_t)2 * DEC_STAGES * KV_TILE + recv_floats(heads) * 4; }
+  // every rank's share of [ROWS][D], rounded up to fours of columns, and maxima and sums of the rows
+  static constexpr int RECV_BYTES = (ROWS * D + 4 * CLUSTER_MAX + CLUSTER_MAX * ROWS * 2) * 4;
+  static constexpr int FIRST = RECV_BYTES > 16 * ROW_BYTES ? RECV_BYTES : 16 * ROW_BYTES;
+  static constexpr size_t BYTES = FIRST + (TMA ? 1024 : 16) + (size_t)2 * DEC_STAGES * KV_TILE;
 };
 
 __device__ __forceinline__ uint32_t transposed(uint32_t a) {
@@ -573,6 +572,20 @@ __device__ __forceinline__ void add_scaled4(float (&sum)[4], float factor, const
   const float4 v = *reinterpret_cast<const float4*>(shared);
   sum[0] = fmaf(factor, v.x, sum[0]); sum[1] = fmaf(factor, v.y, sum[1]);
   sum[2] = fmaf(factor, v.z, sum[2]); sum[3] = fmaf(factor, v.w, sum[3]);
+}
+
+// Values of the keys from j_hi on, of a warp's 16 (rows key0 .. of a tile that came by TMA), become zeros
+__device__ __forceinline__ void clear_values(char* vs, int key0, int jbase, int j_hi, int lane) {
+  if (jbase + 16 <= j_hi) return;
+  if (jbase + (lane >> 1) >= j_hi) {       // two lanes a row
+    const int row = key0 + (lane >> 1);
+#pragma unroll
+    for (int k = 0; k < CH / 2; ++k) {
+      const int piece = (lane & 1) * (CH / 2) + k;
+      *reinterpret_cast<uint4*>(vs + (piece >> 3) * (BN * 128) + row * 128 + (((piece & 7) ^ (row & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
+    }
+  }
+  __syncwarp();
 }
 
 // The end of a decode block: the partial sums of its warps (sm_o: rows of STRIDE floats, `o_rows` rows a warp; sm_ml: maximum
@@ -743,15 +756,15 @@ __device__ __forceinline__ void decode_keys(float (&o)[NH][D / 16][4], float (&m
 template <bool TMA, int NH>
 __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const CUtensorMap* map_k,
                                                  const CUtensorMap* map_v) {
-  using S = DecShared<TMA>;
+  using S = DecShared<TMA, 8 * NH>;
   constexpr int KV_TILE = S::KV_TILE;
   constexpr bool Q_REGS = D <= 128 && NH == 1;
   extern __shared__ __align__(16) char smem[];
   char* Qs = smem;                                   // [16][ROW_BYTES]
-  char* Ks = TMA ? reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(Qs + S::Q_BYTES) + 1023) & ~uintptr_t(1023))
-                 : Qs + S::Q_BYTES;                  // [DEC_STAGES][KV_TILE]
+  char* Ks = TMA ? reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(Qs + S::FIRST) + 1023) & ~uintptr_t(1023))
+                 : Qs + S::FIRST;                    // [DEC_STAGES][KV_TILE]
   char* Vs = Ks + DEC_STAGES * KV_TILE;              // [DEC_STAGES][KV_TILE]
-  float* recv = reinterpret_cast<float*>(Vs + DEC_STAGES * KV_TILE);       // peers' sums: [rank][this block's share]
+  float* recv = reinterpret_cast<float*>(Qs);        // peers' sums: [rank][this block's share]
   __shared__ uint64_t full[DEC_STAGES];              // the tile's bytes have landed
   __shared__ int abort_flag_s;
   volatile int* abort_flag = &abort_flag_s;
@@ -770,8 +783,6 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
   __syncthreads();
 
   pdl_trigger();
-  // (peers may be written to once they have all started; the wait for that comes before the first such write)
-  if (p.cluster_merge) cluster_arrive();
   // The lengths, the block table and every cached key but the newest were written before this
   // step's kernels began: the first tiles are fetched before pdl_wait(), while the kernels that
   // make this token's query, key and value still run.  The tile with the newest key and the
@@ -877,6 +888,8 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
     }
   }
 
+  // (peers write to this block's memory when every thread of the cluster has read its query rows)
+  if (Q_REGS && p.cluster_merge) cluster_arrive();
   const int key0 = warp * 16;
   for (int it = 0; it < n_tiles; ++it) {
     const int stage = it % DEC_STAGES;
@@ -885,13 +898,16 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
     mbar_wait(smem_u32(&full[stage]), (it / DEC_STAGES) & 1, abort_flag);
     __syncwarp();
     const int jbase = tile_of(walk_begin + it) * BN + key0;
-    if (jbase < j_hi)
+    if (jbase < j_hi) {
+      if (TMA) clear_values(Vs + stage * KV_TILE, key0, jbase, j_hi, lane);
       decode_keys<TMA, NH, Q_REGS>(o, m, l, qf, Qs, Ks + stage * KV_TILE, Vs + stage * KV_TILE, key0, jbase, qpos, j_lo, keep, p, sl, lane);
+    }
     if (it + DEC_STAGES < n_tiles) {
       __syncthreads();
       load_tile(it + DEC_STAGES);
     }
   }
+  if (!Q_REGS && p.cluster_merge) cluster_arrive();
   __syncthreads();
   if (traced) timeline_mark_thread(44, split);          // all key tiles done
 
@@ -933,10 +949,11 @@ template <bool TMA>
 __device__ __forceinline__ void attn_decode_qkv_body(const MmaAttnParams& p, const CUtensorMap* map_k,
                                                  const CUtensorMap* map_v) {
   extern __shared__ __align__(16) char smem[];
-  constexpr int KV_TILE = TMA ? BN * D * 2 : BN * ROW_BYTES;      // bytes of the keys (or values) of a stage
+  using S = DecShared<TMA, 16>;
+  constexpr int KV_TILE = S::KV_TILE;
   char* Qs = smem;                                   // [16][ROW_BYTES]
-  char* Ks = TMA ? reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(Qs + 16 * ROW_BYTES) + 1023) & ~uintptr_t(1023))
-                 : Qs + 16 * ROW_BYTES;              // [DEC_STAGES][KV_TILE]
+  char* Ks = TMA ? reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(Qs + S::FIRST) + 1023) & ~uintptr_t(1023))
+                 : Qs + S::FIRST;                    // [DEC_STAGES][KV_TILE]
   char* Vs = Ks + DEC_STAGES * KV_TILE;              // [DEC_STAGES][KV_TILE]
   __shared__ uint64_t full[DEC_STAGES];              // (TMA) the stage's bytes have landed
   __shared__ int abort_flag_s;
@@ -949,7 +966,6 @@ __device__ __forceinline__ void attn_decode_qkv_body(const MmaAttnParams& p, con
   if (TMA) __syncthreads();
 
   pdl_trigger();
-  if (p.cluster_merge) cluster_arrive();
   // The lengths, the block table and every cached key but the newest were written before this
   // step's kernels began: the first tiles are fetched before pdl_wait(), while the kernels that
   // make this token's query, key and value still run.  The tile with the newest key and the
@@ -1065,6 +1081,14 @@ __device__ __forceinline__ void attn_decode_qkv_body(const MmaAttnParams& p, con
 #pragma unroll
     for (int e = 0; e < 4; ++e) o[dt][e] = 0.f;
   uint32_t qf[Q_IN_REGS ? D / 16 : 1][4];
+  if (Q_IN_REGS) {
+    const int mi = lane >> 3, r = lane & 7;
+#pragma unroll
+    for (int kstep = 0; kstep < D / 16; ++kstep)
+      ldmatrix_x4(qf[kstep], smem_u32(Qs + ((mi & 1) * 8 + r) * ROW_BYTES + (kstep * 2 + (mi >> 1)) * 16));
+    // (peers write to this block's memory when every thread of the cluster has read its query rows)
+    if (p.cluster_merge) cluster_arrive();
+  }
 
   for (int it = 0; it < n_tiles; ++it) {
     const int nxt = it + DEC_STAGES - 1;
@@ -1090,15 +1114,10 @@ __device__ __forceinline__ void attn_decode_qkv_body(const MmaAttnParams& p, con
       }
       __syncthreads();
     }
-    if (Q_IN_REGS && it == 0) {
-      const int mi = lane >> 3, r = lane & 7;
-#pragma unroll
-      for (int kstep = 0; kstep < D / 16; ++kstep)
-        ldmatrix_x4(qf[kstep], smem_u32(Qs + ((mi & 1) * 8 + r) * ROW_BYTES + (kstep * 2 + (mi >> 1)) * 16));
-    }
     const int buf = it % DEC_STAGES;
     const int jbase = tile_of(walk_begin + it) * BN + warp * 16;
     if (jbase < j_hi) {
+      if (TMA) clear_values(Vs + buf * KV_TILE, warp * 16, jbase, j_hi, lane);
       float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
       qk_tile<2, TMA>(s, Qs, qf, Ks + buf * KV_TILE, warp * 16, lane);
       softmax_tile<2>(s, o, m, l, pos, lo, jbase, p.scale_log2, lane);
@@ -1107,6 +1126,7 @@ __device__ __forceinline__ void attn_decode_qkv_body(const MmaAttnParams& p, con
     __syncthreads();
   }
   cp_async_wait<0>();
+  if (!Q_IN_REGS && p.cluster_merge) cluster_arrive();
   __syncthreads();
   if (traced) timeline_mark_thread(44, split);          // all key tiles done
 
@@ -1114,7 +1134,7 @@ __device__ __forceinline__ void attn_decode_qkv_body(const MmaAttnParams& p, con
   constexpr int SROW = D + 8;                                  // (8 mod 16: two floats a lane do not collide)
   float* sm_o = reinterpret_cast<float*>(Ks);                  // [4][16][SROW]
   float* sm_ml = sm_o + 4 * 16 * SROW;                         // [4][16][2]
-  float* recv = reinterpret_cast<float*>(Vs + DEC_STAGES * KV_TILE);
+  float* recv = reinterpret_cast<float*>(Qs);
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     float sum = l[h];
@@ -1289,7 +1309,7 @@ namespace {
 // one of the decode kernels; NH 0: the one that makes its rows from the projection
 template <bool TMA, int NH, typename... Args>
 int launch_decode_kernel(void (*kernel)(Args...), const MmaAttnParams& p, dim3 grid, cudaStream_t stream, Args... args) {
-  const size_t smem = DecShared<TMA>::bytes(NH == 1 ? 8 : 16);
+  const size_t smem = DecShared<TMA, NH == 1 ? 8 : 16>::BYTES;
   static bool configured = false;
   if (!configured) {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1347,9 +1367,9 @@ int paged_attention_mma_impl(const MmaAttnParams* from_qkv, const void* q, void*
     const int nh = p.from_qkv ? 0 : G <= 8 ? 1 : 2, heads = nh == 1 ? 8 : 16;
     p.heads_per_tile = heads; p.queries_per_tile = 1; p.head_tiles = (G + heads - 1) / heads;
     // whole pages by TMA where the sizes allow it
-    // (pages of 32 and 64 keys: measured on B200, 64 requests x 4096 keys, pages of 64: 6.67 TB/s by
-    // TMA against 5.78 by cp.async; with pages of 16 both reach 5.4: the 4 KB pieces are what limits)
-    const bool tma = TMA_HEAD && num_pages > 0 && page_size >= 32 && page_size <= BN &&
+    // (pages of 16, 32 and 64 keys; by cp.async -> by TMA, us: pages of 64, 64 requests x 4,096 keys 5.78 -> 6.67 TB/s; pages
+    // of 16, 32 heads over 8, 32 requests of 4,000 keys 156 -> 99, 8 of 4,000 48 -> 29; 64 over 8, 6 of 2,000 45 -> 30, 2 of 500 11.4 -> 8.8)
+    const bool tma = TMA_HEAD && num_pages > 0 && page_size >= 16 && page_size <= BN &&
                      ((uintptr_t)k_cache | (uintptr_t)v_cache) % 16 == 0;
     CUtensorMap mk, mv;
     if (tma) {
