@@ -1188,21 +1188,29 @@ __global__ void attention_combine_kernel(const float* __restrict__ part_o, const
   const size_t row = blockIdx.x;
   if (tokens && tokens[blockIdx.x / H] < 0) return;
   const size_t out_row = tokens ? (size_t)tokens[blockIdx.x / H] * H + blockIdx.x % H : row;
-  const float* ml = part_ml + row * num_splits * 2;
-  float mx = -INFINITY;
-  for (int s = 0; s < num_splits; ++s) mx = fmaxf(mx, ml[2 * s]);
-  float den = 0.f;
-  for (int s = 0; s < num_splits; ++s) den += ml[2 * s] == -INFINITY ? 0.f : exp2f(ml[2 * s] - mx) * ml[2 * s + 1];
+  // Two trips to memory: a lane takes a range's maximum and sum (every warp for itself; up to 64 ranges), then the columns'
+  // partial sums come eight ranges at a time.  (One range after the other: 6.3 us for 2 x 16 rows of 18 ranges in a decode step.)
+  const int lane = threadIdx.x & 31;
+  const float2* ml = reinterpret_cast<const float2*>(part_ml) + row * num_splits;
+  const float2 none = make_float2(-INFINITY, 0.f);
+  const float2 a = lane < num_splits ? __ldcg(ml + lane) : none, b = lane + 32 < num_splits ? __ldcg(ml + lane + 32) : none;
+  const float mx = warp_max(fmaxf(a.x, b.x));
+  const float wa = a.x == -INFINITY ? 0.f : exp2f(a.x - mx), wb = b.x == -INFINITY ? 0.f : exp2f(b.x - mx);
+  const float den = warp_sum(wa * a.y + wb * b.y);
   const float inv = den > 0.f ? 1.f / den : 0.f;
   const int pos = turn.cos ? turn.positions[out_row / H] : 0;
   for (int d0 = 0; d0 < D; d0 += blockDim.x) {       // (whole warps take every round)
     const int d = d0 + threadIdx.x;
+    const float* src = part_o + row * num_splits * D + min(d, D - 1);
     float v = 0.f;
-    if (d < D)
-      for (int s = 0; s < num_splits; ++s) {
-        const float w = ml[2 * s] == -INFINITY ? 0.f : exp2f(ml[2 * s] - mx);
-        v = fmaf(w, part_o[(row * num_splits + s) * D + d], v);
-      }
+#pragma unroll 1
+    for (int s0 = 0; s0 < num_splits; s0 += 8) {
+      float part[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) part[k] = s0 + k < num_splits ? __ldcg(src + (s0 + k) * D) : 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v = fmaf(__shfl_sync(0xffffffffu, s0 < 32 ? wa : wb, (s0 + k) & 31), part[k], v);
+    }
     v *= inv;
     if (turn.cos) {
       const float mate = __shfl_xor_sync(0xffffffffu, v, 1);
