@@ -1492,8 +1492,9 @@ TS_EXPORT int ts_qk_norm_rope_kvwrite(int dtype, const void* qkv, void* q_out, c
                           reinterpret_cast<uintptr_t>(q_weight) | reinterpret_cast<uintptr_t>(k_weight)) % 16 == 0;
   // From 128 tokens on (16 / 32 / 64 heads, us, a warp per head -> eight elements per lane: 96 tokens 1.6 -> 1.8, 2.0 -> 2.2,
   // 3.2 -> 2.3; 203 tokens 2.9 -> 2.3, 3.8 -> 2.2, 5.5 -> 2.3); from 512 on there are blocks enough for two tokens each.
-  constexpr int ROWS8_MIN = 128, ROWS8_TOK = 2;
-  if (vec && aligned16 && num_tokens >= ROWS8_MIN && partials == nullptr && (D == 64 || D == 128 || D == 256) &&
+  // (32-bit rows have twice the bytes to a lane: from 256 on.)
+  constexpr int ROWS8_TOK = 2;
+  if (vec && aligned16 && num_tokens >= (dtype == TS_BF16 ? 128 : 256) && partials == nullptr && (D == 64 || D == 128 || D == 256) &&
       (dtype == TS_F32 || dtype == TS_BF16)) {
     const int per_warp = 512 / D, need = (heads_total + per_warp - 1) / per_warp;
     const int tok = num_tokens >= 512 ? ROWS8_TOK : 1;

@@ -196,6 +196,8 @@ __device__ void hist_choose(Histogram& h, unsigned long long before, unsigned lo
   __syncthreads();
 }
 
+constexpr int LIST = 1024;            // most tokens of a block that top-k leaves and the passes after it keep apart
+
 struct SampleArgs {
   const float* logits;      // [rows, row_stride]
   long long row_stride;
@@ -219,6 +221,11 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
   __shared__ float f_scratch[33];
   __shared__ Histogram h;
   __shared__ unsigned long long shared_word;      // what this block tells the cluster (a maximum, or its best token)
+  // the tokens that top-k leaves of this block's range, where they are so few: the passes after it go over these alone
+  // (151,936 tokens, top-k 50 and top-p, us: 1 row 87 -> 64, 16 143 -> 100, 64 249 -> 171)
+  __shared__ int list_token[LIST];
+  __shared__ float list_value[LIST];
+  __shared__ int list_count;
 
   pdl_trigger();
   pdl_wait();
@@ -303,6 +310,7 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
   const float top_p = a.top_p ? a.top_p[row] : 1.f;
   uint32_t keep_from = 0;   // tokens with sort_key(x / temp) >= keep_from are kept
   int buf = 0;
+  bool listed = false;
 
   if (k > 0 && k < V) {
     // radix select of the k-th largest key, one byte per pass
@@ -329,12 +337,33 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
       __syncthreads();
     }
     keep_from = prefix;
+    if (threadIdx.x == 0) list_count = 0;
+    __syncthreads();
+    for (int base = v0 + threadIdx.x * 4; base < v1; base += THREADS * 4) {
+      float q[4];
+      load4(base, q);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float y = q[j] * inv_temp;
+        if (base + j < v1 && sort_key(y) >= keep_from) {
+          const int at = atomicAdd(&list_count, 1);
+          if (at < LIST) {
+            list_token[at] = base + j;
+            list_value[at] = y;
+          }
+        }
+      }
+    }
+    __syncthreads();
+    listed = list_count <= LIST;       // (equal logits may leave more than k tokens)
   }
+  const int list_n = listed ? list_count : 0;
 
   if (top_p < 1.f) {
     // weights exp(x - max) as 32.32 fixed point: sums are exact and order-independent
     float mx = -INFINITY;
-    for (int base = v0 + threadIdx.x * 4; base < v1; base += THREADS * 4) {
+    for (int i = threadIdx.x; i < list_n; i += THREADS) mx = fmaxf(mx, list_value[i]);
+    for (int base = v0 + threadIdx.x * 4; !listed && base < v1; base += THREADS * 4) {
       float q[4];
       load4(base, q);
 #pragma unroll
@@ -355,7 +384,12 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
     for (int byte = 3; byte >= 0; --byte, buf ^= 1) {
       if (threadIdx.x < 256) h.own[buf][threadIdx.x] = 0ull;
       __syncthreads();
-      for (int base = v0; base < v1; base += THREADS * 4) {
+      for (int i = threadIdx.x; i < list_n; i += THREADS) {
+        const uint32_t key = sort_key(list_value[i]);
+        const unsigned long long w = (key & mask) == prefix ? (unsigned long long)(expf(list_value[i] - mx) * 4294967296.f) : 0ull;
+        if (w != 0ull) atomicAdd(&h.own[buf][(key >> (8 * byte)) & 255u], w);
+      }
+      for (int base = v0; !listed && base < v1; base += THREADS * 4) {
         const int v = base + threadIdx.x * 4;
         float q[4];
         load4(v, q);
@@ -370,8 +404,11 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
       }
       hist_combine<CLUSTER>(h, buf, blocks);
       if (byte == 3) {
-        unsigned long long total = 0;
-        for (int b = 0; b < 256; ++b) total += h.all[b];
+        unsigned long long total = 0;      // (every warp for itself; a sum of integers)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) total += h.all[(threadIdx.x & 31) + 32 * i];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
         limit = (unsigned long long)((double)top_p * (double)total);
       }
       hist_choose(h, above, limit, true);
@@ -388,7 +425,15 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
   const unsigned long long stream = a.stream[row];
   const uint32_t step = a.step[row];
   Best b{-INFINITY, 0x7fffffff};
-  for (int base = v0 + threadIdx.x * 4; base < v1; base += THREADS * 4) {
+  for (int i = threadIdx.x; i < list_n; i += THREADS) {
+    const int v = list_token[i];
+    if (sort_key(list_value[i]) < keep_from) continue;
+    uint32_t c[4] = {(uint32_t)(v >> 2), step, (uint32_t)stream, (uint32_t)(stream >> 32)};
+    philox4x32_10(c, k0, k1);
+    const uint32_t noise = (v & 2) ? ((v & 1) ? c[3] : c[2]) : ((v & 1) ? c[1] : c[0]);
+    b = better(b, Best{list_value[i] + gumbel(noise), v});
+  }
+  for (int base = v0 + threadIdx.x * 4; !listed && base < v1; base += THREADS * 4) {
     uint32_t c[4] = {(uint32_t)(base >> 2), step, (uint32_t)stream, (uint32_t)(stream >> 32)};
     philox4x32_10(c, k0, k1);
     float q[4];
