@@ -34,9 +34,11 @@ _TORCH_DTYPES = {"bfloat16": torch.bfloat16, "float32": torch.float32}
 PENDING = -1     # a token id that is still on the device (see ModelRunner.slot_tokens)
 
 
-# Token counts for which steps that hold prompt portions are captured as graphs: above the
-# largest a step is busy enough with arithmetic that its launches hardly matter, and runs eagerly
-# (tinyserve's buckets are every 16 tokens up to 512, serve.py:1951-1962).
+# Token counts for which steps that hold prompt portions are captured as graphs (tinyserve's buckets
+# are every 16 tokens up to 512, serve.py:1951-1962).  Above the largest a step is captured only where decoded
+# tokens stand beside portions that use up the token budget, as in the steps of a burst: it needs no padding of
+# tokens then.  (Eagerly such a step of 2,048 tokens at the 0.6B shapes is bounded by its 250 launches: 96 requests in a
+# burst 160.6 ms, 155.4 with graphs.  Portions alone gain nothing: the captured shape has a decode launch of its own.)
 MIXED_GRAPH_TOKENS = (16, 32, 48, 64, 96, 128, 192, 256, 384, 512)
 MIXED_GRAPHS_KEPT = 16           # captured shapes kept; the one replayed longest ago goes first
 MIXED_GRAPH_SIGHTINGS = 2        # steps of a shape that run eagerly before the shape is captured
@@ -504,8 +506,11 @@ class ModelRunner:
             return None
         T = sum(len(e.tokens) for e in entries)
         B = len(entries)
+        budget = self.cfg.max_num_batched_tokens
         tokens = next((t for t in MIXED_GRAPH_TOKENS if t >= T), None)
-        if tokens is None or tokens > self.cfg.max_num_batched_tokens or B > self.cfg.max_num_seqs:
+        if T == budget and any(len(e.tokens) == 1 for e in entries):
+            tokens = budget
+        if tokens is None or tokens > budget or B > self.cfg.max_num_seqs:
             return None
         # one request more than the step holds: the empty one that unused work-list entries name
         S = self.cfg.max_num_seqs
