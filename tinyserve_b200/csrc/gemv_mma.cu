@@ -6,7 +6,8 @@
 // mma.sync takes them (64 a lane); after the wait there is one trip to memory for x, 16 MMAs in four accumulators, one
 // meeting of the block's warps in shared memory (K is cut over the warps of a block, never over blocks) and the epilogue.
 // The tcgen05 kernel (gemm_tcgen05.cu) has x brought by TMA, MMAs committed to a barrier, tensor memory read back and a
-// cluster that meets twice behind its wait.
+// cluster that meets twice behind its wait.  In a decode step at the 0.6B shapes (weights of 4 to 13 MB) a product takes
+// 2.8 us of the critical path, 5.1 by that kernel; the step, us: 1 request of 90 tokens 810 -> 622, 8 of 300 932 -> 808.
 // A lane's 16 bytes of a row are eight neighbouring k; the MMA's k are dealt to lanes in another order, but x is loaded
 // in the same one, and a sum does not depend on the names of its terms.
 //
