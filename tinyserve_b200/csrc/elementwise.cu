@@ -64,7 +64,8 @@ __global__ void block_table_scatter_kernel(int* __restrict__ resident, long long
 __global__ void block_table_gather_kernel(const int* __restrict__ resident, int* __restrict__ step_tables,
                                           const int* __restrict__ state_slots, int num_slots, int max_requests,
                                           int max_blocks) {
-  pdl_trigger();
+  // (no early trigger: the decode attention reads these tables before its dependency wait, and with small kernels in between
+  // it could start while this one still writes.  So nothing behind it is launched until its blocks are done.)
   pdl_wait();
   const int b = blockIdx.x, g = blockIdx.y;
   int slot = state_slots[b];
@@ -72,6 +73,7 @@ __global__ void block_table_gather_kernel(const int* __restrict__ resident, int*
   const int* src = resident + ((size_t)g * (num_slots + 1) + slot) * max_blocks;
   int* dst = step_tables + ((size_t)g * max_requests + b) * max_blocks;
   for (int i = threadIdx.x; i < max_blocks; i += blockDim.x) dst[i] = src[i];
+  __threadfence();
 }
 
 // resident [groups][num_slots + 1][max_blocks]; pairs [capacity][2] and num_pairs [1] on the device;
