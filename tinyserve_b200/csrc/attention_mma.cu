@@ -1,7 +1,7 @@
 // Paged grouped-query attention on the tensor cores for bfloat16, one head size per build
 // (-DTS_HEAD_DIM=..., a multiple of 16 up to 256).
 //
-// Two kernels share the tile code:
+// Three kernels:
 //   prefill: a block of 4 warps handles 64 rows = (query, head of one KV group) pairs and walks
 //            the visible keys in tiles of 64, K and V double-buffered in shared memory by cp.async;
 //            tiles that lie wholly below a warp's rows skip the mask;
@@ -9,7 +9,8 @@
 //            rows) and one of `num_splits` key ranges; its 4 warps take 16 keys each of every
 //            64-key tile (3 stages in flight) and merge their partial softmax at the end.  Up
 //            to 8 ranges are the blocks of a cluster and merge through distributed shared memory;
-//            more are merged by attention_combine_kernel.
+//            more are merged by attention_combine_kernel.  One kernel for finished query rows, one that
+//            makes them, the newest key and the newest value from the projection.
 // Scores, running maxima, sums and the output accumulate in 32-bit; exp2 with scale * log2(e);
 // the probabilities are rounded to bfloat16 for P * V, as tinykernels.py:386-413 and 993 do.
 // Visibility as serve.py:668-680: key j is seen by the query at position p iff j <= p and, with a
@@ -788,7 +789,12 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
   // step's kernels began: the first tiles are fetched before pdl_wait(), while the kernels that
   // make this token's query, key and value still run.  The tile with the newest key and the
   // query follow after it.
-  if (q_end - q_begin != 1) return;
+  if (q_end - q_begin != 1) {
+    // (in a captured shape every entry may be unused: one block waits all the same, or this kernel would be complete, and the
+    // next one's wait return, before what ran ahead of it is)
+    if ((blockIdx.x | blockIdx.y | blockIdx.z) == 0) pdl_wait();
+    return;
+  }
   const int G = p.H / p.Hkv, g0 = head_tile * 8 * NH, ng = min(8 * NH, G - g0);
   const int qpos = kv_len - 1;
   const int j_hi = kv_len;
