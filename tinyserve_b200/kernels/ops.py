@@ -512,6 +512,8 @@ def gemm_pair_error() -> int:
     return _gemm_pair().ts_gemm_pair_error()
 
 
+#: Most that a cut tile of the paired product takes: 256 x 256 partial sums and two counters.
+PAIR_TILE_FLOATS, PAIR_TILE_COUNTERS = 2 * 128 * 256, 2
 _pair_scratch: dict = {}
 _pair_count: list = []
 
@@ -527,22 +529,29 @@ def gemm_pairs() -> int:
 
 def _pair_workspace(lib, M, N, K, pairs, halves, out_float32, device):
     """Where the parts of the cut tiles of the last wave are added up, and their counters: zero
-    between products (the kernel leaves them so).  One buffer per device, grown on demand:
-    products of one stream run one after the other."""
+    between products (the kernel leaves them so).  One buffer per device, made as large as any
+    product can need (fewer cut tiles than pairs, two halves of 128 x 256 floats each: 19 MB for 74
+    pairs; more pairs than the device holds at once get one of their own) and never replaced:
+    captured graphs hold its address, and what a product needs does not grow with its tokens (at 74
+    pairs 51200 x 5120 takes 1.2 M floats for 4,096 tokens, 3.5 M for 2,816).  Products of one
+    stream run one after the other."""
+    usual = max(gemm_pairs(), num_sms() // 2)
+    room = max(pairs, usual)
+    key = str(device) if pairs <= usual else (str(device), pairs)
+    have = _pair_scratch.get(key)
+    if have is None:
+        if torch.cuda.is_current_stream_capturing():
+            # (a buffer made during a capture belongs to the graph's pool: it must not outlive it here)
+            raise RuntimeError("the paired product's scratch would have to be made inside a graph capture: "
+                               "run a paired product once before the capture")
+        have = (torch.zeros(room * PAIR_TILE_FLOATS, dtype=torch.float32, device=device),
+                torch.zeros(room * PAIR_TILE_COUNTERS, dtype=torch.int32, device=device))
+        _pair_scratch[key] = have
     counters = c_int(0)
     lib.ts_gemm_pair_scratch.restype = c_longlong
     need = lib.ts_gemm_pair_scratch(c_int(M), c_int(N), c_int(K), c_int(pairs), c_int(halves), c_int(1 if out_float32 else 0), ctypes.byref(counters))
-    key = str(device)
-    have = _pair_scratch.get(key)
-    if have is None or have[0].numel() < need or have[1].numel() < counters.value:
-        if torch.cuda.is_current_stream_capturing():
-            # (a buffer made during a capture belongs to the graph's pool: it must not outlive it here)
-            raise RuntimeError("the paired product's scratch would have to grow inside a graph capture: "
-                               "run the shape once before it is captured")
-        grow = max(need, have[0].numel() if have else 0, 1)
-        have = (torch.zeros(grow, dtype=torch.float32, device=device),
-                torch.zeros(max(counters.value, 1024), dtype=torch.int32, device=device))
-        _pair_scratch[key] = have
+    if need > have[0].numel() or counters.value > have[1].numel():
+        raise RuntimeError(f"paired product of {M} x {N} x {K}: {need} floats of scratch, {have[0].numel()} at most were expected")
     return have
 
 
