@@ -785,9 +785,9 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
   __syncthreads();
 
   pdl_trigger();
-  // The lengths, the block table and every cached key but the newest were written before this
-  // step's kernels began: the first tiles are fetched before pdl_wait(), while the kernels that
-  // make this token's query, key and value still run.  The tile with the newest key and the
+  // The lengths, the block table and every cached key but the newest are complete before any kernel of
+  // the step's layers is launched (the kernels that write the step's indices have no early trigger): the
+  // first tiles are fetched before pdl_wait(), while the kernels that make this token's query, key and value still run.  The tile with the newest key and the
   // query follow after it.
   if (q_end - q_begin != 1) {
     // (in a captured shape every entry may be unused: one block waits all the same, or this kernel would be complete, and the
@@ -976,9 +976,9 @@ __device__ __forceinline__ void attn_decode_qkv_body(const MmaAttnParams& p, con
   if (TMA) __syncthreads();
 
   pdl_trigger();
-  // The lengths, the block table and every cached key but the newest were written before this
-  // step's kernels began: the first tiles are fetched before pdl_wait(), while the kernels that
-  // make this token's query, key and value still run.  The tile with the newest key and the
+  // The lengths, the block table and every cached key but the newest are complete before any kernel of
+  // the step's layers is launched (the kernels that write the step's indices have no early trigger): the
+  // first tiles are fetched before pdl_wait(), while the kernels that make this token's query, key and value still run.  The tile with the newest key and the
   // query follow after it.
   const int b = blockIdx.z, split = blockIdx.y;
   const int kvh = blockIdx.x / p.head_tiles, head_tile = blockIdx.x % p.head_tiles;

@@ -97,10 +97,11 @@ TS_EXPORT int ts_block_tables_step(int* resident, const int* pairs, const int* n
 // harmless one (token 0, position 0, row 0, "no cache slot", the null page, an empty request), so
 // that no later kernel reads or writes out of bounds, and its kind is stored in the status words
 // (common.cuh), which the engine turns into an error.  Off in serving; tests switch it on.
+// (No early trigger in either kernel, as in the gather above: later kernels read the positions, slots, lengths
+// and block tables before their dependency wait.)
 __global__ void sanitize_step_kernel(int* token_ids, int T, int vocab, int* slot_tokens, int num_state_slots,
                                      int* positions, int num_positions, int* logit_rows, int W, int* cu_q,
                                      int* kv_lens, int B, int max_kv_len, int* state_slots) {
-  pdl_trigger();
   pdl_wait();
   for (int t = threadIdx.x; t < T; t += blockDim.x) {
     const int id = token_ids[t];
@@ -148,11 +149,11 @@ __global__ void sanitize_step_kernel(int* token_ids, int T, int vocab, int* slot
       if (b < B) kv_lens[b] = 0;
     }
   }
+  __threadfence();
 }
 
 __global__ void sanitize_group_kernel(int* slot_mapping, int T, long long total_slots, int* block_table, int B,
                                       int max_blocks, int row_stride, int num_pages) {
-  pdl_trigger();
   pdl_wait();
   for (int t = threadIdx.x; t < T; t += blockDim.x)
     if (slot_mapping[t] < -1 || slot_mapping[t] >= total_slots) {
@@ -166,6 +167,7 @@ __global__ void sanitize_group_kernel(int* slot_mapping, int T, long long total_
       *entry = 0;
     }
   }
+  __threadfence();
 }
 
 // token_ids, positions [T]; logit_rows [W]; cu_q [B + 1]; kv_lens, state_slots [B]; slot_tokens
