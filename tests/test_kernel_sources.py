@@ -41,3 +41,15 @@ def test_nothing_is_launched_ahead_of_the_step_indices(kernel):
     _, body = kernels()[("elementwise.cu", kernel)]
     assert "pdl_wait();" in body and "pdl_trigger" not in body
     assert body.rstrip().endswith("__threadfence();")
+
+
+# what no kernel of a step writes: the embedding, tables of angles, logits of attention sinks
+CONSTANTS = {"table", "cos", "sin", "vcos", "vsin", "sinks"}
+
+
+def test_what_a_predecessor_wrote_is_not_declared_constant():
+    """A load through a `const ... __restrict__` parameter may be brought forward over the dependency wait."""
+    for (name, kernel), (parameters, body) in kernels().items():
+        declared = set(re.findall(r"const\s+[\w:<>]+\s*\*\s*__restrict__\s+(\w+)", parameters))
+        assert declared <= CONSTANTS, f"{name}: {kernel} declares {sorted(declared - CONSTANTS)} constant"
+        assert "griddepcontrol" not in body        # (kernels wait through pdl_wait)

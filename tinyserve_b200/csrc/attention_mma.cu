@@ -1190,9 +1190,9 @@ attn_decode_qkv_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
 // out[row] = sum_s 2^(m_s - m) o_s / sum_s 2^(m_s - m) l_s over the key ranges of a row
 // (block x merges partial row x into output row x, or into head x % H of token tokens[x / H];
 // a negative token marks an unused entry of the list)
-__global__ void attention_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
+__global__ void attention_combine_kernel(const float* part_o, const float* part_ml,
                                          bf16* __restrict__ out, int num_splits, int H,
-                                         const int* __restrict__ tokens, TurnBack turn) {
+                                         const int* tokens, TurnBack turn) {
   pdl_trigger();
   pdl_wait();
   const size_t row = blockIdx.x;

@@ -252,8 +252,8 @@ __global__ void __launch_bounds__(WARPS * 32) paged_attention_kernel(AttnParams 
 
 // out[row] = sum_s exp(m_s - m) o_s / sum_s exp(m_s - m) l_s over the splits of a row
 template <typename T>
-__global__ void attention_combine_kernel(const float* __restrict__ part_o,
-                                         const float* __restrict__ part_ml, T* __restrict__ out,
+__global__ void attention_combine_kernel(const float* part_o,
+                                         const float* part_ml, T* __restrict__ out,
                                          int num_splits, const float* __restrict__ sinks, int H, TurnBack turn) {
   pdl_trigger();
   pdl_wait();

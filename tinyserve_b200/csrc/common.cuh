@@ -121,7 +121,9 @@ __device__ __forceinline__ void ts_raise_status(int word, int code) {
 // soon as all of this kernel's blocks have started) and pdl_wait() before it reads anything a
 // predecessor wrote and before it writes global memory at all; pdl_wait() returns when the
 // predecessor has completed and its writes are visible.  What a kernel does before pdl_wait()
-// (set-up, fetching weights) overlaps the predecessor.  Set TINYSERVE_PDL=0 to launch plainly.
+// (set-up, fetching weights) overlaps the predecessor.  A parameter that a predecessor writes is never declared
+// `const ... __restrict__`: the compiler takes such memory for constant during the kernel and may move its loads up
+// over the wait (prompts of 512 tokens in 32-bit came out wrong so).  Set TINYSERVE_PDL=0 to launch plainly.
 __device__ __forceinline__ void pdl_trigger() {
   timeline_mark(0);
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");

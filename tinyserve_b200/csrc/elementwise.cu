@@ -12,9 +12,9 @@ TS_DEFINE_LAST_ERROR()
 // An id < 0 stands for a token that is still on the device: -1 - slot names the state slot of the
 // request, whose last sampled token the sampler left in slot_tokens[slot].
 template <typename T>
-__global__ void embed_lookup_kernel(const T* __restrict__ table, const int* __restrict__ ids,
+__global__ void embed_lookup_kernel(const T* __restrict__ table, const int* ids,
                                     float* __restrict__ out, int n, int vocab,
-                                    const int* __restrict__ slot_tokens, float scale) {
+                                    const int* slot_tokens, float scale) {
   pdl_trigger();
   pdl_wait();
   const int t = blockIdx.x;
@@ -50,7 +50,7 @@ TS_EXPORT int ts_embed_lookup(int dtype, const void* table, const int* ids, floa
 // tables that the attention kernels index by request.  The number of pairs is read from device
 // memory, so that a captured graph serves any step.
 __global__ void block_table_scatter_kernel(int* __restrict__ resident, long long resident_size,
-                                           const int* __restrict__ pairs, const int* __restrict__ num_pairs,
+                                           const int* pairs, const int* num_pairs,
                                            int capacity) {
   pdl_trigger();
   pdl_wait();
@@ -61,8 +61,8 @@ __global__ void block_table_scatter_kernel(int* __restrict__ resident, long long
   }
 }
 
-__global__ void block_table_gather_kernel(const int* __restrict__ resident, int* __restrict__ step_tables,
-                                          const int* __restrict__ state_slots, int num_slots, int max_requests,
+__global__ void block_table_gather_kernel(const int* resident, int* __restrict__ step_tables,
+                                          const int* state_slots, int num_slots, int max_requests,
                                           int max_blocks) {
   // (no early trigger: the decode attention reads these tables before its dependency wait, and with small kernels in between
   // it could start while this one still writes.  So nothing behind it is launched until its blocks are done.)
@@ -197,9 +197,9 @@ TS_EXPORT int ts_sanitize_group(int* slot_mapping, int T, long long total_slots,
 // input row rows[i].  The order of the sum depends on n and the block size only.  With `xs` (one
 // factor per column, null: none) x is multiplied by it, in 32-bit, before it is added.
 template <typename T>
-__global__ void add_rmsnorm_kernel(const T* __restrict__ x, float* __restrict__ residual,
+__global__ void add_rmsnorm_kernel(const T* x, float* __restrict__ residual,
                                    VecParam w, float eps, T* __restrict__ out,
-                                   const int* __restrict__ rows, int n, int write_residual, PartialSrc ps,
+                                   const int* rows, int n, int write_residual, PartialSrc ps,
                                    VecParam xs) {
   __shared__ float scratch[33];
   pdl_trigger();
@@ -263,8 +263,8 @@ template <> struct Quad<__nv_bfloat16> {
 // number of rows in flight per SM, and four element groups per thread would otherwise leave room
 // for two blocks only.
 template <typename T, int ITEMS, int MAX_THREADS = 1024, int MIN_BLOCKS = 1>
-__global__ void __launch_bounds__(MAX_THREADS, MIN_BLOCKS) add_rmsnorm_vec_kernel(const T* __restrict__ x, float* __restrict__ residual, VecParam w,
-                                       float eps, T* __restrict__ out, const int* __restrict__ rows,
+__global__ void __launch_bounds__(MAX_THREADS, MIN_BLOCKS) add_rmsnorm_vec_kernel(const T* x, float* __restrict__ residual, VecParam w,
+                                       float eps, T* __restrict__ out, const int* rows,
                                        int n, int write_residual, PartialSrc ps, VecParam xs) {
   __shared__ float scratch[33];
   pdl_trigger();
@@ -337,8 +337,8 @@ constexpr int NORM_CLUSTER = 8;
 constexpr int PARTIAL_BATCH = 8;      // loads of partial sums in flight per thread
 
 template <typename T>
-__global__ void add_rmsnorm_cluster_kernel(const T* __restrict__ x, float* __restrict__ residual, VecParam w,
-                                           float eps, T* __restrict__ out, const int* __restrict__ rows,
+__global__ void add_rmsnorm_cluster_kernel(const T* x, float* __restrict__ residual, VecParam w,
+                                           float eps, T* __restrict__ out, const int* rows,
                                            int n, int quads_per_block, int write_residual, PartialSrc ps,
                                            VecParam xs) {
   __shared__ float scratch[33];
@@ -488,7 +488,7 @@ __device__ __forceinline__ float branch_addend1(const BranchAddends& a, size_t r
 
 template <typename T>
 __global__ void branch_norm_kernel(BranchAddends a, float* __restrict__ residual, VecParam w1, VecParam w2, float eps,
-                                   T* __restrict__ out1, T* __restrict__ out2, const int* __restrict__ rows, int n,
+                                   T* __restrict__ out1, T* __restrict__ out2, const int* rows, int n,
                                    int write_residual) {
   __shared__ float scratch[33];
   pdl_trigger();
@@ -517,7 +517,7 @@ __device__ __forceinline__ void quad_param(const VecParam& w, int c, float (&v)[
 template <typename T, int ITEMS, bool CLUSTER, int MAX_THREADS = 1024, int MIN_BLOCKS = 1>
 __global__ void __launch_bounds__(MAX_THREADS, MIN_BLOCKS)
 branch_norm_vec_kernel(BranchAddends a, float* __restrict__ residual, VecParam w1, VecParam w2, float eps,
-                       T* __restrict__ out1, T* __restrict__ out2, const int* __restrict__ rows, int n,
+                       T* __restrict__ out1, T* __restrict__ out2, const int* rows, int n,
                        int quads_per_block, int write_residual) {
   __shared__ float scratch[33];
   __shared__ float cluster_part;
@@ -715,7 +715,7 @@ __device__ __forceinline__ void block_sum3(float& a, float& b, float& c, float* 
 }
 
 template <typename T, int HOLD>      // HOLD 0: any row length and alignment, element by element
-__global__ void poly_norm_kernel(const T* __restrict__ z, T* __restrict__ out, VecParam coef, float eps, int n) {
+__global__ void poly_norm_kernel(const T* z, T* __restrict__ out, VecParam coef, float eps, int n) {
   __shared__ float scratch[96];
   pdl_trigger();
   pdl_wait();
@@ -802,7 +802,7 @@ TS_EXPORT int ts_poly_norm(int dtype, const void* z, void* out, const void* coef
 
 // plain RMSNorm of rows stored as T
 template <typename T>
-__global__ void rmsnorm_kernel(const T* __restrict__ x, VecParam w, float eps, T* __restrict__ out,
+__global__ void rmsnorm_kernel(const T* x, VecParam w, float eps, T* __restrict__ out,
                                int n) {
   __shared__ float scratch[33];
   pdl_trigger();
@@ -837,7 +837,7 @@ TS_EXPORT int ts_rmsnorm(int dtype, const void* x, const void* weight, int weigh
 // out[m, :] = x[m, :] * rsqrt(sum_t sumsq[t][m] / n + eps): the normalised rows of what the residual
 // forms of the tcgen05 products leave (x = residual * norm_weight, sums of residual^2 per 128
 // columns, `stride` floats apart)
-__global__ void scale_rows_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ sumsq, int tiles,
+__global__ void scale_rows_kernel(const __nv_bfloat16* x, const float* sumsq, int tiles,
                                   int stride, float eps, __nv_bfloat16* __restrict__ out, int n) {
   pdl_trigger();
   pdl_wait();
@@ -885,7 +885,7 @@ TS_EXPORT int ts_reduce_partials(int dtype, const float* partials, int splits, i
 __device__ __forceinline__ int gate_column(int c, int block) { return block ? (c / block) * 2 * block + c % block : c; }
 
 template <typename T>
-__global__ void gated_activation_kernel(const T* __restrict__ in, T* __restrict__ out, int inter,
+__global__ void gated_activation_kernel(const T* in, T* __restrict__ out, int inter,
                                         int act, int block, float limit) {
   pdl_trigger();
   pdl_wait();
@@ -899,7 +899,7 @@ __global__ void gated_activation_kernel(const T* __restrict__ in, T* __restrict_
 
 // 16 bytes per thread and operand, for widths that are a multiple of 16 / sizeof(T)
 template <typename T>
-__global__ void gated_activation_vec_kernel(const T* __restrict__ in, T* __restrict__ out, int inter, int act,
+__global__ void gated_activation_vec_kernel(const T* in, T* __restrict__ out, int inter, int act,
                                             int block, float limit) {
   constexpr int V = 16 / sizeof(T);
   pdl_trigger();
@@ -1079,12 +1079,12 @@ __device__ __forceinline__ void rope_one_head(int t, int head, int lane, const T
 // one warp per (token, head); with gridDim.y smaller than the number of head groups the warps
 // walk the heads, so that many tokens need few, fatter blocks
 template <typename T>
-__global__ void qk_norm_rope_kvwrite_kernel(const T* __restrict__ qkv, T* __restrict__ q_out,
-                                            const int* __restrict__ positions, RopeArgs rope,
+__global__ void qk_norm_rope_kvwrite_kernel(const T* qkv, T* __restrict__ q_out,
+                                            const int* positions, RopeArgs rope,
                                             VecParam qw, VecParam kw, int has_norm, float eps,
                                             int H, int Hkv, int D, T* __restrict__ k_cache,
                                             T* __restrict__ v_cache,
-                                            const int* __restrict__ slot_mapping, int page_size,
+                                            const int* slot_mapping, int page_size,
                                             int heads_total, PartialSrc ps) {
   pdl_trigger();
   pdl_wait();
@@ -1237,12 +1237,12 @@ __device__ __forceinline__ void rope_apply_vec(const RopeHead<T, STEPS>& h, int 
 }
 
 template <typename T, int STEPS>
-__global__ void qk_norm_rope_kvwrite_vec_kernel(const T* __restrict__ qkv, T* __restrict__ q_out,
-                                                const int* __restrict__ positions, RopeArgs rope,
+__global__ void qk_norm_rope_kvwrite_vec_kernel(const T* qkv, T* __restrict__ q_out,
+                                                const int* positions, RopeArgs rope,
                                                 VecParam qw, VecParam kw, int has_norm, float eps,
                                                 int H, int Hkv, int D, T* __restrict__ k_cache,
                                                 T* __restrict__ v_cache,
-                                                const int* __restrict__ slot_mapping, int page_size,
+                                                const int* slot_mapping, int page_size,
                                                 int heads_total, PartialSrc ps) {
   pdl_trigger();
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1266,12 +1266,12 @@ __global__ void qk_norm_rope_kvwrite_vec_kernel(const T* __restrict__ qkv, T* __
 constexpr int ROPE_UNROLL = 3;
 
 template <typename T, int STEPS>
-__global__ void qk_norm_rope_kvwrite_rows_kernel(const T* __restrict__ qkv, T* __restrict__ q_out,
-                                                 const int* __restrict__ positions, RopeArgs rope,
+__global__ void qk_norm_rope_kvwrite_rows_kernel(const T* qkv, T* __restrict__ q_out,
+                                                 const int* positions, RopeArgs rope,
                                                  VecParam qw, VecParam kw, int has_norm, float eps,
                                                  int H, int Hkv, int D, T* __restrict__ k_cache,
                                                  T* __restrict__ v_cache,
-                                                 const int* __restrict__ slot_mapping, int page_size,
+                                                 const int* slot_mapping, int page_size,
                                                  int heads_total) {
   pdl_trigger();
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1375,10 +1375,10 @@ __device__ __forceinline__ Raw8<__nv_bfloat16> load_raw8(const __nv_bfloat16* p)
 template <typename T, int LPH, int TOK>
 __global__ void __launch_bounds__(512, sizeof(T) == 2 ? 2 : 1)
 qk_norm_rope_kvwrite_rows8_kernel(const T* qkv, T* __restrict__ q_out,
-                                  const int* __restrict__ positions, RopeArgs rope,
+                                  const int* positions, RopeArgs rope,
                                   VecParam qw, VecParam kw, int has_norm, float eps,
                                   int H, int Hkv, T* __restrict__ k_cache, T* __restrict__ v_cache,
-                                  const int* __restrict__ slot_mapping, int page_size, int heads_total, int num_tokens) {
+                                  const int* slot_mapping, int page_size, int heads_total, int num_tokens) {
   constexpr int D = LPH * 16, HALF = D / 2, HPW = 32 / LPH;
   pdl_trigger();
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1559,9 +1559,9 @@ TS_EXPORT int ts_qk_norm_rope_kvwrite(int dtype, const void* qkv, void* q_out, c
 // (row i of the output is row rows[i] of the inputs).  The row waits in shared memory between
 // the passes (mean, deviations, output), so every element is loaded once.
 template <typename T>
-__global__ void add_layernorm_kernel(const T* __restrict__ x1, const T* __restrict__ x2, float* __restrict__ residual,
-                                     VecParam w, const void* __restrict__ bias, int bias_is_f32, float eps,
-                                     T* __restrict__ out, const int* __restrict__ rows, int n, int write_residual) {
+__global__ void add_layernorm_kernel(const T* x1, const T* x2, float* __restrict__ residual,
+                                     VecParam w, const void* bias, int bias_is_f32, float eps,
+                                     T* __restrict__ out, const int* rows, int n, int write_residual) {
   extern __shared__ float ln_row[];
   __shared__ float scratch[33];
   pdl_trigger();
@@ -1623,7 +1623,7 @@ TS_EXPORT int ts_add_layernorm(int dtype, const void* x1, const void* x2, float*
 
 // ------------------------------------------------------------------ sum of two tensors stored as T
 template <typename T>
-__global__ void sum2_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ out, size_t count) {
+__global__ void sum2_kernel(const T* a, const T* b, T* __restrict__ out, size_t count) {
   pdl_trigger();
   pdl_wait();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x)
@@ -1661,8 +1661,8 @@ TS_EXPORT int ts_softcap(float* x, long long count, float cap, float scale, cuda
 // rows, or null): what a block left pending, and the stream as it left the embedding, both added
 // before a group of layers runs again.
 template <typename T>
-__global__ void stream_add_kernel(float* __restrict__ residual, const T* __restrict__ x, PartialSrc ps, VecParam xs,
-                                  const float* __restrict__ first, int n) {
+__global__ void stream_add_kernel(float* __restrict__ residual, const T* x, PartialSrc ps, VecParam xs,
+                                  const float* first, int n) {
   pdl_trigger();
   pdl_wait();
   const size_t m = blockIdx.x;
@@ -1714,8 +1714,8 @@ TS_EXPORT int ts_add_row_vector(float* x, const void* vec, int vec_is_f32, int n
 // are still pending included), columns [n, 2 n) = `first` (the stream as it left the embedding):
 // the input of a product that re-injects the embedding into the stream.
 template <typename T>
-__global__ void stream_concat_kernel(const float* __restrict__ residual, const T* __restrict__ x1,
-                                     const T* __restrict__ x2, const float* __restrict__ first, T* __restrict__ out, int n) {
+__global__ void stream_concat_kernel(const float* residual, const T* x1,
+                                     const T* x2, const float* first, T* __restrict__ out, int n) {
   pdl_trigger();
   pdl_wait();
   const size_t m = blockIdx.x;
@@ -1815,11 +1815,11 @@ TS_EXPORT int ts_mean_of_normed(int dtype, int count, const void* const* xs, con
 // is served by key head g M + m; the value cache holds G / M heads, and the attention kernels give
 // key head i the value head i / M (their `v_share`).
 template <typename T>
-__global__ void rope_unit_kvwrite_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ k, long long ldk,
-                                         const T* __restrict__ v, long long ldv, T* __restrict__ q_out,
-                                         const int* __restrict__ positions, RopeArgs rope, int unit_norm, float eps,
+__global__ void rope_unit_kvwrite_kernel(const T* q, long long ldq, const T* k, long long ldk,
+                                         const T* v, long long ldv, T* __restrict__ q_out,
+                                         const int* positions, RopeArgs rope, int unit_norm, float eps,
                                          int H, int G, int dim, int vdim, int D, T* __restrict__ k_cache,
-                                         T* __restrict__ v_cache, const int* __restrict__ slot_mapping, int page_size,
+                                         T* __restrict__ v_cache, const int* slot_mapping, int page_size,
                                          int heads_total, VecParam qw, VecParam kw, float pre_eps, int maps,
                                          const float* __restrict__ vcos, const float* __restrict__ vsin) {
   pdl_trigger();
@@ -1905,12 +1905,12 @@ __global__ void rope_unit_kvwrite_kernel(const T* __restrict__ q, long long ldq,
 // The same for neighbouring pairs without norms and maps, sizes in multiples of 8: a thread turns eight columns of a
 // stored head (four pairs), 16 bytes of bfloat16 or two times 16 bytes of float in and out.
 template <typename T>
-__global__ void rope_pairs_kvwrite_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ k, long long ldk,
-                                          const T* __restrict__ v, long long ldv, T* __restrict__ q_out,
-                                          const int* __restrict__ positions, const float* __restrict__ cos,
+__global__ void rope_pairs_kvwrite_kernel(const T* q, long long ldq, const T* k, long long ldk,
+                                          const T* v, long long ldv, T* __restrict__ q_out,
+                                          const int* positions, const float* __restrict__ cos,
                                           const float* __restrict__ sin, int R, const float* __restrict__ vcos,
                                           const float* __restrict__ vsin, int H, int G, int dim, int vdim, int D,
-                                          T* __restrict__ k_cache, T* __restrict__ v_cache, const int* __restrict__ slot_mapping,
+                                          T* __restrict__ k_cache, T* __restrict__ v_cache, const int* slot_mapping,
                                           int page_size, int heads_total) {
   pdl_trigger();
   pdl_wait();
@@ -2008,7 +2008,7 @@ TS_EXPORT int ts_rope_unit_kvwrite(int dtype, const void* q, long long ldq, cons
 // ------------------------------------------------------------------ one sigmoid gate per head
 // out [T, H * vdim] = attn [T, H, D][..., :vdim] * sigmoid(gate[t * ldg + h])
 template <typename T>
-__global__ void head_gate_kernel(const T* __restrict__ attn, const T* __restrict__ gate, long long ldg,
+__global__ void head_gate_kernel(const T* attn, const T* gate, long long ldg,
                                  T* __restrict__ out, int H, int D, int vdim) {
   pdl_trigger();
   pdl_wait();
@@ -2037,7 +2037,7 @@ TS_EXPORT int ts_head_gate(int dtype, const void* attn, const void* gate, long l
 // g = h / r, r heads per kv head).  out [T, heads * vdim]: d = a_0 - lambda a_1 over the first vdim
 // columns, then d / sqrt(mean(d^2) + eps) * post.  One warp per (token, head), 32-bit.
 template <typename T>
-__global__ void map_difference_kernel(const T* __restrict__ attn, T* __restrict__ out, int heads, int r, int D, int vdim,
+__global__ void map_difference_kernel(const T* attn, T* __restrict__ out, int heads, int r, int D, int vdim,
                                       float lambda, float eps, float post, int num_tokens) {
   pdl_trigger();
   pdl_wait();

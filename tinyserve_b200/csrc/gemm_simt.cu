@@ -69,7 +69,7 @@ __device__ __forceinline__ int spread(int t, int j) {
 
 template <typename TI, typename TO, int BM, int BN, int TM, int TN, bool VEC>
 __global__ void __launch_bounds__(THREADS)
-gemm_nt_kernel(const TI* __restrict__ A, const TI* __restrict__ W, const TI* __restrict__ bias,
+gemm_nt_kernel(const TI* A, const TI* W, const TI* bias,
                TO* __restrict__ C, int M, int N, int K, size_t lda, size_t ldw, size_t ldc) {
   static_assert((BM / TM) * (BN / TN) == THREADS, "tile does not match the block");
   __shared__ float As[BK][BM + 4];
@@ -148,7 +148,7 @@ __device__ __forceinline__ void copy16_async(uint32_t dst, const void* src, bool
 }
 
 __global__ void __launch_bounds__(SPLIT_THREADS, 2)
-gemm_nt_chains_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
+gemm_nt_chains_kernel(const float* A, const float* W, const float* bias,
                       float* __restrict__ C, int M, int N, int K, size_t lda, size_t ldw, size_t ldc, bool constant_w) {
   extern __shared__ __align__(16) char smem[];
   pdl_trigger();
@@ -316,7 +316,7 @@ constexpr int MAX_CHAINS_SHIFT = 4;  // up to 16 chains of a row at a time: 8 RT
 
 template <int MT, int RT, int STAGES>
 __global__ void __launch_bounds__(SLOTS)
-gemv_nt_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
+gemv_nt_kernel(const float* A, const float* W, const float* bias, float* __restrict__ C,
                int M, int N, int K, size_t lda, size_t ldw, size_t ldc, int cs_shift, bool constant_w) {
   extern __shared__ __align__(16) char smem[];
   const int cs = 1 << cs_shift, groups = SLOTS >> cs_shift;      // chains in flight, groups of rows

@@ -30,9 +30,9 @@ namespace {
 
 // ------------------------------------------------------------------ post-norm, add, pre-norm
 template <typename T>
-__global__ void normed_add_rmsnorm_kernel(const T* __restrict__ y, VecParam w_post, float* __restrict__ residual,
+__global__ void normed_add_rmsnorm_kernel(const T* y, VecParam w_post, float* __restrict__ residual,
                                           VecParam w_pre, float eps_post, float eps_pre, T* __restrict__ out,
-                                          const int* __restrict__ rows, int n, int write_residual) {
+                                          const int* rows, int n, int write_residual) {
   extern __shared__ float row[];
   __shared__ float scratch[33];
   pdl_trigger();
@@ -115,8 +115,8 @@ __global__ void latent_prepare_kernel(LatentPrepare p) {
 // out[t, h, :] = [ carried[h, t, :kv_rank] | rotate(q[t, h, dim : dim + rot_dim]) | 0 ]; the rotation pairs
 // element j with j + rot_dim / 2, or with `interleaved` element 2j with 2j + 1
 template <typename T>
-__global__ void latent_query_kernel(const T* __restrict__ carried, const T* __restrict__ q, long long ldq, int H, int dim,
-                                    int rot_dim, int kv_rank, int stored, const int* __restrict__ positions,
+__global__ void latent_query_kernel(const T* carried, const T* q, long long ldq, int H, int dim,
+                                    int rot_dim, int kv_rank, int stored, const int* positions,
                                     const float* __restrict__ cos, const float* __restrict__ sin, T* __restrict__ out,
                                     int num_tokens, int interleaved) {
   pdl_trigger();
@@ -142,7 +142,7 @@ __global__ void latent_query_kernel(const T* __restrict__ carried, const T* __re
 
 // out[t, h * n + c] = x[h, t, c] * sigmoid(gate[t * ldg + h * n + c]) (gate null: the heads are only laid side by side)
 template <typename T>
-__global__ void gate_heads_kernel(const T* __restrict__ x, const T* __restrict__ gate, long long ldg, T* __restrict__ out,
+__global__ void gate_heads_kernel(const T* x, const T* gate, long long ldg, T* __restrict__ out,
                                   int H, int n, int num_tokens) {
   pdl_trigger();
   pdl_wait();
@@ -334,9 +334,9 @@ __global__ void moe_route_scored_kernel(Router r, float* __restrict__ gates, int
 // warp, into shared memory), as ts_moe_route does: one launch for the router's softmax, its choice
 // and the activation.
 template <typename T>
-__global__ void moe_gated_activate_kernel(const T* __restrict__ a, const float* __restrict__ gates, int E, int ff,
-                                          T* __restrict__ out, int act, float limit, const float* __restrict__ logits,
-                                          const float* __restrict__ bias, int top, int renorm, Router router) {
+__global__ void moe_gated_activate_kernel(const T* a, const float* gates, int E, int ff,
+                                          T* __restrict__ out, int act, float limit, const float* logits,
+                                          const float* bias, int top, int renorm, Router router) {
   extern __shared__ float routed[];      // [E] when the kernel routes (with a scored router: its scratch behind it)
   pdl_trigger();
   pdl_wait();
@@ -364,8 +364,8 @@ __global__ void moe_gated_activate_kernel(const T* __restrict__ a, const float* 
   }
 }
 
-__global__ void moe_route_kernel(const float* __restrict__ logits, float* __restrict__ gates, int num_tokens, int E, int top,
-                                 int renorm, const float* __restrict__ bias) {
+__global__ void moe_route_kernel(const float* logits, float* __restrict__ gates, int num_tokens, int E, int top,
+                                 int renorm, const float* bias) {
   pdl_trigger();
   pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -396,8 +396,8 @@ __device__ __forceinline__ void chunk_store(T* p, const float (&v)[Chunk<T>::N])
 // With `logits` (and top > 0) the block routes its token itself first (its first warp, into shared
 // memory): one launch for the router's softmax, its choice and the activation.
 template <typename T, bool VEC>
-__global__ void moe_activate_kernel(T* __restrict__ a, const float* __restrict__ gates, int E, int ff,
-                                    const float* __restrict__ logits, int top) {
+__global__ void moe_activate_kernel(T* __restrict__ a, const float* gates, int E, int ff,
+                                    const float* logits, int top) {
   extern __shared__ float routed[];      // [E] when the kernel routes
   pdl_trigger();
   pdl_wait();
@@ -435,7 +435,7 @@ __global__ void moe_activate_kernel(T* __restrict__ a, const float* __restrict__
 // then a row for every (token, expert) pair with a gate above zero.  Within a run the rows are in
 // the order the threads arrive; a row's result does not depend on its place.
 constexpr int GROUP_ALIGN = 16;
-__global__ void __launch_bounds__(1024) moe_group_kernel(const float* __restrict__ gates, int num_tokens, int E,
+__global__ void __launch_bounds__(1024) moe_group_kernel(const float* gates, int num_tokens, int E,
                                                          int* __restrict__ row_token, int* __restrict__ pair_row,
                                                          int* __restrict__ ends, int capacity) {
   extern __shared__ int sh[];          // [E] counts, then cursors
@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const float* __restrict
 
 // x_sorted[row] = x[row_token[row]] (zeros where the row is padding)
 template <typename T>
-__global__ void moe_gather_kernel(const T* __restrict__ x, const int* __restrict__ row_token, T* __restrict__ out, int n) {
+__global__ void moe_gather_kernel(const T* x, const int* row_token, T* __restrict__ out, int n) {
   pdl_trigger();
   pdl_wait();
   const size_t row = blockIdx.x;
@@ -484,8 +484,8 @@ __global__ void moe_gather_kernel(const T* __restrict__ x, const int* __restrict
 // out[t] = sum_e gates[t, e] * y[pair_row[t, e]] over the experts the token chose, in expert order
 // (+ rest[t] * h[t], the identity experts, with rest)
 template <typename T, bool VEC>
-__global__ void moe_combine_kernel(const T* __restrict__ y, const float* __restrict__ gates, const int* __restrict__ pair_row,
-                                   T* __restrict__ out, int E, int n, const float* __restrict__ rest, const T* __restrict__ h) {
+__global__ void moe_combine_kernel(const T* y, const float* gates, const int* pair_row,
+                                   T* __restrict__ out, int E, int n, const float* rest, const T* h) {
   pdl_trigger();
   pdl_wait();
   const size_t t = blockIdx.x;
@@ -540,8 +540,8 @@ __global__ void moe_combine_kernel(const T* __restrict__ y, const float* __restr
 // chains of 64 whose results are added in order (as the package's FMA product does)
 constexpr int BT = 32, BKK = 16;
 template <typename T>
-__global__ void __launch_bounds__(256) batched_matmul_kernel(const T* __restrict__ A, long long sab, long long sam, long long sak,
-                                                             const T* __restrict__ B, long long sbb, long long sbk, long long sbn,
+__global__ void __launch_bounds__(256) batched_matmul_kernel(const T* A, long long sab, long long sam, long long sak,
+                                                             const T* B, long long sbb, long long sbk, long long sbn,
                                                              T* __restrict__ C, int M, int N, int K) {
   __shared__ float As[BKK][BT + 1];
   __shared__ float Bs[BKK][BT + 1];

@@ -54,7 +54,7 @@ __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + expf(-
 __device__ __forceinline__ float log_sigmoid_f(float z) { return fminf(z, 0.f) - log1pf(expf(-fabsf(z))); }
 
 // ------------------------------------------------------------------ learned positions
-__global__ void add_position_rows_kernel(float* __restrict__ residual, VecParam table, const int* __restrict__ positions,
+__global__ void add_position_rows_kernel(float* __restrict__ residual, VecParam table, const int* positions,
                                          int num_positions, int n) {
   pdl_trigger();
   pdl_wait();
@@ -320,7 +320,7 @@ constexpr int ROW_HOLD = 8;
 inline int row_threads(int per) { return per >= 1024 ? 256 : (per >= 512 ? 128 : (per >= 256 ? 64 : 32)); }
 
 template <bool ADD>
-__global__ void group_norm_kernel(Rows x, VecParam w, const int* __restrict__ rows, int groups, int n, float eps,
+__global__ void group_norm_kernel(Rows x, VecParam w, const int* rows, int groups, int n, float eps,
                                   RowsOut out, float* __restrict__ residual) {
   __shared__ float scratch[33];
   pdl_trigger();
@@ -574,9 +574,9 @@ __device__ __forceinline__ float2 mlstm_gates_walk(const float* __restrict__ raw
 }
 
 // a warp per (request, head): steps of few tokens a request
-__global__ void mlstm_gates_kernel(const float* __restrict__ raw, long long ld, float cap, float* __restrict__ m_state,
-                                   const int* __restrict__ state_slots, const int* __restrict__ fresh,
-                                   const int* __restrict__ cu_q, int num_requests, int H, float* __restrict__ keep,
+__global__ void mlstm_gates_kernel(const float* raw, long long ld, float cap, float* __restrict__ m_state,
+                                   const int* state_slots, const int* fresh,
+                                   const int* cu_q, int num_requests, int H, float* __restrict__ keep,
                                    float* __restrict__ write, float* __restrict__ floor_) {
   pdl_trigger();
   pdl_wait();
@@ -592,9 +592,9 @@ __global__ void mlstm_gates_kernel(const float* __restrict__ raw, long long ld, 
 
 // a block per (request, head): every warp takes a span of the request's tokens, finds the span's map, learns
 // the maximum before its span from the maps of the spans before it, and walks its span again to write
-__global__ void mlstm_gates_spans_kernel(const float* __restrict__ raw, long long ld, float cap, float* __restrict__ m_state,
-                                         const int* __restrict__ state_slots, const int* __restrict__ fresh,
-                                         const int* __restrict__ cu_q, int H, float* __restrict__ keep,
+__global__ void mlstm_gates_spans_kernel(const float* raw, long long ld, float cap, float* __restrict__ m_state,
+                                         const int* state_slots, const int* fresh,
+                                         const int* cu_q, int H, float* __restrict__ keep,
                                          float* __restrict__ write, float* __restrict__ floor_) {
   __shared__ float span_f[32], span_i[32];
   pdl_trigger();
@@ -625,7 +625,7 @@ __global__ void mlstm_gates_spans_kernel(const float* __restrict__ raw, long lon
 
 // ------------------------------------------------------------------ what follows the scan of a matrix memory
 // raw [T, H, wide] 32-bit: columns [0, vdim) the numerator S^T q, column vdim the product n . q
-__global__ void mlstm_finish_kernel(const float* __restrict__ raw, int wide, const float* __restrict__ floor_,
+__global__ void mlstm_finish_kernel(const float* raw, int wide, const float* floor_,
                                     VecParam weight, Rows gate, float eps, RowsOut out, int H, int vdim, int num_tokens) {
   pdl_trigger();
   pdl_wait();
@@ -652,7 +652,7 @@ __global__ void mlstm_finish_kernel(const float* __restrict__ raw, int wide, con
 }
 
 // raw [T, H vdim] 32-bit y of the scan; x the scan's values; z the gate; a block per (token, norm group)
-__global__ void ssm_finish_kernel(const float* __restrict__ raw, Rows x, VecParam skip, Rows z, VecParam weight, int groups,
+__global__ void ssm_finish_kernel(const float* raw, Rows x, VecParam skip, Rows z, VecParam weight, int groups,
                                   float eps, RowsOut out, int H, int vdim) {
   __shared__ float scratch[33];
   pdl_trigger();
