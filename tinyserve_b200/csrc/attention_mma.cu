@@ -542,7 +542,8 @@ __device__ __forceinline__ void build_head(const MmaAttnParams& p, int t, int co
 // keys): one warp fetches whole pages as boxes of page x 64 columns with the 128-byte swizzle;
 // an SM streams about half as much again this way
 // as through its load/store unit's miss queue.  Whole pages come, also the keys past the
-// request's length in its last page: their scores are masked and their values made zero in shared memory.
+// request's length in its last page and those before the window in its first: their scores are masked and their values made
+// zero in shared memory, as those that cp.async leaves out are.
 constexpr int DEC_THREADS = 128, DEC_WARPS = DEC_THREADS / 32;
 constexpr int SUM_ROW = D + 4;                       // floats of a row of partial sums (4 mod 16: no bank conflicts)
 
@@ -576,16 +577,20 @@ __device__ __forceinline__ void add_scaled4(float (&sum)[4], float factor, const
   sum[2] = fmaf(factor, v.z, sum[2]); sum[3] = fmaf(factor, v.w, sum[3]);
 }
 
-// Values of the keys from j_hi on, of a warp's 16 (rows key0 .. of a tile that came by TMA), become zeros
-__device__ __forceinline__ void clear_values(char* vs, int key0, int jbase, int j_hi, int lane) {
-  if (jbase + 16 <= j_hi) return;
-  if (jbase + (lane >> 1) >= j_hi) {       // two lanes a row
+// Values of the keys that the query does not see (past the end, or before the window and not kept), of a warp's 16 (rows
+// key0 .. of a tile that came by TMA), become zeros: whatever lies there, a probability of zero leaves it out
+__device__ __forceinline__ void clear_values(char* vs, int key0, int jbase, int j_lo, int j_hi, int keep, int lane) {
+  if (jbase + 16 <= j_hi && (jbase >= j_lo || jbase + 16 <= keep)) return;
+  const int j = jbase + (lane >> 1);       // two lanes a row
+  if (j >= j_hi || (j < j_lo && j >= keep)) {
     const int row = key0 + (lane >> 1);
 #pragma unroll
     for (int k = 0; k < CH / 2; ++k) {
       const int piece = (lane & 1) * (CH / 2) + k;
       *reinterpret_cast<uint4*>(vs + (piece >> 3) * (BN * 128) + row * 128 + (((piece & 7) ^ (row & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
     }
+    // (a tile before the window's end is followed by another in its stage: these stores come before that copy)
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   }
   __syncwarp();
 }
@@ -906,7 +911,7 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
     __syncwarp();
     const int jbase = tile_of(walk_begin + it) * BN + key0;
     if (jbase < j_hi) {
-      if (TMA) clear_values(Vs + stage * KV_TILE, key0, jbase, j_hi, lane);
+      if (TMA) clear_values(Vs + stage * KV_TILE, key0, jbase, j_lo, j_hi, keep, lane);
       decode_keys<TMA, NH, Q_REGS>(o, m, l, qf, Qs, Ks + stage * KV_TILE, Vs + stage * KV_TILE, key0, jbase, qpos, j_lo, keep, p, sl, lane);
     }
     if (it + DEC_STAGES < n_tiles) {
@@ -1127,7 +1132,7 @@ __device__ __forceinline__ void attn_decode_qkv_body(const MmaAttnParams& p, con
     const int buf = it % DEC_STAGES;
     const int jbase = tile_of(walk_begin + it) * BN + warp * 16;
     if (jbase < j_hi) {
-      if (TMA) clear_values(Vs + buf * KV_TILE, warp * 16, jbase, j_hi, lane);
+      if (TMA) clear_values(Vs + buf * KV_TILE, warp * 16, jbase, j_lo, j_hi, 0, lane);
       float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
       qk_tile<2, TMA>(s, Qs, qf, Ks + buf * KV_TILE, warp * 16, lane);
       softmax_tile<2>(s, o, m, l, pos, lo, jbase, p.scale_log2, lane);
