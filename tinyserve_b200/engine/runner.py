@@ -500,22 +500,30 @@ class ModelRunner:
     def _mixed_shape_for(self, entries):
         """The captured shape (tokens, requests, logit rows, context bound) that a step with prompt
         portions is padded to, or None where it runs as it is: graphs are off, or the step is
-        larger than the largest captured token count.  Logit rows: one per request (what serving
-        asks for) or, where more are wanted, one per token."""
+        larger than the largest captured token count and does not use up the token budget.  Logit
+        rows: one per request (what serving asks for) or, where more are wanted, one per token (in a
+        step of the budget's size that would be a product with the whole vocabulary for every token: it
+        runs as it is)."""
         if not self.mixed_graphs_enabled:
             return None
         T = sum(len(e.tokens) for e in entries)
         B = len(entries)
         budget = self.cfg.max_num_batched_tokens
-        tokens = next((t for t in MIXED_GRAPH_TOKENS if t >= T), None)
-        if T == budget and any(len(e.tokens) == 1 for e in entries):
+        wanted = sum(len(e.want) for e in entries)
+        tokens = next((t for t in MIXED_GRAPH_TOKENS if T <= t <= budget), None)
+        whole_budget = tokens is None
+        if whole_budget:
+            if T != budget or all(len(e.tokens) > 1 for e in entries):
+                return None
             tokens = budget
-        if tokens is None or tokens > budget or B > self.cfg.max_num_seqs:
+        if B > self.cfg.max_num_seqs:
             return None
         # one request more than the step holds: the empty one that unused work-list entries name
         S = self.cfg.max_num_seqs
         requests = next((r for r in (2, 4, 8, 16, 32, 64, 128, 256, 512, 1024) if B < r <= S), S + 1)
-        rows = requests if sum(len(e.want) for e in entries) <= requests else tokens
+        if whole_budget and wanted > requests:
+            return None
+        rows = requests if wanted <= requests else tokens
         mgr = self.manager
         longest = max(mgr.num_computed(e.rid) + len(e.tokens) for e in entries)
         bound = next((b for b in self.context_bounds() if b >= longest), None)
