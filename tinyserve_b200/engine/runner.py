@@ -85,6 +85,7 @@ class ModelRunner:
         # graphs of steps with prompt portions, captured when a shape comes up the second time
         self.mixed_graphs: dict = {}
         self.mixed_graphs_enabled = False
+        self.budget_graphs_enabled = True        # among them those of steps that use up a budget that is not listed
         self.mixed_graph_replays = 0
         self._graph_pool = None
         self._capture_stream = None
@@ -513,7 +514,7 @@ class ModelRunner:
         tokens = next((t for t in MIXED_GRAPH_TOKENS if T <= t <= budget), None)
         whole_budget = tokens is None
         if whole_budget:
-            if T != budget or all(len(e.tokens) > 1 for e in entries):
+            if not self.budget_graphs_enabled or T != budget or all(len(e.tokens) > 1 for e in entries):
                 return None
             tokens = budget
         if B > self.cfg.max_num_seqs:
@@ -558,10 +559,17 @@ class ModelRunner:
                     finally:
                         graph.capture_end()
             except torch.cuda.OutOfMemoryError:
-                # no room left for another graph's buffers beside the cache: steps with portions
-                # run eagerly from now on (this one too: the caller gets no graph)
-                self.mixed_graphs_enabled = False
-                self.mixed_graphs.pop(key, None)
+                # no room left for another graph's buffers beside the cache (the caller gets no graph: this step
+                # runs eagerly).  The graphs of the whole budget go first, which hold most; where there are none,
+                # steps with portions run eagerly from now on
+                large = [k for k in self.mixed_graphs if k[0] not in MIXED_GRAPH_TOKENS]
+                if large:
+                    self.budget_graphs_enabled = False
+                    for k in large:
+                        del self.mixed_graphs[k]
+                else:
+                    self.mixed_graphs_enabled = False
+                    self.mixed_graphs.pop(key, None)
                 del graph
                 torch.cuda.current_stream(self.device).wait_stream(self._capture_stream)
                 return None
