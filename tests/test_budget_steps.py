@@ -43,3 +43,33 @@ def test_a_whole_budget_with_more_places_than_requests_runs_as_it_is(budget):
     assert r._mixed_shape_for(step([1, budget - 1], [1, budget - 1])) is None
     # smaller steps are padded to a row per token, as they always were
     assert r._mixed_shape_for(step([1, 39], [1, 39]))[:3] == (48, 4, 48)
+
+
+@pytest.mark.parametrize("graphs", [False, True])
+def test_the_cache_leaves_room_for_the_graphs_of_a_whole_budget(graphs, monkeypatch):
+    """The captured step's activations and the kept logits beside those of an eager step; a cache that just holds the longest
+    request is not refused for it."""
+    import torch
+    from tinyserve_b200.cache.device import DeviceCache
+    per_page, page = 1 << 20, 64
+    r = runner(4096, 64, 4096, num_blocks=0, gpu_memory_utilization=0.9, use_cuda_graphs=graphs)
+    r.page_size, r.max_blocks, r.device, r.dtype = page, 1 << 20, "cuda:0", torch.bfloat16
+    r.model = NS(vocab_size=151936, capturable=True)
+    r._activation_bytes_per_token = lambda: 400_000
+    monkeypatch.setattr(DeviceCache, "bytes_per_page", staticmethod(lambda *a: [per_page]))
+    total = 180 << 30
+    step, logits = 4096 * 400_000, 64 * 151936 * 4
+
+    def pages(free):
+        monkeypatch.setattr(torch.cuda, "mem_get_info", lambda device: (free, total))
+        return r._size_cache()
+
+    left = int(0.9 * total) - (1 << 30)          # (a card with nothing on it)
+    assert pages(total) * per_page + step + 2 * logits + (step + 16 * logits if graphs else 0) <= left
+    # little room: as many pages as without graphs, up to those of the longest request
+    few = int(0.1 * total) + step + 2 * logits + (1 << 30)
+    assert pages(few + 65 * per_page + 4096) == 65
+    assert pages(few + 80 * per_page + 4096) == (65 if graphs else 80)
+    from tinyserve_b200.cache.manager import CacheError
+    with pytest.raises(CacheError):
+        pages(few + 64 * per_page + 4096)

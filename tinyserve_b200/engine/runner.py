@@ -108,10 +108,18 @@ class ModelRunner:
             return 2
         free, total = torch.cuda.mem_get_info(self.device)
         # leave room for activations of a full step and for logits
-        reserve = cfg.max_num_batched_tokens * self._activation_bytes_per_token() + \
-            cfg.max_num_seqs * self.model.vocab_size * 8 + (1 << 30)
+        step = cfg.max_num_batched_tokens * self._activation_bytes_per_token()
+        rows = cfg.max_num_seqs * self.model.vocab_size
+        reserve = step + rows * 8 + (1 << 30)
         budget = min(total * cfg.gpu_memory_utilization - (total - free), free) - reserve
         pages = int(budget // per_page)
+        if cfg.use_cuda_graphs and self.model.capturable:
+            # and for the graphs: their pool holds the activations of one captured step, up to the whole budget's, beside
+            # those of a step that runs eagerly, and the logits of every shape that is kept.  (Not at the
+            # price of the longest request's pages: a capture that finds no room is given up)
+            graphs = step + MIXED_GRAPHS_KEPT * rows * 4
+            enough = -(-cfg.max_model_len // self.page_size) + 1
+            pages = max(int((budget - graphs) // per_page), min(pages, enough))
         if (pages - 1) * self.page_size < cfg.max_model_len:
             raise CacheError(
                 f"the cache would hold {max(0, pages - 1) * self.page_size} tokens, fewer than "
