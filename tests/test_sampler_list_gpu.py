@@ -41,3 +41,22 @@ def test_list_after_top_k(V, k, ties):
             masked[b][y < y.sort(descending=True).values[k - 1]] = -float("inf")
     assert torch.equal(ops.sample(masked, temp, streams, steps, 7).cpu(), only_k)
     assert torch.equal(ops.sample(masked, temp, streams, steps, 7, top_p=top_p).cpu(), both)
+
+
+@pytest.mark.parametrize("k", [8191, 8192, 8193, 20000])
+def test_list_of_eight_blocks(k):
+    """Up to eight times the length of a block's list top-k may leave lists, above there are none."""
+    from tinyserve_b200.kernels import ops
+    B, V = 2, 151936
+    g = torch.Generator().manual_seed(k)
+    x = (torch.randn(B, V, generator=g) * 3).cuda()
+    temp, streams, steps = torch.full((B,), 0.8).cuda(), torch.arange(B).cuda(), torch.arange(B, dtype=torch.int32).cuda()
+    top_k, top_p = torch.full((B,), k, dtype=torch.int32).cuda(), torch.full((B,), 0.9).cuda()
+    inverse = (1.0 / torch.tensor(0.8)).cuda()
+    masked = x.clone()
+    for b in range(B):
+        y = x[b] * inverse
+        masked[b][y < y.sort(descending=True).values[k - 1]] = -float("inf")
+    assert torch.equal(ops.sample(masked, temp, streams, steps, 7), ops.sample(x, temp, streams, steps, 7, top_k=top_k))
+    assert torch.equal(ops.sample(masked, temp, streams, steps, 7, top_p=top_p),
+                       ops.sample(x, temp, streams, steps, 7, top_k=top_k, top_p=top_p))

@@ -337,25 +337,29 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
       __syncthreads();
     }
     keep_from = prefix;
-    if (threadIdx.x == 0) list_count = 0;
-    __syncthreads();
-    for (int base = v0 + threadIdx.x * 4; base < v1; base += THREADS * 4) {
-      float q[4];
-      load4(base, q);
+    // (More tokens than the blocks' lists hold leave no list, and the pass over the row would be for nothing: k = 9,000 and
+    // top-p, with the pass / without, 1 row 103.5 / 100.2, 16 179 / 173, 64 325 / 311; top-k alone 64 rows 211 / 197.)
+    if (k <= LIST * (int)blocks) {
+      if (threadIdx.x == 0) list_count = 0;
+      __syncthreads();
+      for (int base = v0 + threadIdx.x * 4; base < v1; base += THREADS * 4) {
+        float q[4];
+        load4(base, q);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float y = q[j] * inv_temp;
-        if (base + j < v1 && sort_key(y) >= keep_from) {
-          const int at = atomicAdd(&list_count, 1);
-          if (at < LIST) {
-            list_token[at] = base + j;
-            list_value[at] = y;
+        for (int j = 0; j < 4; ++j) {
+          const float y = q[j] * inv_temp;
+          if (base + j < v1 && sort_key(y) >= keep_from) {
+            const int at = atomicAdd(&list_count, 1);
+            if (at < LIST) {
+              list_token[at] = base + j;
+              list_value[at] = y;
+            }
           }
         }
       }
+      __syncthreads();
+      listed = list_count <= LIST;       // (equal logits may leave more than k tokens)
     }
-    __syncthreads();
-    listed = list_count <= LIST;       // (equal logits may leave more than k tokens)
   }
   const int list_n = listed ? list_count : 0;
 

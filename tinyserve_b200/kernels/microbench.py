@@ -1,8 +1,8 @@
 """Time one kernel of the package at a given size, after warm-up, with CUDA events.
 
-    python -m tinyserve_b200.kernels.microbench gemm --m 8 --n 24576 --k 4096 [--splits S] [--impl tcgen05|cublas]
+    python -m tinyserve_b200.kernels.microbench gemm --m 8 --n 24576 --k 4096 [--splits S] [--impl tcgen05|cublas|registers]
     python -m tinyserve_b200.kernels.microbench gemm --m 2048 --n 24576 --k 4096 --impl pair [--mode plain|gated|residual]
-    python -m tinyserve_b200.kernels.microbench attention --batch 8 --q-len 1 --kv-len 640
+    python -m tinyserve_b200.kernels.microbench attention --batch 8 --q-len 1 --kv-len 640 [--from-qkv]
     python -m tinyserve_b200.kernels.microbench norm --rows 8 --n 4096
     python -m tinyserve_b200.kernels.microbench rope --rows 2048
 
@@ -54,6 +54,8 @@ def bench_gemm(a):
     splits = a.splits or ops.gemm_splits(a.m, a.n, a.k)
     if a.impl.startswith("tcgen05"):
         fn = lambda i: ops._linear_tcgen05(x, ws[i], False, splits=splits, partials_only=a.partials_only)
+    elif a.impl == "registers":        # up to 8 tokens and 16 MB of weights
+        fn = lambda i: ops._linear_gemv(x, ws[i], partials_only=a.partials_only)
     elif a.impl == "pair":
         # the paired kernel for many tokens, with the epilogue that the engine uses at this place
         res = torch.randn(a.m, a.n, device="cuda") if a.mode == "residual" else None
@@ -97,6 +99,16 @@ def bench_attention(a):
     sinks = torch.randn(H, device="cuda") if a.bias else None
     fn = lambda i: ops.paged_attention(q, kc, vc, views[i], ctx, D ** -0.5, 0, num_splits=a.splits or None,
                                      backend=a.backend or None, chunk=a.chunk, slopes=slopes, sinks=sinks)
+    if a.from_qkv:
+        # the block that makes its rows, the newest key and value from the projection (decode steps of a few requests)
+        from ..parts.rotary import Rotary
+        rot = Rotary(D, 1e6, "half")
+        rot.cos, rot.sin = (t.cuda() for t in Rotary.tables(D, 1e6, kv_len))
+        qkv = torch.randn(B, (H + 2 * Hkv) * D, device="cuda", dtype=torch.bfloat16)
+        w, last = torch.ones(D, device="cuda", dtype=torch.bfloat16), kv - 1
+        for v in views:
+            v.slot_mapping = (v.block_table[:, (kv_len - 1) // page] * page + (kv_len - 1) % page).contiguous()
+        fn = lambda i: ops.attention_from_qkv(qkv, last, H, Hkv, D, rot, w, w, 1e-6, kc, vc, views[i], ctx, D ** -0.5)
     us = _time(fn, copies, a.iters, a.graph)
     pos = torch.arange(kv_len - q_len, kv_len)
     seen = float((pos % a.chunk + 1).sum()) if a.chunk else float((pos + 1).sum())     # visible (query, key) pairs of a request
@@ -146,7 +158,7 @@ def main(argv=None):
     ap.add_argument("--n", type=int, default=24576)
     ap.add_argument("--k", type=int, default=4096)
     ap.add_argument("--splits", type=int, default=0)
-    ap.add_argument("--impl", choices=["tcgen05", "cublas", "pair"], default="tcgen05")
+    ap.add_argument("--impl", choices=["tcgen05", "cublas", "pair", "registers"], default="tcgen05")
     ap.add_argument("--mode", choices=["plain", "gated", "residual"], default="plain", help="epilogue of --impl pair")
     ap.add_argument("--halves", type=int, default=0, help="--impl pair: tiles of 256 (1) or 512 (2) weight rows, 0: by estimate")
     ap.add_argument("--pairs", type=int, default=0, help="pairs of blocks of --impl pair (default: all the device holds)")
@@ -160,6 +172,7 @@ def main(argv=None):
     ap.add_argument("--backend", choices=["tcgen05", "mma", "simt"], default="",
                     help="attention: a slower kernel than the one the head size selects")
     ap.add_argument("--chunk", type=int, default=0, help="attention: positions per chunk (0: plain causal)")
+    ap.add_argument("--from-qkv", action="store_true", help="attention of one token a request straight from the projection")
     ap.add_argument("--bias", action="store_true", help="attention: a distance slope and a sink per head")
     ap.add_argument("--rows", type=int, default=8)
     ap.add_argument("--copies", type=int, default=0)
