@@ -348,6 +348,19 @@ struct PartialSrc {
   }
 };
 
+// sums[0] + sums[stride] + ... of `tiles` values that a predecessor left, in this order, 32 loads in flight
+__device__ __forceinline__ float sum_of_tiles(const float* sums, int tiles, size_t stride) {
+  float sum = 0.f;
+  for (int t0 = 0; t0 < tiles; t0 += 32) {
+    float part[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) part[i] = t0 + i < tiles ? __ldcg(sums + (t0 + i) * stride) : 0.f;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) sum += part[i];
+  }
+  return sum;
+}
+
 // sum over a block of up to 1024 threads; every thread gets the result.
 // `scratch` holds 33 floats of shared memory.
 __device__ __forceinline__ float block_sum(float v, float* scratch) {

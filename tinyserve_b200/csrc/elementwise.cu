@@ -835,16 +835,14 @@ TS_EXPORT int ts_rmsnorm(int dtype, const void* x, const void* weight, int weigh
 
 // ------------------------------------------------------------------ rows without their norm factor -> rows
 // out[m, :] = x[m, :] * rsqrt(sum_t sumsq[t][m] / n + eps): the normalised rows of what the residual
-// forms of the tcgen05 products leave (x = residual * norm_weight, sums of residual^2 per 128
+// forms of the products leave (x = residual * norm_weight, sums of residual^2 per 128 or 16
 // columns, `stride` floats apart)
 __global__ void scale_rows_kernel(const __nv_bfloat16* x, const float* sumsq, int tiles,
                                   int stride, float eps, __nv_bfloat16* __restrict__ out, int n) {
   pdl_trigger();
   pdl_wait();
   const int m = blockIdx.x;
-  float sum = 0.f;
-  for (int t = 0; t < tiles; ++t) sum += sumsq[(size_t)t * stride + m];
-  const float rstd = rsqrtf(sum / (float)n + eps);
+  const float rstd = rsqrtf(sum_of_tiles(sumsq + m, tiles, stride) / (float)n + eps);
   for (int c = threadIdx.x; c < n; c += blockDim.x)
     out[(size_t)m * n + c] = __float2bfloat16_rn(__bfloat162float(x[(size_t)m * n + c]) * rstd);
 }

@@ -256,18 +256,13 @@ gemm_wx_kernel(const __grid_constant__ MAPS maps, const __grid_constant__ GemmPa
     if (ok && nkb > 0) tcgen05_commit(smem_u32(accum));
   } else {
     pdl_wait();
-    // (the lanes of warps 1..3 that do not issue have time for the rows' norm factors; two lanes
-    // take each row, so that one is left wherever the issuing lane is)
-    const int pair = (warp - 1) * 16 + (lane >> 1);       // 0 .. 47 over warps 1..3
-    if (p.x_sumsq != nullptr && warp >= 1) {
-      for (int j = pair; j < TILE_T; j += 48) {
-        const int m = t_tile * TILE_T + j;
-        float sum = 0.f;
-        if (m < p.M)
-#pragma unroll 8
-          for (int t = 0; t < p.x_tiles; ++t) sum += __ldcg(p.x_sumsq + (size_t)t * SUMSQ_STRIDE + m);
-        row_scale[j] = rsqrtf(sum / (float)p.K + p.x_eps);
-      }
+    // the rows' norm factors, a lane of warps 2 and 3 a row: sums of 32 tiles in one trip to memory, added in the order of the
+    // tiles (rows from gemv_mma.cu have a sum for every 16 columns: 64 of them, eight at a time, took longer than the weights)
+    const int j = (int)threadIdx.x - 64;
+    if (p.x_sumsq != nullptr && j >= 0 && j < TILE_T) {
+      const int m = t_tile * TILE_T + j;
+      const float sum = m < p.M ? sum_of_tiles(p.x_sumsq + m, p.x_tiles, SUMSQ_STRIDE) : 0.f;
+      row_scale[j] = rsqrtf(sum / (float)p.K + p.x_eps);
     }
   }
   __syncthreads();
