@@ -36,13 +36,12 @@ static_assert(D % 16 == 0 && D >= 16 && D <= 256, "head size must be a multiple 
 constexpr int CH = D / 8;                 // 16-byte chunks of a row
 constexpr int ROW_BYTES = D * 2 + 16;     // rows are padded by one chunk: ldmatrix without conflicts
 constexpr int CLUSTER_MAX = 8;            // key ranges that merge in a cluster
-// Key tiles that one block walks without its cluster.  Two, but one in clusters of two blocks where the ranges come by
-// cp.async, the head is wide and the merge short (few query heads a key head).  Clusters of two, 16 requests, 128 keys,
-// in the cluster / alone: heads of 256, one query head 17.8 / 20.4 us, four 22.9 / 22.5, eight 29.7 / 25.3; by TMA
-// 14.1 / 13.1; heads of 96 6.5 / 6.8, of 80 6.2 / 5.8.  In clusters of three and more alone is always the faster.
-__device__ __forceinline__ int alone_tiles(int cluster, int group, bool tma) {
-  return cluster > 2 || D <= 80 || tma || group >= 4 ? 2 : 1;
-}
+// Key tiles that one block walks without its cluster: two, but one in clusters of two blocks with wide heads, which share two
+// tiles evenly.  128 keys, in the cluster / alone, us: eight blocks (1 request, 32 heads over 8 of 128) 5.1 / 4.9, four (8
+// requests) 6.3 / 5.8, three (12, 8 over 8 of 96) 10.2 / 6.3; two (16 requests) heads of 64 5.3 / 5.0, of 80 5.9 / 6.2, of 96
+// 6.6 / 7.4, of 128 6.0 / 6.3, 32 over 8 of 128 6.8 / 7.4, of 256 12.6 / 13.5.  One tile is always faster alone (3.8 / 4.7 for
+// 1 request, 16 over 8 of 128); three are not in clusters of four and more (5.2 / 5.9 and 6.5 / 7.0).
+__device__ __forceinline__ int alone_tiles(int cluster) { return cluster > 2 || D <= 64 ? 2 : 1; }
 #ifndef TS_PREFILL_WARPS
 #define TS_PREFILL_WARPS 4
 #endif
@@ -811,7 +810,7 @@ __device__ __forceinline__ void attn_decode_body(const MmaAttnParams& p, const C
   const int total = (j_hi + BN - 1) / BN - first_tile + kept_tiles;
   auto tile_of = [&](int w) { return w < kept_tiles ? w : first_tile + (w - kept_tiles); };
   // A short walk is one block's: the ranges of a cluster cost their merge.  (All blocks of the cluster see the same.)
-  const bool alone = p.cluster_merge && total <= alone_tiles(p.num_splits, G, TMA);
+  const bool alone = p.cluster_merge && total <= alone_tiles(p.num_splits);
   const int per_split = alone ? total : (total + p.num_splits - 1) / p.num_splits;
   if (alone && split > 0) return;
   const int walk_begin = split * per_split;
@@ -998,10 +997,10 @@ __device__ __forceinline__ void attn_decode_qkv_body(const MmaAttnParams& p, con
   const int j_lo = p.window > 0 ? max(0, qpos - p.window + 1) : 0;
   const int first_tile = j_lo / BN, total = (j_hi + BN - 1) / BN - first_tile;
   auto tile_of = [&](int w) { return first_tile + w; };
-  // A short walk is one block's: the ranges of a cluster cost their merge (a cluster barrier and a round trip through
-  // distributed shared memory), a tile of 64 keys about 1 us.  One request, 16 heads over 8, 60 / 120 / 180 / 250 keys:
-  // 6.4 us in a cluster of eight, 4.5 / 5.4 / 6.5 / 7.7 alone.  (All blocks of the cluster see the same.)
-  const bool alone = p.cluster_merge && total <= alone_tiles(p.num_splits, G, TMA);
+  // A short walk is one block's: the ranges of a cluster cost their merge (the sums sent and one meeting), a tile of 64 keys
+  // about 0.9 us.  One request, 16 heads over 8, 60 / 120 / 180 / 250 keys: 4.7 us in a cluster of eight, 3.8 / 4.6 / 5.6 / 6.4
+  // alone.  (All blocks of the cluster see the same.)
+  const bool alone = p.cluster_merge && total <= alone_tiles(p.num_splits);
   const int per_split = alone ? total : (total + p.num_splits - 1) / p.num_splits;
   if (alone && split > 0) return;
   const int walk_begin = split * per_split;
