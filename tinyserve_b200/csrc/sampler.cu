@@ -2,7 +2,7 @@
 // to eight, a range of the vocabulary each, which combine their maxima and histograms through
 // distributed shared memory.  All that blocks combine is a maximum or an integer sum, so the result does
 // not depend on how many blocks share a row.  One row of 151,936 logits (600 KB) by one block / by eight:
-// greedy 9.1 / 4.8 us, with a temperature 65 / 12, with top-p 322 / 62, with top-k and top-p 463 / 90.
+// greedy 9.1 / 4.8 us, with a temperature 66 / 12, with top-p 369 / 65, with top-k 50 and top-p 311 / 64.
 //
 //   temperature == 0           -> argmax (serve.py:1521-1522)
 //   temperature > 0            -> x = logit / temperature, optional top-k (keep the k largest),
@@ -508,9 +508,10 @@ TS_EXPORT int ts_sample(const float* logits, long long row_stride, int num_rows,
   TS_REQUIRE((slot_tokens == nullptr) == (slots == nullptr), "sample: slot_tokens and slots come together");
   SampleArgs a{logits, row_stride, vocab, temperature, top_k, top_p, stream_ids, steps, seed, out, slot_tokens, slots};
   // Blocks per row: as many (1, 2, 4 or 8, the portable cluster) as leave every row's cluster a place at once (a second
-  // wave doubles the time: 16 rows of 151,936 tokens with top-k and top-p 147 us in clusters of four, 178 in
-  // clusters of eight, of which 15 fit), a range of at least 2,048 tokens each and no cluster below 8,192
-  // (with top-k and top-p 8,192 tokens 40 / 33 us by one block / by four, 4,096 tokens 29 / 32 by one / by two).
+  // wave doubles the time: 16 rows of 151,936 tokens with top-k and top-p 101 us in clusters of four, 127 in
+  // clusters of eight, of which 15 fit; 64 rows 175 in clusters of two, 204 of four), a range of at least 2,048 tokens each
+  // and no cluster below 8,192 (with top-k and top-p 8,192 tokens 31 / 27 us by one block / by four, 4,096 tokens 23 / 27 by
+  // one / by two; at a temperature alone 5.9 / 4.7 and 4.3 / 4.7).
   int blocks = 1;
   while (blocks < 8 && vocab >= 8192 && vocab / (2 * blocks) >= 2048 && num_rows <= max_clusters(2 * blocks)) blocks *= 2;
   if (blocks == 1) {
