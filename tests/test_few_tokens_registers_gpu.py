@@ -70,3 +70,46 @@ def test_range():
     assert not ops._gemv_fits(9, 128, 128) and not ops._gemv_fits(1, 16, 4104) and not ops._gemv_fits(1, 8193, 1024)
     assert not ops._gemv_fits(1, 128, 2056, gated=True) and not ops._gemv_fits(1, 192, 128, gated=True)
     assert not ops._gemv_fits(1, 1040, 128, residual=True) and not ops._gemv_fits(1, 1000, 128, residual=True)
+
+
+def test_blocks_that_have_a_place():
+    """A block is four warps and more, 16 warps of them a multiprocessor: rows of a short K, blocks of a long one."""
+    from tinyserve_b200.kernels import ops
+    if ops.num_sms() != 148:
+        pytest.skip("the numbers are those of 148 multiprocessors")
+    fits = ops._gemv_fits
+    assert fits(1, 9472, 256) and not fits(1, 9488, 256) and not fits(1, 65536, 64)
+    assert fits(1, 16384, 512) and fits(1, 8192, 1024)                      # (a second wave of small blocks)
+    assert fits(1, 4736, 1536) and not fits(1, 4752, 1536) and not fits(1, 2384, 3072)
+    assert fits(1, 9472, 512, gated=True) and not fits(1, 9600, 512, gated=True) and not fits(1, 4864, 1536, gated=True)
+    assert fits(1, 2048, 4096, residual=True) and not fits(1, 2064, 2048, residual=True) and not fits(1, 2048, 256, residual=True)
+
+
+# sums of squares of 64, 65, 96 and 128 tiles, which come 32 at a time
+@pytest.mark.parametrize("M", [1, 8])
+@pytest.mark.parametrize("N,K", [(1024, 3072), (1040, 512), (1536, 1536), (2048, 1024)])
+def test_residual_then_a_product_by_tcgen05(M, N, K):
+    """The next product's weights are too large for this kernel; the norm factor comes from the sums per 16 columns."""
+    from tinyserve_b200.kernels import ops
+    F = (1 << 23) // N // 64 * 64
+    assert ops._gemv_fits(M, N, K, residual=True) and not ops._gemv_fits(M, 2 * F, N) and not ops._gemv_fits(M, 2 * F, N, gated=True)
+    x, w = operands(M, N, K, 2)
+    g = torch.Generator().manual_seed(6)
+    res = torch.randn(M, N, generator=g).cuda()
+    norm = (1 + 0.1 * torch.randn(N, generator=g)).bfloat16().cuda()
+    want = res.double() + x.double() @ w.double().T
+    scaled = ops.add_rmsnorm(ops.linear(x, w, allow_pending=True), res, norm, 1e-6, torch.bfloat16, scaled_ok=True)
+    assert isinstance(scaled, ops.ScaledRows) and scaled.tiles == N // 16
+    normed = want * (want.square().mean(1, keepdim=True) + 1e-6).rsqrt() * norm.double()
+    w2 = (torch.randn(2 * F, N, generator=g) / N ** 0.5).bfloat16().cuda()
+    full = normed @ w2.double().T
+    # every normed element carries one rounding to bfloat16
+    slack = U * (normed.abs() @ w2.double().abs().T)
+    assert ((ops.linear(scaled, w2, out_float32=True).double() - full).abs() <= slack + 1e-5).all()
+    act = ops.gated_linear(scaled, w2, "silu", ops.GATED_BLOCK).double()
+    parts, s = full.view(M, F // 64, 2, 64), slack.view(M, F // 64, 2, 64)
+    gate, up = parts[:, :, 0].reshape(M, F), parts[:, :, 1].reshape(M, F)
+    want2 = torch.nn.functional.silu(gate) * up
+    tol = 1.1 * s[:, :, 0].reshape(M, F) * (up.abs() + 1) + s[:, :, 1].reshape(M, F) * gate.abs() + U * want2.abs() + 1e-5
+    assert ((act - want2).abs() <= tol).all()
+    assert ops.gemm_tcgen05_error() == 0

@@ -1,5 +1,6 @@
 // out[M, N] = x[M, K] W[N, K]^T for up to 8 tokens and weights that the whole device holds in registers at once
-// (up to 16 MB): the products of a decode step of a small model, bfloat16.
+// (up to 16 MB in blocks that all have a place; 119 registers a thread, 16 warps a multiprocessor): the products of a decode
+// step of a small model, bfloat16.
 //
 // Such a product takes longer to start and to end than to read its weights, so nothing here is staged: a warp owns 16
 // weight rows and 256 columns of K and loads them before the dependency wait straight into the registers from which

@@ -329,16 +329,32 @@ def _gemv():
 
 
 #: Products of up to this many tokens whose weights the device holds in registers at once run on the kernel that loads
-#: them there before its dependency wait (csrc/gemv_mma.cu).
+#: them there before its dependency wait (csrc/gemv_mma.cu); a multiprocessor holds 16 warps of it (119 registers a thread).
 GEMV_MAX_TOKENS = 8
 GEMV_MAX_BYTES = 1 << 24
 GEMV_MAX_K = 4096
+GEMV_SM_WARPS = 16
 
 
 def _gemv_fits(M, N, K, gated=False, residual=False):
-    """The residual form leaves sums of squares per 16 columns, which the next product adds up: up to 64 of them."""
-    return (M <= GEMV_MAX_TOKENS and 2 * N * K <= GEMV_MAX_BYTES and K <= (GEMV_MAX_K // 2 if gated else GEMV_MAX_K)
-            and (not gated or N % 128 == 0) and (not residual or (N % 16 == 0 and N <= 1024)))
+    """All blocks have a place at once: a block has four warps or more, one for 256 columns of K (twice as many in the gated
+    form), so with a short K it is the rows that count, with a long K how many blocks a multiprocessor holds.  By this
+    kernel / by the tcgen05 one, one token, us: 9472 x 256 2.0 / 2.6, 12288 x 256 3.2 / 2.8, 32768 x 256 6.7 / 4.4;
+    gated 8192 x 512 2.9 / 3.8, 16384 x 512 5.6 / 4.9.  A second wave of blocks of four warps still pays where the
+    tcgen05 kernel has to cut K (16384 x 512 4.7 / 5.9); one of larger blocks is served late behind the other products of a
+    layer: o 2560 x 1024, gate_up 4096, down 2048, qkv 3072 x 2560 with the last by this kernel 27.6, without 23.7.
+    The residual form leaves a sum of squares per 16 columns, which the next product adds up: all four products of a layer with
+    the residuals by this kernel / by tcgen05: 1024 columns (ff 3072) 11.8 / 18.3, 1536 (8960) 26.4 / 28.3, 2048 (6144)
+    31.6 / 33.3, 2560 (6912) 40.7 / 38.8, 3072 (2048) 33.2 / 27.9."""
+    if M > GEMV_MAX_TOKENS or 2 * N * K > GEMV_MAX_BYTES or K > (GEMV_MAX_K // 2 if gated else GEMV_MAX_K):
+        return False
+    if gated and N % 128:
+        return False
+    if residual and (N % 16 or N > 2048 or (N > 1024 and K < 512)):          # (wide rows of a short K: not measured)
+        return False
+    warps = max(4, -(-K // 256)) * (2 if gated else 1)
+    blocks = N // 32 if gated else -(-N // 16)
+    return blocks <= num_sms() * (GEMV_SM_WARPS // warps) or (512 <= K <= 1024 and not gated)
 
 
 def _linear_gemv(x, weight, out_float32=False, partials_only=False, scale=None, gated=0, limit=0.0, residual=None, norm_weight=None):
@@ -983,7 +999,10 @@ def _tma_pages(k_cache, v_cache):
 
 def decode_splits(num_requests, max_kv_len, num_heads, num_kv_heads):
     """Key ranges for the tensor-core decode kernel: as many as fit in one wave of blocks (two
-    per SM), with at least two tiles of 64 keys per range."""
+    per SM), with at least two tiles of 64 keys per range.  One tile a range would be faster where the
+    clusters are few (1 request of 540 keys, 32 heads over 8, us: four ranges 7.0, eight 5.4), slower where
+    they are many (6 of 500, 64 over 8: three 9.0, six 15.4) or no cluster any more (1 of 2,000: 16 ranges 7.0,
+    32 7.7).  Captured graphs take the longest context of their bound: eight ranges for one request up to 1,024 keys."""
     blocks = num_kv_heads * -(-(num_heads // num_kv_heads) // 16) * num_requests
     return max(1, min(2 * num_sms() // blocks, max_kv_len // 128, 32))
 
